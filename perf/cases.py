@@ -139,7 +139,7 @@ def prepare(case, seed):
     if case["op"] != "device" or case.get("learned"):
         state["x"] = np.ascontiguousarray(x.cpu().numpy())
     if case.get("learned"):  # a model trained once and kept by the program
-        ext._mlp_train(state.pop("x"), k, sample=min(n, 40_000), epochs=30, quantile=0.01)
+        ext._mlp_train(state.pop("x"), k, sample=min(n, 100_000), epochs=40, quantile=0.01)
         state["model"] = ext._mlp_get()
     most = (2 if case["op"] == "csr" else 1) * n * k
     if case["op"] == "device":
