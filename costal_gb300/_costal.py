@@ -14,7 +14,7 @@ Differences from the reference, all documented:
     "accelerate" is Apple-only and unavailable here, as it is for the reference on Linux.
   - `row_block`, `col_block`, `sort_by_norm` and `n_threads` are accepted and validated but do not
     change the GPU tiling (the reference: they change speed only, knn.rs:39-44). `prune` (speed
-    only, as in the reference) switches the exact early stop of the bf16 backend's block lists.
+    only, as in the reference) switches the exact early stop of the block lists.
   - The GPU keeps at most 128 candidates a row: k + margin above 128 runs with margin 128 − k, and
     k ≥ 128 with the exact f64 scan of every candidate (the output is the same; the margin in effect
     is reported in the stats).

@@ -68,7 +68,7 @@ struct Context {
     DevBuf x, norms, xsT, cand_idx, cand_score, tau, out_idx, out_cos, out_w, fb_rows, fb_minsim, misc;
     DevBuf fu_scratch, rows, cols, wout, idx_in, cos_in, norms_in, w_in, jac, f32out, tc_ws, tc_rows, prune_ws;
     DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows;
-    DevBuf part_idx, part_score, part_tau, tfloor;
+    DevBuf fp32_ws, tfloor, xsW;
     DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_perm, tani_ws, rm_ws, rm_out;
     MlpState mlp;
 };
@@ -160,6 +160,37 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 
 constexpr int MLP_CHUNK = 262144;  // rows per feature/forward chunk at inference
 
+// An FP32 coarse pass over all rows and columns, with its workspace; callers narrow it down.
+Fp32Job fp32_job(Context& c, int n, int np, int dp, int cap) {
+    Fp32Job j{};
+    j.xsT = c.xsT.as<float>();
+    j.n = n;
+    j.np = np;
+    j.dp = dp;
+    j.cap = cap;
+    j.nq = n;
+    j.tnorm = c.tnorm.as<float2>();
+    j.cand_idx = c.cand_idx.as<uint32_t>();
+    j.cand_score = c.cand_score.as<float>();
+    j.tau = c.tau.as<float>();
+    j.timeout_flag = &c.misc.as<Misc>()->timeout_flag;
+    return j;
+}
+void coarse_fp32(Context& c, const Fp32Job& j, cudaStream_t s) {
+    if (j.nq <= 0) return;
+    CK(ensure(c.fp32_ws, coarse_fp32_ws_bytes(j, c.sm_count)));
+    CK(launch_coarse_fp32(j, c.fp32_ws.p, c.sm_count, s));
+}
+// The queries `rows` only (nq of them, on the device), optionally with a floor for each row.
+void coarse_fp32_rows(Context& c, int n, int np, int dp, int cap, const uint32_t* rows, int nq, const float* tfloor,
+                      cudaStream_t s) {
+    Fp32Job j = fp32_job(c, n, np, dp, cap);
+    j.rows = rows;
+    j.nq = nq;
+    j.tfloor = tfloor;
+    coarse_fp32(c, j, s);
+}
+
 // Learned thresholds: the model's prediction for every row, then t_Q = min over each query block.
 cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) {
     const int n = pp.n, d = pp.d, F = c.mlp.F;
@@ -179,6 +210,35 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
             return e;
     }
     return mlp::block_min(c.mlp_pred.as<float>(), pp.perm, n, pp.tq, s);
+}
+
+// Whether the FP32 pass visits its columns by lists, nearest blocks first with the exact early stop,
+// instead of all tiles in order: where the tiles and admissions it saves cost more than the order stage
+// (measured, whole kNN, lists / all tiles: 20,000 × 32 2.2 / 1.7 ms, 40,000 × 20 3.3 / 4.4, 80,000 × 32
+// 8.0 / 12.6, 161,443 × 32 16.6 / 39.8).
+bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 32768; }
+
+// The FP32 pass's working order and column lists: the same cells, bounds and lists as the tensor-core
+// path (the per-row bounds come from its split operands, with their margin), and the rows' transposed
+// copy in the working order (c.xsW).
+void build_fp32_lists(Context& c, int n, int np, int d, int dp, prune::Plan& pp, cudaStream_t s) {
+    Misc* dm = c.misc.as<Misc>();
+    CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
+    CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), n, np, d, s, pp));
+    CK(ensure(c.tc_ws, tc::workspace_bytes(n, d, false)));
+    tc::Plan plan{};
+    CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), n, np, dp, d, pp.perm, s, plan, false, pp.wrows));
+    if (tc::rowmax_supported(plan)) {
+        CK(ensure(c.rm_ws, tc::rowmax_bytes(pp.ncb, d)));
+        CK(ensure(c.rm_out, (size_t)pp.nqb * pp.ncb * 4));
+        CK(tc::launch_rowmax(plan, pp.ccenter_f, pp.ncb, c.rm_ws.p, c.rm_out.as<float>(), &pp.rm_delta,
+                             &dm->timeout_flag, s));
+        pp.rowmax = c.rm_out.as<float>();
+    }
+    pp.tq = nullptr;
+    CK(prune::build_lists(pp, &dm->blocks_skipped, s));
+    CK(ensure(c.xsW, (size_t)dp * np * 4));
+    CK(launch_work_cols(pp.wrows, n, np, d, dp, c.xsW.as<float>(), s));
 }
 
 // One shard of the query rows (a multi-GPU run gives each rank one): the rows are cut into query
@@ -300,8 +360,9 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                                          c.tani_ws.p, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                          c.tau.as<float>(), &dm->blocks_skipped, s));
         } else {
-            CK(launch_coarse_fp32_tanimoto(c.xsT.as<float>(), n, np, dp, cap, d_norms, c.tnorm.as<float2>(),
-                                           c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(), c.tau.as<float>(), s));
+            Fp32Job j = fp32_job(c, n, np, dp, cap);
+            j.norms = d_norms;
+            coarse_fp32(c, j, s);
         }
         CK(cudaEventRecord(c.ev[2], s));
         CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
@@ -394,20 +455,10 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             CK(cudaStreamSynchronize(s));
             const int nfail = (int)c.h_misc->tc_fail_count;
             if (nfail > 0) {
-                const int segs = coarse_fp32_segments(nfail, np, c.sm_count);
-                if (segs > 1) {
-                    CK(ensure(c.part_idx, (size_t)segs * nfail * cap * 4));
-                    CK(ensure(c.part_score, (size_t)segs * nfail * cap * 4));
-                    CK(ensure(c.part_tau, (size_t)segs * nfail * 4));
-                }
                 CK(ensure(c.tfloor, (size_t)n * 4));
                 CK(launch_rerun_floor(c.tc_rows.as<uint32_t>(), &dm->tc_fail_count, nfail, cap, c.tau.as<float>(),
                                       c.cand_score.as<float>(), plan.row_eps, eps, c.tfloor.as<float>(), s));
-                CK(launch_coarse_fp32_split(c.xsT.as<float>(), n, np, dp, cap, cap, c.tc_rows.as<uint32_t>(),
-                                            &dm->tc_fail_count, nfail, segs, c.tfloor.as<float>(),
-                                            c.part_idx.as<uint32_t>(),
-                                            c.part_score.as<float>(), c.part_tau.as<float>(), c.cand_idx.as<uint32_t>(),
-                                            c.cand_score.as<float>(), c.tau.as<float>(), s));
+                coarse_fp32_rows(c, n, np, dp, cap, c.tc_rows.as<uint32_t>(), nfail, c.tfloor.as<float>(), s);
                 CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                   c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps, cap < n - 1, 0,
                                   c.tc_rows.as<uint32_t>(), &dm->tc_fail_count, d_idx, d_cos, d_w,
@@ -418,13 +469,26 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             if (coarse_fp32_smem(dp, cap) > 227 * 1024)
                 throw Fail{COSTAL_EUNSUPPORTED, "d and k + margin too large for the FP32 coarse kernel"};
             if (!shard) {
-                CK(launch_coarse_fp32(c.xsT.as<float>(), n, np, dp, cap, cap, nullptr, nullptr,
-                                      c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(), c.tau.as<float>(), s));
+                Fp32Job j = fp32_job(c, n, np, dp, cap);
+                prune::Plan pp{};
+                if (o.prune && cap < n - 1 && fp32_lists_pay(n, d)) {
+                    build_fp32_lists(c, n, np, d, dp, pp, s);
+                    list_cb = pp.cb;
+                    j.xsT = c.xsW.as<float>();
+                    j.perm = pp.perm;
+                    j.lists = pp.lists;
+                    j.list_ub = pp.list_ub;
+                    j.counts = pp.counts;
+                    j.ncb = pp.ncb;
+                    j.list_cb = pp.cb;
+                    j.eps = std::nextafterf((float)eps, INFINITY);
+                    j.stopped_total = &dm->blocks_stopped;
+                    CK(cudaEventRecord(c.ev[5], s));
+                }
+                coarse_fp32(c, j, s);
             } else if (nrows > 0) {  // the shard's rows, listed, against all columns
                 CK(launch_iota(srows, qb0 * 128, nrows, s));
-                CK(launch_coarse_fp32_split(c.xsT.as<float>(), n, np, dp, cap, cap, srows, scount, nrows, 1, nullptr,
-                                            nullptr, nullptr, nullptr, c.cand_idx.as<uint32_t>(),
-                                            c.cand_score.as<float>(), c.tau.as<float>(), s));
+                coarse_fp32_rows(c, n, np, dp, cap, srows, nrows, nullptr, s);
             }
             CK(cudaEventRecord(c.ev[2], s));
             if (nrows > 0)
@@ -448,11 +512,11 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     const Misc& hm = *c.h_misc;
     if (hm.bad_row != ~0ull) throw Fail{COSTAL_EINVAL, "row " + std::to_string(hm.bad_row) + " contains NaN or inf"};
     if (hm.timeout_flag == 2) throw Fail{COSTAL_ECUDA, "internal error: a column-block list entry out of range"};
-    if (hm.timeout_flag) throw Fail{COSTAL_ETIMEOUT, "a bounded device wait in the tensor-core kernel gave up"};
+    if (hm.timeout_flag) throw Fail{COSTAL_ETIMEOUT, "a bounded device wait in the coarse kernel gave up"};
     if (st) {
         st->fallback_rows = hm.fb_count;
         st->row_block = 128;
-        st->col_block = used_tc ? (uint64_t)(list_cb ? list_cb : tc::BLOCK_N) : 128;
+        st->col_block = list_cb ? (uint64_t)list_cb : (used_tc ? (uint64_t)tc::BLOCK_N : 128);
         st->blocks_skipped = hm.blocks_skipped;
         st->blocks_stopped = hm.blocks_stopped;
         st->blocks_total = (uint64_t)(qb1 - qb0) * (uint64_t)((n + st->col_block - 1) / st->col_block);
@@ -916,8 +980,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(launch_stride_rows(rows, m, N, s));
         unsigned hm = (unsigned)m;
         CK(cudaMemcpyAsync(&dm->tc_fail_count, &hm, 4, cudaMemcpyHostToDevice, s));
-        CK(launch_coarse_fp32(c.xsT.as<float>(), N, np, dp, cap, cap, rows, &dm->tc_fail_count, c.cand_idx.as<uint32_t>(),
-                              c.cand_score.as<float>(), c.tau.as<float>(), s));
+        coarse_fp32_rows(c, N, np, dp, cap, rows, m, nullptr, s);
         const double eps = ((double)d + 4.0) * F32_EPS;
         CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                           c.tau.as<float>(), c.norms.as<double>(), nullptr, nullptr, nullptr, eps, cap < N - 1, 0, rows,
@@ -956,6 +1019,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(cudaStreamSynchronize(s));
         if (c.h_misc->bad_row != ~0ull)
             throw Fail{COSTAL_EINVAL, "row " + std::to_string(c.h_misc->bad_row) + " contains NaN or inf"};
+        if (c.h_misc->timeout_flag) throw Fail{COSTAL_ETIMEOUT, "a bounded device wait in the coarse kernel gave up"};
         double loss = 0.0, mae = 0.0;
         size_t below = 0;
         for (int i = 0; i < m; ++i) {

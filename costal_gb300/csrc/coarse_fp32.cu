@@ -1,19 +1,13 @@
-// The FP32 coarse pass: every (query block × column tile) dot product on the CUDA cores, fused with
-// the per-query top-cap selection (crates/costal-core/src/knn.rs:603-660 tiles, :758-787 the
-// threshold scan, :791-875 the per-row heaps).
+// Tanimoto selection by norm windows (knn.rs:197-284, :595-644), the merge of column segments' lists and
+// the floors of re-run rows. The FP32 pass itself is in fp32_tiles.cu.
 //
-// Layout: 256 threads per CTA own 128 query rows; each thread holds an 8 × 8 register tile (queries
-// ty·4+i and 64+ty·4+i, columns tx·4+j and 64+tx·4+j), so all 128 columns of a query's tile row are
-// computed inside ONE warp. The normalised rows are read transposed (xsT, d_pad × n_pad) so that a
-// tile is d_pad contiguous 512-byte rows, staged by cp.async in a 3-stage shared-memory ring: one
-// block barrier per tile, and the top-cap merges are warp-local (no block barrier).
-//
-// Selection: each query keeps its best `cap` columns by (score desc, index asc) in shared memory,
-// with τ = the worst kept score (−∞ until full). A column is admitted when its score is strictly
-// above the τ of the tile start; since every earlier tile holds smaller column indices, that is the
-// reference's strict `v > th` test and the kept set is exactly the top-cap (knn.rs:774-780).
-// Admissions go to a 16-entry buffer per query; a query whose buffer overflows (early tiles) has its
-// tile row recomputed by its warp in the same FMA order and inserted column by column.
+// Layout of the windowed kernel: 256 threads per CTA own 128 query rows; each thread holds an 8 × 8
+// register tile (queries ty·4+i and 64+ty·4+i, columns tx·4+j and 64+tx·4+j), so all 128 columns of a
+// query's tile row are computed inside ONE warp. The normalised rows are read transposed (d_pad × n_pad),
+// staged by cp.async in a 3-stage shared-memory ring; the top-cap merges are warp-local. Each query
+// keeps its best `cap` columns by (score desc, index asc), τ = the worst kept score (−∞ until full);
+// admissions go to a 16-entry buffer per query, and a query whose buffer overflows has its tile row
+// recomputed by its warp in the same FMA order and inserted column by column.
 
 #include <cuda_runtime.h>
 
@@ -34,10 +28,6 @@ constexpr int NT = 256;
 constexpr int BUF = 16;
 constexpr int STAGES = 3;
 
-#ifndef COSTAL_FP32_PAIRED
-#define COSTAL_FP32_PAIRED 1
-#endif
-
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -50,28 +40,6 @@ __device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsign
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
-}
-
-// The CTA's lists out: by row (lstride per row), or, with column segments (part_stride > 0), by
-// list slot into segment blockIdx.y's part of the output (cap per slot), for k_merge_parts.
-template <class RowOf>
-__device__ __forceinline__ void write_lists(const float* L_s, const uint32_t* L_i, const float* tau_s, int lcap, int cap,
-                                            int lstride, int n, int nq, int q0, int part_stride, RowOf row_of,
-                                            uint32_t* cand_idx, float* cand_score, float* tau_out) {
-    const int tid = threadIdx.x;
-    for (int e = tid; e < BM * cap; e += NT) {
-        const int qi = e / cap, p = e % cap, q = row_of(qi);
-        if (q < 0 || q >= n) continue;
-        const size_t o = part_stride ? ((size_t)blockIdx.y * part_stride + q0 + qi) * cap + p : (size_t)q * lstride + p;
-        cand_idx[o] = L_i[qi * lcap + p];
-        cand_score[o] = L_s[qi * lcap + p];
-    }
-    for (int qi = tid; qi < BM; qi += NT) {
-        const int q = row_of(qi);
-        if (q < 0 || q >= n) continue;
-        tau_out[part_stride ? (size_t)blockIdx.y * part_stride + q0 + qi : (size_t)q] = tau_s[qi];
-    }
-    (void)nq;
 }
 
 // The selection of one 128 × 128 tile, shared by both FP32 kernels: the admission test of the
@@ -186,7 +154,6 @@ __device__ __forceinline__ void tani_tile(float (&acc)[8][8], const float2* __re
 // (queries ty·4+i and 64+ty·4+i of A_s, columns tx·4+j and 64+tx·4+j of the stage Bst).
 template <int DPC>
 __device__ __forceinline__ void tile_fma(const float* A_s, const float* Bst, int dp, int tx, int ty, float (&acc)[8][8]) {
-#if COSTAL_FP32_PAIRED
     // Blackwell's paired FP32 FMA: one instruction does two independent single-rounding FMAs,
     // so the values are those of the scalar fmaf chain below.
     unsigned long long acc2[8][4];
@@ -213,126 +180,6 @@ __device__ __forceinline__ void tile_fma(const float* A_s, const float* Bst, int
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) unpack2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
-#else
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-#pragma unroll(DPC ? DPC : 4)
-    for (int t = 0; t < dp; ++t) {
-        const float4 a0 = *reinterpret_cast<const float4*>(A_s + t * BM + ty * 4);
-        const float4 a1 = *reinterpret_cast<const float4*>(A_s + t * BM + 64 + ty * 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(Bst + t * BN + tx * 4);
-        const float4 b1 = *reinterpret_cast<const float4*>(Bst + t * BN + 64 + tx * 4);
-        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-#endif
-}
-
-template <int SLOTS, int DPC, bool TANI>
-__global__ void __launch_bounds__(NT, 1)
-    k_coarse_fp32(const float* __restrict__ xsT, int n, int np, int dp_rt, int cap, int lstride,
-                  const uint32_t* __restrict__ qlist, const unsigned* __restrict__ qcount, int part_stride,
-                  const float* __restrict__ tfloor, const float2* __restrict__ tnorm, uint32_t* __restrict__ cand_idx,
-                  float* __restrict__ cand_score, float* __restrict__ tau_out) {
-    constexpr int LCAP = 32 * SLOTS;
-    const int dp = DPC ? DPC : dp_rt;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* A_s = reinterpret_cast<float*>(smem_raw);            // [dp][BM]
-    float* B_s = A_s + (size_t)dp * BM;                          // [STAGES][dp][BN]
-    float* L_s = B_s + (size_t)STAGES * dp * BN;                 // [BM][LCAP]
-    uint32_t* L_i = reinterpret_cast<uint32_t*>(L_s + BM * LCAP);
-    float* buf_s = reinterpret_cast<float*>(L_i + BM * LCAP);   // [BM][BUF]
-    uint32_t* buf_i = reinterpret_cast<uint32_t*>(buf_s + BM * BUF);
-    int* cnt_s = reinterpret_cast<int*>(buf_i + BM * BUF);       // [BM]
-    int* len_s = cnt_s + BM;                                     // [BM]
-    float* tau_s = reinterpret_cast<float*>(len_s + BM);         // [BM]
-    float* floor_s = tau_s + BM;                                 // [BM]
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tx = tid & 15, ty = tid >> 4;
-    // The block's 128 consecutive query rows, or 128 entries of a device-side row list.
-    const int q0 = blockIdx.x * BM;
-    const int nq = qlist ? min(BM, (int)*qcount - q0) : BM;
-    if (nq <= 0) return;
-    auto row_of = [&](int qi) -> int { return qlist ? (qi < nq ? (int)qlist[q0 + qi] : -1) : q0 + qi; };
-    // Column segment blockIdx.y of gridDim.y (one segment: all tiles).
-    const int all_tiles = np / BN, tps = (all_tiles + gridDim.y - 1) / gridDim.y;
-    const int tile0 = blockIdx.y * tps, ntiles = max(0, min(all_tiles, tile0 + tps) - tile0);
-
-    auto load_tile = [&](float* dst, int c0) {
-        for (int ch = tid; ch < dp * (BN / 4); ch += NT) {
-            const int t = ch / (BN / 4), c4 = ch % (BN / 4);
-            cp_async16(dst + t * BN + c4 * 4, xsT + (size_t)t * np + c0 + c4 * 4);
-        }
-    };
-    if (qlist) {
-        for (int e = tid; e < dp * BM; e += NT) {
-            const int t = e / BM, qi = e % BM;
-            A_s[t * BM + qi] = qi < nq ? xsT[(size_t)t * np + qlist[q0 + qi]] : 0.0f;
-        }
-    } else {
-        load_tile(A_s, q0);
-    }
-    if (ntiles > 0) load_tile(B_s, tile0 * BN);
-    cp_async_commit();
-    if (ntiles > 1) load_tile(B_s + (size_t)dp * BN, (tile0 + 1) * BN);
-    cp_async_commit();
-    for (int q = tid; q < BM; q += NT) {
-        cnt_s[q] = 0;
-        len_s[q] = 0;
-        const int r = row_of(q);
-        floor_s[q] = tfloor && r >= 0 ? tfloor[r] : -CUDART_INF_F;
-        tau_s[q] = floor_s[q];
-    }
-    // Unfilled slots read back as index 0xffffffff with score −inf: an empty slot for the rescoring
-    // (a list can stay short only with NaN input or a floor at a tie).
-    for (int e = tid; e < BM * LCAP; e += NT) {
-        L_s[e] = -CUDART_INF_F;
-        L_i[e] = 0xffffffffu;
-    }
-
-    for (int tl = 0; tl < ntiles; ++tl) {
-        cp_async_wait<1>();
-        __syncthreads();  // tile's stage landed for every thread; stage (tl+2)%3 is free again
-        if (tl + 2 < ntiles) load_tile(B_s + (size_t)((tl + 2) % STAGES) * dp * BN, (tile0 + tl + 2) * BN);
-        cp_async_commit();
-        const float* Bst = B_s + (size_t)(tl % STAGES) * dp * BN;
-        const int c0 = (tile0 + tl) * BN;
-
-        float acc[8][8];
-        tile_fma<DPC>(A_s, Bst, dp, tx, ty, acc);
-        if constexpr (TANI) {
-            int rows8[8];  // this thread's 8 query rows (their norms enter the Tanimoto scores)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = row_of(i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-                rows8[i] = r < n ? r : -1;
-            }
-            tani_tile(acc, tnorm, c0, n, tx, ty, rows8);
-        }
-        select_tile<SLOTS>(acc, c0, n, cap, L_s, L_i, buf_s, buf_i, cnt_s, len_s, tau_s, floor_s, warp, lane, tx, ty,
-                           row_of,
-                           [&](int qi, int cl) {
-                               float sv = 0.0f;
-#pragma unroll(DPC ? DPC : 4)
-                               for (int t = 0; t < dp; ++t) sv = fmaf(A_s[t * BM + qi], Bst[t * BN + cl], sv);
-                               if constexpr (TANI) {
-                                   const int q = row_of(qi), col = c0 + cl;
-                                   sv = tani_coarse_f32(sv, q >= 0 ? tnorm[q] : make_float2(0.0f, 0.0f),
-                                                    col < n ? tnorm[col] : make_float2(0.0f, 0.0f));
-                               }
-                               return sv;
-                           });
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    write_lists(L_s, L_i, tau_s, LCAP, cap, lstride, n, nq, q0, part_stride, row_of, cand_idx, cand_score, tau_out);
 }
 
 // Tanimoto selection with the norm window (knn.rs:197-284 `Tanimoto`, :595-644 `coarse_block`):
@@ -606,234 +453,10 @@ __global__ void k_tile_norm_envelope(int ntiles, double* __restrict__ lo, double
     for (int t = 1; t < ntiles; ++t) hi[t] = fmax(hi[t], hi[t - 1]);
 }
 
-// The same pass for any depth: the dimensions stream through the 3-stage ring in chunks of KC rows
-// of the transposed copy (query chunk and column chunk per stage), and the 8 × 8 register tile
-// accumulates across the chunks of a tile in dimension order, so every score is the same FMA chain
-// as in k_coarse_fp32. A query whose buffer overflows is recomputed from global memory.
-template <int SLOTS, int KC, bool TANI>
-__global__ void __launch_bounds__(NT, 1)
-    k_coarse_fp32_kc(const float* __restrict__ xsT, int n, int np, int dp, int cap, int lstride,
-                     const uint32_t* __restrict__ qlist, const unsigned* __restrict__ qcount, int part_stride,
-                     const float* __restrict__ tfloor, const float2* __restrict__ tnorm, uint32_t* __restrict__ cand_idx,
-                     float* __restrict__ cand_score, float* __restrict__ tau_out) {
-    constexpr int LCAP = 32 * SLOTS;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* S_s = reinterpret_cast<float*>(smem_raw);            // [STAGES][KC][BM + BN]
-    float* L_s = S_s + (size_t)STAGES * KC * (BM + BN);          // [BM][LCAP]
-    uint32_t* L_i = reinterpret_cast<uint32_t*>(L_s + BM * LCAP);
-    float* buf_s = reinterpret_cast<float*>(L_i + BM * LCAP);   // [BM][BUF]
-    uint32_t* buf_i = reinterpret_cast<uint32_t*>(buf_s + BM * BUF);
-    int* cnt_s = reinterpret_cast<int*>(buf_i + BM * BUF);       // [BM]
-    int* len_s = cnt_s + BM;                                     // [BM]
-    float* tau_s = reinterpret_cast<float*>(len_s + BM);         // [BM]
-    float* floor_s = tau_s + BM;                                 // [BM]
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int q0 = blockIdx.x * BM;
-    const int nq = qlist ? min(BM, (int)*qcount - q0) : BM;
-    if (nq <= 0) return;
-    auto row_of = [&](int qi) -> int { return qlist ? (qi < nq ? (int)qlist[q0 + qi] : -1) : q0 + qi; };
-    const int all_tiles = np / BN, tps = (all_tiles + gridDim.y - 1) / gridDim.y;
-    const int tile0 = blockIdx.y * tps, ntiles = max(0, min(all_tiles, tile0 + tps) - tile0);
-    const int nch = (dp + KC - 1) / KC;
-    const int nsteps = ntiles * nch;
-
-    // Stage of step s = (tile, chunk): rows [chunk·KC, +KC) of the queries' and the tile's columns.
-    auto load_step = [&](int step) {
-        float* A = S_s + (size_t)(step % STAGES) * KC * (BM + BN);
-        float* B = A + KC * BM;
-        const int tile = tile0 + step / nch, t0 = (step % nch) * KC;
-        for (int ch = tid; ch < KC * (BM / 4); ch += NT) {
-            const int t = ch / (BM / 4), c4 = ch % (BM / 4);
-            if (t0 + t < dp) {
-                if (qlist) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int qi = c4 * 4 + u;
-                        A[t * BM + qi] = qi < nq ? xsT[(size_t)(t0 + t) * np + qlist[q0 + qi]] : 0.0f;
-                    }
-                } else {
-                    cp_async16(A + t * BM + c4 * 4, xsT + (size_t)(t0 + t) * np + q0 + c4 * 4);
-                }
-                cp_async16(B + t * BN + c4 * 4, xsT + (size_t)(t0 + t) * np + tile * BN + c4 * 4);
-            } else {
-                *reinterpret_cast<float4*>(A + t * BM + c4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4*>(B + t * BN + c4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-    };
-    if (nsteps > 0) load_step(0);
-    cp_async_commit();
-    if (nsteps > 1) load_step(1);
-    cp_async_commit();
-    for (int q = tid; q < BM; q += NT) {
-        cnt_s[q] = 0;
-        len_s[q] = 0;
-        const int r = row_of(q);
-        floor_s[q] = tfloor && r >= 0 ? tfloor[r] : -CUDART_INF_F;
-        tau_s[q] = floor_s[q];
-    }
-    // Unfilled slots read back as index 0xffffffff with score −inf: an empty slot for the rescoring
-    // (a list can stay short only with NaN input or a floor at a tie).
-    for (int e = tid; e < BM * LCAP; e += NT) {
-        L_s[e] = -CUDART_INF_F;
-        L_i[e] = 0xffffffffu;
-    }
-
-    for (int tl = 0; tl < ntiles; ++tl) {
-        const int c0 = (tile0 + tl) * BN;
-        unsigned long long acc2[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc2[i][j] = 0ull;
-        for (int ch = 0; ch < nch; ++ch) {
-            const int step = tl * nch + ch;
-            cp_async_wait<1>();
-            __syncthreads();  // this step's stage landed for every thread; stage (step+2)%3 is free
-            if (step + 2 < nsteps) load_step(step + 2);
-            cp_async_commit();
-            const float* A = S_s + (size_t)(step % STAGES) * KC * (BM + BN);
-            const float* B = A + KC * BM;
-#pragma unroll 4
-            for (int t = 0; t < KC; ++t) {
-                const float4 a0 = *reinterpret_cast<const float4*>(A + t * BM + ty * 4);
-                const float4 a1 = *reinterpret_cast<const float4*>(A + t * BM + 64 + ty * 4);
-                const float4 b0 = *reinterpret_cast<const float4*>(B + t * BN + tx * 4);
-                const float4 b1 = *reinterpret_cast<const float4*>(B + t * BN + 64 + tx * 4);
-                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const unsigned long long bp[4] = {pack2(b0.x, b0.y), pack2(b0.z, b0.w), pack2(b1.x, b1.y),
-                                                  pack2(b1.z, b1.w)};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const unsigned long long ap = pack2(a[i], a[i]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc2[i][j] = ffma2(ap, bp[j], acc2[i][j]);
-                }
-            }
-        }
-        float acc[8][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) unpack2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
-        if constexpr (TANI) {
-            int rows8[8];  // this thread's 8 query rows (their norms enter the Tanimoto scores)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = row_of(i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-                rows8[i] = r < n ? r : -1;
-            }
-            tani_tile(acc, tnorm, c0, n, tx, ty, rows8);
-        }
-        select_tile<SLOTS>(acc, c0, n, cap, L_s, L_i, buf_s, buf_i, cnt_s, len_s, tau_s, floor_s, warp, lane, tx, ty,
-                           row_of,
-                           [&](int qi, int cl) {
-                               // zero padding beyond dp adds exact zeros: the chain over dp is the same
-                               const int q = row_of(qi);
-                               float sv = 0.0f;
-                               if (q >= 0)
-                                   for (int t = 0; t < dp; ++t)
-                                       sv = fmaf(xsT[(size_t)t * np + q], xsT[(size_t)t * np + c0 + cl], sv);
-                               if constexpr (TANI) {
-                                   const int col = c0 + cl;
-                                   sv = tani_coarse_f32(sv, q >= 0 ? tnorm[q] : make_float2(0.0f, 0.0f),
-                                                    col < n ? tnorm[col] : make_float2(0.0f, 0.0f));
-                               }
-                               return sv;
-                           });
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    write_lists(L_s, L_i, tau_s, LCAP, cap, lstride, n, nq, q0, part_stride, row_of, cand_idx, cand_score, tau_out);
-}
-
-constexpr int kc_for(int slots) { return slots <= 2 ? 32 : 16; }
-
-size_t coarse_smem_bytes_kc(int slots) {
-    const size_t lcap = 32 * (size_t)slots;
-    return (size_t)STAGES * kc_for(slots) * (BM + BN) * 4 + (size_t)BM * lcap * 8 + (size_t)BM * BUF * 8 + BM * 4 * 4;
-}
-
-template <int S>
-cudaError_t launch_kc(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                      const unsigned* qcount, int segs, int grid_rows, int part_stride, const float* tfloor, const float2* tnorm,
-                      uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st) {
-    constexpr int KC = kc_for(S);
-    const size_t smem = coarse_smem_bytes_kc(S);
-    auto kern = tnorm ? k_coarse_fp32_kc<S, KC, true> : k_coarse_fp32_kc<S, KC, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<dim3(grid_rows ? (grid_rows + BM - 1) / BM : np / BM, segs), NT, smem, st>>>(
-        xsT, n, np, dp, cap, lstride, qlist, qcount, part_stride, tfloor, tnorm, cand_idx, cand_score, tau);
-    note_launch();
-    return cudaGetLastError();
-}
-
 size_t coarse_smem_bytes(int dp, int slots) {
     const size_t lcap = 32 * (size_t)slots;
     return (size_t)dp * BM * 4 + (size_t)STAGES * dp * BN * 4 + (size_t)BM * lcap * 8 + (size_t)BM * BUF * 8 +
            BM * 4 * 4;
-}
-
-template <int S, int D>
-cudaError_t launch_one(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                       const unsigned* qcount, int segs, int grid_rows, int part_stride, const float* tfloor,
-                       const float2* tnorm, uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st) {
-    const size_t smem = coarse_smem_bytes(dp, S);
-    // (the Tanimoto variant is built only for a run-time depth: dispatch_d sends it there)
-    auto kern = k_coarse_fp32<S, D, false>;
-    if constexpr (D == 0)
-        if (tnorm) kern = k_coarse_fp32<S, 0, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<dim3(grid_rows ? (grid_rows + BM - 1) / BM : np / BM, segs), NT, smem, st>>>(
-        xsT, n, np, dp, cap, lstride, qlist, qcount, part_stride, tfloor, tnorm, cand_idx, cand_score, tau);
-    note_launch();
-    return cudaGetLastError();
-}
-
-template <int S>
-cudaError_t dispatch_d(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                       const unsigned* qcount, int segs, int grid_rows, int part_stride, const float* tfloor,
-                       const float2* tnorm, uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st) {
-#define COSTAL_D(D)                                                                                            \
-    case D:                                                                                                    \
-        return launch_one<S, D>(xsT, n, np, dp, cap, lstride, qlist, qcount, segs, grid_rows, part_stride, tfloor, \
-                                tnorm, cand_idx, cand_score, tau, st);
-    if (tnorm)
-        return launch_one<S, 0>(xsT, n, np, dp, cap, lstride, qlist, qcount, segs, grid_rows, part_stride, tfloor,
-                                tnorm, cand_idx, cand_score, tau, st);
-    switch (dp) {
-        COSTAL_D(8) COSTAL_D(16) COSTAL_D(24) COSTAL_D(32) COSTAL_D(40) COSTAL_D(48) COSTAL_D(56) COSTAL_D(64)
-        default:
-            return launch_one<S, 0>(xsT, n, np, dp, cap, lstride, qlist, qcount, segs, grid_rows, part_stride,
-                                    tfloor, tnorm, cand_idx, cand_score, tau, st);
-    }
-#undef COSTAL_D
-}
-
-cudaError_t launch_any(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                       const unsigned* qcount, int segs, int grid_rows, int part_stride, const float* tfloor,
-                       const float2* tnorm, uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st) {
-#define COSTAL_ARGS xsT, n, np, dp, cap, lstride, qlist, qcount, segs, grid_rows, part_stride, tfloor, tnorm, cand_idx, \
-    cand_score, tau, st
-    if (dp > 64) {  // deep rows: the chunked kernel
-        switch (coarse_slots(cap)) {
-            case 1: return launch_kc<1>(COSTAL_ARGS);
-            case 2: return launch_kc<2>(COSTAL_ARGS);
-            case 4: return launch_kc<4>(COSTAL_ARGS);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (coarse_slots(cap)) {
-        case 1: return dispatch_d<1>(COSTAL_ARGS);
-        case 2: return dispatch_d<2>(COSTAL_ARGS);
-        case 4: return launch_one<4, 0>(COSTAL_ARGS);
-        default: return cudaErrorInvalidValue;
-    }
-#undef COSTAL_ARGS
 }
 
 // One warp per listed row: the union of its segments' lists (segs · cap entries) as (score desc,
@@ -866,7 +489,7 @@ __global__ void k_merge_parts(const uint32_t* __restrict__ qlist, int count, int
         }
         warp_sort_keys<8>(key, lane);
     }
-    const uint32_t q = qlist[r];
+    const uint32_t q = qlist ? qlist[r] : (uint32_t)r;
     uint64_t kth = 0;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
@@ -885,33 +508,10 @@ __global__ void k_merge_parts(const uint32_t* __restrict__ qlist, int count, int
 }  // namespace plain
 
 size_t coarse_fp32_smem(int dp, int cap) {
-    return dp > 64 ? plain::coarse_smem_bytes_kc(coarse_slots(cap)) : plain::coarse_smem_bytes(dp, coarse_slots(cap));
+    return dp > 64 ? 0 : plain::coarse_smem_bytes(dp, coarse_slots(cap));
 }
 
 int coarse_dpad(int d) { return d <= 64 ? ((d < 1 ? 1 : d) + 7) / 8 * 8 : (d + 3) / 4 * 4; }
-
-cudaError_t launch_coarse_fp32(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                               const unsigned* qcount, uint32_t* cand_idx, float* cand_score, float* tau,
-                               cudaStream_t st) {
-    return plain::launch_any(xsT, n, np, dp, cap, lstride, qlist, qcount, 1, 0, 0, nullptr, nullptr, cand_idx, cand_score,
-                             tau, st);
-}
-
-// The rows' f32 norm and squared norm from the f64 norms (knn.rs:207-212 rounds ‖x‖² to f32).
-__global__ void k_tani_norms(const double* __restrict__ norms, int n, float2* __restrict__ tnorm) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double a = norms[i];
-        tnorm[i] = make_float2((float)a, (float)(a * a));
-    }
-}
-
-cudaError_t launch_coarse_fp32_tanimoto(const float* xsT, int n, int np, int dp, int cap, const double* norms,
-                                        float2* tnorm, uint32_t* cand_idx, float* cand_score, float* tau,
-                                        cudaStream_t st) {
-    k_tani_norms<<<(n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024, 256, 0, st>>>(norms, n, tnorm); note_launch();
-    return plain::launch_any(xsT, n, np, dp, cap, cap, nullptr, nullptr, 1, 0, 0, nullptr, tnorm, cand_idx, cand_score,
-                             tau, st);
-}
 
 namespace {
 inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -956,29 +556,11 @@ cudaError_t launch_coarse_tani_window(const float* xsT, int n, int np, int dp, i
     return cudaGetLastError();
 }
 
-int coarse_fp32_segments(int count, int np, int sm_count) {
-    // enough CTAs for two per SM; the merge reads segs · cap entries per row, 256 − cap at a time
-    const int qblocks = (count + plain::BM - 1) / plain::BM, all = np / plain::BN;
-    int segs = (2 * sm_count + qblocks - 1) / qblocks;
-    segs = std::min(segs, 64);
-    segs = std::min(segs, all / 2);
-    if (segs <= 1) return 1;
-    const int tps = (all + segs - 1) / segs;
-    return (all + tps - 1) / tps;  // no empty segment
-}
-
-cudaError_t launch_coarse_fp32_split(const float* xsT, int n, int np, int dp, int cap, int lstride,
-                                     const uint32_t* qlist, const unsigned* qcount, int count, int segs,
-                                     const float* tfloor, uint32_t* part_idx, float* part_score, float* part_tau,
-                                     uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st) {
-    if (segs <= 1)
-        return plain::launch_any(xsT, n, np, dp, cap, lstride, qlist, qcount, 1, count, 0, tfloor, nullptr, cand_idx,
-                                 cand_score, tau, st);
-    cudaError_t e = plain::launch_any(xsT, n, np, dp, cap, lstride, qlist, qcount, segs, count, count, tfloor, nullptr,
-                                      part_idx, part_score, part_tau, st);
-    if (e != cudaSuccess) return e;
-    plain::k_merge_parts<<<(count + 7) / 8, 256, 0, st>>>(qlist, count, segs, cap, part_idx, part_score, tfloor,
-                                                          lstride, cand_idx, cand_score, tau);
+cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
+                               const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
+                               float* tau, cudaStream_t st) {
+    plain::k_merge_parts<<<(count + 7) / 8, 256, 0, st>>>(rows, count, segs, cap, part_idx, part_score, tfloor, cap,
+                                                          cand_idx, cand_score, tau);
     note_launch();
     return cudaGetLastError();
 }

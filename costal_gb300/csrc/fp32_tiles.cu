@@ -1,0 +1,741 @@
+// The FP32 coarse pass: every (query block × column tile) dot product on the CUDA cores, fused with
+// the per-query top-cap selection (crates/costal-core/src/knn.rs:603-660 tiles, :758-787 the
+// threshold scan, :791-875 the per-row heaps).
+//
+//   tile      4 consumer warps own 128 query rows; each thread holds a 16 × 8 register tile (16 queries in
+//             groups of 4, columns tx·4+j and 64+tx·4+j), so a warp owns 32 queries and sees all 128
+//             columns of a tile for them. Two queries share one paired FP32 FMA (two independent
+//             single-rounding FMAs per instruction), so the query pairs come straight from shared
+//             memory and only the 8 column values are duplicated in registers. Every score is one
+//             FMA chain over the depth in dimension order. The shape is set by shared-memory
+//             bandwidth: a 16-byte load costs a warp 2 wavefronts when a half warp shares its address
+//             and 4 when it does not, so a depth step costs 16 wavefronts for 64 paired FMAs (128
+//             pipe cycles); an 8 × 8 tile costs 12 for 32 (16 with the queries stored twice), as many
+//             as the FMAs of 8 warps.
+//   pipeline  warp 4 streams column tiles with TMA into a ring of stages (full / empty mbarriers), kc
+//             dimensions a stage. The consumer warps never meet at a block barrier: one warp's
+//             selection overlaps another's FMAs, and a stage is handed back before its scores are
+//             looked at. Two CTAs per SM wherever their shared memory fits. For d_pad ≤ 64 the query
+//             operand stays resident; deeper rows stream both operands.
+//   select    A row whose tile maximum exceeds its query's τ appends its columns above τ to the query's
+//             buffer in shared memory; a buffer about to overflow is cut to its best cap by a warp-wide
+//             radix select, and τ rises to the cap-th score. Everything outside the buffer scored ≤ τ
+//             when it was seen or cut, and τ only grows: the certificate s_k > τ + ε (k_rescore) covers
+//             it. The first tile seeds τ: the cap-th largest of its column-group maxima is reached by
+//             cap distinct columns.
+//   lists     With prune.cu's lists the rows and columns are in the working order and a CTA visits the
+//             column blocks of its list, nearest first: τ is near its final value after the first
+//             tiles, and the CTA stops at the first block whose bound is below every query's τ − ε (its
+//             columns' coarse scores are ≤ bound + ε, so none could be admitted; later bounds are no
+//             larger).
+//   segments  Few query blocks: the columns are split over gridDim.y CTAs per block and the segments'
+//             lists merged per row (k_merge_parts), so that no SM idles in a nearly empty last wave.
+//             The segments of a query share their thresholds whenever one of them cuts its buffer.
+//
+// Every mbarrier wait is bounded (ptx.cuh); a wait that gives up raises timeout_flag.
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <math_constants.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "ptx.cuh"
+#include "topk.cuh"
+
+namespace costal {
+namespace fp32 {
+
+constexpr int BM = 128;
+constexpr int BN = 128;
+constexpr int CONS_WARPS = 4;                // consumer warps, 32 queries each
+// One warpgroup of consumers and one for the producer (one thread of it works): a launch at 128
+// registers a thread, of which the producers give up all but 40 and the consumers take 208. (A lone
+// producer warp would be the third warp of a scheduler in two CTAs and cap every thread at 168.)
+constexpr int NT = 256;
+constexpr int REGS_PRODUCER = 40, REGS_CONSUMER = 208;
+static_assert((REGS_PRODUCER + REGS_CONSUMER) * 128 <= NT * 128, "the split stays within the launch's registers");
+constexpr int MAX_STAGES = 6;
+constexpr size_t SMEM_ONE = 227 * 1024;      // shared memory of a CTA alone on its SM
+constexpr size_t SMEM_TWO = 113 * 1024;      // of each of two
+
+struct __align__(8) Bars {
+    uint64_t a_full;
+    uint64_t full[MAX_STAGES];
+    uint64_t empty[MAX_STAGES];
+    int c0[MAX_STAGES];  // first column of the stage's tile, −1: no more tiles
+    float warp_floor[CONS_WARPS];  // per consumer warp: min over its queries of τ − ε (never decreases)
+};
+
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float lo_of(unsigned long long r) { return __uint_as_float((uint32_t)r); }
+__device__ __forceinline__ float hi_of(unsigned long long r) { return __uint_as_float((uint32_t)(r >> 32)); }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+__device__ __forceinline__ unsigned long long twice(float x) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+
+// 8 depth steps of the register tile. A: [t][128] queries, B: [t][128] columns, 16 bytes an element
+// here; acc[p][j] holds queries 2p and 2p + 1 of the thread's 16 and column j of its 8.
+__device__ __forceinline__ void fma8(const ulonglong2* A, const float4* B, int tx, int ty,
+                                     unsigned long long (&acc)[8][8]) {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const ulonglong2 a0 = A[t * 32 + ty], a1 = A[t * 32 + 8 + ty], a2 = A[t * 32 + 16 + ty], a3 = A[t * 32 + 24 + ty];
+        const float4 b0 = B[t * 32 + tx], b1 = B[t * 32 + 16 + tx];
+        const unsigned long long a[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
+        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const unsigned long long bb = twice(b[j]);
+#pragma unroll
+            for (int p = 0; p < 8; ++p) acc[p][j] = ffma2(a[p], bb, acc[p][j]);
+        }
+    }
+}
+
+// The cap-th largest of a half warp's 16·R values (R per lane): a bitonic sorting network over the
+// 16 lanes, both halves of the warp at once. Out of line: it runs once per row of the first tile.
+template <int R>
+__device__ __noinline__ float half_kth(float v0, float v1, float v2, float v3, int cap, int lane) {
+    float v[4] = {v0, v1, v2, v3};
+    const int l = lane & 15;
+#pragma unroll
+    for (int size = 2; size <= 16 * R; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= 16) {
+#pragma unroll
+                for (int s = 0; s < R; ++s) {
+                    const int t = s ^ (stride >> 4);
+                    if (t > s) {
+                        const bool desc = ((s * 16 + l) & size) == 0;
+                        const float hi = fmaxf(v[s], v[t]), lo = fminf(v[s], v[t]);
+                        v[s] = desc ? hi : lo;
+                        v[t] = desc ? lo : hi;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < R; ++s) {
+                    const float o = __shfl_xor_sync(COSTAL_FULL_MASK, v[s], stride);
+                    const bool keep_max = ((l & stride) == 0) == (((s * 16 + l) & size) == 0);
+                    v[s] = keep_max ? fmaxf(v[s], o) : fminf(v[s], o);
+                }
+            }
+        }
+    }
+    float pick = v[0];
+#pragma unroll
+    for (int s = 1; s < R; ++s)
+        if (s == (cap - 1) >> 4) pick = v[s];
+    return __shfl_sync(COSTAL_FULL_MASK, pick, (lane & 16) | ((cap - 1) & 15));
+}
+
+// Cut one query's buffer (cnt > cap entries) to its best cap, in place, and return the cap-th largest
+// score: a warp-wide radix select on order-preserving keys, bit by bit from the highest bit where the
+// buffer's keys differ, done as soon as exactly cap keys lie at or above the prefix. Of entries equal
+// to the cap-th score the first in the buffer stay.
+template <int SLB>
+__device__ __noinline__ float cut_buffer(float* bs, uint32_t* bi, int cnt, int cap, int lane) {
+    float sc[SLB];
+    uint32_t id[SLB], key[SLB];
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+#pragma unroll
+    for (int s = 0; s < SLB; ++s) {
+        const int p = s * 32 + lane;
+        const bool v = p < cnt;
+        sc[s] = v ? bs[p] : 0.0f;
+        id[s] = v ? bi[p] : 0u;
+        const uint32_t u = __float_as_uint(sc[s]);
+        key[s] = v ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;  // 0: below every valid key
+        if (v) {
+            kmin = min(kmin, key[s]);
+            kmax = max(kmax, key[s]);
+        }
+    }
+    kmin = __reduce_min_sync(COSTAL_FULL_MASK, kmin);
+    kmax = __reduce_max_sync(COSTAL_FULL_MASK, kmax);
+    const uint32_t diff = kmin ^ kmax;
+    const int top = diff ? 31 - __clz(diff) : -1;
+    uint32_t T = top >= 0 ? (kmax & ~((2u << top) - 1u)) : kmax;
+    bool whole = false;  // exactly cap keys are ≥ T
+    for (int b = top; b >= 0; --b) {
+        const uint32_t c = T | (1u << b);
+        int n_ge = 0;
+#pragma unroll
+        for (int s = 0; s < SLB; ++s) n_ge += __popc(__ballot_sync(COSTAL_FULL_MASK, key[s] >= c));
+        if (n_ge >= cap) T = c;
+        if (n_ge == cap) {
+            whole = true;
+            break;
+        }
+    }
+    if (whole) {  // the cap-th score is the smallest key at or above the prefix
+        uint32_t m = 0xffffffffu;
+#pragma unroll
+        for (int s = 0; s < SLB; ++s)
+            if (key[s] >= T) m = min(m, key[s]);
+        T = __reduce_min_sync(COSTAL_FULL_MASK, m);
+    }
+    int n_gt = 0;
+#pragma unroll
+    for (int s = 0; s < SLB; ++s) n_gt += __popc(__ballot_sync(COSTAL_FULL_MASK, key[s] > T));
+    const unsigned below = (1u << lane) - 1u;
+    int eq = 0, kept = 0;
+    bool keep[SLB];
+    int pos[SLB];
+#pragma unroll
+    for (int s = 0; s < SLB; ++s) {
+        const unsigned meq = __ballot_sync(COSTAL_FULL_MASK, key[s] == T);
+        const bool k = key[s] > T || (key[s] == T && eq + __popc(meq & below) < cap - n_gt);
+        const unsigned mk = __ballot_sync(COSTAL_FULL_MASK, k);
+        keep[s] = k;
+        pos[s] = kept + __popc(mk & below);
+        eq += __popc(meq);
+        kept += __popc(mk);
+    }
+    __syncwarp();  // every lane has read its entries before any is overwritten
+#pragma unroll
+    for (int s = 0; s < SLB; ++s) {
+        if (keep[s]) {
+            bs[pos[s]] = sc[s];
+            bi[pos[s]] = id[s];
+        }
+    }
+    __syncwarp();
+    return __uint_as_float((T & 0x80000000u) ? (T & 0x7fffffffu) : ~T);
+}
+
+struct Args {
+    int n;          // columns
+    int nq;         // query slots in use
+    int cap, bcap, dp, kc, tiles, stages;
+    const uint32_t* rows;  // the queries' column ids (NULL: slot q is column q)
+    int part_stride;       // > 0: segment lists out, by slot
+    const uint32_t* perm;  // working → original row (NULL: identity)
+    const uint32_t* lists; // [query blocks][ncb] column blocks, nearest first (NULL: all tiles)
+    const float* list_ub;  // their bounds, not increasing (NULL: no early stop)
+    const uint32_t* counts;
+    int ncb, epc;          // list stride; 128-column tiles per list entry
+    float eps;             // the coarse error bound, rounded up
+    unsigned long long* stopped_total;
+    uint32_t* tau_shared;  // with segments: order key of each slot's largest threshold so far
+    const float* tfloor;   // by row: no column at or below it can be among the best cap (NULL: none)
+    const float2* tnorm;   // Tanimoto: f32 norm and squared norm of every column
+    uint32_t* cand_idx;
+    float* cand_score;
+    float* tau_out;
+    unsigned long long* timeout_flag;
+};
+
+__device__ __forceinline__ uint32_t okey(float v) {
+    const uint32_t u = __float_as_uint(v);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float okey_inv(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// Tanimoto: T > τ > 0 needs a cosine above τ/(1+τ)·(ρ + 1/ρ) ≥ 2τ/(1+τ), ρ the norms' quotient
+// (knn.rs:239-283); the factor 1 − 2⁻¹⁶ covers every f32 rounding of T and of this threshold.
+__device__ __forceinline__ float tani_cos_floor(float tau) {
+    return !(tau > 0.0f)         ? -CUDART_INF_F
+           : tau == CUDART_INF_F ? CUDART_INF_F
+                                 : 2.0f * __fdividef(tau, 1.0f + tau) * (1.0f - 0x1p-16f);
+}
+
+template <int SLB, bool STREAM, bool TANI>
+__global__ void __launch_bounds__(NT, 2)
+    k_fp32_tiles(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Args P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127);
+    const int kc = P.kc, bcap = P.bcap, cap = P.cap;
+    const uint32_t chunk = (uint32_t)kc * BN * 4;  // one operand's kc dimensions
+    const uint32_t stage_bytes = STREAM ? 2 * chunk : chunk;
+    unsigned char* a_res = smem;                                          // resident query operand
+    unsigned char* ring = STREAM ? smem : smem + (size_t)P.dp * BM * 4;   // stages × (A chunk, B chunk) or × B chunk
+    float* buf_s = reinterpret_cast<float*>(ring + (size_t)P.stages * stage_bytes);  // [BM][bcap]
+    uint32_t* buf_i = reinterpret_cast<uint32_t*>(buf_s + BM * bcap);
+    int* cnt_s = reinterpret_cast<int*>(buf_i + BM * bcap);
+    float* tau_s = reinterpret_cast<float*>(cnt_s + BM);
+    int* own_s = reinterpret_cast<int*>(tau_s + BM);  // the query's own column, −1: no query
+    Bars* bars = reinterpret_cast<Bars*>(own_s + BM);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int q0 = blockIdx.x * BM;
+    const int nch = (P.dp + kc - 1) / kc;
+    if (tid == 0) {
+        mbar_init(&bars->a_full, 1);
+        for (int s = 0; s < P.stages; ++s) {
+            mbar_init(&bars->full[s], 1);
+            mbar_init(&bars->empty[s], CONS_WARPS);
+        }
+        for (int w = 0; w < CONS_WARPS; ++w) bars->warp_floor[w] = -CUDART_INF_F;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int q = tid; q < BM; q += NT) {
+        const int own = q0 + q < P.nq ? (P.rows ? (int)P.rows[q0 + q] : q0 + q) : -1;
+        own_s[q] = own;
+        cnt_s[q] = 0;
+        tau_s[q] = own < 0 ? CUDART_INF_F : (P.tfloor ? P.tfloor[own] : -CUDART_INF_F);  // no query: never admits
+    }
+    __syncthreads();
+
+    if (warp >= CONS_WARPS) {
+        // ------------------------------------------------------------------ TMA producer
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_PRODUCER));
+        if (tid != CONS_WARPS * 32) return;
+        if (!STREAM) {
+            mbar_expect_tx(&bars->a_full, (uint32_t)P.dp * BM * 4);
+            for (int t = 0; t < P.dp; t += kc) tma_load_2d(a_res + (size_t)t * BM * 4, &map_a, q0, t, &bars->a_full);
+        }
+        int s = 0;
+        uint32_t ph = 1;
+        auto next_stage = [&]() {
+            if (++s == P.stages) {
+                s = 0;
+                ph ^= 1u;
+            }
+        };
+        auto send_tile = [&](int c0) -> bool {
+            for (int ch = 0; ch < nch; ++ch) {
+                if (!mbar_wait(&bars->empty[s], ph, P.timeout_flag, true)) return false;
+                unsigned char* dst = ring + (size_t)s * stage_bytes;
+                bars->c0[s] = c0;
+                mbar_expect_tx(&bars->full[s], stage_bytes);
+                if (STREAM) tma_load_2d(dst + chunk, &map_a, q0, ch * kc, &bars->full[s]);
+                tma_load_2d(dst, &map_b, c0, ch * kc, &bars->full[s]);
+                next_stage();
+            }
+            return true;
+        };
+        const int seg = (int)blockIdx.y, segs = (int)gridDim.y;
+        if (P.lists) {  // the segment's list entries: every segs-th one
+            const uint32_t* list = P.lists + (size_t)blockIdx.x * P.ncb;
+            const float* ub = P.list_ub ? P.list_ub + (size_t)blockIdx.x * P.ncb : nullptr;
+            const int count = min((int)P.counts[blockIdx.x], P.ncb);
+            const int limit_c = P.tiles * BN;
+            for (int e = seg; e < count; e += segs) {
+                if (ub) {
+                    volatile float* wf = bars->warp_floor;  // may be stale, i.e. lower: that only delays the stop
+                    if (ub[e] < fminf(fminf(wf[0], wf[1]), fminf(wf[2], wf[3]))) {
+                        if (P.stopped_total) atomicAdd(P.stopped_total, (unsigned long long)((count - e + segs - 1) / segs));
+                        break;
+                    }
+                }
+                for (int h = 0; h < P.epc; ++h) {
+                    const long long c0 = ((long long)list[e] * P.epc + h) * BN;
+                    if (c0 < limit_c && !send_tile((int)c0)) return;
+                }
+            }
+        } else {
+            const int tps = (P.tiles + segs - 1) / segs;
+            for (int t = seg * tps; t < min(P.tiles, (seg + 1) * tps); ++t)
+                if (!send_tile(t * BN)) return;
+        }
+        if (!mbar_wait(&bars->empty[s], ph, P.timeout_flag, true)) return;
+        bars->c0[s] = -1;
+        mbar_arrive(&bars->full[s]);  // completes the phase without data (release)
+        return;
+    }
+
+    // ---------------------------------------------------------------------- consumers
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_CONSUMER));
+    const int tx = lane & 15, ty = 2 * warp + (lane >> 4);
+    auto qi_at = [&](int i, int y) { return (i >> 2) * 32 + y * 4 + (i & 3); };  // query i of thread row y
+    auto cj_of = [&](int j) { return j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4); };
+    const int limit = cap + (bcap - cap) * 3 / 4;
+    if (!STREAM && !mbar_wait(&bars->a_full, 0, P.timeout_flag, false)) return;
+    int s = 0;
+    uint32_t ph = 0;
+    for (bool first = true;; first = false) {
+        unsigned long long acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+        int c0 = 0;
+        for (int ch = 0; ch < nch; ++ch) {
+            if (!mbar_wait(&bars->full[s], ph, P.timeout_flag, false)) return;
+            c0 = *reinterpret_cast<volatile int*>(&bars->c0[s]);
+            if (c0 < 0) break;
+            const unsigned char* st = ring + (size_t)s * stage_bytes;
+            const ulonglong2* A = reinterpret_cast<const ulonglong2*>(STREAM ? st + chunk : a_res + (size_t)ch * chunk);
+            const float4* B = reinterpret_cast<const float4*>(st);
+#pragma unroll 1
+            for (int k = 0; k < kc; k += 8) fma8(A + k * 32, B + k * 32, tx, ty, acc);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->empty[s]);
+            if (++s == P.stages) {
+                s = 0;
+                ph ^= 1u;
+            }
+        }
+        if (c0 < 0) break;
+        auto score = [&](int i, int j) { return i & 1 ? hi_of(acc[i >> 1][j]) : lo_of(acc[i >> 1][j]); };
+        // rows whose tile maximum is above their threshold (Tanimoto: above the cosine that threshold needs)
+        unsigned m = 0;
+        if (!first) {
+#pragma unroll
+            for (int i4 = 0; i4 < 4; ++i4) {
+                const float4 tr = *reinterpret_cast<const float4*>(tau_s + i4 * 32 + ty * 4);
+                const float t4[4] = {tr.x, tr.y, tr.z, tr.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = i4 * 4 + u;
+                    const float top = max3(max3(score(i, 0), score(i, 1), score(i, 2)),
+                                           max3(score(i, 3), score(i, 4), score(i, 5)), fmaxf(score(i, 6), score(i, 7)));
+                    m |= (top > (TANI ? tani_cos_floor(t4[u]) : t4[u]) ? 1u : 0u) << i;
+                }
+            }
+            m = __reduce_or_sync(COSTAL_FULL_MASK, m);
+            if (m == 0) continue;
+        } else {
+            m = 0xffffu;
+        }
+        // a tile with the queries' own columns or the padding: those columns never count
+        const bool edge = P.rows != nullptr || c0 + BN > P.n || c0 == q0;
+        // (One copy of this path, the row's scores picked by a jump: unrolled over the rows its code
+        // overflows the instruction cache, 4.8 against 1.7 ms at 20,000 × 32.)
+#pragma unroll 1
+        while (m) {
+            const int i = __ffs(m) - 1;  // warp-uniform
+            m &= m - 1;
+            float sv[8];
+            switch (i) {
+#define COSTAL_ROW(r)                                     \
+    case r:                                               \
+        _Pragma("unroll") for (int j = 0; j < 8; ++j) sv[j] = score(r, j); \
+        break;
+                COSTAL_ROW(0) COSTAL_ROW(1) COSTAL_ROW(2) COSTAL_ROW(3) COSTAL_ROW(4) COSTAL_ROW(5) COSTAL_ROW(6)
+                COSTAL_ROW(7) COSTAL_ROW(8) COSTAL_ROW(9) COSTAL_ROW(10) COSTAL_ROW(11) COSTAL_ROW(12)
+                COSTAL_ROW(13) COSTAL_ROW(14)
+                default: COSTAL_ROW(15)
+#undef COSTAL_ROW
+            }
+            const int qi = qi_at(i, ty), own = own_s[qi];
+            float* bs = buf_s + qi * bcap;
+            uint32_t* bi = buf_i + qi * bcap;
+            float tau = tau_s[qi];
+            const float2 qn = TANI && own >= 0 ? P.tnorm[own] : make_float2(0.f, 0.f);
+            const float cf = TANI && !first ? tani_cos_floor(tau) : -CUDART_INF_F;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int col = c0 + cj_of(j);
+                if (TANI) sv[j] = sv[j] > cf ? tani_coarse_f32(sv[j], qn, col < P.n ? P.tnorm[col] : make_float2(0.f, 0.f))
+                                             : -CUDART_INF_F;
+                if (edge && (col >= P.n || col == own)) sv[j] = -CUDART_INF_F;
+            }
+            if (first && cap <= 64) {
+                // the seed: the cap-th largest of 32 maxima of 4 columns (cap ≤ 32), or of 64 of 2
+                float t0;
+                if (cap <= 32)
+                    t0 = half_kth<2>(fmaxf(max3(sv[0], sv[1], sv[2]), sv[3]), fmaxf(max3(sv[4], sv[5], sv[6]), sv[7]), 0.f,
+                                     0.f, cap, lane);
+                else
+                    t0 = half_kth<4>(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]), fmaxf(sv[4], sv[5]), fmaxf(sv[6], sv[7]),
+                                     cap, lane);
+                if (t0 > -CUDART_INF_F) tau = fmaxf(tau, nextafterf(t0, -CUDART_INF_F));
+                if (tx == 0) tau_s[qi] = tau;
+            }
+            unsigned pend = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) pend |= (sv[j] > tau ? 1u : 0u) << j;
+            while (__any_sync(COSTAL_FULL_MASK, pend != 0)) {
+                int pos = pend ? atomicAdd(&cnt_s[qi], __popc(pend)) : 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (pend >> j & 1u) {
+                        if (pos < bcap) {
+                            bs[pos] = sv[j];
+                            bi[pos] = (uint32_t)(c0 + cj_of(j));
+                            pend &= ~(1u << j);
+                        }
+                        ++pos;
+                    }
+                }
+                __syncwarp();
+                const int c = cnt_s[qi];
+                const unsigned over = __ballot_sync(COSTAL_FULL_MASK, c > limit);
+                if (over) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        if (!(over >> (16 * h) & 1u)) continue;
+                        const int qh = qi_at(i, 2 * warp + h);
+                        float T = cut_buffer<SLB>(buf_s + qh * bcap, buf_i + qh * bcap,
+                                                  min(bcap, __shfl_sync(COSTAL_FULL_MASK, c, 16 * h)), cap, lane);
+                        if (lane == 0) {
+                            if (P.tau_shared) {
+                                const uint32_t k = okey(T);
+                                T = okey_inv(max(k, atomicMax(&P.tau_shared[q0 + qh], k)));
+                            }
+                            cnt_s[qh] = cap;
+                            tau_s[qh] = T;
+                        }
+                    }
+                    __syncwarp();
+                    tau = tau_s[qi];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (!(sv[j] > tau)) pend &= ~(1u << j);
+                }
+            }
+        }
+        __syncwarp();  // every lane sees the thresholds before the next tile's test
+        if (P.list_ub) {  // the warp's floor for the producer's stop test (signed-int order of the f32)
+            int key = __float_as_int(__fsub_rd(tau_s[qi_at(lane & 15, ty)], P.eps));
+            key = __reduce_min_sync(COSTAL_FULL_MASK, key >= 0 ? key : key ^ 0x7fffffff);
+            if (lane == 0)
+                *reinterpret_cast<volatile float*>(&bars->warp_floor[warp]) = __int_as_float(key >= 0 ? key : key ^ 0x7fffffff);
+        }
+    }
+
+    // the warp's 32 queries out: by row, or by slot into the segment's part
+    __syncwarp();
+#pragma unroll 1
+    for (int e = 0; e < 32; ++e) {
+        const int qi = qi_at(e & 15, 2 * warp + (e >> 4)), own = own_s[qi];
+        if (own < 0) continue;
+        int c = min(bcap, cnt_s[qi]);
+        float tau = tau_s[qi];
+        if (c > cap) {
+            tau = fmaxf(tau, cut_buffer<SLB>(buf_s + qi * bcap, buf_i + qi * bcap, c, cap, lane));
+            c = cap;
+        }
+        const size_t row = P.part_stride ? (size_t)blockIdx.y * P.part_stride + q0 + qi
+                                         : (size_t)(P.perm ? P.perm[own] : (uint32_t)own);
+        for (int p = lane; p < cap; p += 32) {
+            const uint32_t col = p < c ? buf_i[qi * bcap + p] : 0xffffffffu;
+            P.cand_idx[row * cap + p] = p < c && P.perm ? P.perm[col] : col;
+            P.cand_score[row * cap + p] = p < c ? buf_s[qi * bcap + p] : -CUDART_INF_F;
+        }
+        if (lane == 0) P.tau_out[row] = tau;
+    }
+}
+
+// The rows in working order (row-major [n][d]) as the transposed copy out[t][w], zero for w ≥ n and
+// t ≥ d: a CTA per 128 rows, staged through shared memory so that both sides are coalesced.
+__global__ void __launch_bounds__(256) k_work_cols(const float* __restrict__ wrows, int n, int np, int d, int dp,
+                                                   float* __restrict__ out) {
+    extern __shared__ float tile[];  // [BM][d + 1]
+    const int w0 = blockIdx.x * BM, rows = min(BM, n - w0);
+    for (int e = threadIdx.x; e < rows * d; e += 256) tile[(e / d) * (d + 1) + e % d] = wrows[(size_t)w0 * d + e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < dp * BM; e += 256) {
+        const int t = e / BM, r = e % BM;
+        out[(size_t)t * np + w0 + r] = r < rows && t < d ? tile[r * (d + 1) + t] : 0.0f;
+    }
+}
+
+// The listed queries' columns of xsT, side by side: out[t][q] = value t of row rows[q], zero for
+// q ≥ nq; mp = the slots rounded up to a whole block.
+__global__ void k_gather_cols(const float* __restrict__ xsT, int np, int dp, const uint32_t* __restrict__ rows, int nq,
+                              int mp, float* __restrict__ out) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= mp) return;
+    const uint32_t c = q < nq ? rows[q] : 0u;
+    for (int t = blockIdx.y; t < dp; t += gridDim.y) out[(size_t)t * mp + q] = q < nq ? xsT[(size_t)t * np + c] : 0.0f;
+}
+
+// The rows' f32 norm and squared norm from the f64 norms (knn.rs:207-212 rounds ‖x‖² to f32).
+__global__ void k_tani_norms(const double* __restrict__ norms, int n, float2* __restrict__ tnorm) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double a = norms[i];
+        tnorm[i] = make_float2((float)a, (float)(a * a));
+    }
+}
+
+// The launch shape for a depth and a candidate count: the query operand resident or streamed, the
+// buffer's entries, the dimensions and number of the ring's stages, CTAs per SM. Two CTAs per SM with
+// buffers of cap + 32 entries if they fit, else down to cap + 16, else one CTA per SM.
+struct Shape {
+    bool stream;
+    int bcap, kc, stages, ctas;
+    size_t smem;
+};
+
+static Shape shape_of(int dp, int cap) {
+    for (int ctas = 2; ctas >= 1; --ctas)
+        for (int extra = 32; extra >= 16; extra -= 8) {
+            Shape s{};
+            s.ctas = ctas;
+            s.stream = dp > 64;
+            s.bcap = (cap + extra + 3) / 4 * 4;
+            const size_t lim = ctas == 2 ? SMEM_TWO : SMEM_ONE;
+            const size_t fixed = 128 + (size_t)BM * s.bcap * 8 + BM * 12 + sizeof(Bars) + (s.stream ? 0 : (size_t)dp * BM * 4);
+            if (fixed >= lim) continue;
+            // the deepest stage of which two fit (whole tiles), else three
+            const int most = s.stream ? 16 : dp;
+            for (int kc = most; kc >= 8; kc -= 8) {
+                if (!s.stream && dp % kc) continue;
+                const size_t per = (size_t)kc * BN * 4 * (s.stream ? 2 : 1);
+                const int stages = (int)std::min<size_t>(MAX_STAGES, (lim - fixed) / per);
+                if (stages < (kc == dp ? 2 : 3)) continue;
+                s.kc = kc;
+                s.stages = stages;
+                s.smem = fixed + stages * per;
+                return s;
+            }
+        }
+    return Shape{};
+}
+
+// [rows][cols] f32 with boxes of box_cols × box_rows.
+static bool make_map(CUtensorMap* m, const void* base, size_t cols, int rows, int box_cols, int box_rows) {
+    auto fn = tensor_map_encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Column segments for nq queries against `tiles` column tiles: the number whose last wave of CTAs
+// (`slots` at a time) ends first, a CTA costing its tiles plus `start` tiles' worth of time for loading
+// its queries, seeding and writing its lists (and the merge reading one more list).
+static int segments(int nq, int tiles, int dp, int slots) {
+    const int blocks = (nq + BM - 1) / BM;
+    const double start = 1.0 + 64.0 / dp;
+    int best = 1;
+    double best_t = 1e300;
+    for (int s = 1; s <= std::min(64, tiles); ++s) {
+        const int tps = (tiles + s - 1) / s;
+        if ((tiles + tps - 1) / tps != s) continue;  // an empty segment
+        const double waves = (double)(((long long)blocks * s + slots - 1) / slots);
+        const double t = waves * (tps + start) * (1.0 + 1e-3 * s);
+        if (t < best_t * 0.98) {
+            best_t = t;
+            best = s;
+        }
+    }
+    return best;
+}
+
+static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+}  // namespace fp32
+
+namespace fp32 {
+struct Ws {
+    float* a;             // the listed queries' operand
+    uint32_t* part_idx;   // with segments: their lists, and the shared thresholds
+    float* part_score;
+    float* part_tau;
+    uint32_t* tau_shared;
+    size_t bytes;
+};
+static Ws carve(void* base, int dp, int cap, bool listed, int nq, int segs) {
+    const size_t mp = (size_t)(nq + BM - 1) / BM * BM;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char* p = static_cast<char*>(base) + off;
+        off += al256(bytes);
+        return p;
+    };
+    Ws w{};
+    w.a = reinterpret_cast<float*>(take(listed ? (size_t)dp * mp * 4 : 0));
+    const size_t per = segs > 1 ? (size_t)segs * nq : 0;
+    w.part_idx = reinterpret_cast<uint32_t*>(take(per * cap * 4));
+    w.part_score = reinterpret_cast<float*>(take(per * cap * 4));
+    w.part_tau = reinterpret_cast<float*>(take(per * 4));
+    w.tau_shared = reinterpret_cast<uint32_t*>(take(segs > 1 ? mp * 4 : 0));
+    w.bytes = off;
+    return w;
+}
+}  // namespace fp32
+
+cudaError_t launch_work_cols(const float* wrows, int n, int np, int d, int dp, float* xsW, cudaStream_t st) {
+    fp32::k_work_cols<<<np / fp32::BM, 256, (size_t)fp32::BM * (d + 1) * 4, st>>>(wrows, n, np, d, dp, xsW); note_launch();
+    return cudaGetLastError();
+}
+
+// (with lists, about a third of the tiles is visited)
+static int segs_of(const Fp32Job& J, const fp32::Shape& sh, int sm_count) {
+    const int tiles = J.np / fp32::BN;
+    return fp32::segments(J.nq, J.lists ? std::max(1, tiles / 3) : tiles, J.dp, sm_count * sh.ctas);
+}
+
+size_t coarse_fp32_ws_bytes(const Fp32Job& J, int sm_count) {
+    const fp32::Shape sh = fp32::shape_of(J.dp, J.cap);
+    const int segs = segs_of(J, sh, sm_count);
+    return fp32::carve(nullptr, J.dp, J.cap, J.rows != nullptr, J.nq, segs).bytes;
+}
+
+cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStream_t st) {
+    using namespace fp32;
+    if (J.nq <= 0) return cudaSuccess;
+    const Shape sh = shape_of(J.dp, J.cap);
+    if (sh.stages < 2) return cudaErrorInvalidValue;
+    const int mp = (J.nq + BM - 1) / BM * BM, tiles = J.np / BN;
+    const int segs = segs_of(J, sh, sm_count);
+    const Ws w = carve(ws, J.dp, J.cap, J.rows != nullptr, J.nq, segs);
+    cudaError_t e;
+    if (J.norms) {
+        k_tani_norms<<<std::min((J.n + 255) / 256, 1024), 256, 0, st>>>(J.norms, J.n, J.tnorm); note_launch();
+    }
+    if (J.rows) {
+        k_gather_cols<<<dim3(mp / BM, std::min(J.dp, 64)), BM, 0, st>>>(J.xsT, J.np, J.dp, J.rows, J.nq, mp, w.a);
+        note_launch();
+    }
+    if (segs > 1 && (e = cudaMemsetAsync(w.tau_shared, 0, (size_t)mp * 4, st)) != cudaSuccess) return e;
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, J.rows ? w.a : J.xsT, J.rows ? mp : J.np, J.dp, BM, sh.kc) ||
+        !make_map(&mb, J.xsT, J.np, J.dp, BN, sh.kc))
+        return cudaErrorInvalidValue;
+    Args P{};
+    P.n = J.n;
+    P.nq = J.nq;
+    P.cap = J.cap;
+    P.bcap = sh.bcap;
+    P.dp = J.dp;
+    P.kc = sh.kc;
+    P.tiles = tiles;
+    P.stages = sh.stages;
+    P.rows = J.rows;
+    P.perm = J.perm;
+    P.lists = J.lists;
+    P.list_ub = J.lists ? J.list_ub : nullptr;
+    P.counts = J.counts;
+    P.ncb = J.ncb;
+    P.epc = J.list_cb / BN;
+    P.eps = J.eps;
+    P.stopped_total = J.stopped_total;
+    P.part_stride = segs > 1 ? J.nq : 0;
+    P.tau_shared = segs > 1 ? w.tau_shared : nullptr;
+    P.tfloor = J.tfloor;
+    P.tnorm = J.norms ? J.tnorm : nullptr;
+    P.cand_idx = segs > 1 ? w.part_idx : J.cand_idx;
+    P.cand_score = segs > 1 ? w.part_score : J.cand_score;
+    P.tau_out = segs > 1 ? w.part_tau : J.tau;
+    P.timeout_flag = J.timeout_flag;
+    const int slb = (sh.bcap + 31) / 32;
+#define COSTAL_K(S)                                                                               \
+    (sh.stream ? (J.norms ? k_fp32_tiles<S, true, true> : k_fp32_tiles<S, true, false>)            \
+               : (J.norms ? k_fp32_tiles<S, false, true> : k_fp32_tiles<S, false, false>))
+    auto kern = slb <= 2 ? COSTAL_K(2) : slb == 3 ? COSTAL_K(3) : COSTAL_K(5);
+#undef COSTAL_K
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem)) != cudaSuccess) return e;
+    kern<<<dim3(mp / BM, segs), NT, sh.smem, st>>>(ma, mb, P); note_launch();
+    if (segs > 1)
+        return launch_merge_parts(J.rows ? J.rows : J.perm, J.nq, segs, J.cap, w.part_idx, w.part_score, J.tfloor, J.cand_idx, J.cand_score,
+                                  J.tau, st);
+    return cudaGetLastError();
+}
+
+}  // namespace costal

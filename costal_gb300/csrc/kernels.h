@@ -15,24 +15,39 @@ int coarse_slots(int cap);
 // d_pad of the working copy: a multiple of 8 up to 64 (compile-time tile depths), else of 4.
 int coarse_dpad(int d);
 size_t coarse_fp32_smem(int dp, int cap);
-// qlist/qcount (optional): run only the rows listed on the device (128 per CTA, grid sized for n).
-cudaError_t launch_coarse_fp32(const float* xsT, int n, int np, int dp, int cap, int lstride, const uint32_t* qlist,
-                               const unsigned* qcount, uint32_t* cand_idx, float* cand_score, float* tau,
-                               cudaStream_t st);
-// Few listed rows: the columns split into `segs` segments (one CTA per 128 rows per segment), their
-// lists merged per row. part_* hold segs × count × cap entries (τ: segs × count).
-int coarse_fp32_segments(int count, int np, int sm_count);
-// tfloor (optional, by row): a per-row threshold below which no column can be among the best cap.
-cudaError_t launch_coarse_fp32_split(const float* xsT, int n, int np, int dp, int cap, int lstride,
-                                     const uint32_t* qlist, const unsigned* qcount, int count, int segs,
-                                     const float* tfloor, uint32_t* part_idx, float* part_score, float* part_tau,
-                                     uint32_t* cand_idx, float* cand_score, float* tau, cudaStream_t st);
-// Tanimoto selection (knn.rs:197-284): the same FP32 pass over all columns with the coarse score
-// T = a·b·ĉ / (A + B − a·b·ĉ) from the normalised tile and the rows' norms (tnorm: n entries of
-// scratch, filled here); within 2(d+12)·2⁻²³ of the exact T.
-cudaError_t launch_coarse_fp32_tanimoto(const float* xsT, int n, int np, int dp, int cap, const double* norms,
-                                        float2* tnorm, uint32_t* cand_idx, float* cand_score, float* tau,
-                                        cudaStream_t st);
+// The FP32 coarse pass (fp32_tiles.cu): the queries (all n rows, or nq listed ones) against all columns.
+struct Fp32Job {
+    const float* xsT;      // [dp][np] the normalised rows, transposed
+    int n, np, dp, cap;
+    const uint32_t* rows;  // the queries' row ids on the device (NULL: all rows, nq = n)
+    int nq;
+    const float* tfloor;   // optional, by row: no column at or below it can be among the best cap
+    // Tanimoto selection (knn.rs:197-284): the f64 norms (NULL: cosine) and n entries of scratch for
+    // their f32 form; the coarse score is T = a·b·ĉ / (A + B − a·b·ĉ), within 2(d+12)·2⁻²³ of the exact T.
+    const double* norms;
+    float2* tnorm;
+    // Column lists (prune.cu), with xsT in the working order: perm, the lists of nqb query blocks with
+    // their bounds, list_cb (128 or 256) rows a column block, the coarse error bound rounded up to f32.
+    const uint32_t* perm;
+    const uint32_t* lists;
+    const float* list_ub;
+    const uint32_t* counts;
+    int ncb, list_cb;
+    float eps;
+    unsigned long long* stopped_total;
+    uint32_t* cand_idx;    // [n][cap], by original row, original column ids
+    float* cand_score;
+    float* tau;            // [n]
+    unsigned long long* timeout_flag;
+};
+size_t coarse_fp32_ws_bytes(const Fp32Job& job, int sm_count);
+cudaError_t launch_coarse_fp32(const Fp32Job& job, void* ws, int sm_count, cudaStream_t st);
+// The transposed copy of the rows in working order (prune::Plan::wrows, [n][d]): xsW [dp][np].
+cudaError_t launch_work_cols(const float* wrows, int n, int np, int d, int dp, float* xsW, cudaStream_t st);
+// The lists of `segs` column segments (segs × count × cap entries, τ: segs × count) merged per row.
+cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
+                               const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
+                               float* tau, cudaStream_t st);
 // Tanimoto selection with the norm window (knn.rs:595-644): rows in the norm order `perm` (working →
 // original, prune::norm_order), each query block walking outward from its own norms and stopping a
 // side once its norms leave every row's window; d_pad ≤ 64. ws holds tani_window_bytes(n, np, dp)

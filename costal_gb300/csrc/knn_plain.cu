@@ -4,7 +4,7 @@
 //   k_prep      — knn.rs:315-323 row_norms64 (f64, dimension order) and knn.rs:420-436 the
 //                 L2-normalised f32 working copy, written transposed (d_pad × n_pad) for the tiles;
 //                 also knn.rs:325-342's non-finite check (first bad row).
-//   (the FP32 coarse kernel, knn.rs:603-660 + 758-875, lives in coarse_fp32.cu)
+//   (the FP32 coarse kernel, knn.rs:603-660 + 758-875, lives in fp32_tiles.cu)
 //   k_rescore   — knn.rs:688-720 + 746-753: f64 rescoring of the cap candidates, the sort, the
 //                 ε-certificate s_k > τ + (d+4)·2⁻²³, and (fused) the Tanimoto edge weight of
 //                 weight.rs:30-37 for the k survivors.

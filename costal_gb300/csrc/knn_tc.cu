@@ -36,7 +36,6 @@
 #include <algorithm>
 
 #include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
@@ -46,6 +45,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "knn_tc.h"
+#include "ptx.cuh"
 #include "topk.cuh"
 
 namespace costal {
@@ -59,52 +59,6 @@ constexpr int B_HALF_BYTES = HALF_N * 128;     // 16 KB: the second half of a K 
 constexpr int EPI_WARPS = 4;
 constexpr int NTHREADS = (EPI_WARPS + 2) * 32;  // 4 epilogue warps, 1 TMA warp, 1 MMA warp
 constexpr uint32_t TMEM_COLS = 512;    // two 256-column FP32 accumulators
-constexpr long long WAIT_LIMIT = 1ll << 22;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// ---- mbarrier --------------------------------------------------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: false (and the flag raised) if the phase never completes. Every 1024 polls the wait
-// also checks the global flag, so once any thread of any CTA has given up, every later wait of the
-// launch returns at once and the kernel drains in microseconds.
-// Roles that are not the bottleneck (TMA, MMA issue) sleep between polls so that they do not take
-// issue slots from the epilogue warps that share their schedulers.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long* timeout_flag,
-                                          bool sleep) {
-    for (long long i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (sleep) __nanosleep(64);
-        if ((i & 1023) == 1023 && *reinterpret_cast<volatile unsigned long long*>(timeout_flag)) return false;
-    }
-    atomicExch(timeout_flag, 1ull);
-    return false;
-}
-
-// ---- TMA ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-        : "memory");
-}
 
 // ---- tcgen05 -----------------------------------------------------------------------------------
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
@@ -1270,22 +1224,10 @@ size_t workspace_bytes(int n, int d, bool fp8) {
 }
 
 namespace {
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        cudaDriverEntryPointQueryResult q;
-        void* p = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-    return fn;
-}
-
 // A 2-D map of an operand ([rows][kp] elements of bf16 or e4m3 bytes) with 128-byte boxes of
 // box_rows rows (one K block: 64 bf16 or 128 e4m3).
 bool make_map(CUtensorMap* m, const void* base, int kp, int rows, int box_rows, bool fp8 = false) {
-    auto fn = encode_fn();
+    auto fn = tensor_map_encode_fn();
     if (!fn) return false;
     const int esize = fp8 ? 1 : 2;
     cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows};

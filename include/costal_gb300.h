@@ -54,8 +54,8 @@ typedef struct costal_knn_opts {
     uint32_t row_block;    /* accepted for compatibility (knn.rs:35-37); speed-only, 0 = derive */
     uint32_t col_block;    /* idem */
     int32_t sort_by_norm;  /* idem (knn.rs:41): output-independent */
-    int32_t prune;         /* idem (knn.rs:44): output-independent; on the bf16 backend it enables the
-                              exact early stop of each query block's column list */
+    int32_t prune;         /* idem (knn.rs:44): output-independent; it enables the exact early stop of each
+                              query block's column list (bf16 backend; FP32 from 32,768 rows, d <= 64) */
     int32_t learned_prune; /* 1 = use the trained block-pruning model if one is loaded (bf16 backend) */
 } costal_knn_opts;
 
@@ -71,10 +71,10 @@ typedef struct costal_knn_stats {
     uint64_t pruned_fallback_rows; /* learned pruning: rows whose skip was not certified, rescanned */
     double max_coarse_err;     /* max |coarse score - f64 rescored score| over all kept candidates */
     double ms_prep, ms_coarse, ms_rescore, ms_fallback, ms_total; /* CUDA-event times of the stages */
-    double ms_order;           /* bf16 backend: locality order, block bounds and lists (inside ms_total) */
+    double ms_order;           /* locality order, block bounds and lists, where used (inside ms_total) */
     double ms_kernel;          /* the coarse tile + selection kernel alone (inside ms_coarse) */
-    uint64_t blocks_stopped;   /* bf16 backend: list blocks left out because every row's threshold
-                                  already exceeded their bound (exact; no certificate needed) */
+    uint64_t blocks_stopped;   /* list blocks left out because every row's threshold already exceeded
+                                  their bound (exact; no certificate needed) */
     double max_err_ratio;      /* max over the rescored candidates of |coarse - f64 score| divided by the
                                   bound the row's certificate used (E_i on the bf16 backend, the FP32
                                   epsilon otherwise): the certificate is sound while this stays below 1 */
