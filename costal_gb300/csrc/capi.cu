@@ -68,7 +68,7 @@ struct Context {
     DevBuf x, norms, xsT, cand_idx, cand_score, tau, out_idx, out_cos, out_w, fb_rows, fb_minsim, misc;
     DevBuf fu_scratch, rows, cols, wout, idx_in, cos_in, norms_in, w_in, jac, f32out, tc_ws, tc_rows, prune_ws;
     DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows;
-    DevBuf fp32_ws, tfloor, xsW;
+    DevBuf fp32_ws, tfloor, xsW, xsR;
     DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_perm, tani_ws, rm_ws, rm_out;
     MlpState mlp;
 };
@@ -214,9 +214,9 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 
 // Whether the FP32 pass visits its columns by lists, nearest blocks first with the exact early stop,
 // instead of all tiles in order: where the tiles and admissions it saves cost more than the order stage
-// (measured, whole kNN, lists / all tiles: 20,000 × 32 2.2 / 1.7 ms, 40,000 × 20 3.3 / 4.4, 80,000 × 32
-// 8.0 / 12.6, 161,443 × 32 16.6 / 39.8).
-bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 32768; }
+// (measured, whole kNN, lists / all tiles: 12,000 × 32 0.94 / 0.78 ms, 20,000 × 32 1.5 / 1.7,
+// 40,000 × 20 2.5 / 4.4, 80,000 × 32 6.5 / 12.6, 161,443 × 32 14.9 / 39.8).
+bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 16384; }
 
 // The FP32 pass's working order and column lists: the same cells, bounds and lists as the tensor-core
 // path (the per-row bounds come from its split operands, with their margin), and the rows' transposed
@@ -224,7 +224,7 @@ bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 32768; }
 void build_fp32_lists(Context& c, int n, int np, int d, int dp, prune::Plan& pp, cudaStream_t s) {
     Misc* dm = c.misc.as<Misc>();
     CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
-    CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), n, np, d, s, pp));
+    CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), n, np, d, s, pp));
     CK(ensure(c.tc_ws, tc::workspace_bytes(n, d, false)));
     tc::Plan plan{};
     CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), n, np, dp, d, pp.perm, s, plan, false, pp.wrows));
@@ -312,17 +312,24 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     CK(ensure(c.fb_rows, (size_t)n * 4));
     CK(ensure(c.fb_minsim, (size_t)n * 8));
     CK(cudaEventRecord(c.ev[0], s));
-    CK(launch_prep(d_x, n, d, np, dp, d_norms, c.xsT.as<float>(), &dm->bad_row, s));
+    const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
+    const bool tc_backend = o.backend == COSTAL_BACKEND_BF16 || o.backend == COSTAL_BACKEND_BF16X3 ||
+                            o.backend == COSTAL_BACKEND_FP8;
+    // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
+    const bool fp32_lists = !tc_backend && !tanimoto && !scan_all && !shard && o.prune && cap < n - 1 && fp32_lists_pay(n, d);
+    float* xsR = nullptr;
+    if (fp32_lists || (tc_backend && !tanimoto && !scan_all && prune::supported(d))) {
+        CK(ensure(c.xsR, (size_t)n * d * 4));
+        xsR = c.xsR.as<float>();
+    }
+    CK(launch_prep(d_x, n, d, np, dp, d_norms, c.xsT.as<float>(), xsR, &dm->bad_row, s));
     CK(cudaEventRecord(c.ev[1], s));
     CK(cudaEventRecord(c.ev[5], s));
-    const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
     bool used_tc = false;
     int list_cb = 0;  // rows of a column block of the tensor-core path's lists (0: no lists)
     // The split-FP8 kind: its coarse scores are ~2⁻⁸ coarser than split BF16's, so it keeps 64
     // candidates a row whatever the margin (the output does not depend on it) to let the certificate
     // hold for nearly every row.
-    const bool tc_backend = o.backend == COSTAL_BACKEND_BF16 || o.backend == COSTAL_BACKEND_BF16X3 ||
-                            o.backend == COSTAL_BACKEND_FP8;
     bool fp8 = !tanimoto && !scan_all && (o.backend == COSTAL_BACKEND_FP8 || (o.backend == COSTAL_BACKEND_BF16 && d >= 512));
     if (fp8) {
         const int cap8 = std::max(cap, std::min(64, n - 1));
@@ -392,7 +399,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             bool learned = false;
             if (ordered) {
                 CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
-                CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), n, np, d, s, pp));
+                CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), n, np, d, s, pp));
             }
             CK(ensure(c.tc_ws, tc::workspace_bytes(n, d, fp8)));
             CK(ensure(c.tc_rows, (size_t)n * 4));
@@ -471,7 +478,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             if (!shard) {
                 Fp32Job j = fp32_job(c, n, np, dp, cap);
                 prune::Plan pp{};
-                if (o.prune && cap < n - 1 && fp32_lists_pay(n, d)) {
+                if (fp32_lists) {
                     build_fp32_lists(c, n, np, d, dp, pp, s);
                     list_cb = pp.cb;
                     j.xsT = c.xsW.as<float>();
@@ -677,7 +684,7 @@ int costal_knn_bruteforce(const float* x, uint64_t n, uint32_t d, uint32_t k, ui
         Misc* dm = c.misc.as<Misc>();
         CK(cudaMemsetAsync(&dm->bad_row, 0xff, 8, s));
         CK(cudaMemcpyAsync(c.x.p, x, n * d * 4ull, cudaMemcpyHostToDevice, s));
-        CK(launch_prep(c.x.as<float>(), (int)n, (int)d, np, dp, c.norms.as<double>(), c.xsT.as<float>(), &dm->bad_row, s));
+        CK(launch_prep(c.x.as<float>(), (int)n, (int)d, np, dp, c.norms.as<double>(), c.xsT.as<float>(), nullptr, &dm->bad_row, s));
         if (gather_smem(k, d, dp) > 227 * 1024) throw Fail{COSTAL_EUNSUPPORTED, "k too large for the GPU scan kernel"};
         CK(launch_gather(c.x.as<float>(), c.xsT.as<float>(), (int)n, np, (int)d, dp, (int)k, c.norms.as<double>(),
                          nullptr, nullptr, nullptr, 1, select == COSTAL_SELECT_TANIMOTO ? 1 : 0,
@@ -970,11 +977,12 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(cudaMemsetAsync(&dm->bad_row, 0xff, 8, s));
         CK(cudaMemcpyAsync(c.x.p, x, n * d * 4ull, cudaMemcpyHostToDevice, s));
         CK(cudaEventRecord(c.ev[0], s));
-        CK(launch_prep(c.x.as<float>(), N, D, np, dp, c.norms.as<double>(), c.xsT.as<float>(), &dm->bad_row, s));
+        CK(ensure(c.xsR, n * d * 4ull));
+        CK(launch_prep(c.x.as<float>(), N, D, np, dp, c.norms.as<double>(), c.xsT.as<float>(), c.xsR.as<float>(), &dm->bad_row, s));
         // the same cells (and so the same features) as the pruned kNN computes for this data
         CK(ensure(c.prune_ws, prune::workspace_bytes(N, D)));
         prune::Plan pp{};
-        CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), N, np, D, s, pp));
+        CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), N, np, D, s, pp));
         // labels: the exact k-th-neighbour cosine of every sampled row, from the plain FP32 path
         uint32_t* rows = c.mlp_rows.as<uint32_t>();
         CK(launch_stride_rows(rows, m, N, s));
@@ -1144,10 +1152,11 @@ int costal_block_bounds(const float* x, uint64_t n, uint32_t d, uint32_t* perm, 
         CK(cudaMemsetAsync(dm, 0, sizeof(Misc), s));
         CK(cudaMemsetAsync(&dm->bad_row, 0xff, 8, s));
         CK(cudaMemcpyAsync(c.x.p, x, n * d * 4ull, cudaMemcpyHostToDevice, s));
-        CK(launch_prep(c.x.as<float>(), N, D, np, dp, c.norms.as<double>(), c.xsT.as<float>(), &dm->bad_row, s));
+        CK(ensure(c.xsR, n * d * 4ull));
+        CK(launch_prep(c.x.as<float>(), N, D, np, dp, c.norms.as<double>(), c.xsT.as<float>(), c.xsR.as<float>(), &dm->bad_row, s));
         CK(ensure(c.prune_ws, prune::workspace_bytes(N, D)));
         prune::Plan pp{};
-        CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), N, np, D, s, pp));
+        CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), N, np, D, s, pp));
         CK(ensure(c.tc_ws, tc::workspace_bytes(N, D, false)));
         tc::Plan plan{};
         CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), N, np, dp, D, pp.perm, s, plan, false, pp.wrows));

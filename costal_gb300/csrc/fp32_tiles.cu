@@ -41,6 +41,7 @@
 #include <stdint.h>
 
 #include "common.cuh"
+#include "fp32_tile.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
 #include "topk.cuh"
@@ -68,44 +69,6 @@ struct __align__(8) Bars {
     int c0[MAX_STAGES];  // first column of the stage's tile, −1: no more tiles
     float warp_floor[CONS_WARPS];  // per consumer warp: min over its queries of τ − ε (never decreases)
 };
-
-__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float lo_of(unsigned long long r) { return __uint_as_float((uint32_t)r); }
-__device__ __forceinline__ float hi_of(unsigned long long r) { return __uint_as_float((uint32_t)(r >> 32)); }
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-
-__device__ __forceinline__ unsigned long long twice(float x) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
-}
-
-// 8 depth steps of the register tile. A: [t][128] queries, B: [t][128] columns, 16 bytes an element
-// here; acc[p][j] holds queries 2p and 2p + 1 of the thread's 16 and column j of its 8.
-__device__ __forceinline__ void fma8(const ulonglong2* A, const float4* B, int tx, int ty,
-                                     unsigned long long (&acc)[8][8]) {
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        const ulonglong2 a0 = A[t * 32 + ty], a1 = A[t * 32 + 8 + ty], a2 = A[t * 32 + 16 + ty], a3 = A[t * 32 + 24 + ty];
-        const float4 b0 = B[t * 32 + tx], b1 = B[t * 32 + 16 + tx];
-        const unsigned long long a[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const unsigned long long bb = twice(b[j]);
-#pragma unroll
-            for (int p = 0; p < 8; ++p) acc[p][j] = ffma2(a[p], bb, acc[p][j]);
-        }
-    }
-}
 
 // The cap-th largest of a half warp's 16·R values (R per lane): a bitonic sorting network over the
 // 16 lanes, both halves of the warp at once. Out of line: it runs once per row of the first tile.
@@ -355,8 +318,8 @@ __global__ void __launch_bounds__(NT, 2)
     // ---------------------------------------------------------------------- consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_CONSUMER));
     const int tx = lane & 15, ty = 2 * warp + (lane >> 4);
-    auto qi_at = [&](int i, int y) { return (i >> 2) * 32 + y * 4 + (i & 3); };  // query i of thread row y
-    auto cj_of = [&](int j) { return j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4); };
+    auto qi_at = [&](int i, int y) { return tile_row(i, y); };  // query i of thread row y
+    auto cj_of = [&](int j) { return tile_col(j, tx); };
     const int limit = cap + (bcap - cap) * 3 / 4;
     if (!STREAM && !mbar_wait(&bars->a_full, 0, P.timeout_flag, false)) return;
     int s = 0;
@@ -385,7 +348,7 @@ __global__ void __launch_bounds__(NT, 2)
             }
         }
         if (c0 < 0) break;
-        auto score = [&](int i, int j) { return i & 1 ? hi_of(acc[i >> 1][j]) : lo_of(acc[i >> 1][j]); };
+        auto score = [&](int i, int j) { return tile_score(acc, i, j); };
         // rows whose tile maximum is above their threshold (Tanimoto: above the cosine that threshold needs)
         unsigned m = 0;
         if (!first) {

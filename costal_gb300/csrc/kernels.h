@@ -8,7 +8,8 @@
 namespace costal {
 
 // ---- knn_plain.cu ------------------------------------------------------------------------------
-cudaError_t launch_prep(const float* x, int n, int d, int np, int dp, double* norms, float* xsT,
+// xsR (optional): the normalised rows row-major [n][d] too.
+cudaError_t launch_prep(const float* x, int n, int d, int np, int dp, double* norms, float* xsT, float* xsR,
                         unsigned long long* bad_row, cudaStream_t st);
 cudaError_t launch_row_l2_norms_f32(const float* x, int n, int d, float* out, cudaStream_t st);
 int coarse_slots(int cap);

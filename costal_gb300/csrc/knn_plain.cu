@@ -38,7 +38,7 @@ constexpr int PREP_TCHUNK = 64;
 // so the f64 sum has exactly the reference's order.
 __global__ void __launch_bounds__(PREP_ROWS) k_prep(const float* __restrict__ x, int n, int d, int np, int dp,
                                                     double* __restrict__ norms, float* __restrict__ xsT,
-                                                    unsigned long long* __restrict__ bad_row) {
+                                                    float* __restrict__ xsR, unsigned long long* __restrict__ bad_row) {
     __shared__ float tile[PREP_ROWS * (PREP_TCHUNK + 1)];
     const int r0 = blockIdx.x * PREP_ROWS;
     const int r = r0 + threadIdx.x;
@@ -83,8 +83,18 @@ __global__ void __launch_bounds__(PREP_ROWS) k_prep(const float* __restrict__ x,
         if (r < np) {
             for (int tt = 0; tt < tend; ++tt) {
                 float v = 0.0f;
-                if (r < n && t0 + tt < d) v = (float)(f64_of(tile[threadIdx.x * (PREP_TCHUNK + 1) + tt]) * inv);
+                if (r < n && t0 + tt < d) {
+                    v = (float)(f64_of(tile[threadIdx.x * (PREP_TCHUNK + 1) + tt]) * inv);
+                    if (xsR) tile[threadIdx.x * (PREP_TCHUNK + 1) + tt] = v;
+                }
                 xsT[(size_t)(t0 + tt) * np + r] = v;
+            }
+        }
+        if (xsR && tc > 0) {  // the row-major copy (the order stage gathers whole rows of it)
+            __syncthreads();
+            for (int e = threadIdx.x; e < rows * tc; e += PREP_ROWS) {
+                const int rr = e / tc, tt = e % tc;
+                xsR[(size_t)(r0 + rr) * d + t0 + tt] = tile[rr * (PREP_TCHUNK + 1) + tt];
             }
         }
     }
@@ -497,10 +507,10 @@ __global__ void __launch_bounds__(GT)
 // launchers
 // =================================================================================================
 
-cudaError_t launch_prep(const float* x, int n, int d, int np, int dp, double* norms, float* xsT,
+cudaError_t launch_prep(const float* x, int n, int d, int np, int dp, double* norms, float* xsT, float* xsR,
                         unsigned long long* bad_row, cudaStream_t st) {
     const int blocks = (np + PREP_ROWS - 1) / PREP_ROWS;
-    k_prep<<<blocks, PREP_ROWS, 0, st>>>(x, n, d, np, dp, norms, xsT, bad_row); note_launch();
+    k_prep<<<blocks, PREP_ROWS, 0, st>>>(x, n, d, np, dp, norms, xsT, xsR, bad_row); note_launch();
     return cudaGetLastError();
 }
 

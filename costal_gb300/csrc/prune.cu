@@ -31,80 +31,119 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
+#include "fp32_tile.cuh"
 #include "kernels.h"
 #include "prune.h"
 
 namespace costal {
 namespace prune {
 
-constexpr int KM_BLOCK = 128;
-
 // ---- k-means ----------------------------------------------------------------------------------
 
-// Rows of xsT (d × np, transposed) listed in `rows` → a row-major [m][d] copy.
-__global__ void k_gather_rows(const float* __restrict__ xsT, int np, int d, const uint32_t* __restrict__ rows, int m,
-                              float* __restrict__ out) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m * d; e += gridDim.x * blockDim.x) {
-        const int i = e / d, t = e % d;
-        out[e] = xsT[(size_t)t * np + rows[i]];
+// The sample (row j of it: row ⌊j·n/m⌋), row-major [m][d] and transposed [dp][mp] (zero padded), and the
+// initial centroids: K evenly spaced sample rows, row-major and transposed [dp][K].
+__global__ void k_sample(const float* __restrict__ xsR, int n, int d, int dp, int m, int mp, int K, float* __restrict__ rows,
+                         float* __restrict__ rowsT, float* __restrict__ cent, float* __restrict__ centT) {
+    auto source = [&](int j) { return (size_t)(((unsigned long long)j * (unsigned long long)n) / (unsigned long long)m); };
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < mp * dp; e += gridDim.x * blockDim.x) {
+        const int t = e / mp, j = e - t * mp;  // (transposed: lanes run over the rows)
+        const float v = j < m && t < d ? xsR[source(j) * d + t] : 0.0f;
+        rowsT[e] = v;
+        if (j < m && t < d) rows[(size_t)j * d + t] = v;
+    }
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K * dp; e += gridDim.x * blockDim.x) {
+        const int t = e / K, c = e - t * K;
+        const float v = t < d ? xsR[source((int)(((long long)c * m) / K)) * d + t] : 0.0f;
+        centT[e] = v;
+        if (t < d) cent[(size_t)c * d + t] = v;
     }
 }
 
-// Best centroid (largest dot with the unit centroid) of every row; rows are either a row-major
-// [m][d] array (rows_rm) or the columns of xsT. Centroids live in shared memory, rows padded to a
-// multiple of 4 with zeros, read 16 bytes at a time (every thread reads the same centroid: a
-// broadcast); the dot keeps the dimension order.
-__global__ void __launch_bounds__(KM_BLOCK) k_assign(const float* __restrict__ rows_rm, const float* __restrict__ xsT,
-                                                     int np, int m, int d, const float* __restrict__ cent, int K,
-                                                     uint32_t* __restrict__ assign) {
-    extern __shared__ float4 c_s4[];  // [K][dq/4]
-    float* c_s = reinterpret_cast<float*>(c_s4);
-    const int dq = (d + 3) & ~3, q4 = dq >> 2;
-    for (int e = threadIdx.x; e < K * dq; e += blockDim.x) {
-        const int c = e / dq, t = e - c * dq;
-        c_s[e] = t < d ? cent[c * d + t] : 0.0f;
+// Best centroid (largest dot with the unit centroid, ties to the smallest index) of every column of
+// rowsT [dp][mp]: 128 rows per CTA against the 256 centroids (centT [dp][256]) on the 16 × 8 register
+// tile, in two halves of 128 centroids. Every dot is one FMA chain in dimension order. One row per
+// thread against broadcast centroids took a 16-byte shared load for every 4 FMAs: 1.83 ms at
+// 2,000,000 × 40, 100 us for a 65,536-row sample; this tile 1 per 8 paired FMAs.
+constexpr int KM_ROWS = 128;
+__global__ void __launch_bounds__(128, 2) k_assign(const float* __restrict__ rowsT, int mp, int m, int dp,
+                                                   const float* __restrict__ centT, uint32_t* __restrict__ assign) {
+    using namespace fp32;
+    static_assert(K_CENTROIDS == 256, "two halves of 128 centroids");
+    extern __shared__ float4 km_s[];
+    float* rows_s = reinterpret_cast<float*>(km_s);  // [dp][128]
+    float* cent_s = rows_s + dp * KM_ROWS;           // [2][dp][128]
+    const int r0 = blockIdx.x * KM_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e = threadIdx.x; e < dp * 32; e += 128)
+        cp_async16(rows_s + e * 4, rowsT + (size_t)(e >> 5) * mp + r0 + (e & 31) * 4);
+    for (int e = threadIdx.x; e < dp * 64; e += 128) {
+        const int t = e >> 6, c4 = e & 63;
+        cp_async16(cent_s + ((c4 >> 5) * dp + t) * 128 + (c4 & 31) * 4, centT + (size_t)t * 256 + c4 * 4);
     }
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    float x[64];
+    const int tx = lane & 15, ty = 2 * warp + (lane >> 4);
+    float best[16];
+    int arg[16];
 #pragma unroll
-    for (int t = 0; t < 64; ++t) x[t] = t < d ? (rows_rm ? rows_rm[(size_t)i * d + t] : xsT[(size_t)t * np + i]) : 0.0f;
-    float best = -CUDART_INF_F;
-    uint32_t arg = 0;
-    for (int c = 0; c < K; ++c) {
-        float s = 0.0f;
-#pragma unroll
-        for (int t4 = 0; t4 < 16; ++t4) {
-            if (t4 < q4) {
-                const float4 w = c_s4[c * q4 + t4];
-                s = fmaf(x[4 * t4], w.x, s);
-                s = fmaf(x[4 * t4 + 1], w.y, s);
-                s = fmaf(x[4 * t4 + 2], w.z, s);
-                s = fmaf(x[4 * t4 + 3], w.w, s);
-            }
-        }
-        if (s > best) {
-            best = s;
-            arg = (uint32_t)c;
-        }
+    for (int i = 0; i < 16; ++i) {
+        best[i] = -CUDART_INF_F;
+        arg[i] = 0;
     }
-    assign[i] = arg;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        unsigned long long acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+#pragma unroll 1
+        for (int t = 0; t < dp; t += 8)
+            fma8(reinterpret_cast<const ulonglong2*>(rows_s) + t * 32,
+                 reinterpret_cast<const float4*>(cent_s + h * dp * 128) + t * 32, tx, ty, acc);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {  // ascending centroid indices
+                const float v = tile_score(acc, i, j);
+                if (v > best[i]) {
+                    best[i] = v;
+                    arg[i] = h * 128 + tile_col(j, tx);
+                }
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(COSTAL_FULL_MASK, best[i], o);
+            const int oa = __shfl_xor_sync(COSTAL_FULL_MASK, arg[i], o);
+            const bool take = ob > best[i] || (ob == best[i] && oa < arg[i]);
+            best[i] = take ? ob : best[i];
+            arg[i] = take ? oa : arg[i];
+        }
+        const int r = r0 + tile_row(i, ty);
+        if (tx == i && r < m) assign[r] = (uint32_t)arg[i];
+    }
 }
 
 // One CTA per centroid: the normalised sum of its rows, summed in a fixed order (deterministic): the
 // rows fall into 128 classes by (row / 4) mod 128, each class adds its rows in row order, and the 128
-// class sums are combined by a fixed pairwise tree. Warp w takes classes 16w … 16w+15 one after the
-// other, lane t holding dimensions t and t + 32: the class's assignment words are loaded four per
+// class sums are combined by a fixed pairwise tree. Warp w takes classes 4w … 4w+3 one after the
+// other (the adds wait for their rows: 32 warps a centroid hide that, 8 did not), lane t holding dimensions t and t + 32: the class's assignment words are loaded four per
 // lane at once and its matches found by ballots, so the warp's branches are uniform and a row is read
 // coalesced. An empty cluster keeps its previous centroid.
-constexpr int UPD_T = 256;
+constexpr int UPD_T = 1024;
 constexpr int UPD_CLASSES = 128;
 constexpr int UPD_GROUPS = 128;  // word groups of a class: m ≤ 4 · 128 · 128 rows
 static_assert(4 * UPD_CLASSES * UPD_GROUPS >= SAMPLE, "the centroid update covers the k-means sample");
 __global__ void __launch_bounds__(UPD_T) k_centroid_update(const float* __restrict__ rows, int m, int d,
-                                                           const uint32_t* __restrict__ assign, float* __restrict__ cent) {
+                                                           const uint32_t* __restrict__ assign, float* __restrict__ cent,
+                                                           float* __restrict__ centT) {
     constexpr int NW = UPD_T / 32, CPW = UPD_CLASSES / NW;
     __shared__ float part[UPD_CLASSES][65];
     __shared__ int cnt_s[UPD_CLASSES];
@@ -169,105 +208,175 @@ __global__ void __launch_bounds__(UPD_T) k_centroid_update(const float* __restri
         nrm = (float)sqrt(nn);
     }
     __syncthreads();
-    if ((int)threadIdx.x < d && nrm > 0.0f) cent[(size_t)c * d + threadIdx.x] = part[0][threadIdx.x] / nrm;
+    if ((int)threadIdx.x < d && nrm > 0.0f) {
+        const float v = part[0][threadIdx.x] / nrm;
+        cent[(size_t)c * d + threadIdx.x] = v;
+        centT[(size_t)threadIdx.x * K_CENTROIDS + c] = v;
+    }
 }
 
 // ---- working order: stable counting sort of rows by cell -------------------------------------
 
+// Chunks of 1,024 rows, one warp each: a histogram per chunk (hist [K][chunks]), every cell's counts
+// scanned over the chunks, and the scatter: within a chunk a row's rank among the equal cells before it
+// comes from a warp match. (One thread per chunk, walking its rows, took 0.5–0.8 ms at any n.)
 constexpr int CHUNK = 1024;
+constexpr int SORT_WARPS = 4;
 
-__global__ void k_cell_hist(const uint32_t* __restrict__ cell, int n, int K, uint32_t* __restrict__ hist) {
-    // one thread per chunk, sequential over its rows (deterministic)
-    const int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nch = (n + CHUNK - 1) / CHUNK;
+__global__ void __launch_bounds__(32 * SORT_WARPS) k_cell_hist(const uint32_t* __restrict__ cell, int n, int K, int nch,
+                                                               uint32_t* __restrict__ hist) {
+    extern __shared__ uint32_t sort_s[];  // [SORT_WARPS][K]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ch = blockIdx.x * SORT_WARPS + warp;
+    uint32_t* h = sort_s + warp * K;
+    for (int c = lane; c < K; c += 32) h[c] = 0u;
+    __syncwarp();
     if (ch >= nch) return;
-    uint32_t* h = hist + (size_t)ch * K;
-    for (int c = 0; c < K; ++c) h[c] = 0;
     const int end = min(n, (ch + 1) * CHUNK);
-    for (int i = ch * CHUNK; i < end; ++i) h[cell[i]] += 1;
+    for (int i = ch * CHUNK + lane; i < end; i += 32) atomicAdd(&h[cell[i]], 1u);
+    __syncwarp();
+    for (int c = lane; c < K; c += 32) hist[(size_t)c * nch + ch] = h[c];
 }
 
-// Exclusive offsets in (cell, chunk) order: thread c totals its cell over the chunks, one warp
-// scans the K totals, then thread c rewrites its column of the histogram as offsets.
-__global__ void k_cell_scan(uint32_t* __restrict__ hist, int nch, int K, uint32_t* __restrict__ cell_start) {
-    __shared__ uint32_t tot[1024];
-    const int c = threadIdx.x;
-    uint32_t s = 0;
-    if (c < K)
-        for (int ch = 0; ch < nch; ++ch) s += hist[(size_t)ch * K + c];
-    tot[c] = s;
-    __syncthreads();
-    if (c == 0) {
-        uint32_t acc = 0;
-        for (int j = 0; j < K; ++j) {
-            const uint32_t v = tot[j];
-            tot[j] = acc;
-            acc += v;
+// One CTA per cell: its chunk counts become exclusive offsets within the cell; total[c] = its rows.
+__global__ void __launch_bounds__(256) k_cell_scan(uint32_t* __restrict__ hist, int nch, uint32_t* __restrict__ total) {
+    __shared__ uint32_t wsum[8];
+    uint32_t* row = hist + (size_t)blockIdx.x * nch;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (int b = 0; b < nch; b += 256) {
+        const int e = b + threadIdx.x;
+        const uint32_t v = e < nch ? row[e] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(COSTAL_FULL_MASK, x, o);
+            if (lane >= o) x += y;
         }
-        cell_start[K] = acc;
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        uint32_t before = carry, all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            before += w < warp ? wsum[w] : 0u;
+            all += wsum[w];
+        }
+        if (e < nch) row[e] = before + x - v;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+__global__ void __launch_bounds__(32 * SORT_WARPS) k_cell_scatter(const uint32_t* __restrict__ cell, int n, int K, int nch,
+                                                                  const uint32_t* __restrict__ hist,
+                                                                  const uint32_t* __restrict__ total,
+                                                                  uint32_t* __restrict__ perm) {
+    extern __shared__ uint32_t sort_s[];  // [K] cell starts, then [SORT_WARPS][K] the chunks' next positions
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ch = blockIdx.x * SORT_WARPS + warp;
+    uint32_t* start = sort_s;
+    if (warp == 0) {  // exclusive scan of the cells' totals
+        uint32_t carry = 0;
+        for (int b = 0; b < K; b += 32) {
+            const uint32_t v = b + lane < K ? total[b + lane] : 0u;
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(COSTAL_FULL_MASK, x, o);
+                if (lane >= o) x += y;
+            }
+            if (b + lane < K) start[b + lane] = carry + x - v;
+            carry += __shfl_sync(COSTAL_FULL_MASK, x, 31);
+        }
     }
     __syncthreads();
-    if (c < K) {
-        uint32_t acc = tot[c];
-        cell_start[c] = acc;
-        for (int ch = 0; ch < nch; ++ch) {
-            const uint32_t v = hist[(size_t)ch * K + c];
-            hist[(size_t)ch * K + c] = acc;
-            acc += v;
+    if (ch >= nch) return;
+    uint32_t* next = sort_s + (1 + warp) * K;
+    for (int c = lane; c < K; c += 32) next[c] = start[c] + hist[(size_t)c * nch + ch];
+    __syncwarp();
+    const int end = min(n, (ch + 1) * CHUNK);
+    for (int i0 = ch * CHUNK; i0 < end; i0 += 32) {
+        const int i = i0 + lane;
+        const bool live = i < end;
+        const uint32_t c = live ? cell[i] : 0xffffffffu;
+        const unsigned peers = __match_any_sync(COSTAL_FULL_MASK, c);
+        uint32_t base = 0;
+        if (live) base = next[c];
+        __syncwarp();
+        if (live) {
+            perm[base + __popc(peers & ((1u << lane) - 1u))] = (uint32_t)i;
+            if (lane == __ffs(peers) - 1) next[c] = base + __popc(peers);
         }
+        __syncwarp();
     }
 }
 
-__global__ void k_cell_scatter(const uint32_t* __restrict__ cell, int n, int K, uint32_t* __restrict__ hist,
-                               uint32_t* __restrict__ perm) {
-    const int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nch = (n + CHUNK - 1) / CHUNK;
-    if (ch >= nch) return;
-    uint32_t* h = hist + (size_t)ch * K;
-    const int end = min(n, (ch + 1) * CHUNK);
-    for (int i = ch * CHUNK; i < end; ++i) perm[h[cell[i]]++] = (uint32_t)i;
+// The stable order of n rows by cell (K cells). hist: K·⌈n/CHUNK⌉ words, total: K.
+static cudaError_t sort_by_cell(const uint32_t* cell, int n, int K, uint32_t* hist, uint32_t* total, uint32_t* perm,
+                                cudaStream_t st) {
+    const int nch = (n + CHUNK - 1) / CHUNK, blocks = (nch + SORT_WARPS - 1) / SORT_WARPS;
+    k_cell_hist<<<blocks, 32 * SORT_WARPS, (size_t)SORT_WARPS * K * 4, st>>>(cell, n, K, nch, hist); note_launch();
+    k_cell_scan<<<K, 256, 0, st>>>(hist, nch, total); note_launch();
+    k_cell_scatter<<<blocks, 32 * SORT_WARPS, (size_t)(SORT_WARPS + 1) * K * 4, st>>>(cell, n, K, nch, hist, total, perm);
+    note_launch();
+    return cudaGetLastError();
+}
+
+// The rows in working order, row-major: wrows[w] = xsR[perm[w]], whole rows at a time.
+__global__ void k_gather_rows(const float* __restrict__ xsR, int d, const uint32_t* __restrict__ perm, int n,
+                              float* __restrict__ wrows) {
+    const size_t total = (size_t)n * d;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const size_t w = e / d;
+        wrows[e] = xsR[(size_t)perm[w] * d + (e - w * d)];
+    }
 }
 
 // ---- block geometry -------------------------------------------------------------------------------
 
 // One CTA per block of `bs` consecutive working rows (wrows: the normalised rows in working order,
-// row-major [n][d]): centre = normalised f64 sum (row order), radius = the largest angle between a row
-// and the centre (f64). Rows past n are ignored.
-__global__ void k_block_geom(const float* __restrict__ wrows, int d, int n, int bs, double* __restrict__ center,
-                             double* __restrict__ radius, float* __restrict__ center_f, float* __restrict__ radius_f) {
+// row-major [n][d]; staged through shared memory): centre = normalised f64 sum (row order), radius = the
+// largest angle between a row and the centre (f64). Rows past n are ignored. With center_f, the centre
+// and radius go out in f32 too (transposed, and rounded up).
+__global__ void __launch_bounds__(128) k_block_geom(const float* __restrict__ wrows, int d, int n, int bs,
+                                                    double* __restrict__ center, double* __restrict__ radius,
+                                                    float* __restrict__ center_f, float* __restrict__ radius_f) {
+    extern __shared__ float rows_s[];  // [bs][d | 1]: an odd stride, so a warp's rows fall in 32 banks
     __shared__ double c_s[64];
-    __shared__ double red[256];
-    const int b = blockIdx.x;
-    const int r0 = b * bs, r1 = min(n, r0 + bs);
-    if (threadIdx.x < d) {
+    __shared__ double inv_s;
+    __shared__ float cf_s[64];
+    __shared__ float red[4];
+    const int b = blockIdx.x, ds = d | 1;
+    const int r0 = b * bs, nr = min(n, r0 + bs) - r0;
+    for (int e = threadIdx.x; e < nr * d; e += 128) rows_s[(e / d) * ds + e % d] = wrows[(size_t)r0 * d + e];
+    __syncthreads();
+    if ((int)threadIdx.x < d) {
         double s = 0.0;
-        for (int w = r0; w < r1; ++w) s += (double)wrows[(size_t)w * d + threadIdx.x];
+        for (int w = 0; w < nr; ++w) s += f64_of(rows_s[w * ds + threadIdx.x]);
         c_s[threadIdx.x] = s;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         double nn = 0.0;
         for (int t = 0; t < d; ++t) nn += c_s[t] * c_s[t];
-        const double inv = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
-        for (int t = 0; t < d; ++t) c_s[t] *= inv;
+        inv_s = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
     }
     __syncthreads();
-    if (threadIdx.x < d) {
-        center[(size_t)b * d + threadIdx.x] = c_s[threadIdx.x];
-        if (center_f) center_f[(size_t)threadIdx.x * gridDim.x + b] = (float)c_s[threadIdx.x];  // [d][blocks]
+    if ((int)threadIdx.x < d) {
+        const double c = c_s[threadIdx.x] * inv_s;
+        center[(size_t)b * d + threadIdx.x] = c;
+        cf_s[threadIdx.x] = (float)c;
+        if (center_f) center_f[(size_t)threadIdx.x * gridDim.x + b] = (float)c;  // [d][blocks]
     }
+    __syncthreads();
     // The radius in f32 with a rigorous margin: the rows are unit vectors to within (d + 2)·2⁻²⁴, the
     // f32 centre is the f64 one to 2⁻²⁴ per component, and the f32 dot and norm accumulate at most
     // d·2⁻²⁴ of relative error each, so the f32 cosine is within (2d + 8)·2⁻²⁴ of the exact one; twice
     // that is subtracted before acosf (itself within a few ulp, covered by 1e-6 rad), and every step
     // rounds up. A zero row has cosine 0 with everything: angle π/2 covers it.
-    __shared__ float cf_s[64];
-    if (threadIdx.x < d) cf_s[threadIdx.x] = (float)c_s[threadIdx.x];
-    __syncthreads();
     const float margin = (float)(2 * d + 8) * 0x1p-23f;
     float worst = 0.0f;
-    for (int w = r0 + threadIdx.x; w < r1; w += blockDim.x) {
-        const float* row = wrows + (size_t)w * d;
+    for (int w = threadIdx.x; w < nr; w += 128) {
+        const float* row = rows_s + w * ds;
         float dot = 0.0f, nn = 0.0f;
         for (int t = 0; t < d; ++t) {
             const float v = row[t];
@@ -281,19 +390,14 @@ __global__ void k_block_geom(const float* __restrict__ wrows, int d, int n, int 
         }
         worst = fmaxf(worst, ang);
     }
-    red[threadIdx.x] = (double)worst;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(COSTAL_FULL_MASK, worst, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = worst;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        radius[b] = red[0];
-        if (radius_f) {
-            float rf = (float)red[0];
-            if ((double)rf < red[0]) rf = nextafterf(rf, CUDART_INF_F);  // rounded up
-            radius_f[b] = rf;
-        }
+        worst = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+        radius[b] = (double)worst;
+        if (radius_f) radius_f[b] = worst;
     }
 }
 
@@ -596,100 +700,90 @@ inline size_t a256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 bool supported(int d) { return d >= 1 && d <= 64; }
 
-size_t workspace_bytes(int n, int d) {
-    const int cb = col_block(n);
-    const size_t nqb = (size_t)(n + QB - 1) / QB, ncb = (size_t)(n + cb - 1) / cb;
-    const size_t m = (size_t)(n < SAMPLE ? n : SAMPLE), nch = (size_t)(n + CHUNK - 1) / CHUNK;
-    return a256(n * 4ull) * 2 + a256((size_t)K_CENTROIDS * d * 4) + a256(nqb * d * 8) + a256(nqb * 8) +
-           a256(ncb * d * 8) + a256(ncb * 8) + a256(ncb * d * 4) + a256(ncb * 4) + 2 * a256(nqb * ncb * 4) +
-           a256(nqb * 4) + a256(nqb * 4) + a256(n * 8ull) + a256(nqb * 4) + a256(m * d * 4) + a256(m * 4) + a256(nch * K_CENTROIDS * 4) + a256((K_CENTROIDS + 1) * 4) +
-           a256(m * 4) + a256((size_t)n * d * 4) + 4096;
-}
-
 namespace {
 struct Scratch {
-    float* sample_rows;
-    uint32_t* sample_assign;
-    uint32_t* hist;
-    uint32_t* cell_start;
-    uint32_t* sample_idx;
+    float *sample_rows, *sample_T, *centT;
+    uint32_t *sample_assign, *hist, *total;
 };
 
-__global__ void k_sample_idx(uint32_t* idx, int m, int n) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < m) idx[j] = (uint32_t)(((unsigned long long)j * (unsigned long long)n) / (unsigned long long)m);
-}
-
-// Initial centroids: K evenly spaced sample rows (deterministic).
-__global__ void k_init_centroids(const float* rows, int m, int d, int K, float* cent) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= K * d) return;
-    const int c = e / d, t = e % d;
-    const int i = (int)(((long long)c * m) / K);
-    cent[e] = rows[(size_t)i * d + t];
-}
-}  // namespace
-
-cudaError_t build_order(void* ws, const float* xsT, int n, int np, int d, cudaStream_t st, Plan& P) {
-    const int K = K_CENTROIDS;
-    const int cb = col_block(n);
-    const int nqb = (n + QB - 1) / QB, ncb = (n + cb - 1) / cb;
-    const int m = n < SAMPLE ? n : SAMPLE, nch = (n + CHUNK - 1) / CHUNK;
-    char* p = static_cast<char*>(ws);
-    auto take = [&](size_t bytes) {
-        char* r = p;
-        p += a256(bytes);
-        return r;
+// The workspace's layout (base NULL: only its size).
+size_t carve(void* base, int n, int d, Plan& P, Scratch& S) {
+    const int K = K_CENTROIDS, cb = col_block(n), dp = coarse_dpad(d);
+    const int m = n < SAMPLE ? n : SAMPLE, mp = (m + KM_ROWS - 1) / KM_ROWS * KM_ROWS;
+    const size_t nqb = (size_t)(n + QB - 1) / QB, ncb = (size_t)(n + cb - 1) / cb, nch = (size_t)(n + CHUNK - 1) / CHUNK;
+    size_t off = 0;
+    auto take = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(static_cast<char*>(base) + off);
+        off += a256(count * sizeof(*p));
     };
     P.n = n;
     P.d = d;
     P.K = K;
-    P.nqb = nqb;
-    P.ncb = ncb;
+    P.nqb = (int)nqb;
+    P.ncb = (int)ncb;
     P.cb = cb;
-    P.perm = reinterpret_cast<uint32_t*>(take(n * 4ull));
-    P.cell = reinterpret_cast<uint32_t*>(take(n * 4ull));
-    P.centroids = reinterpret_cast<float*>(take((size_t)K * d * 4));
-    P.qcenter = reinterpret_cast<double*>(take((size_t)nqb * d * 8));
-    P.qradius = reinterpret_cast<double*>(take((size_t)nqb * 8));
-    P.ccenter = reinterpret_cast<double*>(take((size_t)ncb * d * 8));
-    P.cradius = reinterpret_cast<double*>(take((size_t)ncb * 8));
-    P.ccenter_f = reinterpret_cast<float*>(take((size_t)ncb * d * 4));
-    P.cradius_f = reinterpret_cast<float*>(take((size_t)ncb * 4));
-    P.lists = reinterpret_cast<uint32_t*>(take((size_t)nqb * ncb * 4));
-    P.list_ub = reinterpret_cast<float*>(take((size_t)nqb * ncb * 4));
-    P.counts = reinterpret_cast<uint32_t*>(take((size_t)nqb * 4));
-    P.ub_skip = reinterpret_cast<float*>(take((size_t)nqb * 4));
-    P.row_ub = reinterpret_cast<double*>(take(n * 8ull));
-    P.tq = reinterpret_cast<float*>(take((size_t)nqb * 4));
-    Scratch S;
-    S.sample_rows = reinterpret_cast<float*>(take((size_t)m * d * 4));
-    S.sample_assign = reinterpret_cast<uint32_t*>(take((size_t)m * 4));
-    S.hist = reinterpret_cast<uint32_t*>(take((size_t)nch * K * 4));
-    S.cell_start = reinterpret_cast<uint32_t*>(take((size_t)(K + 1) * 4));
-    S.sample_idx = reinterpret_cast<uint32_t*>(take((size_t)m * 4));
-    P.wrows = reinterpret_cast<float*>(take((size_t)n * d * 4));
-    P.scratch = S.sample_rows;
-
-    const size_t csm = (size_t)K * ((d + 3) & ~3) * 4;
-    cudaError_t e = cudaFuncSetAttribute(k_assign, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    if (e != cudaSuccess) return e;
-    k_sample_idx<<<(m + 255) / 256, 256, 0, st>>>(S.sample_idx, m, n); note_launch();
-    k_gather_rows<<<1024, 256, 0, st>>>(xsT, np, d, S.sample_idx, m, S.sample_rows); note_launch();
-    k_init_centroids<<<(K * d + 255) / 256, 256, 0, st>>>(S.sample_rows, m, d, K, P.centroids); note_launch();
-    for (int it = 0; it < LLOYD_STEPS; ++it) {
-        k_assign<<<(m + KM_BLOCK - 1) / KM_BLOCK, KM_BLOCK, csm, st>>>(S.sample_rows, nullptr, np, m, d, P.centroids, K,
-                                                                         S.sample_assign); note_launch();
-        k_centroid_update<<<K, UPD_T, 0, st>>>(S.sample_rows, m, d, S.sample_assign, P.centroids); note_launch();
+    take(P.perm, n);
+    take(P.cell, n);
+    take(P.centroids, (size_t)K * d);
+    take(P.ccenter, ncb * d);
+    take(P.cradius, ncb);
+    take(P.ccenter_f, ncb * d);
+    take(P.cradius_f, ncb);
+    if (cb == QB) {  // query and column blocks are the same rows
+        P.qcenter = P.ccenter;
+        P.qradius = P.cradius;
+    } else {
+        take(P.qcenter, nqb * d);
+        take(P.qradius, nqb);
     }
-    k_assign<<<(n + KM_BLOCK - 1) / KM_BLOCK, KM_BLOCK, csm, st>>>(nullptr, xsT, np, n, d, P.centroids, K, P.cell); note_launch();
-    k_cell_hist<<<(nch + 127) / 128, 128, 0, st>>>(P.cell, n, K, S.hist); note_launch();
-    k_cell_scan<<<1, K, 0, st>>>(S.hist, nch, K, S.cell_start); note_launch();
-    k_cell_scatter<<<(nch + 127) / 128, 128, 0, st>>>(P.cell, n, K, S.hist, P.perm); note_launch();
-    // the rows in working order, row-major, for the block geometry's contiguous reads
-    k_gather_rows<<<std::min((n * d + 255) / 256, 8 * 1024), 256, 0, st>>>(xsT, np, d, P.perm, n, P.wrows); note_launch();
-    k_block_geom<<<nqb, 256, 0, st>>>(P.wrows, d, n, QB, P.qcenter, P.qradius, nullptr, nullptr); note_launch();
-    k_block_geom<<<ncb, 256, 0, st>>>(P.wrows, d, n, cb, P.ccenter, P.cradius, P.ccenter_f, P.cradius_f); note_launch();
+    take(P.lists, nqb * ncb);
+    take(P.list_ub, nqb * ncb);
+    take(P.counts, nqb);
+    take(P.ub_skip, nqb);
+    take(P.row_ub, n);
+    take(P.tq, nqb);
+    take(P.wrows, (size_t)n * d);
+    take(S.sample_rows, (size_t)m * d);
+    take(S.sample_T, (size_t)mp * dp);
+    take(S.centT, (size_t)K * dp);
+    take(S.sample_assign, m);
+    take(S.hist, nch * K);
+    take(S.total, K);
+    return off;
+}
+}  // namespace
+
+size_t workspace_bytes(int n, int d) {
+    Plan P{};
+    Scratch S{};
+    return carve(nullptr, n, d, P, S);
+}
+
+cudaError_t build_order(void* ws, const float* xsT, const float* xsR, int n, int np, int d, cudaStream_t st, Plan& P) {
+    const int K = K_CENTROIDS, dp = coarse_dpad(d);
+    const int m = n < SAMPLE ? n : SAMPLE, mp = (m + KM_ROWS - 1) / KM_ROWS * KM_ROWS;
+    Scratch S{};
+    carve(ws, n, d, P, S);
+    const size_t asm_ = (size_t)dp * (KM_ROWS + K) * 4;
+    const size_t gsm = (size_t)P.cb * (d | 1) * 4;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_assign, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asm_)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_block_geom, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm)) != cudaSuccess) return e;
+    k_sample<<<std::min((mp * dp + 255) / 256, 4096), 256, 0, st>>>(xsR, n, d, dp, m, mp, K, S.sample_rows, S.sample_T,
+                                                                    P.centroids, S.centT); note_launch();
+    for (int it = 0; it < LLOYD_STEPS; ++it) {
+        k_assign<<<mp / KM_ROWS, 128, asm_, st>>>(S.sample_T, mp, m, dp, S.centT, S.sample_assign); note_launch();
+        k_centroid_update<<<K, UPD_T, 0, st>>>(S.sample_rows, m, d, S.sample_assign, P.centroids, S.centT); note_launch();
+    }
+    k_assign<<<np / KM_ROWS, 128, asm_, st>>>(xsT, np, n, dp, S.centT, P.cell); note_launch();
+    if ((e = sort_by_cell(P.cell, n, K, S.hist, S.total, P.perm, st)) != cudaSuccess) return e;
+    k_gather_rows<<<(unsigned)std::min<size_t>(((size_t)n * d + 255) / 256, 16 * 1024), 256, 0, st>>>(xsR, d, P.perm, n,
+                                                                                                      P.wrows); note_launch();
+    k_block_geom<<<P.ncb, 128, gsm, st>>>(P.wrows, d, n, P.cb, P.ccenter, P.cradius, P.ccenter_f, P.cradius_f); note_launch();
+    if (P.cb != QB) {
+        k_block_geom<<<P.nqb, 128, (size_t)QB * (d | 1) * 4, st>>>(P.wrows, d, n, QB, P.qcenter, P.qradius, nullptr, nullptr);
+        note_launch();
+    }
     return cudaGetLastError();
 }
 
@@ -751,10 +845,7 @@ cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cud
     if (e != cudaSuccess) return e;
     k_norm_range<<<std::min((n + 255) / 256, 1024), 256, 0, st>>>(norms, n, range); note_launch();
     k_norm_bucket<<<(n + 255) / 256, 256, 0, st>>>(norms, n, range, cell); note_launch();
-    k_cell_hist<<<(nch + 127) / 128, 128, 0, st>>>(cell, n, NORM_BUCKETS, hist); note_launch();
-    k_cell_scan<<<1, NORM_BUCKETS, 0, st>>>(hist, nch, NORM_BUCKETS, start); note_launch();
-    k_cell_scatter<<<(nch + 127) / 128, 128, 0, st>>>(cell, n, NORM_BUCKETS, hist, perm); note_launch();
-    return cudaGetLastError();
+    return sort_by_cell(cell, n, NORM_BUCKETS, hist, start, perm, st);
 }
 
 cudaError_t build_lists(Plan& P, unsigned long long* skipped_total, cudaStream_t st) {

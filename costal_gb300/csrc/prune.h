@@ -44,13 +44,13 @@ struct Plan {
     float* wrows;        // [n][d] the normalised rows in working order, row-major
     const float* rowmax;    // [nqb][ncb] per-row bound data (tc::launch_rowmax), or NULL: cone bound only
     const float* rm_delta;  // its error margin (device scalar)
-    void* scratch;       // k-means sample, histograms
 };
 
 size_t workspace_bytes(int n, int d);
 bool supported(int d);
-// Cells, working order and block geometry from the normalised rows (xsT, d_pad × np).
-cudaError_t build_order(void* ws, const float* xsT, int n, int np, int d, cudaStream_t st, Plan& plan);
+// Cells, working order and block geometry from the normalised rows (xsT, d_pad × np, and xsR, the same
+// rows row-major [n][d]).
+cudaError_t build_order(void* ws, const float* xsT, const float* xsR, int n, int np, int d, cudaStream_t st, Plan& plan);
 // Per-query-block column lists with the thresholds in plan.tq (NULL: keep all, nearest first).
 cudaError_t build_lists(Plan& plan, unsigned long long* skipped_total, cudaStream_t st);
 

@@ -55,7 +55,7 @@ typedef struct costal_knn_opts {
     uint32_t col_block;    /* idem */
     int32_t sort_by_norm;  /* idem (knn.rs:41): output-independent */
     int32_t prune;         /* idem (knn.rs:44): output-independent; it enables the exact early stop of each
-                              query block's column list (bf16 backend; FP32 from 32,768 rows, d <= 64) */
+                              query block's column list (bf16 backend; FP32 from 16,384 rows, d <= 64) */
     int32_t learned_prune; /* 1 = use the trained block-pruning model if one is loaded (bf16 backend) */
 } costal_knn_opts;
 

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
     (257, 64, 16, None), (1000, 64, 32, None), (385, 63, 20, 13),                # resident, 2 stages; cap 32 | 33
     (300, 5, 64, None), (700, 40, 50, 14), (900, 8, 64, 64),                     # cap 64 and 128: streamed
     (640, 65, 10, None), (513, 72, 30, None), (513, 130, 60, 60), (129, 2000, 15, None),
-    (20_011, 17, 10, None),                                                      # several segments a block
+    (12_011, 17, 10, None),                                                      # several segments a block
 ])
 @pytest.mark.parametrize("select", ["cosine", "tanimoto"])
 def test_fp32_pass_at_its_edges(ext, oracle, n, d, k, margin, select):
@@ -44,7 +44,7 @@ def test_fp32_pass_with_repeated_and_zero_rows(ext, oracle, d):
             np.testing.assert_array_equal(a, b)
 
 
-@pytest.mark.parametrize("n,d,k,margin", [(33_001, 2, 10, None), (40_000, 33, 30, None), (33_100, 64, 10, 3),
+@pytest.mark.parametrize("n,d,k,margin", [(16_384, 2, 10, None), (40_000, 33, 30, None), (33_100, 64, 10, 3),
                                           (36_000, 17, 70, None)])
 def test_fp32_pass_by_lists(ext, oracle, n, d, k, margin):
     """Enough rows for the column lists and the early stop (ragged last blocks, repeated rows): the
