@@ -53,6 +53,7 @@ struct Misc {  // small device-side results read back at the end of a call
     unsigned long long blocks_stopped;
     unsigned long long conv_mismatches;
     unsigned nnz;
+    unsigned norm_share[2];
     unsigned shard_rows;  // rows of the shard being computed (the rescoring's device-side row count)
 };
 
@@ -69,7 +70,7 @@ struct Context {
     DevBuf fu_scratch, rows, cols, wout, idx_in, cos_in, norms_in, w_in, jac, f32out, tc_ws, tc_rows, prune_ws;
     DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows;
     DevBuf fp32_ws, tfloor, xsW, xsR;
-    DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_perm, tani_ws, rm_ws, rm_out;
+    DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_ws, tani_ranges, rm_ws, rm_out;
     MlpState mlp;
 };
 
@@ -218,27 +219,60 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 // 40,000 × 20 2.5 / 4.4, 80,000 × 32 6.5 / 12.6, 161,443 × 32 14.9 / 39.8).
 bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 16384; }
 
-// The FP32 pass's working order and column lists: the same cells, bounds and lists as the tensor-core
-// path (the per-row bounds come from its split operands, with their margin), and the rows' transposed
-// copy in the working order (c.xsW).
-void build_fp32_lists(Context& c, int n, int np, int d, int dp, prune::Plan& pp, cudaStream_t s) {
+// The FP32 pass by lists: the working order, the column lists and the rows' transposed copy in that order
+// (c.xsW) into the job. Cosine selection, and Tanimoto selection of enough rows, use the cells, bounds
+// and lists of the tensor-core path (the per-row bounds come from its split operands, with their
+// margin); Tanimoto selection bounds each block pair's score by its cosine bound and norm ranges, or
+// by the norm ranges alone in the norm order (knn.rs:595-644): with few rows, or where the norms are
+// spread so far that the window of a score of 0.9 leaves out more than half of all pairs (a block of
+// one cell spans its rows' whole norm range, so the cells' order cannot use the window: of 20,000 × 12
+// rows spread 8-fold in norm the norm order leaves out 45 % of the tiles, the cells' order 0.1 %;
+// of 100,003 × 15 cytometry-like rows the norm order 6 %, the cells' order 75 %).
+void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani_norms, double eps, Fp32Job& j, cudaStream_t s) {
     Misc* dm = c.misc.as<Misc>();
+    prune::Plan pp{};
     CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
-    CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), n, np, d, s, pp));
-    CK(ensure(c.tc_ws, tc::workspace_bytes(n, d, false)));
-    tc::Plan plan{};
-    CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), n, np, dp, d, pp.perm, s, plan, false, pp.wrows));
-    if (tc::rowmax_supported(plan)) {
-        CK(ensure(c.rm_ws, tc::rowmax_bytes(pp.ncb, d)));
-        CK(ensure(c.rm_out, (size_t)pp.nqb * pp.ncb * 4));
-        CK(tc::launch_rowmax(plan, pp.ccenter_f, pp.ncb, c.rm_ws.p, c.rm_out.as<float>(), &pp.rm_delta,
-                             &dm->timeout_flag, s));
-        pp.rowmax = c.rm_out.as<float>();
+    bool by_norm = tani_norms && !fp32_lists_pay(n, d);
+    if (tani_norms && !by_norm) {
+        CK(prune::norm_window_share(tani_norms, n, dm->norm_share, s));
+        CK(cudaMemcpyAsync(c.h_misc->norm_share, dm->norm_share, 8, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        by_norm = 2ull * c.h_misc->norm_share[1] < c.h_misc->norm_share[0];
+    }
+    if (by_norm) {
+        CK(ensure(c.tani_ws, prune::norm_order_bytes(n)));
+        CK(prune::norm_plan(c.prune_ws.p, tani_norms, n, d, c.tani_ws.p, s, pp));
+    } else {
+        CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), n, np, d, s, pp));
+        CK(ensure(c.tc_ws, tc::workspace_bytes(n, d, false)));
+        tc::Plan plan{};
+        CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), n, np, dp, d, pp.perm, s, plan, false, pp.wrows));
+        if (tc::rowmax_supported(plan)) {
+            CK(ensure(c.rm_ws, tc::rowmax_bytes(pp.ncb, d)));
+            CK(ensure(c.rm_out, (size_t)pp.nqb * pp.ncb * 4));
+            CK(tc::launch_rowmax(plan, pp.ccenter_f, pp.ncb, c.rm_ws.p, c.rm_out.as<float>(), &pp.rm_delta,
+                                 &dm->timeout_flag, s));
+            pp.rowmax = c.rm_out.as<float>();
+        }
+    }
+    if (tani_norms) {
+        CK(ensure(c.tani_ranges, (size_t)(pp.ncb + pp.nqb) * 8));
+        CK(prune::block_norms(tani_norms, pp, c.tani_ranges.as<float2>(), s));
     }
     pp.tq = nullptr;
-    CK(prune::build_lists(pp, &dm->blocks_skipped, s));
+    CK(prune::build_lists(pp, nullptr, s));
     CK(ensure(c.xsW, (size_t)dp * np * 4));
-    CK(launch_work_cols(pp.wrows, n, np, d, dp, c.xsW.as<float>(), s));
+    CK(launch_work_cols(c.xsR.as<float>(), pp.perm, n, np, d, dp, c.xsW.as<float>(), s));
+    j.xsT = c.xsW.as<float>();
+    j.perm = pp.perm;
+    j.lists = pp.lists;
+    j.list_ub = pp.list_ub;
+    j.counts = pp.counts;
+    j.ncb = pp.ncb;
+    j.list_cb = pp.cb;
+    j.eps = std::nextafterf((float)eps, INFINITY);
+    // (Tanimoto selection's left-out blocks are reported as skipped, as its norm window's are)
+    j.stopped_total = tani_norms ? &dm->blocks_skipped : &dm->blocks_stopped;
 }
 
 // One shard of the query rows (a multi-GPU run gives each rank one): the rows are cut into query
@@ -274,7 +308,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     // the FP32 kernel holds that still exceeds k (rows the certificate then fails take the regather);
     // when none does, every candidate is scanned exactly in f64 (knn.rs:884-924).
     bool scan_all = false;
-    auto fits = [&](int c) { return coarse_slots(c) != 0 && coarse_fp32_smem(dp, c) <= 227 * 1024; };
+    auto fits = [&](int c) { return coarse_fp32_holds(dp, c); };
     if (!fits(cap)) {
         int smaller = 0;
         for (int c : {128, 64, 32})
@@ -316,7 +350,8 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     const bool tc_backend = o.backend == COSTAL_BACKEND_BF16 || o.backend == COSTAL_BACKEND_BF16X3 ||
                             o.backend == COSTAL_BACKEND_FP8;
     // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
-    const bool fp32_lists = !tc_backend && !tanimoto && !scan_all && !shard && o.prune && cap < n - 1 && fp32_lists_pay(n, d);
+    const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
+                            (tanimoto ? prune::supported(d) : !tc_backend && fp32_lists_pay(n, d));
     float* xsR = nullptr;
     if (fp32_lists || (tc_backend && !tanimoto && !scan_all && prune::supported(d))) {
         CK(ensure(c.xsR, (size_t)n * d * 4));
@@ -333,7 +368,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     bool fp8 = !tanimoto && !scan_all && (o.backend == COSTAL_BACKEND_FP8 || (o.backend == COSTAL_BACKEND_BF16 && d >= 512));
     if (fp8) {
         const int cap8 = std::max(cap, std::min(64, n - 1));
-        if (tc::supported_fp8(d, cap8) && coarse_slots(cap8) != 0 && coarse_fp32_smem(dp, cap8) <= 227 * 1024) {
+        if (tc::supported_fp8(d, cap8) && coarse_fp32_holds(dp, cap8)) {
             cap = cap8;
             margin = (uint64_t)(cap - k);
         } else {
@@ -358,19 +393,14 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
         CK(ensure(c.tau, (size_t)n * 4));
         CK(ensure(c.tnorm, (size_t)n * 8));
         const double eps_t = 2.0 * ((double)d + 12.0) * F32_EPS;
-        if (o.prune && cap < n - 1 && dp <= 64) {
-            // the norm window (knn.rs:595-644): rows in norm order, each query block walking outward
-            CK(ensure(c.tani_perm, (size_t)n * 4));
-            CK(ensure(c.tani_ws, std::max(prune::norm_order_bytes(n), tani_window_bytes(n, np, dp))));
-            CK(prune::norm_order(d_norms, n, c.tani_ws.p, c.tani_perm.as<uint32_t>(), s));
-            CK(launch_coarse_tani_window(c.xsT.as<float>(), n, np, dp, cap, d_norms, c.tani_perm.as<uint32_t>(),
-                                         c.tani_ws.p, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
-                                         c.tau.as<float>(), &dm->blocks_skipped, s));
-        } else {
-            Fp32Job j = fp32_job(c, n, np, dp, cap);
-            j.norms = d_norms;
-            coarse_fp32(c, j, s);
+        Fp32Job j = fp32_job(c, n, np, dp, cap);
+        j.norms = d_norms;
+        if (fp32_lists) {
+            fp32_lists_job(c, n, np, d, dp, d_norms, eps_t, j, s);
+            list_cb = j.list_cb;
+            CK(cudaEventRecord(c.ev[5], s));
         }
+        coarse_fp32(c, j, s);
         CK(cudaEventRecord(c.ev[2], s));
         CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                           c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps_t, cap < n - 1, 1, nullptr,
@@ -454,8 +484,6 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                                   &dm->prune_fail_count, 0.0, cap < n - 1, 0, srows, scount, d_idx, d_cos, d_w,
                                   c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count,
                                   dm->max_err_bits, s));
-            if (coarse_fp32_smem(dp, cap) > 227 * 1024)
-                throw Fail{COSTAL_EUNSUPPORTED, "d and k + margin too large for the FP32 re-run of uncertified rows"};
             // How many rows failed decides the re-run's shape (few rows: the columns split across CTAs).
             CK(cudaMemcpyAsync(&c.h_misc->tc_fail_count, &dm->tc_fail_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
                                s));
@@ -473,23 +501,11 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             }
             CK(cudaEventRecord(c.ev[3], s));
         } else {
-            if (coarse_fp32_smem(dp, cap) > 227 * 1024)
-                throw Fail{COSTAL_EUNSUPPORTED, "d and k + margin too large for the FP32 coarse kernel"};
             if (!shard) {
                 Fp32Job j = fp32_job(c, n, np, dp, cap);
-                prune::Plan pp{};
                 if (fp32_lists) {
-                    build_fp32_lists(c, n, np, d, dp, pp, s);
-                    list_cb = pp.cb;
-                    j.xsT = c.xsW.as<float>();
-                    j.perm = pp.perm;
-                    j.lists = pp.lists;
-                    j.list_ub = pp.list_ub;
-                    j.counts = pp.counts;
-                    j.ncb = pp.ncb;
-                    j.list_cb = pp.cb;
-                    j.eps = std::nextafterf((float)eps, INFINITY);
-                    j.stopped_total = &dm->blocks_stopped;
+                    fp32_lists_job(c, n, np, d, dp, nullptr, eps, j, s);
+                    list_cb = j.list_cb;
                     CK(cudaEventRecord(c.ev[5], s));
                 }
                 coarse_fp32(c, j, s);
@@ -946,7 +962,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         const int dp = coarse_dpad(D), np = round_up(N, 128);
         const uint64_t margin = o.margin == UINT32_MAX ? (uint64_t)k : (uint64_t)o.margin;
         const int cap = (int)std::min<uint64_t>((uint64_t)k + margin, n - 1);
-        if (coarse_slots(cap) == 0 || coarse_fp32_smem(dp, cap) > 227 * 1024)
+        if (!coarse_fp32_holds(dp, cap))
             throw Fail{COSTAL_EUNSUPPORTED, "k + margin too large for the FP32 label pass"};
         const int m = (int)std::min<uint64_t>(o.sample ? o.sample : n, n);
         const int F = D + MLP_TOPC;

@@ -489,13 +489,15 @@ __global__ void __launch_bounds__(NT, 2)
     }
 }
 
-// The rows in working order (row-major [n][d]) as the transposed copy out[t][w], zero for w ≥ n and
-// t ≥ d: a CTA per 128 rows, staged through shared memory so that both sides are coalesced.
-__global__ void __launch_bounds__(256) k_work_cols(const float* __restrict__ wrows, int n, int np, int d, int dp,
-                                                   float* __restrict__ out) {
+// The transposed copy in working order: out[t][w] = xsR[perm[w]][t] (xsR row-major [n][d]), zero for w ≥ n
+// and t ≥ d: a CTA per 128 rows, staged through shared memory so that whole rows are read and both
+// sides are coalesced.
+__global__ void __launch_bounds__(256) k_work_cols(const float* __restrict__ xsR, const uint32_t* __restrict__ perm, int n,
+                                                   int np, int d, int dp, float* __restrict__ out) {
     extern __shared__ float tile[];  // [BM][d + 1]
     const int w0 = blockIdx.x * BM, rows = min(BM, n - w0);
-    for (int e = threadIdx.x; e < rows * d; e += 256) tile[(e / d) * (d + 1) + e % d] = wrows[(size_t)w0 * d + e];
+    for (int e = threadIdx.x; e < rows * d; e += 256)
+        tile[(e / d) * (d + 1) + e % d] = xsR[(size_t)perm[w0 + e / d] * d + e % d];
     __syncthreads();
     for (int e = threadIdx.x; e < dp * BM; e += 256) {
         const int t = e / BM, r = e % BM;
@@ -513,12 +515,59 @@ __global__ void k_gather_cols(const float* __restrict__ xsT, int np, int dp, con
     for (int t = blockIdx.y; t < dp; t += gridDim.y) out[(size_t)t * mp + q] = q < nq ? xsT[(size_t)t * np + c] : 0.0f;
 }
 
-// The rows' f32 norm and squared norm from the f64 norms (knn.rs:207-212 rounds ‖x‖² to f32).
-__global__ void k_tani_norms(const double* __restrict__ norms, int n, float2* __restrict__ tnorm) {
+// The rows' f32 norm and squared norm from the f64 norms (knn.rs:207-212 rounds ‖x‖² to f32), in working order.
+__global__ void k_tani_norms(const double* __restrict__ norms, int n, const uint32_t* __restrict__ perm,
+                             float2* __restrict__ tnorm) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double a = norms[i];
+        const double a = norms[perm ? perm[i] : (uint32_t)i];
         tnorm[i] = make_float2((float)a, (float)(a * a));
     }
+}
+
+// One warp per listed row: the union of its segments' lists (segs · cap entries) as (score desc,
+// index asc) keys, 256 at a time: after each warp sort the first cap positions hold the best so far
+// and the other 256 − cap take the next entries. The best cap go to the row's candidates, and τ is
+// the cap-th score (≥ every segment's own τ, since a full segment list holds cap entries at or above
+// it), or the row's floor when the segments hold fewer than cap together.
+__global__ void k_merge_parts(const uint32_t* __restrict__ qlist, int count, int segs, int cap,
+                              const uint32_t* __restrict__ part_idx, const float* __restrict__ part_score,
+                              const float* __restrict__ tfloor, int lstride, uint32_t* __restrict__ cand_idx,
+                              float* __restrict__ cand_score, float* __restrict__ tau_out) {
+    const int lane = threadIdx.x & 31;
+    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (r >= count) return;
+    const int total = segs * cap;
+    auto load = [&](int e) {
+        if (e >= total) return PAD_KEY;
+        const size_t o = ((size_t)(e / cap) * count + r) * cap + e % cap;
+        return order_key(part_score[o], part_idx[o]);
+    };
+    uint64_t key[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) key[s] = load(s * 32 + lane);
+    warp_sort_keys<8>(key, lane);
+    for (int next = 256; next < total; next += 256 - cap) {  // warp-uniform
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const int p = s * 32 + lane;
+            if (p >= cap) key[s] = load(next + p - cap);
+        }
+        warp_sort_keys<8>(key, lane);
+    }
+    const uint32_t q = qlist ? qlist[r] : (uint32_t)r;
+    uint64_t kth = 0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int p = s * 32 + lane;
+        if (p < cap) {
+            cand_idx[(size_t)q * lstride + p] = key_index(key[s]);
+            cand_score[(size_t)q * lstride + p] = key_score(key[s]);
+        }
+        if (s == (cap - 1) >> 5) kth = key[s];
+    }
+    const uint64_t t = __shfl_sync(COSTAL_FULL_MASK, kth, (cap - 1) & 31);
+    // with fewer than cap candidates in all segments together, the row's floor still bounds the rest
+    if (lane == 0) tau_out[q] = fmaxf(key_score(t), tfloor ? tfloor[q] : -CUDART_INF_F);
 }
 
 // The launch shape for a depth and a candidate count: the query operand resident or streamed, the
@@ -572,12 +621,12 @@ static bool make_map(CUtensorMap* m, const void* base, size_t cols, int rows, in
 // Column segments for nq queries against `tiles` column tiles: the number whose last wave of CTAs
 // (`slots` at a time) ends first, a CTA costing its tiles plus `start` tiles' worth of time for loading
 // its queries, seeding and writing its lists (and the merge reading one more list).
-static int segments(int nq, int tiles, int dp, int slots) {
+static int segments(int nq, int tiles, int dp, int slots, int most) {
     const int blocks = (nq + BM - 1) / BM;
     const double start = 1.0 + 64.0 / dp;
     int best = 1;
     double best_t = 1e300;
-    for (int s = 1; s <= std::min(64, tiles); ++s) {
+    for (int s = 1; s <= std::min(most, tiles); ++s) {
         const int tps = (tiles + s - 1) / s;
         if ((tiles + tps - 1) / tps != s) continue;  // an empty segment
         const double waves = (double)(((long long)blocks * s + slots - 1) / slots);
@@ -623,21 +672,56 @@ static Ws carve(void* base, int dp, int cap, bool listed, int nq, int segs) {
 }
 }  // namespace fp32
 
-cudaError_t launch_work_cols(const float* wrows, int n, int np, int d, int dp, float* xsW, cudaStream_t st) {
-    fp32::k_work_cols<<<np / fp32::BM, 256, (size_t)fp32::BM * (d + 1) * 4, st>>>(wrows, n, np, d, dp, xsW); note_launch();
+cudaError_t launch_work_cols(const float* xsR, const uint32_t* perm, int n, int np, int d, int dp, float* xsW,
+                             cudaStream_t st) {
+    fp32::k_work_cols<<<np / fp32::BM, 256, (size_t)fp32::BM * (d + 1) * 4, st>>>(xsR, perm, n, np, d, dp, xsW);
+    note_launch();
     return cudaGetLastError();
 }
 
-// (with lists, about a third of the tiles is visited)
+// With lists about a third of the tiles is visited, and a segment keeps at least 24 entries: its stop
+// comes a ring of stages after its thresholds have risen.
 static int segs_of(const Fp32Job& J, const fp32::Shape& sh, int sm_count) {
     const int tiles = J.np / fp32::BN;
-    return fp32::segments(J.nq, J.lists ? std::max(1, tiles / 3) : tiles, J.dp, sm_count * sh.ctas);
+    if (!J.lists) return fp32::segments(J.nq, tiles, J.dp, sm_count * sh.ctas, 64);
+    return fp32::segments(J.nq, std::max(1, tiles / 3), J.dp, sm_count * sh.ctas, std::max(1, J.ncb / 24));
 }
 
 size_t coarse_fp32_ws_bytes(const Fp32Job& J, int sm_count) {
     const fp32::Shape sh = fp32::shape_of(J.dp, J.cap);
     const int segs = segs_of(J, sh, sm_count);
     return fp32::carve(nullptr, J.dp, J.cap, J.rows != nullptr, J.nq, segs).bytes;
+}
+
+cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
+                               const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
+                               float* tau, cudaStream_t st) {
+    fp32::k_merge_parts<<<(count + 7) / 8, 256, 0, st>>>(rows, count, segs, cap, part_idx, part_score, tfloor, cap,
+                                                          cand_idx, cand_score, tau);
+    note_launch();
+    return cudaGetLastError();
+}
+
+// The re-run's floor for each listed row, from the tensor-core pass it follows: when that pass kept a
+// full list of cap candidates above its threshold τ, their exact cosines are ≥ τ − E_i, so the row's
+// cap-th FP32 score is ≥ τ − E_i − ε; below that no column can be among the best cap (rounded down).
+__global__ void k_rerun_floor(const uint32_t* __restrict__ rows, const unsigned* __restrict__ count, int cap,
+                              const float* __restrict__ tau, const float* __restrict__ cand_score,
+                              const double* __restrict__ row_eps, double eps, float* __restrict__ tfloor) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= (int)*count) return;
+    const uint32_t i = rows[r];
+    const bool full = cand_score[(size_t)i * cap + cap - 1] > -CUDART_INF_F;
+    tfloor[i] = full ? __double2float_rd(__dsub_rd(__dsub_rd((double)tau[i], row_eps[i]), eps)) : -CUDART_INF_F;
+}
+
+cudaError_t launch_rerun_floor(const uint32_t* rows, const unsigned* count, int nmax, int cap, const float* tau,
+                               const float* cand_score, const double* row_eps, double eps, float* tfloor,
+                               cudaStream_t st) {
+    if (nmax <= 0) return cudaSuccess;
+    k_rerun_floor<<<(nmax + 255) / 256, 256, 0, st>>>(rows, count, cap, tau, cand_score, row_eps, eps, tfloor);
+    note_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStream_t st) {
@@ -650,7 +734,7 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     const Ws w = carve(ws, J.dp, J.cap, J.rows != nullptr, J.nq, segs);
     cudaError_t e;
     if (J.norms) {
-        k_tani_norms<<<std::min((J.n + 255) / 256, 1024), 256, 0, st>>>(J.norms, J.n, J.tnorm); note_launch();
+        k_tani_norms<<<std::min((J.n + 255) / 256, 1024), 256, 0, st>>>(J.norms, J.n, J.perm, J.tnorm); note_launch();
     }
     if (J.rows) {
         k_gather_cols<<<dim3(mp / BM, std::min(J.dp, 64)), BM, 0, st>>>(J.xsT, J.np, J.dp, J.rows, J.nq, mp, w.a);
@@ -700,5 +784,9 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
                                   J.tau, st);
     return cudaGetLastError();
 }
+
+int coarse_dpad(int d) { return d <= 64 ? ((d < 1 ? 1 : d) + 7) / 8 * 8 : (d + 3) / 4 * 4; }
+
+bool coarse_fp32_holds(int dp, int cap) { return cap <= 128 && fp32::shape_of(dp, cap).stages >= 2; }
 
 }  // namespace costal

@@ -15,7 +15,8 @@ cudaError_t launch_row_l2_norms_f32(const float* x, int n, int d, float* out, cu
 int coarse_slots(int cap);
 // d_pad of the working copy: a multiple of 8 up to 64 (compile-time tile depths), else of 4.
 int coarse_dpad(int d);
-size_t coarse_fp32_smem(int dp, int cap);
+// Whether the FP32 pass holds cap candidates a row at this depth (up to 128 at any).
+bool coarse_fp32_holds(int dp, int cap);
 // The FP32 coarse pass (fp32_tiles.cu): the queries (all n rows, or nq listed ones) against all columns.
 struct Fp32Job {
     const float* xsT;      // [dp][np] the normalised rows, transposed
@@ -43,20 +44,13 @@ struct Fp32Job {
 };
 size_t coarse_fp32_ws_bytes(const Fp32Job& job, int sm_count);
 cudaError_t launch_coarse_fp32(const Fp32Job& job, void* ws, int sm_count, cudaStream_t st);
-// The transposed copy of the rows in working order (prune::Plan::wrows, [n][d]): xsW [dp][np].
-cudaError_t launch_work_cols(const float* wrows, int n, int np, int d, int dp, float* xsW, cudaStream_t st);
+// The transposed copy in working order: xsW [dp][np] from the row-major rows xsR [n][d].
+cudaError_t launch_work_cols(const float* xsR, const uint32_t* perm, int n, int np, int d, int dp, float* xsW,
+                             cudaStream_t st);
 // The lists of `segs` column segments (segs × count × cap entries, τ: segs × count) merged per row.
 cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
                                const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
                                float* tau, cudaStream_t st);
-// Tanimoto selection with the norm window (knn.rs:595-644): rows in the norm order `perm` (working →
-// original, prune::norm_order), each query block walking outward from its own norms and stopping a
-// side once its norms leave every row's window; d_pad ≤ 64. ws holds tani_window_bytes(n, np, dp)
-// (the norm-ordered working copy, norms and tile ranges); the lists are written in input order.
-size_t tani_window_bytes(int n, int np, int dp);
-cudaError_t launch_coarse_tani_window(const float* xsT, int n, int np, int dp, int cap, const double* norms,
-                                      const uint32_t* perm, void* ws, uint32_t* cand_idx, float* cand_score,
-                                      float* tau, unsigned long long* skipped_total, cudaStream_t st);
 // The floor of rows re-run after the tensor-core pass (rows[0..*count), cand_* and tau of that pass).
 cudaError_t launch_rerun_floor(const uint32_t* rows, const unsigned* count, int nmax, int cap, const float* tau,
                                const float* cand_score, const double* row_eps, double eps, float* tfloor,

@@ -477,6 +477,19 @@ __device__ __forceinline__ float row_ub_f32(float m, float delta, float rb) {
     return fminf(1.0f, __fadd_ru(cosf(th), 1e-6f));
 }
 
+// Tanimoto selection (knn.rs:239-283): with ρ the quotient of two rows' norms, T = c / (ρ + 1/ρ − c) grows
+// with their cosine c > 0, so over two blocks whose cosines are ≤ u and whose norms lie in [a.x, a.y] and
+// [b.x, b.y], T ≤ u / (m − u) with m = the smallest ρ + 1/ρ there (2 where the ranges meet), and T ≤ 0 for
+// u ≤ 0. Roundings go outward (the ranges arrive rounded outward to f32).
+__device__ __forceinline__ float tani_ub_f32(float u, float2 a, float2 b) {
+    if (u <= 0.0f) return 0.0f;
+    float r = 1.0f;
+    if (a.x > b.y) r = __fdiv_rd(a.x, b.y);
+    else if (b.x > a.y) r = __fdiv_rd(b.x, a.y);
+    const float m = r > 1.0f ? __fadd_rd(r, __fdiv_rd(1.0f, r)) : 2.0f;  // (r = +inf: no pair of live rows)
+    return fminf(1.0f, __fdiv_ru(u, __fsub_rd(fmaxf(m, 2.0f), u)));
+}
+
 // Compare-exchange of list keys (descending) at a register distance S within a thread's run.
 template <int S, int KPT>
 __device__ __forceinline__ void cx_regs(uint32_t (&v)[KPT], int base, int size) {
@@ -574,11 +587,12 @@ __device__ __forceinline__ void compact_keys(const uint32_t (&all)[KPT_ALL], uin
 // levels — a bitonic sort of 32-bit keys, 16 per thread, exchanged in registers, by warp shuffles or
 // through shared memory by distance — and the largest UB of a skipped block. Lists longer than the
 // shape's N stay in block order with bounds +inf.
-template <int KPT_ALL>
+template <int KPT_ALL, bool TANI>
 __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
     k_block_lists(const double* __restrict__ qcenter, const double* __restrict__ qradius,
                   const float* __restrict__ ccenter_f, const float* __restrict__ cradius_f, int nqb, int ncb, int d,
                   const float* __restrict__ tq, const float* __restrict__ rowmax, const float* __restrict__ rm_delta,
+                  const float2* __restrict__ qnorm, const float2* __restrict__ cnorm, int use_cos,
                   uint32_t* __restrict__ lists, float* __restrict__ list_ub, uint32_t* __restrict__ counts,
                   float* __restrict__ ub_skip, unsigned long long* __restrict__ skipped_total) {
     using LS = ListShape<KPT_ALL>;
@@ -587,22 +601,33 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
     __shared__ unsigned kept, slot;
     __shared__ int skip_max_bits;
     const int Q = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-    if (tid < d) cq[tid] = (float)qcenter[(size_t)Q * d + tid];
+    if ((!TANI || use_cos) && tid < d) cq[tid] = (float)qcenter[(size_t)Q * d + tid];
     if (tid == 0) {
         kept = 0;
         slot = 0;
         skip_max_bits = __float_as_int(-CUDART_INF_F);
     }
     __syncthreads();
-    float rq = (float)qradius[Q];
-    if ((double)rq < qradius[Q]) rq = nextafterf(rq, CUDART_INF_F);
+    float rq = 0.0f;
+    if (!TANI || use_cos) {
+        rq = (float)qradius[Q];
+        if ((double)rq < qradius[Q]) rq = nextafterf(rq, CUDART_INF_F);
+    }
+    const float2 nq = TANI ? qnorm[Q] : make_float2(0.0f, 0.0f);
     const float t = tq ? tq[Q] : -CUDART_INF_F;
     const float* rm = rowmax ? rowmax + (size_t)Q * ncb : nullptr;
     const float delta = rowmax ? *rm_delta : 0.0f;
-    // the smaller of the cone bound and the per-row bound
+    // the smaller of the cone bound and the per-row bound (without cosine bounds 1, all at one angle);
+    // for Tanimoto selection the bound on T that it and the blocks' norms give
     auto bound = [&](int b, float* phi) {
-        const float u = block_ub_f32(cq, rq, ccenter_f + b, ncb, cradius_f[b], d, phi);
-        return rm ? fminf(u, row_ub_f32(rm[b], delta, cradius_f[b])) : u;
+        float u = 1.0f;
+        if (!TANI || use_cos) {
+            u = block_ub_f32(cq, rq, ccenter_f + b, ncb, cradius_f[b], d, phi);
+            if (rm) u = fminf(u, row_ub_f32(rm[b], delta, cradius_f[b]));
+        } else if (phi) {
+            *phi = 0.0f;
+        }
+        return TANI ? tani_ub_f32(u, nq, cnorm[b]) : u;
     };
     uint32_t* out = lists + (size_t)Q * ncb;
     float* out_ub = list_ub + (size_t)Q * ncb;
@@ -825,6 +850,67 @@ __global__ void k_norm_bucket(const double* __restrict__ norms, int n, const uns
     cell[i] = b;
 }
 
+// The norm range of each block of `bs` working rows, rounded outward to f32 (one warp per block).
+__global__ void k_block_norms(const double* __restrict__ norms, const uint32_t* __restrict__ perm, int n, int bs, int nb,
+                              float2* __restrict__ range) {
+    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb) return;
+    float lo = CUDART_INF_F, hi = 0.0f;
+    for (int w = b * bs + lane; w < min(n, (b + 1) * bs); w += 32) {
+        const double a = norms[perm[w]];
+        lo = fminf(lo, __double2float_rd(a));
+        hi = fmaxf(hi, __double2float_ru(a));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(COSTAL_FULL_MASK, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(COSTAL_FULL_MASK, hi, o));
+    }
+    if (lane == 0) range[b] = make_float2(lo, hi);
+}
+
+cudaError_t block_norms(const double* norms, Plan& P, float2* ranges, cudaStream_t st) {
+    k_block_norms<<<(P.ncb + 7) / 8, 256, 0, st>>>(norms, P.perm, P.n, P.cb, P.ncb, ranges); note_launch();
+    P.cnorm = P.qnorm = ranges;
+    if (P.cb != QB) {
+        k_block_norms<<<(P.nqb + 7) / 8, 256, 0, st>>>(norms, P.perm, P.n, QB, P.nqb, ranges + P.ncb); note_launch();
+        P.qnorm = ranges + P.ncb;
+    }
+    return cudaGetLastError();
+}
+
+// Over a strided sample of up to 1,024 rows: share[0] = the pairs of live rows, share[1] = those whose
+// norms' quotient lies inside the window of a Tanimoto score of 0.9 (ρ + 1/ρ ≤ 1.9 / 0.9).
+__global__ void __launch_bounds__(1024) k_norm_window_share(const double* __restrict__ norms, int n, unsigned* __restrict__ share) {
+    __shared__ float a_s[1024];
+    const int m = min(n, 1024), i = threadIdx.x;
+    a_s[i] = i < m ? (float)norms[(size_t)i * n / m] : 0.0f;
+    __syncthreads();
+    unsigned all = 0, in = 0;
+    if (a_s[i] > 0.0f)
+        for (int j = 0; j < m; ++j) {
+            const float b = a_s[j], a = a_s[i];
+            if (b > 0.0f) {
+                ++all;
+                in += a * a + b * b <= (1.9f / 0.9f) * a * b ? 1u : 0u;
+            }
+        }
+    atomicAdd(&share[0], all);
+    atomicAdd(&share[1], in);
+}
+
+cudaError_t norm_window_share(const double* norms, int n, unsigned* share, cudaStream_t st) {
+    k_norm_window_share<<<1, 1024, 0, st>>>(norms, n, share); note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& P) {
+    Scratch S{};
+    carve(ws, n, d, P, S);
+    P.norm_only = true;
+    return norm_order(norms, n, norm_ws, P.perm, st);
+}
+
 size_t norm_order_bytes(int n) {
     const size_t nch = (size_t)(n + CHUNK - 1) / CHUNK;
     return a256((size_t)n * 4) + a256(nch * NORM_BUCKETS * 4) + a256((NORM_BUCKETS + 1) * 4) + 256;
@@ -852,12 +938,13 @@ cudaError_t build_lists(Plan& P, unsigned long long* skipped_total, cudaStream_t
     // up to 8,192 column blocks: 16 keys a thread, two CTAs per SM; up to 16,384: 32 keys a thread;
     // beyond that (n > 4,194,304 with blocks of 256) the lists stay in block order (no early stop)
     const bool wide = P.ncb > ListShape<16>::N;
-    auto kern = wide ? k_block_lists<32> : k_block_lists<16>;
+    auto kern = P.qnorm ? (wide ? k_block_lists<32, true> : k_block_lists<16, true>)
+                        : (wide ? k_block_lists<32, false> : k_block_lists<16, false>);
     const size_t smem = (size_t)(wide ? ListShape<32>::N : ListShape<16>::N) * 4;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     kern<<<P.nqb, LIST_T, smem, st>>>(P.qcenter, P.qradius, P.ccenter_f, P.cradius_f, P.nqb, P.ncb, P.d, P.tq,
-                                      P.rowmax, P.rm_delta, P.lists, P.list_ub, P.counts, P.ub_skip, skipped_total);
+                                      P.rowmax, P.rm_delta, P.qnorm, P.cnorm, P.norm_only ? 0 : 1, P.lists, P.list_ub, P.counts, P.ub_skip, skipped_total);
     note_launch();
     k_row_ub<<<(P.n + 255) / 256, 256, 0, st>>>(P.perm, P.n, P.ub_skip, P.row_ub); note_launch();
     return cudaGetLastError();

@@ -42,6 +42,8 @@ struct Plan {
     double* row_ub;      // [n] (original order) pruning floor of the certificate
     float* tq;           // [nqb] per-query-block thresholds (NULL = keep every block)
     float* wrows;        // [n][d] the normalised rows in working order, row-major
+    const float2 *qnorm, *cnorm;  // Tanimoto selection: the blocks' norm ranges (block_norms), or NULL
+    bool norm_only;         // the working order is the norm order: no cosine bounds
     const float* rowmax;    // [nqb][ncb] per-row bound data (tc::launch_rowmax), or NULL: cone bound only
     const float* rm_delta;  // its error margin (device scalar)
 };
@@ -56,11 +58,19 @@ cudaError_t build_lists(Plan& plan, unsigned long long* skipped_total, cudaStrea
 
 // Rows grouped by norm for Tanimoto selection's norm window (knn.rs:413-418 sorts by norm): a stable
 // counting sort into NORM_BUCKETS buckets spaced evenly in log(norm) between the smallest and the
-// largest positive norm (zero rows first). Within a bucket rows keep their input order; the window
-// test only needs each column tile's exact norm range, so the order inside a bucket does not matter.
+// largest positive norm (zero rows first). Within a bucket rows keep their input order; the bounds
+// only need each block's exact norm range, so the order inside a bucket does not matter.
 constexpr int NORM_BUCKETS = 1024;
 size_t norm_order_bytes(int n);
 cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cudaStream_t st);
+// How much of the data a norm window leaves: of the pairs of a row sample (share[0], zeroed by the
+// caller), those inside the window of a Tanimoto score of 0.9 (share[1]).
+cudaError_t norm_window_share(const double* norms, int n, unsigned* share, cudaStream_t st);
+// A plan whose working order is that norm order (no cells, no geometry), for lists by norm ranges alone.
+cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& plan);
+// The blocks' norm ranges into ranges[ncb + nqb], and into the plan: build_lists then bounds the
+// Tanimoto score instead of the cosine.
+cudaError_t block_norms(const double* norms, Plan& plan, float2* ranges, cudaStream_t st);
 
 }  // namespace prune
 }  // namespace costal

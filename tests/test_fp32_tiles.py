@@ -58,3 +58,23 @@ def test_fp32_pass_by_lists(ext, oracle, n, d, k, margin):
         for a, b in zip((idx.view(np.uint32), cos, norms), want):
             np.testing.assert_array_equal(a, b)
         assert prune or st["blocks_stopped"] == 0
+
+
+@pytest.mark.parametrize("n,d,k,spread,signed", [(130, 3, 5, 4.0, False), (5001, 30, 10, 9.0, False), (16_383, 7, 12, 3.0, True),
+                                                 (16_385, 5, 10, 6.0, False), (30_001, 40, 30, 2.0, False),
+                                                 (25_000, 64, 70, 5.0, True)])
+def test_tanimoto_by_lists(ext, oracle, n, d, k, spread, signed):
+    """Tanimoto selection by the norm order's lists (few rows) and by cosine bounds with norm ranges
+    (16,384 rows and more): zero rows, repeated rows, thresholds below zero."""
+    rng = np.random.default_rng(n)
+    x = clustered(n, d, n + d) - (2.0 if signed else 0.0)
+    x = x * np.exp(rng.uniform(0, np.log(spread), size=(n, 1)))
+    x[n // 2:n // 2 + 40] = x[4]
+    x[:2] = 0.0
+    x = np.ascontiguousarray(x, dtype=np.float32)
+    want, _ = oracle.knn_exact(x, k, select="tanimoto")
+    for prune in (True, False):
+        got, st = ext._knn_exact(x, k, select="tanimoto", prune=prune)
+        for a, b in zip((got[0].view(np.uint32), got[1], got[2]), want):
+            np.testing.assert_array_equal(a, b)
+        assert prune or st["blocks_skipped"] == 0
