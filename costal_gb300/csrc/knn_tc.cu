@@ -15,12 +15,12 @@
 //             [hi | hi] × B's [hi | lo], then A's [lo] × B's leading [hi].
 //   kernel    One CTA per 128 query rows (M = 128, one TMEM lane per query), column tiles of N = 256.
 //             Warp 4 streams B tiles with TMA (128-byte swizzle) into a ring of shared-memory
-//             stages; warp 5 issues the MMAs (one elected thread) into two 256-column TMEM
-//             accumulators; warps 0-3 read the accumulators back (tcgen05.ld, 64 columns at a time,
-//             the next load in flight while one is scanned), reject whole slices with a 3-input max
-//             tree against the query's threshold, and append the rare survivors to per-query buffers
-//             that the warp shrinks cooperatively to the best cap (strict `v > τ` admission,
-//             knn.rs:774-780).
+//             stages; warps 5 and 6 issue the MMAs (one thread each) into a 256-column TMEM
+//             accumulator each (K loop: warp 5 into both in turn); warps 0-3 read the accumulators
+//             back (tcgen05.ld.red, 64 columns at a time with their row maximum), reject whole slices
+//             by that maximum against the query's threshold, and append the rare survivors to
+//             per-query buffers that the warp shrinks cooperatively to the best cap (strict `v > τ`
+//             admission, knn.rs:774-780).
 //   bound     Every query row i gets a rigorous bound E_i on |coarse − exact cosine| (k_row_eps):
 //             split remainder ‖a_lo‖·max‖b_lo‖ + ‖a_hi+a_lo‖·max‖r_b‖ + ‖r_a‖·max‖b_hi+b_lo‖ + ‖r_a‖·max‖r_b‖
 //             (Cauchy–Schwarz), plus the tensor-core accumulation (K + 16)·2⁻²¹·Σ|products| (four
@@ -57,7 +57,7 @@ constexpr int B_KB_BYTES = BLOCK_N * 128;  // 32 KB per K block of a column tile
 constexpr int HALF_N = BLOCK_N / 2;            // columns of one TMA box of a column tile
 constexpr int B_HALF_BYTES = HALF_N * 128;     // 16 KB: the second half of a K block
 constexpr int EPI_WARPS = 4;
-constexpr int NTHREADS = (EPI_WARPS + 2) * 32;  // 4 epilogue warps, 1 TMA warp, 1 MMA warp
+constexpr int NTHREADS = (EPI_WARPS + 3) * 32;  // 4 epilogue warps, 1 TMA warp, 2 MMA warps
 constexpr uint32_t TMEM_COLS = 512;    // two 256-column FP32 accumulators
 
 // ---- tcgen05 -----------------------------------------------------------------------------------
@@ -123,6 +123,17 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
         : "r"(taddr)
         : "memory");
 }
+// The same load with the hardware's row reduction: also the largest of the 64 values.
+__device__ __forceinline__ void tmem_ld64_max(uint32_t taddr, uint32_t (&r)[64], uint32_t& top) {
+    asm volatile(
+        "tcgen05.ld.red.sync.aligned.32x32b.x64.max.f32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"
+        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,"
+        "%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, %64, [%65];"
+        : COSTAL_R8(0), COSTAL_R8(8), COSTAL_R8(16), COSTAL_R8(24), COSTAL_R8(32), COSTAL_R8(40), COSTAL_R8(48),
+          COSTAL_R8(56), "=r"(top)
+        : "r"(taddr)
+        : "memory");
+}
 // Wait for this thread's outstanding TMEM loads. The registers are in/out operands, so no use of
 // them can be scheduled before the wait.
 __device__ __forceinline__ void tmem_wait(uint32_t (&r)[64]) {
@@ -132,21 +143,32 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[64]) {
                  :
                  : "memory");
 }
-#undef COSTAL_R8
+// Two slices at once (the wait covers every outstanding load; the second statement only ties its
+// registers to it).
+__device__ __forceinline__ void tmem_wait2(uint32_t (&ra)[64], uint32_t (&rb)[64], uint32_t& ta, uint32_t& tb) {
+    tmem_wait(ra);
+    uint32_t(&r)[64] = rb;
+    asm volatile(""
+                 : COSTAL_W8(0), COSTAL_W8(8), COSTAL_W8(16), COSTAL_W8(24), COSTAL_W8(32), COSTAL_W8(40),
+                   COSTAL_W8(48), COSTAL_W8(56), "+r"(ta), "+r"(tb)
+                 :
+                 : "memory");
+}
 #undef COSTAL_W8
 
-// 8 TMEM columns at a run-time column offset, loaded and waited for.
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-    uint32_t r[8];
+// The largest of 32 consecutive TMEM columns of this thread's lane, loaded and waited for.
+__device__ __forceinline__ float tmem_max32(uint32_t taddr) {
+    uint32_t r[32], top;
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+        "tcgen05.ld.red.sync.aligned.32x32b.x32.max.f32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"
+        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, %32, [%33];\n"
         "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : COSTAL_R8(0), COSTAL_R8(8), COSTAL_R8(16), COSTAL_R8(24), "=r"(top)
         : "r"(taddr)
         : "memory");
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+    return __uint_as_float(top);
 }
+#undef COSTAL_R8
 
 __device__ __forceinline__ float max3f(float a, float b, float c) {
     float r;
@@ -211,12 +233,24 @@ __device__ __noinline__ float flush_one(float* B_s, uint32_t* B_i, int qL, int c
     const uint32_t diff = kmin ^ kmax;
     const int top = diff ? 31 - __clz(diff) : -1;
     uint32_t T = top >= 0 ? (kmax & ~((2u << top) - 1u)) : kmax;
+    bool whole = false;  // exactly cap keys are ≥ T: the cap-th score is the smallest of them
     for (int b = top; b >= 0; --b) {
         const uint32_t c = T | (1u << b);
         int n_ge = 0;
 #pragma unroll
         for (int s = 0; s < SL; ++s) n_ge += __popc(__ballot_sync(COSTAL_FULL_MASK, key[s] >= c));
         if (n_ge >= cap) T = c;
+        if (n_ge == cap) {
+            whole = true;
+            break;
+        }
+    }
+    if (whole) {
+        uint32_t m = 0xffffffffu;
+#pragma unroll
+        for (int s = 0; s < SL; ++s)
+            if (key[s] >= T) m = min(m, key[s]);
+        T = __reduce_min_sync(COSTAL_FULL_MASK, m);
     }
     // keep key > T, and the first (cap − #{key > T}) entries with key == T
     int n_gt = 0;
@@ -313,52 +347,46 @@ __device__ __forceinline__ void group_max4(const uint32_t (&r)[64], float* gm) {
                       __uint_as_float(r[4 * g + 3]));
 }
 
-// One 64-column slice held in registers: a per-lane 8-bit mask of the 8-column groups whose maximum
-// is above the lane's threshold, OR-ed over the warp. Returns the warp's mask.
-__device__ __forceinline__ unsigned slice_mask(const uint32_t (&r)[64], float tau) {
-    unsigned m = 0;
-#pragma unroll
-    for (int g = 0; g < 8; ++g) m |= (max8(r + 8 * g) > tau ? 1u : 0u) << g;
-    return __reduce_or_sync(COSTAL_FULL_MASK, m);
-}
-
-// The 8-column groups of a slice that some lane of the warp needs: re-read each from TMEM (at a
-// run-time column) and append each lane's survivors (strictly above τ, in range, not the query
-// itself). Kept out of line: the rare path stays off the hot loop's instruction footprint.
+// A 64-column slice held in registers: append each lane's survivors (strictly above τ, in range, not the
+// query itself). Every lane walks its own 8-column groups whose maximum is above its τ, all lanes at
+// once, the group's values picked by selects: as many turns as the busiest lane has such groups.
+// (Walking the union of the lanes' groups, each re-read from TMEM, took the epilogue warps 1.1 of the
+// 1.5 M cycles of a query block at 600,000 × 40.)
 template <int SL>
-__device__ __noinline__ void admit_groups(unsigned gmask, uint32_t taddr, int cb, int n, int q, int qi, int qbase,
-                                          int lane, int cap, int q_lo, float* B_s, uint32_t* B_i,
-                                          int* cnt_io, float* tau_io) {
-    constexpr int BCAP = 32 * SL;
-    int cnt = *cnt_io;
-    float tau = *tau_io;
-    while (gmask) {
-        const int g = __ffs(gmask) - 1;
-        gmask &= gmask - 1;
-        float v[8];
-        tmem_ld8(taddr + (uint32_t)(8 * g), v);
+__device__ __forceinline__ void admit_slice(const uint32_t (&r)[64], int cb, int n, int q, int qi, int qbase, int lane,
+                                            int cap, int q_lo, int limit, float* B_s, uint32_t* B_i, int& cnt, float& tau) {
+    unsigned gm = 0;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) gm |= (max8(r + 8 * g) > tau ? 1u : 0u) << g;
+    const bool clean = cb + 64 <= n && (cb + 64 <= q_lo || cb >= q_lo + 32);  // warp-uniform
+    while (__any_sync(COSTAL_FULL_MASK, gm != 0)) {
+        const int g = gm ? __ffs(gm) - 1 : 0;
+        const bool live = gm != 0;
+        gm &= gm - 1;
         const int c = cb + 8 * g;
-        const bool clean = c + 8 <= n && (c + 8 <= q_lo || c >= q_lo + 32);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+            const uint32_t a = g & 1 ? r[8 + j] : r[j], b = g & 1 ? r[24 + j] : r[16 + j];
+            const uint32_t d = g & 1 ? r[40 + j] : r[32 + j], e = g & 1 ? r[56 + j] : r[48 + j];
+            const uint32_t ab = g & 2 ? b : a, de = g & 2 ? e : d;
+            const float v = __uint_as_float(g & 4 ? de : ab);
             const int col = c + j;
-            if (v[j] > tau && (clean || (col < n && col != q))) {
-                B_s[cnt * BSTRIDE + qi] = v[j];
+            if (live && v > tau && (clean || (col < n && col != q))) {
+                B_s[cnt * BSTRIDE + qi] = v;
                 B_i[cnt * BSTRIDE + qi] = (uint32_t)col;
                 ++cnt;
             }
         }
-        flush_full<SL>(B_s, B_i, qbase, lane, cap, BCAP - 8, cnt, tau);
+        flush_full<SL>(B_s, B_i, qbase, lane, cap, limit, cnt, tau);
     }
-    *cnt_io = cnt;
-    *tau_io = tau;
 }
 
 template <int SLOTS, bool KLOOP, bool FP8 = false, bool PAIR = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_coarse_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_bw, int n, int np,
-                int nkb, int nkb_b, int ksteps, int k1s, int stages, int cap, const uint32_t* __restrict__ perm,
+                int nkb, int nkb_b, int ksteps, int k1s, int stages, int cap, int probes, int mma_warps,
+                const uint32_t* __restrict__ perm,
                 const uint32_t* __restrict__ lists, const float* __restrict__ list_ub,
                 const uint32_t* __restrict__ counts, int ncb, const double* __restrict__ row_eps,
                 uint32_t* __restrict__ cand_idx, float* __restrict__ cand_score, float* __restrict__ tau_out,
@@ -375,9 +403,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // 1024-byte alignment for the swizzled tiles
     const uint32_t base_u32 = smem_u32(smem_raw);
     unsigned char* smem = smem_raw + ((1024 - (base_u32 & 1023)) & 1023);
-    // Resident A: the query tile (nkb K blocks) once, then `stages` column tiles of nkb_b K blocks. K loop (deep rows, KLOOP): every stage holds one K block of the query tile
+    // Resident A: the query tile (nkb K blocks) once, then `stages` stages of one K block of a column tile
+    // (finer than a tile: a block's refill starts when its own MMAs are done). K loop (deep rows, KLOOP): every stage holds one K block of the query tile
     // and of the column tile, and a tile's MMA chain runs over nkb stages.
-    const uint32_t stage_bytes = KLOOP ? (uint32_t)(A_KB_BYTES + B_KB_BYTES) : (uint32_t)nkb_b * B_KB_BYTES;
+    const uint32_t stage_bytes = (uint32_t)(KLOOP ? A_KB_BYTES + B_KB_BYTES : B_KB_BYTES);
     unsigned char* a_tile = smem;                                            // nkb × 16 KB (resident A)
     unsigned char* b_tiles = KLOOP ? smem : a_tile + (size_t)nkb * A_KB_BYTES;  // stages × stage_bytes
     float* B_s = reinterpret_cast<float*>(b_tiles + (size_t)stages * stage_bytes);  // [BCAP][BSTRIDE]
@@ -400,29 +429,39 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int nentries = lists ? (int)counts[qb] : 0;
     const int ntiles = lists ? (nentries + EPC - 1) / EPC : np / BLOCK_N;
     const uint32_t* my_list = lists ? lists + (size_t)qb * ncb : nullptr;
-    auto tile_cols = [&](int t, int& c0, int& c1) -> bool {
+    // A tile's list entries are read one tile ahead by every role that needs them: read when they were
+    // needed, their latency stood in every tile (850 of the epilogue's 2,690 cycles at 2,000,000 × 40).
+    struct Entry {
+        uint32_t e0, e1;
+    };
+    auto tile_entry = [&](int t) -> Entry {
+        if (t >= ntiles) return Entry{0u, 0u};
+        if (!my_list) return Entry{(uint32_t)t, 0u};
+        if constexpr (PAIR) return Entry{my_list[2 * t], my_list[min(2 * t + 1, nentries - 1)]};
+        return Entry{my_list[t], 0u};
+    };
+    // The first columns of its halves; false: its second half has no list entry.
+    auto tile_cols = [&](int t, const Entry& en, int& c0, int& c1) -> bool {
         if constexpr (PAIR) {
             const bool two = 2 * t + 1 < nentries;
-            c0 = (int)my_list[2 * t] * HALF_N;
-            c1 = two ? (int)my_list[2 * t + 1] * HALF_N : c0;
+            c0 = (int)en.e0 * HALF_N;
+            c1 = two ? (int)en.e1 * HALF_N : c0;
             return two;
         } else {
-            c0 = (my_list ? (int)my_list[t] : t) * BLOCK_N;
+            c0 = (int)en.e0 * BLOCK_N;
             c1 = c0 + HALF_N;
             return true;
         }
     };
-    // the list entries of tile t lie inside the operands (the list kernel never writes others)
-    auto tile_ok = [&](int t) -> bool {
-        if (!my_list) return true;
-        if constexpr (PAIR) {
-            const unsigned lim = (unsigned)(np / HALF_N);
-            return my_list[2 * t] < lim && (2 * t + 1 >= nentries || my_list[2 * t + 1] < lim);
-        } else {
-            return my_list[t] < (unsigned)(np / BLOCK_N);
-        }
+    // the list entries of a tile lie inside the operands (the list kernel never writes others)
+    auto entry_ok = [&](const Entry& en) -> bool {
+        const uint32_t lim = (uint32_t)(np / (PAIR ? HALF_N : BLOCK_N));
+        return en.e0 < lim && en.e1 < lim;
     };
-    const uint32_t a_bytes = (uint32_t)nkb * A_KB_BYTES, b_bytes = (uint32_t)nkb_b * B_KB_BYTES;
+    // The CTA's visits: its first P tiles once for their slice maxima alone (the starting threshold), then
+    // all tiles from the first. Rings, accumulators and the stop go by visits.
+    const int P = KLOOP ? 0 : min(probes, ntiles), nvisits = P + ntiles;
+    const uint32_t a_bytes = (uint32_t)nkb * A_KB_BYTES;
     (void)a_bytes;
 
     if (threadIdx.x == 0) {
@@ -435,7 +474,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(&bars->t_full[b], 1);
             mbar_init(&bars->t_empty[b], EPI_WARPS);
         }
-        bars->stop_tile = ntiles;
+        bars->stop_tile = nvisits;
         for (int w = 0; w < EPI_WARPS; ++w) bars->warp_floor[w] = -CUDART_INF_F;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -455,14 +494,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (KLOOP && lane == 0) {
             const float* my_ub = list_ub ? list_ub + (size_t)qb * ncb : nullptr;
             bool go = true;
+            int s = 0;
+            uint32_t ph = 1;
             for (int t = 0; go && t < ntiles; ++t) {
-                const bool ok = tile_ok(t);
+                const Entry en = tile_entry(t);
+                const bool ok = entry_ok(en);
                 int c0 = 0, c1 = 0;
-                if (ok) tile_cols(t, c0, c1);
+                if (ok) tile_cols(t, en, c0, c1);
                 for (int kb = 0; kb < nkb; ++kb) {
-                    const int g = t * nkb + kb, s = g % stages;
-                    const uint32_t ph = (uint32_t)(g / stages) & 1u;
-                    if (!mbar_wait(&bars->b_empty[s], ph ^ 1u, timeout_flag, true)) {
+                    if (!mbar_wait(&bars->b_empty[s], ph, timeout_flag, false)) {
                         go = false;
                         break;
                     }
@@ -496,6 +536,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         tma_load_2d(dst + A_KB_BYTES, &map_b, kb * KBE, c0, &bars->b_full[s]);
                         tma_load_2d(dst + A_KB_BYTES + B_HALF_BYTES, &map_b, kb * KBE, c1, &bars->b_full[s]);
                     }
+                    if (++s == stages) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
             }
         }
@@ -503,62 +547,81 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_expect_tx(&bars->a_full, a_bytes);
             for (int kb = 0; kb < nkb; ++kb) tma_load_2d(a_tile + kb * A_KB_BYTES, &map_a, kb * KBE, q0, &bars->a_full);
             const float* my_ub = list_ub ? list_ub + (size_t)qb * ncb : nullptr;
-            for (int t = 0; t < ntiles; ++t) {
-                const int s = t % stages;
-                const uint32_t ph = (uint32_t)(t / stages) & 1u;
-                if (!mbar_wait(&bars->b_empty[s], ph ^ 1u, timeout_flag, true)) break;
-                if (!tile_ok(t)) {
-                    // a list entry outside the operands (never produced by the list kernel): report it
-                    // and stop the CTA here like an early stop, so no role reads past the operands
-                    atomicExch(timeout_flag, 2ull);
-                    *reinterpret_cast<volatile int*>(&bars->stop_tile) = t;
-                    mbar_arrive(&bars->b_full[s]);
-                    break;
-                }
-                if (t > 0 && my_ub) {
-                    // Every column of the tile's first list entry (and of all later ones: the bounds do
-                    // not increase) has cosine ≤ its bound; its coarse score is ≤ bound + E_i. When that
-                    // is below every row's threshold τ_i, none of them can be admitted: stop here. The
-                    // floors read may be stale, i.e. lower, which only delays the stop.
-                    volatile float* wf = bars->warp_floor;
-                    const float fl = fminf(fminf(wf[0], wf[1]), fminf(wf[2], wf[3]));
-                    if (my_ub[t * EPC] < fl) {
-                        *reinterpret_cast<volatile int*>(&bars->stop_tile) = t;
-                        if (stopped_total) atomicAdd(stopped_total, (unsigned long long)(nentries - t * EPC));
-                        mbar_arrive(&bars->b_full[s]);  // completes the phase without data (release)
+            int s = 0;  // the ring's next stage and phase: one K block (32 KB) of a column tile per stage
+            uint32_t ph = 1;
+            bool go = true;
+            Entry next = tile_entry(0);
+            float next_ub = CUDART_INF_F;
+            for (int v = 0; go && v < nvisits; ++v) {
+                const int t = v < P ? v : v - P, tn = v + 1 < P ? v + 1 : v + 1 - P;
+                const Entry en = next;
+                const float ub = next_ub;
+                next = tile_entry(tn);
+                if (my_ub && tn < ntiles) next_ub = my_ub[tn * EPC];
+                int c0 = 0, c1 = 0;
+                for (int kb = 0; kb < nkb_b; ++kb) {
+                    if (!mbar_wait(&bars->b_empty[s], ph, timeout_flag, false)) {
+                        go = false;
                         break;
                     }
-                }
-                mbar_expect_tx(&bars->b_full[s], b_bytes);
-                unsigned char* dst = b_tiles + (size_t)s * b_bytes;
-                int c0, c1;
-                tile_cols(t, c0, c1);
-                // (the last K block may reach past the operand's row: TMA fills those columns with zeros
-                // and reads nothing for them)
-                if (c1 == c0 + HALF_N) {  // adjacent halves: one 256-row box per K block
-                    for (int kb = 0; kb < nkb_b; ++kb)
-                        tma_load_2d(dst + kb * B_KB_BYTES, &map_bw, kb * KBE, c0, &bars->b_full[s]);
-                } else {
-                    for (int kb = 0; kb < nkb_b; ++kb) {
-                        tma_load_2d(dst + kb * B_KB_BYTES, &map_b, kb * KBE, c0, &bars->b_full[s]);
-                        tma_load_2d(dst + kb * B_KB_BYTES + B_HALF_BYTES, &map_b, kb * KBE, c1, &bars->b_full[s]);
+                    if (kb == 0) {
+                        bool stop = false;
+                        if (!entry_ok(en)) {
+                            // a list entry outside the operands (never produced by the list kernel): report
+                            // it and stop the CTA here like an early stop, so no role reads past the operands
+                            atomicExch(timeout_flag, 2ull);
+                            stop = true;
+                        } else if (t > 0 && v >= P && my_ub) {
+                            // Every column of the tile's first list entry (and of all later ones: the bounds
+                            // do not increase) has cosine ≤ its bound; its coarse score is ≤ bound + E_i. When
+                            // that is below every row's threshold τ_i, none of them can be admitted: stop here.
+                            // The floors read may be stale, i.e. lower, which only delays the stop.
+                            volatile float* wf = bars->warp_floor;
+                            const float fl = fminf(fminf(wf[0], wf[1]), fminf(wf[2], wf[3]));
+                            if (ub < fl) {
+                                stop = true;
+                                if (stopped_total) atomicAdd(stopped_total, (unsigned long long)(nentries - t * EPC));
+                            }
+                        }
+                        if (stop) {
+                            *reinterpret_cast<volatile int*>(&bars->stop_tile) = v;
+                            mbar_arrive(&bars->b_full[s]);  // completes the phase without data (release)
+                            go = false;
+                            break;
+                        }
+                        tile_cols(t, en, c0, c1);
+                    }
+                    mbar_expect_tx(&bars->b_full[s], (uint32_t)B_KB_BYTES);
+                    unsigned char* dst = b_tiles + (size_t)s * B_KB_BYTES;
+                    // (the last K block may reach past the operand's row: TMA fills those columns with zeros
+                    // and reads nothing for them)
+                    if (c1 == c0 + HALF_N) {  // adjacent halves: one 256-row box
+                        tma_load_2d(dst, &map_bw, kb * KBE, c0, &bars->b_full[s]);
+                    } else {
+                        tma_load_2d(dst, &map_b, kb * KBE, c0, &bars->b_full[s]);
+                        tma_load_2d(dst + B_HALF_BYTES, &map_b, kb * KBE, c1, &bars->b_full[s]);
+                    }
+                    if (++s == stages) {
+                        s = 0;
+                        ph ^= 1u;
                     }
                 }
             }
         }
-    } else if (warp == EPI_WARPS + 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        if (KLOOP && lane == 0) {
+    } else if (KLOOP && warp == EPI_WARPS + 1) {
+        // ------------------------------------------------------------------ MMA issuer, K loop
+        if (lane == 0) {
             bool go = true;
+            const uint64_t st_desc = sw128_desc(smem_u32(b_tiles));
+            int s = 0;
+            uint32_t ph = 0;
             for (int t = 0; go && t < ntiles; ++t) {
                 const int buf = t & 1;
                 const uint32_t bph = (uint32_t)(t >> 1) & 1u;
-                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, true)) break;
+                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, false)) break;
                 const uint32_t d = tmem + (uint32_t)(buf * BLOCK_N);
                 for (int kb = 0; kb < nkb; ++kb) {
-                    const int g = t * nkb + kb, s = g % stages;
-                    const uint32_t ph = (uint32_t)(g / stages) & 1u;
-                    if (!mbar_wait(&bars->b_full[s], ph, timeout_flag, true)) {
+                    if (!mbar_wait(&bars->b_full[s], ph, timeout_flag, false)) {
                         go = false;
                         break;
                     }
@@ -568,49 +631,92 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         go = false;
                         break;
                     }
-                    const uint32_t a_base = smem_u32(b_tiles + (size_t)s * stage_bytes);
-                    const uint32_t b_base = a_base + A_KB_BYTES;
-                    const int nks = min(4, ksteps - 4 * kb);
-                    for (int ks = 0; ks < nks; ++ks) {
-                        const uint32_t koff = (uint32_t)(ks * 32);  // 16 bf16 = 32 bytes inside the swizzle row
-                        mma_kind<FP8>(d, sw128_desc(a_base + koff), sw128_desc(b_base + koff), (kb | ks) ? 1u : 0u);
-                    }
+                    const uint64_t ad = st_desc + (uint64_t)(s * ((A_KB_BYTES + B_KB_BYTES) >> 4));
+                    const uint64_t bd = ad + (uint64_t)(A_KB_BYTES >> 4);
+                    const int nks = ksteps - 4 * kb;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)  // 16 bf16 = 32 bytes inside the swizzle row
+                        if (u < nks) mma_kind<FP8>(d, ad + 2 * u, bd + 2 * u, (kb | u) ? 1u : 0u);
                     mma_commit(&bars->b_empty[s]);
+                    if (++s == stages) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
                 if (!go) break;
                 mma_commit(&bars->t_full[buf]);
             }
         }
-        if (!KLOOP && lane == 0) {
+    }
+    if (!KLOOP && warp > EPI_WARPS) {
+        // ------------------------------------------------------------------ MMA issuers, resident query tile
+        // Each of the two warps owns one accumulator and every other visit: while one has its MMAs in the
+        // tensor pipe the other waits for its tile and its accumulator. (The 8 MMAs of a tile at d = 40 take
+        // 1,025 cycles, but a visit costs its issuing thread ~700 more of waits, fences and commits: with one
+        // thread for both accumulators the pipe idled meanwhile, 157 against 141 ms at 2,000,000 × 40.) A wait
+        // by phase parity may trail the barrier by one phase at most, so a stage has to stay with one warp:
+        // two warps need a ring of an even number of tiles, else warp 5 issues every visit.
+        const int mw = warp - (EPI_WARPS + 1);
+        if (lane == 0 && mw < mma_warps) {
             bool ok = mbar_wait(&bars->a_full, 0, timeout_flag, true);
             tc_fence_after();
-            const uint32_t a_base = smem_u32(a_tile);
-            for (int t = 0; ok && t < ntiles; ++t) {
-                const int s = t % stages, buf = t & 1;
-                const uint32_t ph = (uint32_t)(t / stages) & 1u, bph = (uint32_t)(t >> 1) & 1u;
-                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, true)) break;
-                if (!mbar_wait(&bars->b_full[s], ph, timeout_flag, true)) break;
-                tc_fence_after();
-                if (*reinterpret_cast<volatile int*>(&bars->stop_tile) == t) {
-                    mbar_arrive(&bars->t_full[buf]);  // pass the stop on to the epilogue warps
-                    break;
+            // The descriptors of the first K step; a step is 32 bytes further (2 in their 16-byte units).
+            const uint64_t a_desc = sw128_desc(smem_u32(a_tile)), b_desc = sw128_desc(smem_u32(b_tiles));
+            volatile int* stop = &bars->stop_tile;
+            long long budget = 0;
+            int s = 0;
+            uint32_t ph = 0;
+            auto advance = [&](int k) {
+                s += k;
+                while (s >= stages) {
+                    s -= stages;
+                    ph ^= 1u;
                 }
-                const uint32_t b_base = smem_u32(b_tiles + (size_t)s * b_bytes);
+            };
+            if (mw) advance(nkb_b);
+            for (int v = mw; ok && v < nvisits; v += mma_warps) {
+                const int buf = v & 1;
                 const uint32_t d = tmem + (uint32_t)(buf * BLOCK_N);
-                // Two chains into one accumulator: steps [0, k1s) pair A's [hi | hi] with B's [hi | lo];
-                // steps [k1s, ksteps) pair A's [lo] with B's leading [hi] (A's zero padding cancels
-                // whatever of B's lo those steps also cover). 16 bf16 = 32 bytes inside a swizzle row.
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const int kb = ks < k1s ? ks : ks - k1s;
-                    const uint64_t ad = sw128_desc(a_base + (uint32_t)(ks >> 2) * A_KB_BYTES + (uint32_t)((ks & 3) * 32));
-                    const uint64_t bd = sw128_desc(b_base + (uint32_t)(kb >> 2) * B_KB_BYTES + (uint32_t)((kb & 3) * 32));
-                    mma_kind<FP8>(d, ad, bd, ks > 0 ? 1u : 0u);
+                // One chain over the K blocks of a 3d-wide tile; compact operands (one K block): two chains
+                // into one accumulator, steps [0, k1s) pairing A's [hi | hi] with B's [hi | lo] and steps
+                // [k1s, ksteps) A's [lo] with B's leading [hi] (A's zero padding cancels whatever of B's lo
+                // those steps also cover). 16 bf16 = 32 bytes inside a swizzle row.
+                for (int kb = 0; kb < nkb_b; ++kb) {
+                    // (a stop at an earlier visit, the other warp's, leaves this one's tile unloaded)
+                    while (ok && !mbar_try_wait(&bars->b_full[s], ph)) {
+                        if (kb == 0 && *stop < v) ok = false;
+                        else if (kb == 0 && *stop == v) break;
+                        else if (!wait_budget(timeout_flag, budget)) ok = false;
+                    }
+                    if (!ok) break;
+                    // (the accumulator last: it is what the visit waits for, and its MMAs start at once)
+                    if (kb == 0 && !mbar_wait(&bars->t_empty[buf], ((uint32_t)(v >> 1) & 1u) ^ 1u, timeout_flag, false)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (kb == 0 && *stop == v) {
+                        mbar_arrive(&bars->t_full[buf]);  // pass the stop on to the epilogue warps
+                        ok = false;
+                        break;
+                    }
+                    const uint64_t bd = b_desc + (uint64_t)(s * (B_KB_BYTES >> 4));
+                    const int ks1 = nkb_b == 1 ? ksteps : min(ksteps, 4 * kb + 4);
+#pragma unroll 1
+                    for (int ks = 4 * kb; ks < ks1; ++ks) {
+                        const uint64_t ad = a_desc + (uint64_t)((ks >> 2) * (A_KB_BYTES >> 4) + (ks & 3) * 2);
+                        mma_kind<FP8>(d, ad, bd + (uint64_t)(2 * (ks < k1s ? ks - 4 * kb : ks - k1s)), ks > 0 ? 1u : 0u);
+                    }
+                    mma_commit(&bars->b_empty[s]);
+                    advance(1);
                 }
-                mma_commit(&bars->b_empty[s]);
+                if (!ok) break;
                 mma_commit(&bars->t_full[buf]);
+                if (mma_warps == 2) advance(nkb_b);  // the other warp's visit
             }
         }
-    } else {
+    }
+    if (warp < EPI_WARPS) {
         // ------------------------------------------------------------------ epilogue (warps 0-3)
         const int qbase = warp * 32;
         const int qi = qbase + lane;  // TMEM lane = query row within the block
@@ -621,18 +727,54 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         int cnt = 0;
         const uint32_t lane_addr = tmem + ((uint32_t)qbase << 16);
         uint32_t ra[64], rb[64];
-        int cnt_m = 0;  // cnt and tau round-trip through these when the rare path runs
-        float tau_m = tau;
-        for (int t = 0; t < ntiles; ++t) {
-            const int buf = t & 1;
-            const uint32_t bph = (uint32_t)(t >> 1) & 1u;
+        const int limit = cap + (BCAP - 8 - cap) * 2 / 3;  // a buffer above it is cut
+        if (P > 0)
+            for (int e = 0; e < BCAP; ++e) B_s[e * BSTRIDE + qi] = -CUDART_INF_F;
+        Entry next = tile_entry(0);
+        for (int v = 0; v < nvisits; ++v) {
+            const int t = v < P ? v : v - P, buf = v & 1;
+            const Entry en = next;
+            next = tile_entry(v + 1 < P ? v + 1 : v + 1 - P);
+            const uint32_t bph = (uint32_t)(v >> 1) & 1u;
             if (!mbar_wait(&bars->t_full[buf], bph, timeout_flag, false)) break;
             tc_fence_after();
-            if (*reinterpret_cast<volatile int*>(&bars->stop_tile) == t) break;
+            if (*reinterpret_cast<volatile int*>(&bars->stop_tile) == v) break;
             int c0, c1;
-            const bool two = tile_cols(t, c0, c1);  // false: the tile's second half has no list entry
+            const bool two = tile_cols(t, en, c0, c1);  // false: the tile's second half has no list entry
             const uint32_t tb = lane_addr + (uint32_t)(buf * BLOCK_N);
-            if (t == 0) {
+            if (!KLOOP && v < P) {
+                // The probe: the maxima of the tile's 64-column slices (cap ≤ 32) or 32-column ones into
+                // the still unused buffer, one slot per slice of 16 tiles (a further 16 tiles share the
+                // slots, and 32 tiles are probed). The (cap + 1)-th largest slot is reached by cap + 1 columns, one of them perhaps
+                // the query's own, so no other column below it can be among the query's best cap. (Cut
+                // from 512 columns instead, the threshold lets cap·ln(16) more columns a row through.)
+                constexpr int GROUPS = BCAP / 16;  // per tile
+                for (int g = 0; g < (two ? GROUPS : GROUPS / 2); ++g) {
+                    float top;
+                    if constexpr (GROUPS == 4) {
+                        uint32_t mx;
+                        tmem_ld64_max(tb + (uint32_t)(64 * g), ra, mx);
+                        tmem_wait2(ra, rb, mx, mx);
+                        top = __uint_as_float(mx);
+                    } else {
+                        top = tmem_max32(tb + (uint32_t)(32 * g));
+                    }
+                    float* slot = &B_s[((v % 16) * GROUPS + g) * BSTRIDE + qi];
+                    *slot = fmaxf(*slot, top);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->t_empty[buf]);
+                if (v == P - 1) {
+                    for (int L = 0; L < 32; ++L) {
+                        const float T = flush_one<SL>(B_s, B_i, qbase + L, BCAP, min(cap + 1, BCAP - 1), lane, 0.0f);
+                        if (lane == L && T > -CUDART_INF_F) tau = nextafterf(T, -CUDART_INF_F);
+                    }
+                    __syncwarp();
+                }
+                continue;
+            }
+            if (t == 0 && P == 0) {
                 // A starting threshold from the first tiles: the cap-th largest of their column-group
                 // maxima (64 groups of 8 columns over tiles 0 and 1, 32 over tile 0 alone, or 64 of 4
                 // when cap > 32) is reached by cap distinct columns, so no other column below it can
@@ -647,7 +789,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     tc_fence_after();
                     // (no stop can fall on tile 1: the warps' floors are still −inf when it is issued)
                     int d0, d1;
-                    const bool two1 = tile_cols(1, d0, d1);
+                    const bool two1 = tile_cols(1, next, d0, d1);
                     float gmax[64];
 #pragma unroll
                     for (int h = 0; h < 8; ++h) {
@@ -685,46 +827,36 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     tau = nextafterf(kth_of<64>(gmax, cap), -CUDART_INF_F);
                 }
             }
-            // Four 64-column slices (two per half), as a two-step software pipeline: the next
-            // slice's TMEM load is in flight while one is scanned. A slice costs a max tree and a warp
-            // OR; only the 8-column groups some lane needs are re-read and scanned.
-            tmem_ld64(tb, ra);
-            tmem_wait(ra);
+            // Four 64-column slices, two (a half) at a time, each with its row maximum from the load
+            // itself: a slice costs one compare and a share of the warp's vote; only a slice that some
+            // lane needs is looked at further. (With the slices' maxima taken by 3-input
+            // max trees the epilogue warps were the kernel's bound: 1,322 of 2,546 cycles a tile.)
+            bool any_hit = t == 0;
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
+                if (h == 1 && !two) break;
                 const int ch = h ? c1 : c0;  // the half's first column
-                tmem_ld64(tb + (uint32_t)(HALF_N * h + 64), rb);
-                unsigned gm = slice_mask(ra, tau);
-                if (gm) {
-                    cnt_m = cnt;
-                    tau_m = tau;
-                    admit_groups<SL>(gm, tb + (uint32_t)(HALF_N * h), ch, n, q, qi, qbase, lane, cap, q_lo, B_s, B_i,
-                                     &cnt_m, &tau_m);
-                    cnt = cnt_m;
-                    tau = tau_m;
+                const uint32_t th = tb + (uint32_t)(HALF_N * h);
+                uint32_t ma, mb;
+                tmem_ld64_max(th, ra, ma);
+                tmem_ld64_max(th + 64u, rb, mb);
+                tmem_wait2(ra, rb, ma, mb);
+                if (h == 1 || !two) {
+                    // every TMEM read of this accumulator is complete: hand it back to its MMA warp before
+                    // the admissions, which work on registers
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->t_empty[buf]);
                 }
-                tmem_wait(rb);
-                if (h == 0 && two) tmem_ld64(tb + HALF_N, ra);
-                gm = slice_mask(rb, tau);
-                if (gm) {
-                    cnt_m = cnt;
-                    tau_m = tau;
-                    admit_groups<SL>(gm, tb + (uint32_t)(HALF_N * h + 64), ch + 64, n, q, qi, qbase, lane, cap, q_lo,
-                                     B_s, B_i, &cnt_m, &tau_m);
-                    cnt = cnt_m;
-                    tau = tau_m;
-                }
-                if (h == 0) {
-                    if (!two) break;
-                    tmem_wait(ra);
-                }
+                unsigned hit = (__uint_as_float(ma) > tau ? 1u : 0u) | (__uint_as_float(mb) > tau ? 2u : 0u);
+                hit = __reduce_or_sync(COSTAL_FULL_MASK, hit);
+                if (hit == 0) continue;
+                any_hit = true;
+                if (hit & 1u) admit_slice<SL>(ra, ch, n, q, qi, qbase, lane, cap, q_lo, limit, B_s, B_i, cnt, tau);
+                if (hit & 2u) admit_slice<SL>(rb, ch + 64, n, q, qi, qbase, lane, cap, q_lo, limit, B_s, B_i, cnt, tau);
             }
-            // every TMEM read of this accumulator is complete: hand it back to the MMA warp
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->t_empty[buf]);
             // the warp's floor min(τ − E) for the TMA warp's stop test (signed-int order of the f32)
-            if (list_ub) {
+            if (list_ub && any_hit) {
                 const float f = q < n ? __fsub_rd(tau * OSCALE, row_e) : CUDART_INF_F;
                 int key = __float_as_int(f);
                 key = __reduce_min_sync(COSTAL_FULL_MASK, key >= 0 ? key : key ^ 0x7fffffff);
@@ -767,6 +899,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // issues the MMAs into two 128-column accumulators, warps 0-3 reduce and write M[Q][·].
 constexpr int RM_N = 128;                       // query rows per tile (the MMA's N)
 constexpr int RM_KB_BYTES = 128 * 128;          // one 128-byte K block of 128 operand rows
+constexpr int RM_THREADS = (EPI_WARPS + 2) * 32;  // 4 epilogue warps, 1 TMA warp, 1 MMA warp
 constexpr uint32_t RM_TMEM_COLS = 2 * RM_N;     // two accumulators
 constexpr uint32_t IDESC_RM = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(RM_N >> 3) << 17) |
                               ((uint32_t)(BLOCK_M >> 4) << 24);
@@ -788,7 +921,7 @@ __device__ __forceinline__ void mma_rm(uint32_t tmem_d, uint64_t adesc, uint64_t
         : "memory");
 }
 
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(RM_THREADS, 1)
     k_block_rowmax(const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_q, int n, int ncb,
                    int nkb_c, int nkb_q, int ksteps, int k1s, int stages, float* __restrict__ rowmax,
                    unsigned long long* __restrict__ timeout_flag) {
@@ -876,30 +1009,24 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             if (!mbar_wait(&bars->t_full[buf], bph, timeout_flag, false)) break;
             tc_fence_after();
             const uint32_t tb = lane_addr + (uint32_t)(buf * RM_N);
-            tmem_ld64(tb, ra);
-            tmem_ld64(tb + 64, rb);
-            tmem_wait(ra);
-            tmem_wait(rb);
+            uint32_t ma, mb;
+            tmem_ld64_max(tb, ra, ma);
+            tmem_ld64_max(tb + 64, rb, mb);
+            tmem_wait2(ra, rb, ma, mb);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->t_empty[buf]);
+            float top = fmaxf(__uint_as_float(ma), __uint_as_float(mb));
             if (nv < RM_N) {  // the last block: rows past n do not count
+                top = -CUDART_INF_F;
 #pragma unroll
                 for (int j = 0; j < 64; ++j) {
-                    if (j >= nv) ra[j] = __float_as_uint(-CUDART_INF_F);
-                    if (64 + j >= nv) rb[j] = __float_as_uint(-CUDART_INF_F);
+                    if (j < nv) top = fmaxf(top, __uint_as_float(ra[j]));
+                    if (64 + j < nv) top = fmaxf(top, __uint_as_float(rb[j]));
                 }
             }
-            float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, m2 = -CUDART_INF_F, m3 = -CUDART_INF_F;
-#pragma unroll
-            for (int j = 0; j < 64; j += 4) {
-                m0 = max3f(m0, __uint_as_float(ra[j]), __uint_as_float(rb[j]));
-                m1 = max3f(m1, __uint_as_float(ra[j + 1]), __uint_as_float(rb[j + 1]));
-                m2 = max3f(m2, __uint_as_float(ra[j + 2]), __uint_as_float(rb[j + 2]));
-                m3 = max3f(m3, __uint_as_float(ra[j + 3]), __uint_as_float(rb[j + 3]));
-            }
             const int c = t * BLOCK_M + warp * 32 + lane;
-            if (c < ncb) rowmax[(size_t)Q * ncb + c] = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+            if (c < ncb) rowmax[(size_t)Q * ncb + c] = top;
         }
     }
     tc_fence_before();
@@ -1202,7 +1329,7 @@ static size_t fixed_smem(const Shape& sh, int cap) {
     return 1024 + (sh.resident ? (size_t)sh.nkb_a * A_KB_BYTES : 0) + (size_t)(BLOCK_M + 1) * bcap * 8 + sizeof(Barriers);
 }
 static size_t stage_smem(const Shape& sh) {
-    return sh.resident ? (size_t)sh.nkb_b * B_KB_BYTES : (size_t)(A_KB_BYTES + B_KB_BYTES);
+    return sh.resident ? (size_t)B_KB_BYTES : (size_t)(A_KB_BYTES + B_KB_BYTES);
 }
 
 bool supported(int d, int cap) {
@@ -1321,6 +1448,9 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
     const size_t fixed = fixed_smem(sh, cap), per = stage_smem(sh);
     int stages = 4;
     while (stages > 1 && fixed + (size_t)stages * per > 227 * 1024) --stages;
+    // (resident query tile) an even number of tiles in the ring, if two fit: one MMA warp per accumulator
+    const int ring = sh.resident ? stages / sh.nkb_b : 0, mma_warps = ring >= 2 ? 2 : 1;
+    if (ring >= 2) stages = (ring & ~1) * sh.nkb_b;
     const size_t smem = fixed + (size_t)stages * per;
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
     const int qblocks = (plan.n + BLOCK_M - 1) / BLOCK_M;
@@ -1335,8 +1465,13 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
     if (plan.fp8 && sh.resident) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
+    const int tiles = plan.np / BLOCK_N;
+    // 32 probes (8,192 of the nearest columns) where a list is long enough: 16 / 32 / 64 probes measured
+    // 19.6 / 19.5 / 19.8 ms at 600,000 × 40 (20.2 without), 145.7 / 144.1 / 145.1 at 2,000,000 × 40 (149.7),
+    // but 0.50 against 0.35 ms at 20,000 × 32 (79 tiles).
+    const int probes = lists && sh.resident && tiles >= 128 ? 32 : 0;
     kern<<<qb1 - qb0, NTHREADS, smem, st>>>(ma, mb, mbw, plan.n, plan.np, sh.nkb_a, sh.nkb_b, sh.ksteps, sh.k1s, stages,
-                                            cap, plan.perm, lists, lists ? list_ub : nullptr, counts, ncb, plan.row_eps, cand_idx, cand_score, tau, stopped_total, timeout_flag, qb0);
+                                            cap, probes, mma_warps, plan.perm, lists, lists ? list_ub : nullptr, counts, ncb, plan.row_eps, cand_idx, cand_score, tau, stopped_total, timeout_flag, qb0);
     note_launch();
     return cudaGetLastError();
 }
@@ -1430,7 +1565,7 @@ cudaError_t launch_rowmax(const Plan& plan, const float* centers_fT, int ncb, vo
     if ((e = cudaFuncSetAttribute(k_block_rowmax, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return e;
     const int nqb = (plan.n + RM_N - 1) / RM_N;
-    k_block_rowmax<<<nqb, NTHREADS, smem, st>>>(mc, mq, plan.n, ncb, nkb_c, nkb_q, sh.ksteps, sh.k1s, stages, rowmax,
+    k_block_rowmax<<<nqb, RM_THREADS, smem, st>>>(mc, mq, plan.n, ncb, nkb_c, nkb_q, sh.ksteps, sh.k1s, stages, rowmax,
                                                 timeout_flag);
     note_launch();
     *delta = L.delta;

@@ -36,15 +36,28 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // launch returns at once and the kernel drains in microseconds.
 // Roles that are not the bottleneck (TMA, MMA issue) sleep between polls so that they do not take
 // issue slots from the epilogue warps that share their schedulers.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long* timeout_flag,
-                                          bool sleep) {
-    for (long long i = 0; i < WAIT_LIMIT; ++i) {
+// One more poll of a wait (polls counts them): false once the wait has to give up.
+__device__ __forceinline__ bool wait_budget(unsigned long long* timeout_flag, long long& polls) {
+    if ((++polls & 1023) == 0) {
+        if (*reinterpret_cast<volatile unsigned long long*>(timeout_flag)) return false;
+        if (polls >= WAIT_LIMIT) {
+            atomicExch(timeout_flag, 1ull);
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ bool mbar_wait_long(uint64_t* bar, uint32_t parity, unsigned long long* timeout_flag, bool sleep) {
+    long long polls = 0;
+    while (wait_budget(timeout_flag, polls)) {
         if (mbar_try_wait(bar, parity)) return true;
         if (sleep) __nanosleep(64);
-        if ((i & 1023) == 1023 && *reinterpret_cast<volatile unsigned long long*>(timeout_flag)) return false;
     }
-    atomicExch(timeout_flag, 1ull);
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long* timeout_flag,
+                                          bool sleep) {
+    return mbar_try_wait(bar, parity) || mbar_wait_long(bar, parity, timeout_flag, sleep);
 }
 
 // ---- TMA ---------------------------------------------------------------------------------------
