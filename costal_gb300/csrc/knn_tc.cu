@@ -187,7 +187,12 @@ struct __align__(8) Barriers {
     float warp_floor[4];   // per epilogue warp: min over its rows of τ − E (never decreases)
 };
 
-// Per-query candidate buffer: BCAP = 2·LCAP entries in shared memory, [entry][query] with a row
+// Entries of a query's buffer: 64 for cap ≤ 32, 128 for cap ≤ 64, and 80 for the split-FP8 kind (cap ≤ 64),
+// whose 48 KB stages then are three instead of two.
+__host__ __device__ constexpr int tc_bcap(int slots, bool fp8) { return fp8 && slots == 2 ? 80 : 64 * slots; }
+__host__ __device__ constexpr int tc_slots(int slots, bool fp8) { return (tc_bcap(slots, fp8) + 31) / 32; }
+
+// Per-query candidate buffer: BCAP entries in shared memory, [entry][query] with a row
 // stride of BLOCK_M + 1 words (appends of 32 lanes and the warp's reads of one query are both free
 // of bank conflicts). Survivors are appended with predicated stores; when a buffer could overflow,
 // the warp selects its best `cap` cooperatively (radix select, no sort) and raises τ to the cap-th
@@ -392,13 +397,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 uint32_t* __restrict__ cand_idx, float* __restrict__ cand_score, float* __restrict__ tau_out,
                 unsigned long long* __restrict__ stopped_total, unsigned long long* __restrict__ timeout_flag,
                 int qb0) {
-    constexpr int SL = 2 * SLOTS;  // buffer slots per lane in a flush: BCAP = 2·LCAP entries
+    constexpr int SL = tc_slots(SLOTS, FP8);  // buffer slots per lane in a flush
     // The split-FP8 kind computes on the rows scaled by 2^8, so its accumulators hold 2^16 × the
     // coarse score: thresholds and admissions stay in those units, the lists and floors are scaled
     // back exactly.
     constexpr float OSCALE = FP8 ? 0x1p-16f : 1.0f;
     constexpr int KBE = FP8 ? 128 : KB;  // elements in one 128-byte K block (the TMA x coordinate step)
-    constexpr int BCAP = 32 * SL;
+    constexpr int BCAP = tc_bcap(SLOTS, FP8);
     extern __shared__ unsigned char smem_raw[];
     // 1024-byte alignment for the swizzled tiles
     const uint32_t base_u32 = smem_u32(smem_raw);
@@ -1324,8 +1329,8 @@ static Shape shape_fp8(int d) {
     return s;
 }
 
-static size_t fixed_smem(const Shape& sh, int cap) {
-    const int bcap = cap <= 32 ? 64 : 128;
+static size_t fixed_smem(const Shape& sh, int cap, bool fp8 = false) {
+    const int bcap = tc_bcap(cap <= 32 ? 1 : 2, fp8);
     return 1024 + (sh.resident ? (size_t)sh.nkb_a * A_KB_BYTES : 0) + (size_t)(BLOCK_M + 1) * bcap * 8 + sizeof(Barriers);
 }
 static size_t stage_smem(const Shape& sh) {
@@ -1341,7 +1346,7 @@ bool supported(int d, int cap) {
 bool supported_fp8(int d, int cap) {
     if (d < 1 || cap < 1 || cap > 64 || 3 * d <= 128) return false;
     const Shape sh = shape_fp8(d);
-    return fixed_smem(sh, cap) + stage_smem(sh) <= 227 * 1024;
+    return fixed_smem(sh, cap, true) + stage_smem(sh) <= 227 * 1024;
 }
 
 size_t workspace_bytes(int n, int d, bool fp8) {
@@ -1445,7 +1450,7 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
         !make_map(&mbw, plan.ops_b, plan.kpb, plan.np, BLOCK_N, plan.fp8))
         return cudaErrorInvalidValue;
     const Shape sh = plan.fp8 ? shape_fp8(plan.d) : shape_of(plan.d);
-    const size_t fixed = fixed_smem(sh, cap), per = stage_smem(sh);
+    const size_t fixed = fixed_smem(sh, cap, plan.fp8), per = stage_smem(sh);
     int stages = 4;
     while (stages > 1 && fixed + (size_t)stages * per > 227 * 1024) --stages;
     // (resident query tile) an even number of tiles in the ring, if two fit: one MMA warp per accumulator
