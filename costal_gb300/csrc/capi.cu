@@ -219,6 +219,11 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 // 40,000 × 20 2.5 / 4.4, 80,000 × 32 6.5 / 12.6, 161,443 × 32 14.9 / 39.8).
 bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 16384; }
 
+// The tensor-core pass visits its tiles in row order below this many rows: the order stage costs more than
+// the lists and the earlier thresholds save (whole kNN on the device, row order / locality order:
+// 5,003 × 17 0.21 / 0.51 ms, 16,000 × 32 0.41 / 0.72, 24,000 × 15 0.80 / 0.96).
+constexpr int TC_ORDER_ROWS = 24576;
+
 // The FP32 pass by lists: the working order, the column lists and the rows' transposed copy in that order
 // (c.xsW) into the job. Cosine selection, and Tanimoto selection of enough rows, use the cells, bounds
 // and lists of the tensor-core path (the per-row bounds come from its split operands, with their
@@ -352,8 +357,11 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
     const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
                             (tanimoto ? prune::supported(d) : !tc_backend && fp32_lists_pay(n, d));
+    // the tensor-core pass in the locality order, with lists (a shard is a range of that order)
+    const bool tc_ordered = tc_backend && !tanimoto && !scan_all && prune::supported(d) &&
+                            (n >= TC_ORDER_ROWS || shard || (o.learned_prune && c.mlp.ready && c.mlp.d == d && c.mlp.k == k));
     float* xsR = nullptr;
-    if (fp32_lists || (tc_backend && !tanimoto && !scan_all && prune::supported(d))) {
+    if (fp32_lists || tc_ordered) {
         CK(ensure(c.xsR, (size_t)n * d * 4));
         xsR = c.xsR.as<float>();
     }
@@ -424,7 +432,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             // Locality order (k-means cells) and per-query-block column lists, nearest blocks first;
             // with a learned threshold, blocks whose bound is below it are skipped. Deep rows (the
             // pruning geometry covers d ≤ 64) keep the input order and visit every column block.
-            const bool ordered = prune::supported(d);
+            const bool ordered = tc_ordered;
             prune::Plan pp{};
             bool learned = false;
             if (ordered) {
