@@ -47,17 +47,22 @@ __device__ __forceinline__ double dot64_step(double s, float a, float b) {
     return __fma_rn(f64_of(a), f64_of(b), s);
 }
 
+// ±0.0, told by its bits: a comparison would take the FP64 pipe.
+__device__ __forceinline__ bool is_zero64(double v) {
+    return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0;
+}
+
 // knn.rs:301-312 `cos64`: 0 for a zero row, dot / (n_i·n_j), −0 → +0.
 __device__ __forceinline__ double cos64(double dot, double ni, double nj) {
-    if (ni == 0.0 || nj == 0.0) return 0.0;
+    if (is_zero64(ni) || is_zero64(nj)) return 0.0;
     double c = __ddiv_rn(dot, __dmul_rn(ni, nj));
-    return c == 0.0 ? 0.0 : c;
+    return is_zero64(c) ? 0.0 : c;
 }
 
 // weight.rs:30-37 `tani_from_cos`: d = a·b·cos; 0 when d == 0, else d / (a² + b² − d).
 __device__ __forceinline__ double tani_from_cos(double a, double b, double c) {
     double d = __dmul_rn(__dmul_rn(a, b), c);
-    if (d == 0.0) return 0.0;
+    if (is_zero64(d)) return 0.0;
     double den = __dsub_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), d);
     return __ddiv_rn(d, den);
 }

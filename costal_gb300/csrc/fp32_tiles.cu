@@ -626,7 +626,7 @@ static int segments(int nq, int tiles, int dp, int slots) {
     const double start = 1.0 + 64.0 / dp;
     int best = 1;
     double best_t = 1e300;
-    for (int s = 1; s <= std::min(64, tiles); ++s) {
+    for (int s = 1; s <= std::min(256, tiles); ++s) {
         const int tps = (tiles + s - 1) / s;
         if ((tiles + tps - 1) / tps != s) continue;  // an empty segment
         const double waves = (double)(((long long)blocks * s + slots - 1) / slots);

@@ -202,14 +202,21 @@ __device__ __forceinline__ uint32_t warp_kth_key(const uint32_t (&key)[SLOTS], i
 //     a candidate whose coarse score is below c_k − 2E scores below s_k exactly and can neither enter
 //     the top-k nor change s_k. Only the others are rescored (cosine selection; E the row's coarse
 //     error bound); they are packed into one list for the CTA.
+// (½) Deep rows: one warp per row takes each packed candidate's cosine in f32 over the normalised rows
+//     (lanes over the dimensions, within δ = (d/32 + 22)·2⁻²³ of the exact one: a lane's chain of at most
+//     d/32 + 4 FMAs and five lane sums, 3 roundings for each normalised factor, Cauchy–Schwarz with unit
+//     rows, and a factor two) and drops by it what (0) could not by the coarse score: c'_k − 2δ in place
+//     of c_k − 2E. The split-FP8 kind's E of ~0.007 keeps ~60 candidates a row, δ the top k and a few: the
+//     f64 dots of 100,000 × 2,000 rows fall from 33 to 14 ms with this pass.
 // (1) Every thread rescores entries of that list — all lanes of a warp on real work, since the f64
 //     dot products are the kernel's cost on the GB300's narrow FP64 pipe — into shared memory.
-// (2) One warp per row sorts its cap results (skipped and empty slots as −∞), certifies and writes
-//     the row.
+// (2) One warp per row sorts its cap results (skipped and empty slots as −∞) and certifies; then all
+//     threads write the rows and their weights, 8·k entries packed (a warp instruction of the FP64 pipe
+//     costs the same with 10 lanes as with 32).
 constexpr int RS_ROWS = 8;
 constexpr int RS_MAXCAP = 128;
 
-template <int SLOTS>
+template <int SLOTS, bool DEEP>
 __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x, int n, int d, int k, int cap, int lstride,
               const uint32_t* __restrict__ cand_idx, const float* __restrict__ cand_score,
               const float* __restrict__ tau, const double* __restrict__ norms, const double* __restrict__ row_eps,
@@ -221,7 +228,8 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
     __shared__ double sc_s[RS_ROWS * RS_MAXCAP], cs_s[RS_ROWS * RS_MAXCAP];
     __shared__ uint32_t id_s[RS_ROWS * RS_MAXCAP];
     __shared__ uint16_t work_s[RS_ROWS * RS_MAXCAP];  // packed (row, slot) entries to rescore
-    __shared__ int row_s[RS_ROWS], cnt_s[RS_ROWS];
+    __shared__ float r_s[DEEP ? RS_ROWS * RS_MAXCAP : 1];
+    __shared__ int row_s[RS_ROWS], cnt_s[RS_ROWS], ok_s[RS_ROWS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nrows = rlist ? (int)*rcount : n;
     const int w0 = g * RS_ROWS;
@@ -245,12 +253,12 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
             }
             valid += __popc(__ballot_sync(COSTAL_FULL_MASK, key[s] != 0));
         }
-        double thr = -CUDART_INF;
+        float thr = -CUDART_INF_F;  // (in f32, rounded down: the FP64 pipe is the kernel's bound)
         if (select == 0 && valid >= k) {
             const uint32_t h = warp_kth_key<SLOTS>(key, k);
             const float ck = __uint_as_float((h & 0x80000000u) ? (h & 0x7fffffffu) : ~h);
-            const double e = row_eps ? row_eps[i] : eps;
-            thr = __dsub_rd((double)ck, __dadd_ru(e, e));
+            const float e = __double2float_ru(row_eps ? row_eps[i] : eps);
+            thr = __fsub_rd(ck, __fadd_ru(e, e));
         }
         int n_keep = 0;
 #pragma unroll
@@ -259,7 +267,7 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
             bool kp = false;
             if (key[s] != 0) {
                 const float cf = __uint_as_float((key[s] & 0x80000000u) ? (key[s] & 0x7fffffffu) : ~key[s]);
-                kp = !((double)cf < thr);
+                kp = !(cf < thr);
             }
             keep[s] = __ballot_sync(COSTAL_FULL_MASK, kp);
             if (!kp && p < cap) {
@@ -290,9 +298,107 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
         }
     }
     __syncthreads();
-    // phase 1: the f64 rescoring of the packed entries
     const bool vec4 = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    double err = 0.0, ratio = 0.0;
+    // phase ½: the packed candidates' f32 cosines; fewer entries packed
+    if (DEEP && select == 0) {
+        if (warp < nr) {
+            const int i = row_s[warp], lo = base, hi = base + cnt_s[warp];
+            const float nf = (float)norms[i];
+            const float inv_i = __fdiv_rn(1.0f, nf);
+            const bool row_ok = nf > 1e-15f && nf < 1e15f;
+            const float* xi = x + (size_t)i * d;
+            // (few more than k left by the coarse score: the f64 dots are cheaper than the pass)
+            const bool worth = hi - lo > k + k / 4;
+            for (int w = lo; worth && w < hi; ++w) {
+                const int p = work_s[w] & (RS_MAXCAP - 1);
+                const uint32_t j = cand_idx[(size_t)i * lstride + p];
+                const float mf = (float)norms[j];
+                float s = CUDART_NAN_F;  // (a norm out of range: no estimate, the candidate stays)
+                if (row_ok && mf > 1e-15f && mf < 1e15f) {
+                    const float inv_j = __fdiv_rn(1.0f, mf);
+                    const float* xj = x + (size_t)j * d;
+                    s = 0.0f;
+                    if (vec4) {
+#pragma unroll 4
+                        for (int t = 4 * lane; t < d; t += 128) {
+                            const float4 a = __ldg(reinterpret_cast<const float4*>(xi + t));
+                            const float4 b = __ldg(reinterpret_cast<const float4*>(xj + t));
+                            s = fmaf(a.x * inv_i, b.x * inv_j, s);
+                            s = fmaf(a.y * inv_i, b.y * inv_j, s);
+                            s = fmaf(a.z * inv_i, b.z * inv_j, s);
+                            s = fmaf(a.w * inv_i, b.w * inv_j, s);
+                        }
+                    } else {
+#pragma unroll 4
+                        for (int t = lane; t < d; t += 32) s = fmaf(__ldg(xi + t) * inv_i, __ldg(xj + t) * inv_j, s);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(COSTAL_FULL_MASK, s, o);
+                }
+                if (lane == 0) r_s[warp * RS_MAXCAP + p] = s;
+            }
+            __syncwarp();
+            uint32_t key[SLOTS];
+            int known = 0;
+#pragma unroll
+            for (int s = 0; s < SLOTS; ++s) {
+                const int p = s * 32 + lane;
+                key[s] = 0;  // no estimate, or not packed
+                if (worth && (keep[s] >> lane & 1u)) {
+                    const uint32_t u = __float_as_uint(r_s[warp * RS_MAXCAP + p]);
+                    if ((u & 0x7fffffffu) < 0x7f800000u) key[s] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+                }
+                known += __popc(__ballot_sync(COSTAL_FULL_MASK, key[s] != 0));
+            }
+            if (known >= k) {
+                const uint32_t h = warp_kth_key<SLOTS>(key, k);
+                const float ck = __uint_as_float((h & 0x80000000u) ? (h & 0x7fffffffu) : ~h);
+                const float delta = (float)(d / 32 + 22) * 0x1p-23f;
+                const float thr = __fsub_rd(ck, 2.0f * delta);
+                int n_keep = 0;
+#pragma unroll
+                for (int s = 0; s < SLOTS; ++s) {
+                    const int p = s * 32 + lane;
+                    const bool was = keep[s] >> lane & 1u;
+                    bool kp = was;
+                    if (was && key[s] != 0) kp = !(r_s[warp * RS_MAXCAP + p] < thr);
+                    keep[s] = __ballot_sync(COSTAL_FULL_MASK, kp);
+                    if (was && !kp) {
+                        sc_s[warp * cap + p] = -CUDART_INF;
+                        cs_s[warp * cap + p] = 0.0;
+                        id_s[warp * cap + p] = 0xffffffffu;
+                    }
+                    n_keep += __popc(keep[s]);
+                }
+                if (lane == 0) r_s[warp * RS_MAXCAP] = __int_as_float(n_keep);
+            } else if (lane == 0) {
+                r_s[warp * RS_MAXCAP] = __int_as_float(cnt_s[warp]);
+            }
+        }
+        __syncthreads();  // every warp has read the first packing
+        if (threadIdx.x < RS_ROWS) cnt_s[threadIdx.x] = (int)threadIdx.x < nr ? __float_as_int(r_s[threadIdx.x * RS_MAXCAP]) : 0;
+        __syncthreads();
+        total = 0;
+        base = 0;
+#pragma unroll
+        for (int r = 0; r < RS_ROWS; ++r) {
+            base += r < warp ? cnt_s[r] : 0;
+            total += cnt_s[r];
+        }
+        if (warp < nr) {
+            int off = base;
+#pragma unroll
+            for (int s = 0; s < SLOTS; ++s) {
+                if (keep[s] >> lane & 1u)
+                    work_s[off + __popc(keep[s] & ((1u << lane) - 1u))] = (uint16_t)(warp * RS_MAXCAP + s * 32 + lane);
+                off += __popc(keep[s]);
+            }
+        }
+        __syncthreads();
+    }
+    // phase 1: the f64 rescoring of the packed entries
+    unsigned long long err = 0;  // (non-negative doubles order like their bits)
+    float ratio = 0.0f;          // rounded up
     for (int w = tid; w < total; w += blockDim.x) {
         const int code = work_s[w], r = code / RS_MAXCAP, p = code - r * RS_MAXCAP, e = r * cap + p;
         const int i = row_s[r];
@@ -316,71 +422,83 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
         const double c = cos64(dot, ni, nj);
         const double score = select == 0 ? c : tani_from_cos(ni, nj, c);
         const double diff = fabs((double)cand_score[(size_t)i * lstride + p] - score);
-        err = fmax(err, diff);
-        ratio = fmax(ratio, diff / (row_eps ? row_eps[i] : eps));  // against the bound the certificate used
+        const unsigned long long db = (unsigned long long)__double_as_longlong(diff);
+        err = db > err ? db : err;
+        // against the bound the certificate used
+        ratio = fmaxf(ratio, __fdiv_ru(__double2float_ru(diff), __double2float_rd(row_eps ? row_eps[i] : eps)));
         sc_s[e] = score;
         cs_s[e] = c;
         id_s[e] = j;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        err = fmax(err, __shfl_xor_sync(COSTAL_FULL_MASK, err, o));
-        ratio = fmax(ratio, __shfl_xor_sync(COSTAL_FULL_MASK, ratio, o));
+        const unsigned long long oe = __shfl_xor_sync(COSTAL_FULL_MASK, err, o);
+        err = oe > err ? oe : err;
+        ratio = fmaxf(ratio, __shfl_xor_sync(COSTAL_FULL_MASK, ratio, o));
     }
     // max_err_bits[0]: the largest |coarse − rescored|, [1]: the largest ratio of it to the row's bound
     // (non-negative doubles order like their bits). One address for the whole grid: read it first,
     // so that only a new maximum pays for the atomic.
-    if (lane == 0 && max_err_bits && err > 0.0) {
-        const unsigned long long eb = (unsigned long long)__double_as_longlong(err);
-        if (eb > *reinterpret_cast<volatile unsigned long long*>(max_err_bits)) atomicMax(max_err_bits, eb);
-        const unsigned long long rb = (unsigned long long)__double_as_longlong(ratio);
+    if (lane == 0 && max_err_bits && err > 0) {
+        if (err > *reinterpret_cast<volatile unsigned long long*>(max_err_bits)) atomicMax(max_err_bits, err);
+        const unsigned long long rb = (unsigned long long)__double_as_longlong((double)ratio);
         if (rb > *reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) atomicMax(max_err_bits + 1, rb);
     }
     __syncthreads();
-    if (warp >= nr) return;  // no barrier below
-    const int i = row_s[warp];
-    const double ni = norms[i];
-    double sc[SLOTS], cs[SLOTS];
-    uint32_t id[SLOTS];
+    if (warp < nr) {
+        const int i = row_s[warp];
+        double sc[SLOTS], cs[SLOTS];
+        uint32_t id[SLOTS];
 #pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-        const int p = s * 32 + lane;
-        const bool v = p < cap;
-        sc[s] = v ? sc_s[warp * cap + p] : -CUDART_INF;
-        cs[s] = v ? cs_s[warp * cap + p] : 0.0;
-        id[s] = v ? id_s[warp * cap + p] : 0xffffffffu;
-    }
-    warp_sort<SLOTS>(sc, cs, id, lane);
-    const double s_k = __shfl_sync(COSTAL_FULL_MASK, sc[(k - 1) >> 5], (k - 1) & 31);
-    const double e = row_eps ? row_eps[i] : eps;
-    // knn.rs:704-714: with cap == n−1 nothing was left out; otherwise exact iff s_k > τ + ε. With
-    // block pruning, every column of a skipped block scores at most row_ub: s_k must also beat it.
-    const bool ub_bad = row_ub && s_k <= row_ub[i];
-    if (ub_bad && lane == 0 && ub_fail) atomicAdd(ub_fail, 1u);
-    // fewer than k candidates kept (possible only when a coarse threshold cut the list): regather
-    const bool short_list = s_k == -CUDART_INF;
-    if ((certify && s_k <= __dadd_rn((double)tau[i], e)) || ub_bad || short_list) {
-        if (lane == 0) {
+        for (int s = 0; s < SLOTS; ++s) {
+            const int p = s * 32 + lane;
+            const bool v = p < cap;
+            sc[s] = v ? sc_s[warp * cap + p] : -CUDART_INF;
+            cs[s] = v ? cs_s[warp * cap + p] : 0.0;
+            id[s] = v ? id_s[warp * cap + p] : 0xffffffffu;
+        }
+        warp_sort<SLOTS>(sc, cs, id, lane);
+        const double s_k = __shfl_sync(COSTAL_FULL_MASK, sc[(k - 1) >> 5], (k - 1) & 31);
+        const double e = row_eps ? row_eps[i] : eps;
+        // knn.rs:704-714: with cap == n−1 nothing was left out; otherwise exact iff s_k > τ + ε. With
+        // block pruning, every column of a skipped block scores at most row_ub: s_k must also beat it.
+        const bool ub_bad = row_ub && s_k <= row_ub[i];
+        if (ub_bad && lane == 0 && ub_fail) atomicAdd(ub_fail, 1u);
+        // fewer than k candidates kept (possible only when a coarse threshold cut the list): regather
+        const bool short_list = s_k == -CUDART_INF;
+        const bool fail = (certify && s_k <= __dadd_rn((double)tau[i], e)) || ub_bad || short_list;
+        if (lane == 0) ok_s[warp] = !fail;
+        if (fail && lane == 0) {
             const unsigned slot = atomicAdd(fb_count, 1u);
             fb_rows[slot] = (uint32_t)i;
             fb_minsim[slot] = __dsub_rn(s_k, e);
         }
-        return;
-    }
+        // the row's best k back to its part of the shared arrays (read above)
 #pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-        const int p = s * 32 + lane;
-        if (p < k) {
-            out_idx[(size_t)i * k + p] = id[s];
-            out_cos[(size_t)i * k + p] = cs[s];
-            if (out_w) out_w[(size_t)i * k + p] = tani_from_cos(ni, norms[id[s]], cs[s]);
+        for (int s = 0; s < SLOTS; ++s) {
+            const int p = s * 32 + lane;
+            if (p < k) {
+                cs_s[warp * cap + p] = cs[s];
+                id_s[warp * cap + p] = id[s];
+            }
         }
+    }
+    __syncthreads();
+    for (int e = tid; e < nr * k; e += blockDim.x) {
+        const int r = e / k, p = e - r * k;
+        if (!ok_s[r]) continue;
+        const size_t o = (size_t)row_s[r] * k + p;
+        const uint32_t j = id_s[r * cap + p];
+        const double c = cs_s[r * cap + p];
+        out_idx[o] = j;
+        out_cos[o] = c;
+        if (out_w) out_w[o] = tani_from_cos(norms[row_s[r]], norms[j], c);
     }
 }
 
 // Row groups of RS_ROWS, grid-stride: one group per CTA, or (deep rows) a few CTAs per SM walking
 // many groups, so that the rows each thread streams through stay in L1.
-template <int SLOTS>
+template <int SLOTS, bool DEEP>
 __global__ void __launch_bounds__(256)
     k_rescore(const float* __restrict__ x, int n, int d, int k, int cap, int lstride,
               const uint32_t* __restrict__ cand_idx, const float* __restrict__ cand_score,
@@ -392,7 +510,7 @@ __global__ void __launch_bounds__(256)
               unsigned* __restrict__ fb_count, unsigned long long* __restrict__ max_err_bits) {
     const int nrows = rlist ? (int)*rcount : n;
     for (int g = blockIdx.x; g * RS_ROWS < nrows; g += gridDim.x) {
-        rescore_group<SLOTS>(g, x, n, d, k, cap, lstride, cand_idx, cand_score, tau, norms, row_eps, row_ub, ub_fail,
+        rescore_group<SLOTS, DEEP>(g, x, n, d, k, cap, lstride, cand_idx, cand_score, tau, norms, row_eps, row_ub, ub_fail,
                              eps, certify, select, rlist, rcount, out_idx, out_cos, out_w, fb_rows, fb_minsim, fb_count,
                              max_err_bits);
         __syncthreads();  // the group's shared arrays are free again
@@ -556,20 +674,12 @@ cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lst
     }
     const int groups = (n + RS_ROWS - 1) / RS_ROWS;
     const int blocks = d >= 256 ? std::min(groups, 3 * sms) : groups;
-#define COSTAL_RESCORE(S)                                                                                   \
-    k_rescore<S><<<blocks, 256, 0, st>>>(x, n, d, k, cap, lstride, cand_idx, cand_score, tau, norms, row_eps, \
-                                         row_ub, ub_fail, eps, certify, select, rlist, rcount, out_idx, out_cos, \
-                                         out_w, fb_rows, \
-                                         fb_minsim,                                                           \
-                                         fb_count, max_err_bits); note_launch();
-    if (slots == 1) {
-        COSTAL_RESCORE(1)
-    } else if (slots == 2) {
-        COSTAL_RESCORE(2)
-    } else {
-        COSTAL_RESCORE(4)
-    }
-#undef COSTAL_RESCORE
+    auto kern = d >= 256 ? (slots == 1 ? k_rescore<1, true> : slots == 2 ? k_rescore<2, true> : k_rescore<4, true>)
+                         : (slots == 1 ? k_rescore<1, false> : slots == 2 ? k_rescore<2, false> : k_rescore<4, false>);
+    kern<<<blocks, 256, 0, st>>>(x, n, d, k, cap, lstride, cand_idx, cand_score, tau, norms, row_eps, row_ub, ub_fail, eps,
+                                 certify, select, rlist, rcount, out_idx, out_cos, out_w, fb_rows, fb_minsim, fb_count,
+                                 max_err_bits);
+    note_launch();
     return cudaGetLastError();
 }
 

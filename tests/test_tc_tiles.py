@@ -24,3 +24,19 @@ def test_tc_pass_at_its_edges(ext, oracle, n, d, k, margin, prune):
     for a, b in zip((idx.view(np.uint32), cos, norms), want):
         np.testing.assert_array_equal(a, b)
     assert st["max_err_ratio"] < 1.0 and st["coarse_kind"] == "bf16"
+
+
+@pytest.mark.parametrize("n,d,k,matmul", [(700, 256, 15, "fp32"), (900, 259, 10, "bf16"), (600, 513, 30, "fp8"),
+                                          (500, 1000, 60, "fp32")])
+def test_deep_rescoring_drops_by_f32_cosines(ext, oracle, n, d, k, matmul):
+    """Deep rows: the candidates an f32 cosine rules out are not rescored. Rows whose norms are far out
+    of f32's comfortable range get no such estimate, zero and repeated rows stay exact."""
+    x = clustered(n, d, n + d)
+    x[: n // 4] *= np.float32(1e-18)
+    x[n // 4: n // 2] *= np.float32(1e16)
+    x[n - 40:] = x[n - 1]
+    x[[1, n // 2]] = 0.0
+    want = oracle.knn_bruteforce(x, k)
+    (idx, cos, norms), st = ext._knn_exact(x, k, matmul=matmul)
+    for a, b in zip((idx.view(np.uint32), cos, norms), want):
+        np.testing.assert_array_equal(a, b)
