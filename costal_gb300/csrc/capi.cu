@@ -231,8 +231,8 @@ constexpr int TC_ORDER_ROWS = 24576;
 // by the norm ranges alone in the norm order (knn.rs:595-644): with few rows, or where the norms are
 // spread so far that the window of a score of 0.9 leaves out more than half of all pairs (a block of
 // one cell spans its rows' whole norm range, so the cells' order cannot use the window: of 20,000 × 12
-// rows spread 8-fold in norm the norm order leaves out 45 % of the tiles, the cells' order 0.1 %;
-// of 100,003 × 15 cytometry-like rows the norm order 6 %, the cells' order 75 %).
+// rows spread 8-fold in norm the norm order leaves out 60 % of the tiles, the cells' order 0.1 %;
+// of 100,003 × 15 cytometry-like rows the norm order 6 %, the cells' order 64 %).
 void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani_norms, double eps, Fp32Job& j, cudaStream_t s) {
     Misc* dm = c.misc.as<Misc>();
     prune::Plan pp{};
@@ -273,6 +273,7 @@ void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani
     j.lists = pp.lists;
     j.list_ub = pp.list_ub;
     j.counts = pp.counts;
+    j.order = pp.order;
     j.ncb = pp.ncb;
     j.list_cb = pp.cb;
     j.eps = std::nextafterf((float)eps, INFINITY);
@@ -477,7 +478,8 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             if (nrows > 0)
                 CK(tc::launch_coarse(plan, cap, ordered ? pp.lists : nullptr,
                                      ordered && o.prune ? pp.list_ub : nullptr, ordered ? pp.counts : nullptr,
-                                     ordered ? pp.ncb : 0, ordered ? pp.cb : 0, c.cand_idx.as<uint32_t>(),
+                                     ordered && !shard ? pp.order : nullptr, ordered ? pp.ncb : 0, ordered ? pp.cb : 0,
+                                     c.cand_idx.as<uint32_t>(),
                                      c.cand_score.as<float>(),
                                      c.tau.as<float>(), &dm->blocks_stopped, &dm->timeout_flag, c.sm_count, s, qb0,
                                      qb1));

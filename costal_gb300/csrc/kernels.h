@@ -34,6 +34,7 @@ struct Fp32Job {
     const uint32_t* lists;
     const float* list_ub;
     const uint32_t* counts;
+    const uint32_t* order;  // the query blocks, longest lists first
     int ncb, list_cb;
     float eps;
     unsigned long long* stopped_total;

@@ -393,7 +393,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 int nkb, int nkb_b, int ksteps, int k1s, int stages, int cap, int probes, int mma_warps,
                 const uint32_t* __restrict__ perm,
                 const uint32_t* __restrict__ lists, const float* __restrict__ list_ub,
-                const uint32_t* __restrict__ counts, int ncb, const double* __restrict__ row_eps,
+                const uint32_t* __restrict__ counts, const uint32_t* __restrict__ order, int ncb,
+                const double* __restrict__ row_eps,
                 uint32_t* __restrict__ cand_idx, float* __restrict__ cand_score, float* __restrict__ tau_out,
                 unsigned long long* __restrict__ stopped_total, unsigned long long* __restrict__ timeout_flag,
                 int qb0) {
@@ -421,8 +422,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Rows and columns are in the working order (rows sorted by locality cell; perm maps back to the
     // original index). A CTA visits the column blocks of its list, nearest first, or all of them.
-    // CTA b takes query block qb0 + b (a launch over a contiguous range of query blocks: one shard).
-    const int qb = qb0 + (int)blockIdx.x;
+    // CTA b takes query block qb0 + b (a launch over a contiguous range of query blocks: one shard), or,
+    // over all of them, the b-th by length of its list.
+    const int qb = order ? (int)order[blockIdx.x] : qb0 + (int)blockIdx.x;
     const int q0 = qb * BLOCK_M;
     // A tile's 256 columns are two halves of HALF_N. PAIR (lists of 128-column blocks): the halves are
     // two consecutive list entries, each loaded by its own TMA box unless they are adjacent; an odd
@@ -1438,8 +1440,8 @@ cudaError_t prepare(void* ws, const float* xsT, int n, int np_x, int dp, int d, 
 }
 
 cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, const float* list_ub,
-                          const uint32_t* counts, int ncb, int list_cb, uint32_t* cand_idx, float* cand_score,
-                          float* tau, unsigned long long* stopped_total, unsigned long long* timeout_flag,
+                          const uint32_t* counts, const uint32_t* order, int ncb, int list_cb, uint32_t* cand_idx,
+                          float* cand_score, float* tau, unsigned long long* stopped_total, unsigned long long* timeout_flag,
                           int sm_count, cudaStream_t st, int qb0, int qb1) {
     (void)sm_count;
     if (lists && list_cb != HALF_N && list_cb != BLOCK_N) return cudaErrorInvalidValue;
@@ -1476,7 +1478,7 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
     // but 0.50 against 0.35 ms at 20,000 × 32 (79 tiles).
     const int probes = lists && sh.resident && tiles >= 128 ? 32 : 0;
     kern<<<qb1 - qb0, NTHREADS, smem, st>>>(ma, mb, mbw, plan.n, plan.np, sh.nkb_a, sh.nkb_b, sh.ksteps, sh.k1s, stages,
-                                            cap, probes, mma_warps, plan.perm, lists, lists ? list_ub : nullptr, counts, ncb, plan.row_eps, cand_idx, cand_score, tau, stopped_total, timeout_flag, qb0);
+                                            cap, probes, mma_warps, plan.perm, lists, lists ? list_ub : nullptr, counts, lists ? order : nullptr, ncb, plan.row_eps, cand_idx, cand_score, tau, stopped_total, timeout_flag, qb0);
     note_launch();
     return cudaGetLastError();
 }

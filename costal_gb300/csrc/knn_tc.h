@@ -39,8 +39,8 @@ cudaError_t prepare(void* ws, const float* xsT, int n, int np, int dp, int d, co
 // of its rows. [qb0, qb1) restricts the launch to those query blocks (one shard of the rows); qb1 = -1
 // means all of them.
 cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, const float* list_ub,
-                          const uint32_t* counts, int ncb, int list_cb, uint32_t* cand_idx, float* cand_score,
-                          float* tau, unsigned long long* stopped_total, unsigned long long* timeout_flag,
+                          const uint32_t* counts, const uint32_t* order, int ncb, int list_cb, uint32_t* cand_idx,
+                          float* cand_score, float* tau, unsigned long long* stopped_total, unsigned long long* timeout_flag,
                           int sm_count, cudaStream_t st, int qb0 = 0, int qb1 = -1);
 
 // Per-row block bounds for the column lists (prune.cu): for every query block Q (128 working rows)

@@ -134,9 +134,10 @@ __global__ void __launch_bounds__(128, 2) k_assign(const float* __restrict__ row
 // One CTA per centroid: the normalised sum of its rows, summed in a fixed order (deterministic): the
 // rows fall into 128 classes by (row / 4) mod 128, each class adds its rows in row order, and the 128
 // class sums are combined by a fixed pairwise tree. Warp w takes classes 4w … 4w+3 one after the
-// other (the adds wait for their rows: 32 warps a centroid hide that, 8 did not), lane t holding dimensions t and t + 32: the class's assignment words are loaded four per
-// lane at once and its matches found by ballots, so the warp's branches are uniform and a row is read
-// coalesced. An empty cluster keeps its previous centroid.
+// other (the adds wait for their rows: 32 warps a centroid hide that, 8 did not; the four classes side by
+// side were slower, 24 against 19 us at 20,000 rows), lane t holding dimensions t and t + 32: the class's
+// assignment words are loaded four per lane at once and its matches found by ballots, so the warp's
+// branches are uniform and a row is read coalesced. An empty cluster keeps its previous centroid.
 constexpr int UPD_T = 1024;
 constexpr int UPD_CLASSES = 128;
 constexpr int UPD_GROUPS = 128;  // word groups of a class: m ≤ 4 · 128 · 128 rows
@@ -294,10 +295,19 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_cell_scatter(const uint32_t
     for (int c = lane; c < K; c += 32) next[c] = start[c] + hist[(size_t)c * nch + ch];
     __syncwarp();
     const int end = min(n, (ch + 1) * CHUNK);
+    constexpr int AHEAD = 8;  // cells loaded at once: the ranks are a serial chain, their loads need not be
+    uint32_t ahead[AHEAD];
     for (int i0 = ch * CHUNK; i0 < end; i0 += 32) {
+        const int step = ((i0 - ch * CHUNK) >> 5) & (AHEAD - 1);
+        if (step == 0) {
+#pragma unroll
+            for (int a = 0; a < AHEAD; ++a) ahead[a] = i0 + 32 * a + lane < end ? cell[i0 + 32 * a + lane] : 0xffffffffu;
+        }
         const int i = i0 + lane;
         const bool live = i < end;
-        const uint32_t c = live ? cell[i] : 0xffffffffu;
+        uint32_t c = ahead[0];
+#pragma unroll
+        for (int a = 1; a < AHEAD; ++a) c = step == a ? ahead[a] : c;
         const unsigned peers = __match_any_sync(COSTAL_FULL_MASK, c);
         uint32_t base = 0;
         if (live) base = next[c];
@@ -594,17 +604,19 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
                   const float* __restrict__ tq, const float* __restrict__ rowmax, const float* __restrict__ rm_delta,
                   const float2* __restrict__ qnorm, const float2* __restrict__ cnorm, int use_cos,
                   uint32_t* __restrict__ lists, float* __restrict__ list_ub, uint32_t* __restrict__ counts,
-                  float* __restrict__ ub_skip, unsigned long long* __restrict__ skipped_total) {
+                  uint32_t* __restrict__ weight, float* __restrict__ ub_skip,
+                  unsigned long long* __restrict__ skipped_total) {
     using LS = ListShape<KPT_ALL>;
     extern __shared__ uint32_t xk[];  // [LS::N] exchange buffer
     __shared__ float cq[64];
-    __shared__ unsigned kept, slot;
+    __shared__ unsigned kept, slot, near;
     __shared__ int skip_max_bits;
     const int Q = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     if ((!TANI || use_cos) && tid < d) cq[tid] = (float)qcenter[(size_t)Q * d + tid];
     if (tid == 0) {
         kept = 0;
         slot = 0;
+        near = 0;
         skip_max_bits = __float_as_int(-CUDART_INF_F);
     }
     __syncthreads();
@@ -648,7 +660,7 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
     } else {
         const int base = tid * KPT_ALL;
         uint32_t v[KPT_ALL];
-        unsigned my_kept = 0;
+        unsigned my_kept = 0, my_near = 0;
         int my_skip = __float_as_int(-CUDART_INF_F);
         // keys are computed for blocks j·LIST_T + tid (coalesced reads of the transposed centres); the
         // sort does not care where each key starts
@@ -661,6 +673,7 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
                 const float u = bound(b, &phi);
                 if (u >= t) {
                     ++my_kept;
+                    my_near += u >= 0.9f ? 1u : 0u;
                     // ties of the bound at 1 (e.g. every block of the query's own cluster) go nearest
                     // centre first, then by block
                     v[j] = list_key<KPT_ALL>(u, phi, b);
@@ -671,6 +684,7 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
             }
         }
         atomicAdd(&kept, my_kept);
+        atomicAdd(&near, my_near);
         atomicMax(&skip_max_bits, my_skip);
         __syncthreads();  // kept is final
         const unsigned nk = kept;
@@ -699,9 +713,39 @@ __global__ void __launch_bounds__(LIST_T, KPT_ALL <= 16 ? 2 : 1)
     __syncthreads();
     if (tid == 0) {
         counts[Q] = kept;
+        weight[Q] = near;
         ub_skip[Q] = __int_as_float(skip_max_bits);
         if (skipped_total) atomicAdd(skipped_total, (unsigned long long)(ncb - (int)kept));
     }
+}
+
+// The query blocks by descending weight (the list entries with a bound of 0.9 or more, a guess at how far
+// the block's list will be walked), in 1,024 classes: launched in this order the long lists start first and
+// the short ones fill the last wave. One CTA; the order inside a class does not matter.
+__global__ void __launch_bounds__(1024) k_block_order(const uint32_t* __restrict__ weight, int nqb, int ncb,
+                                                      uint32_t* __restrict__ order) {
+    __shared__ uint32_t next[1024], wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto cls = [&](int Q) { return 1023 - (int)((unsigned long long)weight[Q] * 1023ull / (unsigned)max(ncb, 1)); };
+    next[tid] = 0;
+    __syncthreads();
+    for (int Q = tid; Q < nqb; Q += 1024) atomicAdd(&next[cls(Q)], 1u);
+    __syncthreads();
+    const uint32_t v = next[tid];
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(COSTAL_FULL_MASK, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += wsum[w];
+    __syncthreads();
+    next[tid] = before + x - v;
+    __syncthreads();
+    for (int Q = tid; Q < nqb; Q += 1024) order[atomicAdd(&next[cls(Q)], 1u)] = (uint32_t)Q;
 }
 
 // The per-row certificate floor from pruning: ub_skip of the row's query block, or −∞.
@@ -764,6 +808,8 @@ size_t carve(void* base, int n, int d, Plan& P, Scratch& S) {
     take(P.lists, nqb * ncb);
     take(P.list_ub, nqb * ncb);
     take(P.counts, nqb);
+    take(P.weight, nqb);
+    take(P.order, nqb);
     take(P.ub_skip, nqb);
     take(P.row_ub, n);
     take(P.tq, nqb);
@@ -944,8 +990,9 @@ cudaError_t build_lists(Plan& P, unsigned long long* skipped_total, cudaStream_t
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     kern<<<P.nqb, LIST_T, smem, st>>>(P.qcenter, P.qradius, P.ccenter_f, P.cradius_f, P.nqb, P.ncb, P.d, P.tq,
-                                      P.rowmax, P.rm_delta, P.qnorm, P.cnorm, P.norm_only ? 0 : 1, P.lists, P.list_ub, P.counts, P.ub_skip, skipped_total);
+                                      P.rowmax, P.rm_delta, P.qnorm, P.cnorm, P.norm_only ? 0 : 1, P.lists, P.list_ub, P.counts, P.weight, P.ub_skip, skipped_total);
     note_launch();
+    k_block_order<<<1, 1024, 0, st>>>(P.weight, P.nqb, P.ncb, P.order); note_launch();
     k_row_ub<<<(P.n + 255) / 256, 256, 0, st>>>(P.perm, P.n, P.ub_skip, P.row_ub); note_launch();
     return cudaGetLastError();
 }

@@ -38,6 +38,8 @@ struct Plan {
     uint32_t* lists;     // [nqb][ncb] kept column blocks, nearest first
     float* list_ub;      // [nqb][ncb] the bound of each list entry (non-increasing; +inf when unsorted)
     uint32_t* counts;    // [nqb]
+    uint32_t* weight;    // [nqb] list entries with a bound of 0.9 or more
+    uint32_t* order;     // [nqb] the query blocks by descending weight
     float* ub_skip;      // [nqb]
     double* row_ub;      // [n] (original order) pruning floor of the certificate
     float* tq;           // [nqb] per-query-block thresholds (NULL = keep every block)

@@ -37,3 +37,18 @@ def test_order_is_the_stable_sort_by_cell(ext, n, d):
         cell = _cells(x)[perm]
         runs = 1 + (np.diff(cell) != 0).sum()  # (a few near ties and drifted centroids split runs)
         assert runs <= 256 + n // 20, runs
+
+
+@pytest.mark.parametrize("matmul,n,k", [("fp32", 16385, 5), ("fp32", 131_201, 3), ("bf16", 24_577, 5), ("bf16", 131_073, 3)])
+def test_every_query_block_runs_in_the_list_length_order(ext, matmul, n, k):
+    """Query blocks start by descending list weight, in 1,024 classes: with lists of very different
+    lengths, and with more than 1,024 blocks, every row is still computed exactly once."""
+    d = 12
+    x = clustered(n, d, n)
+    x[: n // 3] += 6.0  # a third of the rows in one narrow cone: long lists beside short ones
+    (idx, cos, norms), st = ext._knn_exact(x, k, matmul=matmul)
+    assert st["blocks_skipped"] + st.get("blocks_stopped", 0) > 0
+    (want, wcos, wnorms), _ = ext._knn_exact(x, k, matmul="fp32", prune=False)
+    np.testing.assert_array_equal(idx, want)
+    np.testing.assert_array_equal(cos, wcos)
+    np.testing.assert_array_equal(norms, wnorms)
