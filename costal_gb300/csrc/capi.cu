@@ -996,8 +996,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(ensure(c.mlp_params_bf, P * 4));
         CK(ensure(c.mlp_m1, P * 4));
         CK(ensure(c.mlp_m2, P * 4));
-        CK(ensure(c.mlp_grad, P * 4));
-        CK(ensure(c.mlp_partial, (size_t)((o.batch + 31) / 32) * P * 4));
+        CK(ensure(c.mlp_partial, (size_t)((std::max<uint32_t>(32, o.batch) + 31) / 32) * P * 4));
         Misc* dm = c.misc.as<Misc>();
         CK(cudaMemsetAsync(dm, 0, sizeof(Misc), s));
         CK(cudaMemsetAsync(&dm->bad_row, 0xff, 8, s));
@@ -1036,11 +1035,9 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         for (uint32_t ep = 0; ep < o.epochs; ++ep) {
             for (int b0 = 0; b0 < m; b0 += B) {
                 const int mb = std::min(B, m - b0);
-                CK(mlp::gradient(c.mlp_params.as<float>(), F, c.mlp_feat.as<float>() + (size_t)b0 * F,
-                                 c.mlp_y.as<float>() + b0, mb, o.quantile, c.mlp_partial.as<float>(),
-                                 c.mlp_grad.as<float>(), s));
-                CK(mlp::adam(c.mlp_params.as<float>(), c.mlp_grad.as<float>(), c.mlp_m1.as<float>(),
-                             c.mlp_m2.as<float>(), P, o.lr, ++t, s));
+                CK(mlp::train_step(c.mlp_params.as<float>(), F, c.mlp_feat.as<float>() + (size_t)b0 * F,
+                                   c.mlp_y.as<float>() + b0, mb, o.quantile, c.mlp_partial.as<float>(),
+                                   c.mlp_m1.as<float>(), c.mlp_m2.as<float>(), o.lr, ++t, s));
             }
         }
         CK(mlp::round_bf16(c.mlp_params.as<float>(), c.mlp_params_bf.as<float>(), P, s));

@@ -22,8 +22,7 @@
 namespace costal {
 namespace mlp {
 
-constexpr int R = 32;    // rows per CTA
-constexpr int T = MLP_H; // threads per CTA (one per hidden unit)
+constexpr int R = 32;  // rows of a gradient group (one CTA)
 
 struct Off {
     size_t w1, b1, w2, b2, w3, b3;
@@ -154,45 +153,6 @@ __global__ void k_features(const float* __restrict__ xsT, int np, int d, const f
             }
         }
     }
-}
-
-// ---- forward (shared by inference and training) ------------------------------------------------
-// CTA: R rows × T hidden units. Leaves h1, h2 in shared memory and returns the outputs in out_s.
-__device__ void forward_block(const float* __restrict__ P, int F, const float* __restrict__ feat, int m, int r0,
-                              float* f_s, float* h1_s, float* h2_s, float* out_s) {
-    const Off o = offsets(F);
-    const int j = threadIdx.x;
-    for (int e = j; e < R * F; e += T) {
-        const int r = e / F, t = e % F;
-        f_s[e] = r0 + r < m ? feat[(size_t)(r0 + r) * F + t] : 0.0f;
-    }
-    __syncthreads();
-    {
-        const float* w = P + o.w1 + (size_t)j * F;
-        const float b = P[o.b1 + j];
-        for (int r = 0; r < R; ++r) {
-            float z = b;
-            for (int t = 0; t < F; ++t) z = fmaf(w[t], f_s[r * F + t], z);
-            h1_s[r * T + j] = fmaxf(z, 0.0f);
-        }
-    }
-    __syncthreads();
-    {
-        const float* w = P + o.w2 + (size_t)j * MLP_H;
-        const float b = P[o.b2 + j];
-        for (int r = 0; r < R; ++r) {
-            float z = b;
-            for (int t = 0; t < MLP_H; ++t) z = fmaf(w[t], h1_s[r * T + t], z);
-            h2_s[r * T + j] = fmaxf(z, 0.0f);
-        }
-    }
-    __syncthreads();
-    if (j < R) {
-        float z = P[o.b3];
-        for (int t = 0; t < MLP_H; ++t) z = fmaf(P[o.w3 + t], h2_s[j * T + t], z);
-        out_s[j] = z;
-    }
-    __syncthreads();
 }
 
 // ---- inference ----------------------------------------------------------------------------------
@@ -328,94 +288,240 @@ __global__ void __launch_bounds__(IT) k_infer(const float* __restrict__ P, int F
     }
 }
 
-// ---- backward ----------------------------------------------------------------------------------
-// Per CTA: forward, the pinball-loss gradient of its rows (mean over all m rows), and the gradient
-// of every parameter summed over the CTA's rows in row order → partial[blockIdx.x][nparams].
-__global__ void __launch_bounds__(T) k_grad_partial(const float* __restrict__ P, int F, const float* __restrict__ feat,
-                                                    const float* __restrict__ y, int m, float quantile,
-                                                    float* __restrict__ partial) {
-    extern __shared__ float sm[];
-    float* f_s = sm;                  // [R][F]
-    float* h1_s = f_s + R * F;        // [R][T]
-    float* h2_s = h1_s + R * T;       // [R][T]
-    float* out_s = h2_s + R * T;      // [R]
+// ---- training -----------------------------------------------------------------------------------
+// Per CTA: the FP32 forward of its 32 rows, the pinball-loss gradient (mean over all m rows), and the
+// gradient of every parameter summed over the CTA's rows in row order → partial[blockIdx.x][nparams].
+// Every sum is one FMA chain in the order of its index (inputs, units or rows), so a tile's shape does
+// not show in the result. Bound by shared-memory loads: both weight matrices and the activations stay
+// in shared memory (row strides of 4 × an odd number of words: conflict-free 16-byte loads down a
+// column of rows), and a thread keeps 4 rows × 4 units (8 × 4 for the weight gradients), so that an
+// operand word serves 4 FMAs. A thread per unit that read its weights' rows from global memory, one
+// load an FMA and lanes F words apart, made a step of 2,048 rows (F = 104, 64 CTAs) take 0.447 ms; with
+// this form it takes 0.045 (this kernel 0.032, k_adam 0.009). W2 arrives while layer 1 runs.
+constexpr int GT = 256;          // threads: 8 warps × 4 rows, lane L's units L, L + 32, L + 64, L + 96
+constexpr int GS = MLP_H + 4;    // row stride (words) of W2 and the hidden activations
+__host__ __device__ inline int grad_stride(int F) {  // of W1 and the features
+    const int q = (F + 3) / 4;
+    return 4 * (q | 1);
+}
+
+__device__ __forceinline__ void cp4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+// acc[i][c] += Σ_t x[row i][t] · w[unit c][t] in t order (i: 4 rows from x, c: units lane + 32c of w).
+__device__ __forceinline__ void layer_tile(float (&acc)[4][4], const float* x, int xs, const float* w, int ws, int n) {
+    int t = 0;
+#pragma unroll 2
+    for (; t + 4 <= n; t += 4) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(x + i * xs + t);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(w + 32 * c * ws + t);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                acc[i][c] = fmaf(b[c].x, a[i].x, acc[i][c]);
+                acc[i][c] = fmaf(b[c].y, a[i].y, acc[i][c]);
+                acc[i][c] = fmaf(b[c].z, a[i].z, acc[i][c]);
+                acc[i][c] = fmaf(b[c].w, a[i].w, acc[i][c]);
+            }
+    }
+    for (; t < n; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(w[32 * c * ws + t], x[i * xs + t], acc[i][c]);
+}
+
+// G[j][t] = Σ_r dz[r][j] · x[r][t] in row order, for the warp's 16 units j and all t < n.
+__device__ __forceinline__ void weight_grad(float* __restrict__ G, const float* dz, const float* x, int xs, int n,
+                                            int warp, int lane) {
+    for (int j0 = 16 * warp; j0 < 16 * warp + 16; j0 += 8) {
+        float acc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+        int tc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tc[c] = min(lane + 32 * c, n - 1);
+#pragma unroll 4
+        for (int r = 0; r < R; ++r) {
+            const float4 lo = *reinterpret_cast<const float4*>(dz + r * GS + j0);
+            const float4 hi = *reinterpret_cast<const float4*>(dz + r * GS + j0 + 4);
+            const float d[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float v = x[r * xs + tc[c]];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][c] = fmaf(d[i], v, acc[i][c]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (lane + 32 * c < n) G[(size_t)(j0 + i) * n + lane + 32 * c] = acc[i][c];
+    }
+}
+
+static size_t grad_smem(int F) {
+    return (size_t)((R + MLP_H) * grad_stride(F) + MLP_H * GS + 3 * R * GS + 2 * R) * 4;
+}
+
+__global__ void __launch_bounds__(GT) k_grad_partial(const float* __restrict__ P, int F, const float* __restrict__ feat,
+                                                     const float* __restrict__ y, int m, float quantile,
+                                                     float* __restrict__ partial) {
+    extern __shared__ __align__(16) float sm[];
+    const int FS = grad_stride(F);
+    float* f_s = sm;                  // [R][FS]
+    float* w1_s = f_s + R * FS;       // [H][FS]
+    float* w2_s = w1_s + MLP_H * FS;  // [H][GS]
+    float* h1_s = w2_s + MLP_H * GS;  // [R][GS]
+    float* h2_s = h1_s + R * GS;      // [R][GS], then dz1
+    float* dz2_s = h2_s + R * GS;     // [R][GS]
+    float* out_s = dz2_s + R * GS;    // [R]
     float* g_s = out_s + R;           // [R] dL/dout
-    float* dz2_s = g_s + R;           // [R][T]
-    float* dz1_s = dz2_s + R * T;     // [R][T]
+    float* dz1_s = h2_s;
     const Off o = offsets(F);
-    const int j = threadIdx.x;
-    const int r0 = blockIdx.x * R;
-    forward_block(P, F, feat, m, r0, f_s, h1_s, h2_s, out_s);
-    if (j < R) {
-        const int i = r0 + j;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r0 = blockIdx.x * R, rw = 4 * warp;
+    for (int r = warp; r < R; r += GT / 32)
+        for (int t = lane; t < F; t += 32) {
+            if (r0 + r < m) cp4(f_s + r * FS + t, feat + (size_t)(r0 + r) * F + t);
+            else f_s[r * FS + t] = 0.0f;
+        }
+    for (int u = warp; u < MLP_H; u += GT / 32)
+        for (int t = lane; t < F; t += 32) cp4(w1_s + u * FS + t, P + o.w1 + (size_t)u * F + t);
+    asm volatile("cp.async.commit_group;");
+    for (int e = tid; e < MLP_H * MLP_H / 4; e += GT)
+        cp16(w2_s + (e >> 5) * GS + 4 * (e & 31), P + o.w2 + 4 * (size_t)e);
+    asm volatile("cp.async.commit_group;");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    auto layer = [&](const float* x, int xs, const float* w, int ws, int n, const float* bias, float* out) {
+        float acc[4][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = acc[2][c] = acc[3][c] = bias[lane + 32 * c];
+        layer_tile(acc, x + rw * xs, xs, w + lane * ws, ws, n);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) out[(rw + i) * GS + lane + 32 * c] = fmaxf(acc[i][c], 0.0f);
+    };
+    layer(f_s, FS, w1_s, FS, F, P + o.b1, h1_s);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    layer(h1_s, GS, w2_s, GS, MLP_H, P + o.b2, h2_s);
+    __syncthreads();
+    if (tid < R) {
+        float z = P[o.b3];
+#pragma unroll 8
+        for (int t = 0; t < MLP_H; t += 4) {
+            const float4 h = *reinterpret_cast<const float4*>(h2_s + tid * GS + t);
+            z = fmaf(P[o.w3 + t], h.x, z);
+            z = fmaf(P[o.w3 + t + 1], h.y, z);
+            z = fmaf(P[o.w3 + t + 2], h.z, z);
+            z = fmaf(P[o.w3 + t + 3], h.w, z);
+        }
+        const int i = r0 + tid;
         // pinball loss ρ(y − out): d/dout = (1 − α) when out > y, −α otherwise
-        g_s[j] = i < m ? (out_s[j] > y[i] ? 1.0f - quantile : -quantile) / (float)m : 0.0f;
+        g_s[tid] = i < m ? (z > y[i] ? 1.0f - quantile : -quantile) / (float)m : 0.0f;
     }
     __syncthreads();
     float* G = partial + (size_t)blockIdx.x * mlp_param_count(F);
-    const float w3j = P[o.w3 + j];
     {
-        float gw3 = 0.0f;
-        for (int r = 0; r < R; ++r) {
-            gw3 = fmaf(g_s[r], h2_s[r * T + j], gw3);
-            dz2_s[r * T + j] = h2_s[r * T + j] > 0.0f ? g_s[r] * w3j : 0.0f;
-        }
-        G[o.w3 + j] = gw3;
-        if (j == 0) {
+        const int j = tid & (MLP_H - 1);
+        const float w3j = P[o.w3 + j];
+        for (int r = tid / MLP_H; r < R; r += GT / MLP_H)
+            dz2_s[r * GS + j] = h2_s[r * GS + j] > 0.0f ? g_s[r] * w3j : 0.0f;
+        if (tid < MLP_H) {
+            float gw3 = 0.0f;
+            for (int r = 0; r < R; ++r) gw3 = fmaf(g_s[r], h2_s[r * GS + j], gw3);
+            G[o.w3 + j] = gw3;
+        } else if (tid == MLP_H) {
             float gb3 = 0.0f;
             for (int r = 0; r < R; ++r) gb3 += g_s[r];
             G[o.b3] = gb3;
         }
     }
     __syncthreads();
-    {
-        // layer 2: dW2[j][t] = Σ_r dz2[r][j] h1[r][t], db2[j] = Σ_r dz2[r][j]
+    // layer 2: dW2[j][t] = Σ_r dz2[r][j] h1[r][t], db2[j] = Σ_r dz2[r][j]
+    weight_grad(G + o.w2, dz2_s, h1_s, GS, MLP_H, warp, lane);
+    if (tid < MLP_H) {
         float gb = 0.0f;
-        for (int r = 0; r < R; ++r) gb += dz2_s[r * T + j];
-        G[o.b2 + j] = gb;
-        for (int t = 0; t < MLP_H; ++t) {
-            float s = 0.0f;
-            for (int r = 0; r < R; ++r) s = fmaf(dz2_s[r * T + j], h1_s[r * T + t], s);
-            G[o.w2 + (size_t)j * MLP_H + t] = s;
-        }
+        for (int r = 0; r < R; ++r) gb += dz2_s[r * GS + tid];
+        G[o.b2 + tid] = gb;
+    }
+    {
         // dh1[r][j] = Σ_u dz2[r][u] W2[u][j], masked by the ReLU of layer 1
-        for (int r = 0; r < R; ++r) {
-            float s = 0.0f;
-            for (int u = 0; u < MLP_H; ++u) s = fmaf(dz2_s[r * T + u], P[o.w2 + (size_t)u * MLP_H + j], s);
-            dz1_s[r * T + j] = h1_s[r * T + j] > 0.0f ? s : 0.0f;
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+#pragma unroll 2
+        for (int u = 0; u < MLP_H; u += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(dz2_s + (rw + i) * GS + u);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float b[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) b[c] = w2_s[(u + q) * GS + lane + 32 * c];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float d = q == 0 ? a[i].x : q == 1 ? a[i].y : q == 2 ? a[i].z : a[i].w;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(d, b[c], acc[i][c]);
+                }
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int e = (rw + i) * GS + lane + 32 * c;
+                dz1_s[e] = h1_s[e] > 0.0f ? acc[i][c] : 0.0f;  // (h2 is no longer read)
+            }
     }
     __syncthreads();
-    {
+    weight_grad(G + o.w1, dz1_s, f_s, FS, F, warp, lane);
+    if (tid < MLP_H) {
         float gb = 0.0f;
-        for (int r = 0; r < R; ++r) gb += dz1_s[r * T + j];
-        G[o.b1 + j] = gb;
-        for (int t = 0; t < F; ++t) {
-            float s = 0.0f;
-            for (int r = 0; r < R; ++r) s = fmaf(dz1_s[r * T + j], f_s[r * F + t], s);
-            G[o.w1 + (size_t)j * F + t] = s;
-        }
+        for (int r = 0; r < R; ++r) gb += dz1_s[r * GS + tid];
+        G[o.b1 + tid] = gb;
     }
+}
+
+// The groups' gradients of one parameter, summed in group order (16 loads in flight).
+__device__ __forceinline__ float sum_groups(const float* __restrict__ partial, int groups, size_t np, size_t p) {
+    float s = 0.0f;
+#pragma unroll 16
+    for (int g = 0; g < groups; ++g) s += partial[(size_t)g * np + p];
+    return s;
 }
 
 __global__ void k_grad_reduce(const float* __restrict__ partial, int groups, size_t np, float* __restrict__ grad) {
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < np; p += (size_t)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int g = 0; g < groups; ++g) s += partial[(size_t)g * np + p];
-        grad[p] = s;
-    }
+    const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (p < np) grad[p] = sum_groups(partial, groups, np, p);
 }
 
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ g, float* __restrict__ m1, float* __restrict__ m2,
-                       size_t np, float lr, float bc1, float bc2) {
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < np; p += (size_t)gridDim.x * blockDim.x) {
-        const float gp = g[p];
-        const float a = 0.9f * m1[p] + 0.1f * gp;
-        const float b = 0.999f * m2[p] + 0.001f * gp * gp;
-        m1[p] = a;
-        m2[p] = b;
-        P[p] -= lr * (a / bc1) / (sqrtf(b / bc2) + 1e-8f);
-    }
+// The gradient sum and the Adam step it feeds, in one launch: a parameter's update needs nothing but
+// its own sum, so the sum does not go through memory.
+__global__ void k_adam(const float* __restrict__ partial, int groups, float* __restrict__ P, float* __restrict__ m1,
+                       float* __restrict__ m2, size_t np, float lr, float bc1, float bc2) {
+    const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    const float gp = sum_groups(partial, groups, np, p);
+    const float a = 0.9f * m1[p] + 0.1f * gp;
+    const float b = 0.999f * m2[p] + 0.001f * gp * gp;
+    m1[p] = a;
+    m2[p] = b;
+    P[p] -= lr * (a / bc1) / (sqrtf(b / bc2) + 1e-8f);
 }
 
 __global__ void k_round_bf16(const float* __restrict__ P, float* __restrict__ Q, size_t np) {
@@ -438,8 +544,6 @@ __global__ void k_block_min(const float* __restrict__ pred, const uint32_t* __re
 }
 
 // ---- launchers ----------------------------------------------------------------------------------
-
-static size_t grad_smem(int F) { return (size_t)(R * F + 4 * R * T + 2 * R) * 4; }
 
 cudaError_t features(const float* xsT, int np, int d, const float* centroids, int K, const uint32_t* rows, int m,
                      float* feat, cudaStream_t st) {
@@ -474,20 +578,31 @@ cudaError_t forward(const float* params, int F, const float* feat, int m, float*
     return cudaGetLastError();
 }
 
-cudaError_t gradient(const float* params, int F, const float* feat, const float* y, int m, float quantile,
-                     float* partial, float* grad, cudaStream_t st) {
-    const int groups = (m + R - 1) / R;
+static cudaError_t launch_partial(const float* params, int F, const float* feat, const float* y, int m, float quantile,
+                                  float* partial, cudaStream_t st) {
     const size_t smem = grad_smem(F);
     cudaError_t e = cudaFuncSetAttribute(k_grad_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_grad_partial<<<groups, T, smem, st>>>(params, F, feat, y, m, quantile, partial); note_launch();
-    k_grad_reduce<<<128, 256, 0, st>>>(partial, groups, mlp_param_count(F), grad); note_launch();
+    k_grad_partial<<<(m + R - 1) / R, GT, smem, st>>>(params, F, feat, y, m, quantile, partial); note_launch();
     return cudaGetLastError();
 }
 
-cudaError_t adam(float* params, const float* grad, float* m1, float* m2, size_t np, float lr, int t, cudaStream_t st) {
+cudaError_t gradient(const float* params, int F, const float* feat, const float* y, int m, float quantile,
+                     float* partial, float* grad, cudaStream_t st) {
+    cudaError_t e = launch_partial(params, F, feat, y, m, quantile, partial, st);
+    if (e != cudaSuccess) return e;
+    const size_t np = mlp_param_count(F);
+    k_grad_reduce<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(partial, (m + R - 1) / R, np, grad); note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t train_step(float* params, int F, const float* feat, const float* y, int m, float quantile, float* partial,
+                       float* m1, float* m2, float lr, int t, cudaStream_t st) {
+    cudaError_t e = launch_partial(params, F, feat, y, m, quantile, partial, st);
+    if (e != cudaSuccess) return e;
     const float bc1 = 1.0f - powf(0.9f, (float)t), bc2 = 1.0f - powf(0.999f, (float)t);
-    k_adam<<<128, 256, 0, st>>>(params, grad, m1, m2, np, lr, bc1, bc2); note_launch();
+    const size_t np = mlp_param_count(F);
+    k_adam<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(partial, (m + R - 1) / R, params, m1, m2, np, lr, bc1, bc2); note_launch();
     return cudaGetLastError();
 }
 

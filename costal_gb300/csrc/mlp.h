@@ -37,8 +37,9 @@ cudaError_t forward(const float* params, int F, const float* feat, int m, float*
 // parameter, summed in a fixed order: grad[nparams]. `partial` holds ⌈m/32⌉ × nparams floats.
 cudaError_t gradient(const float* params, int F, const float* feat, const float* y, int m, float quantile,
                      float* partial, float* grad, cudaStream_t st);
-// One Adam step (β1 0.9, β2 0.999, ε 1e-8) on params with gradient grad, step count t ≥ 1.
-cudaError_t adam(float* params, const float* grad, float* m1, float* m2, size_t np, float lr, int t, cudaStream_t st);
+// One training step: the gradient as above, then Adam (β1 0.9, β2 0.999, ε 1e-8) on params, step count t ≥ 1.
+cudaError_t train_step(float* params, int F, const float* feat, const float* y, int m, float quantile, float* partial,
+                       float* m1, float* m2, float lr, int t, cudaStream_t st);
 // params_bf = bf16-rounded copy of params (inference weights).
 cudaError_t round_bf16(const float* params, float* params_bf, size_t np, cudaStream_t st);
 // Per-query-block thresholds for the pruning lists: t_Q = min over the block's rows of the

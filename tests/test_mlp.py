@@ -32,6 +32,24 @@ def test_forward_and_gradient_match_the_oracle(ext):
         assert np.linalg.norm(g - gw) <= 1e-4 * np.linalg.norm(gw)
 
 
+@pytest.mark.parametrize("F,m", [(1, 1), (2, 31), (33, 32), (65, 33), (67, 65), (104, 2048), (127, 40), (128, 4100)])
+def test_gradient_at_the_tiles_edges(ext, F, m):
+    """Every parameter block of the gradient kernel: inputs that are no multiple of 4 or 32, partial row
+    groups, more groups than SMs. Each value is a chain of f32 FMAs no longer than 128 + 128 + 32 terms
+    plus m / 32 sums, within ~(288 + m / 32) · 2⁻²⁴ ≈ 2.5e-5 of the terms' magnitude: 1e-4 in norm."""
+    from oracle import mlp_oracle as M
+
+    rng = np.random.default_rng(1000 * F + m)
+    params = (rng.standard_normal(M.param_count(F)) * 0.15).astype(np.float32)
+    feat = rng.standard_normal((m, F)).astype(np.float32)
+    y = (10.0 * rng.choice([-1.0, 1.0], m)).astype(np.float32)
+    g = ext._mlp_gradient(params, feat, y, 0.05).astype(np.float64)
+    gw = M.gradient(params, feat, y, 0.05)
+    ends = np.cumsum([128 * F, 128, 128 * 128, 128, 128, 1])
+    for a, b in zip(np.r_[0, ends[:-1]], ends):
+        assert np.linalg.norm(g[a:b] - gw[a:b]) <= 1e-4 * np.linalg.norm(gw[a:b]) + 1e-12, (a, b)
+
+
 @pytest.fixture(scope="module")
 def zipf_case(ext):
     from costal_gb300 import workloads as W
