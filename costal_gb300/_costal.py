@@ -408,7 +408,7 @@ def default_matmul() -> str:
 # ---- the learned block-pruning model (GB300 addition; no counterpart in the reference) ----------
 
 def _mlp_train(x, k, *, sample=200_000, epochs=30, batch=2048, lr=2e-3, quantile=0.05, margin=None, seed=20241203):
-    """Train the k-th-neighbour-cosine model on x (labels from the plain FP32 path); it stays loaded.
+    """Train the k-th-neighbour-cosine model on x (exact labels); it stays loaded.
 
     Returns the training stats (loss, mean absolute error, coverage = share of rows predicted at or
     below their exact k-th cosine, times)."""

@@ -68,7 +68,7 @@ struct Context {
     Misc* h_misc = nullptr;
     DevBuf x, norms, xsT, cand_idx, cand_score, tau, out_idx, out_cos, out_w, fb_rows, fb_minsim, misc;
     DevBuf fu_scratch, rows, cols, wout, idx_in, cos_in, norms_in, w_in, jac, f32out, tc_ws, tc_rows, prune_ws;
-    DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows;
+    DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows, mlp_perm;
     DevBuf fp32_ws, tfloor, xsW, xsR;
     DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_ws, tani_ranges, rm_ws, rm_out;
     MlpState mlp;
@@ -1008,17 +1008,52 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(ensure(c.prune_ws, prune::workspace_bytes(N, D)));
         prune::Plan pp{};
         CK(prune::build_order(c.prune_ws.p, c.xsT.as<float>(), c.xsR.as<float>(), N, np, D, s, pp));
-        // labels: the exact k-th-neighbour cosine of every sampled row, from the plain FP32 path
+        // Labels: the exact k-th-neighbour cosine of every sampled row. The tensor-core pass in an order that
+        // has the sample's rows first computes just their query blocks against every column (32,768 rows ×
+        // 200,000 columns, d = 40: 2.6 ms with the operands; the FP32 pass of those rows 12.4); rows that fail its certificate
+        // go through the FP32 pass, as does everything where k + margin or d is beyond the tensor-core pass.
         uint32_t* rows = c.mlp_rows.as<uint32_t>();
         CK(launch_stride_rows(rows, m, N, s));
-        unsigned hm = (unsigned)m;
-        CK(cudaMemcpyAsync(&dm->tc_fail_count, &hm, 4, cudaMemcpyHostToDevice, s));
-        coarse_fp32_rows(c, N, np, dp, cap, rows, m, nullptr, s);
+        CK(cudaMemcpyAsync(&dm->shard_rows, &m, 4, cudaMemcpyHostToDevice, s));
         const double eps = ((double)d + 4.0) * F32_EPS;
-        CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
-                          c.tau.as<float>(), c.norms.as<double>(), nullptr, nullptr, nullptr, eps, cap < N - 1, 0, rows,
-                          &dm->tc_fail_count, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
-                          c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, s));
+        const uint32_t* frows = rows;  // the rows of the FP32 pass
+        const unsigned* fcount = &dm->shard_rows;
+        int nf = m;
+        const float* tfloor = nullptr;
+        if (tc::supported(D, cap)) {
+            CK(ensure(c.mlp_perm, n * 4ull));
+            CK(launch_sample_first(c.mlp_perm.as<uint32_t>(), m, N, s));
+            CK(ensure(c.tc_ws, tc::workspace_bytes(N, D)));
+            CK(ensure(c.tc_rows, n * 4ull));
+            tc::Plan plan{};
+            CK(tc::prepare(c.tc_ws.p, c.xsT.as<float>(), N, np, dp, D, c.mlp_perm.as<uint32_t>(), s, plan));
+            CK(tc::launch_coarse(plan, cap, nullptr, nullptr, nullptr, nullptr, 0, 0, c.cand_idx.as<uint32_t>(),
+                                 c.cand_score.as<float>(), c.tau.as<float>(), &dm->blocks_stopped, &dm->timeout_flag,
+                                 c.sm_count, s, 0, (m + 127) / 128));
+            CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
+                              c.tau.as<float>(), c.norms.as<double>(), plan.row_eps, nullptr, nullptr, 0.0, cap < N - 1,
+                              0, rows, &dm->shard_rows, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
+                              c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count, nullptr, s));
+            CK(cudaMemcpyAsync(&c.h_misc->tc_fail_count, &dm->tc_fail_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                               s));
+            CK(cudaStreamSynchronize(s));
+            nf = (int)c.h_misc->tc_fail_count;
+            frows = c.tc_rows.as<uint32_t>();
+            fcount = &dm->tc_fail_count;
+            if (nf > 0) {
+                CK(ensure(c.tfloor, n * 4ull));
+                CK(launch_rerun_floor(frows, fcount, nf, cap, c.tau.as<float>(), c.cand_score.as<float>(), plan.row_eps,
+                                      eps, c.tfloor.as<float>(), s));
+                tfloor = c.tfloor.as<float>();
+            }
+        }
+        if (nf > 0) {
+            coarse_fp32_rows(c, N, np, dp, cap, frows, nf, tfloor, s);
+            CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
+                              c.tau.as<float>(), c.norms.as<double>(), nullptr, nullptr, nullptr, eps, cap < N - 1, 0,
+                              frows, fcount, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
+                              c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, s));
+        }
         if (cap < N - 1)
             CK(launch_gather(c.x.as<float>(), c.xsT.as<float>(), N, np, D, dp, K, c.norms.as<double>(),
                              c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, 0, 0,

@@ -78,6 +78,20 @@ cudaError_t launch_stride_rows(uint32_t* out, int m, int n, cudaStream_t st) {
     if (m > 0) { k_stride_rows<<<(m + 255) / 256, 256, 0, st>>>(out, m, n); note_launch(); }
     return cudaGetLastError();
 }
+
+// Those rows (row i·n/m is the sample's i-th) first, in order, then every other row in order: below row
+// r + 1 lie ⌈(r + 1)·m / n⌉ rows of the sample.
+__global__ void k_sample_first(uint32_t* __restrict__ perm, int m, int n) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int before = (int)(((unsigned long long)r * m + n - 1) / n);
+    const int upto = (int)(((unsigned long long)(r + 1) * m + n - 1) / n);
+    perm[upto > before ? before : m + r - upto] = (uint32_t)r;
+}
+cudaError_t launch_sample_first(uint32_t* perm, int m, int n, cudaStream_t st) {
+    k_sample_first<<<(n + 255) / 256, 256, 0, st>>>(perm, m, n); note_launch();
+    return cudaGetLastError();
+}
 // y[j] = cos[rows[j]·k + k − 1]: the k-th neighbour cosine of each listed row.
 __global__ void k_kth(const double* __restrict__ cos, const uint32_t* __restrict__ rows, int m, int k,
                       float* __restrict__ y) {

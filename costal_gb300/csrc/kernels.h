@@ -76,6 +76,8 @@ cudaError_t launch_iota(uint32_t* out, int start, int m, cudaStream_t st);
 cudaError_t launch_take_rows(const uint32_t* rows, int nrows, int k, const uint32_t* idx, const double* cos,
                              const double* w, uint32_t* oidx, double* ocos, double* ow, cudaStream_t st);
 cudaError_t launch_stride_rows(uint32_t* out, int m, int n, cudaStream_t st);
+// perm = those rows first, then the others, each in ascending order.
+cudaError_t launch_sample_first(uint32_t* perm, int m, int n, cudaStream_t st);
 cudaError_t launch_kth(const double* cos, const uint32_t* rows, int m, int k, float* y, cudaStream_t st);
 cudaError_t launch_init_params(float* P, int F, unsigned long long seed, cudaStream_t st);
 cudaError_t launch_check_idx(const int32_t* idx, uint64_t nk, int n, unsigned long long* first_bad, cudaStream_t st);

@@ -185,12 +185,12 @@ typedef struct costal_mlp_stats {
     double loss;        /* final mean pinball loss on the training rows (bf16 weights) */
     double mae;         /* mean |prediction - exact k-th cosine| */
     double coverage;    /* fraction of training rows whose prediction is <= their exact k-th cosine */
-    double ms_labels;   /* exact labels (plain FP32 path) and features */
+    double ms_labels;   /* exact labels and features */
     double ms_train;    /* forward/backward/Adam kernels */
 } costal_mlp_stats;
 
 /* Train the model on X (host, n x d): labels are the exact k-th-neighbour cosines of the sampled rows
- * from the plain FP32 path, features use the same k-means cells as the pruned kNN. The model stays
+ * (a coarse pass and its certificate), features use the same k-means cells as the pruned kNN. The model stays
  * loaded in the library's context. mo may be NULL (defaults). */
 int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const costal_mlp_opts* mo,
                      costal_mlp_stats* stats, char* err, size_t errlen);

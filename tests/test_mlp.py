@@ -50,6 +50,24 @@ def test_gradient_at_the_tiles_edges(ext, F, m):
         assert np.linalg.norm(g[a:b] - gw[a:b]) <= 1e-4 * np.linalg.norm(gw[a:b]) + 1e-12, (a, b)
 
 
+@pytest.mark.parametrize("n,d,k,sample,copies", [(300, 7, 5, 300, 0), (300, 33, 5, 1, 0), (5000, 40, 10, 129, 0),
+                                                 (2999, 64, 5, 127, 0), (40_001, 15, 10, 20_000, 2000)])
+def test_labels_are_exact_on_either_pass(ext, n, d, k, sample, copies):
+    """The training labels (exact k-th cosines) come from the tensor-core pass of the sample's rows where
+    k + margin fits it (64 candidates) and from the FP32 pass above: the trained weights are the same bits.
+    With near-copies of one row, their certificates fail and the FP32 pass re-runs them."""
+    from conftest import clustered
+
+    x = clustered(n, d, n + d)
+    if copies:
+        rng = np.random.default_rng(n)
+        x[:copies] = x[0] * (1.0 + rng.normal(0, 1e-7, (copies, d))).astype(np.float32)
+    ext._mlp_train(x, k, sample=sample, epochs=2, batch=64, margin=k)
+    a = ext._mlp_get()[0]
+    ext._mlp_train(x, k, sample=sample, epochs=2, batch=64, margin=100)
+    np.testing.assert_array_equal(a, ext._mlp_get()[0])
+
+
 @pytest.fixture(scope="module")
 def zipf_case(ext):
     from costal_gb300 import workloads as W
