@@ -240,12 +240,12 @@ def _profile_case(name):
 
 
 PROFILE_CASES = {
-    "coarse_fp32_kc": "k_coarse_fp32_kc: the FP32 pass for deep rows (20,000 x 2,000 scRNA-like)",
+    "coarse_fp32_kc": "k_fp32_tiles: the FP32 pass, query tile streamed for deep rows (20,000 x 2,000 scRNA-like)",
     "split_wide": "k_split_wide: the split-BF16 operands of deep rows (20,000 x 2,000)",
     "coarse_tc_fp8": "k_coarse_tc<.., FP8>: the split-FP8 tensor-core pass (20,000 x 2,000)",
     "gather": "k_gather: the full-row regather (50,000 x 6 integer rows)",
     "merge_parts": "k_merge_parts: column-segment lists of re-run rows merged (200,000 x 16, 300 near-copies)",
-    "tanimoto_window": "k_coarse_tani_window: Tanimoto selection with the norm window (200,000 x 15)",
+    "tanimoto_window": "k_fp32_tiles: Tanimoto selection by lists (200,000 x 15)",
     "jaccard": "k_sort_rows + k_jaccard: Jaccard weights (400,000 x 10 neighbours)",
     "csr": "k_sort_big + k_csr_emit: the Leiden CSR with two hub rows of ~6,000 entries",
 }
@@ -362,7 +362,7 @@ def main():
     weight = L.WEIGHT["tanimoto"]
     stream = torch.cuda.current_stream()
 
-    # ---- the model (trained once on this input, labels from the plain FP32 path; untimed)
+    # ---- the model (trained once on this input with exact labels; untimed)
     train = None
     if learned and args.mlp_load:
         from costal_gb300 import _costal as ext
@@ -537,7 +537,7 @@ def main():
         kms = float(np.mean([s_["ms_kernel"] for s_ in stats]))
         total_blocks = s0["blocks_total"]
         tensor = args.backend != "fp32"
-        skipped = s0["blocks_skipped"] + s0["blocks_stopped"] if tensor else 0
+        skipped = s0["blocks_skipped"] + s0["blocks_stopped"]
         visited = 1.0 - skipped / total_blocks if total_blocks else 1.0
         pairs = float(n) * float(n) * visited  # dense pairs of the visited (query block, column block) tiles
         flops = 2.0 * d * pairs
@@ -545,15 +545,13 @@ def main():
         if tensor and kind == 2:
             # split FP8: e4m3 MMAs, K = 3d padded to 128; the dense FP8 rate is twice the BF16 one
             kpad = (3 * d + 127) // 128 * 128
-            tiles = (total_blocks - skipped)
-            executed = 2.0 * kpad * tiles * 128 * 256
+            executed = 2.0 * kpad * pairs
             bound, peak, unit = "tensor", 2.0 * pk.get("bf16_tflops_sustained", pk["bf16_tflops"]), "TFLOP/s"
             kernel = "k_coarse_tc (split-FP8 e4m3 tcgen05 tiles + top-(k+m) selection)"
             peak_kind = f"fp8 dense = 2 x bf16 dense sustained ({pk_kind}; no fp8 figure is measured)"
         elif tensor:
             kpad = (3 * d + 63) // 64 * 64
-            tiles = (total_blocks - skipped)
-            executed = 2.0 * kpad * tiles * 128 * 256
+            executed = 2.0 * kpad * pairs
             bound, peak, unit = "tensor", pk.get("bf16_tflops_sustained", pk["bf16_tflops"]), "TFLOP/s"
             kernel = "k_coarse_tc (split-BF16 tcgen05 tiles + top-(k+m) selection)"
             peak_kind = f"bf16 dense sustained, {pk_kind}"
@@ -563,7 +561,7 @@ def main():
             # has no CUDA-core figure, so it is derived from the measured max clock.
             bound, unit = "fp32-fma", "TFLOP/s"
             peak = 152 * 128 * 2 * pk.get("sm_max_mhz", 2070.0) * 1e6 / 1e12
-            kernel = "k_coarse_fp32 (FP32 tiles + top-(k+m) selection)"
+            kernel = "k_fp32_tiles (FP32 tiles + top-(k+m) selection)"
             peak_kind = "derived FP32-FFMA peak at max SM clock"
         achieved = flops / (kms * 1e-3) / 1e12
         traffic = traffic_per_launch("bf16" if kind else "fp32", pairs, d) if kind != 2 else None
