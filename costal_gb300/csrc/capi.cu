@@ -487,11 +487,13 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             // The split-BF16 certificate with its per-row bound (and, with pruning, the skipped
             // blocks' bound); rows that fail it are listed in tc_rows, re-run over ALL columns by the
             // FP32 coarse kernel and rescored with the FP32 bound, whose failures in turn take the
-            // full-row regather.
+            // full-row regather. It is asked for at cap = n − 1 too: this pass's starting threshold may come
+            // from the query's own column or from zero padding and so leave columns out of a list that has
+            // room for all of them (the FP32 pass's start never counts those columns).
             if (nrows > 0)
                 CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                   c.tau.as<float>(), d_norms, plan.row_eps, learned ? pp.row_ub : nullptr,
-                                  &dm->prune_fail_count, 0.0, cap < n - 1, 0, srows, scount, d_idx, d_cos, d_w,
+                                  &dm->prune_fail_count, 0.0, 1, 0, srows, scount, d_idx, d_cos, d_w,
                                   c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count,
                                   dm->max_err_bits, s));
             // How many rows failed decides the re-run's shape (few rows: the columns split across CTAs).
@@ -1031,8 +1033,8 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
                                  c.cand_score.as<float>(), c.tau.as<float>(), &dm->blocks_stopped, &dm->timeout_flag,
                                  c.sm_count, s, 0, (m + 127) / 128));
             CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
-                              c.tau.as<float>(), c.norms.as<double>(), plan.row_eps, nullptr, nullptr, 0.0, cap < N - 1,
-                              0, rows, &dm->shard_rows, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
+                              c.tau.as<float>(), c.norms.as<double>(), plan.row_eps, nullptr, nullptr, 0.0, 1, 0, rows,
+                              &dm->shard_rows, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
                               c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count, nullptr, s));
             CK(cudaMemcpyAsync(&c.h_misc->tc_fail_count, &dm->tc_fail_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
                                s));

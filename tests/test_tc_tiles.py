@@ -40,3 +40,31 @@ def test_deep_rescoring_drops_by_f32_cosines(ext, oracle, n, d, k, matmul):
     (idx, cos, norms), st = ext._knn_exact(x, k, matmul=matmul)
     for a, b in zip((idx.view(np.uint32), cos, norms), want):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,d,matmul", [(17, 20, "bf16"), (20, 21, "bf16"), (33, 36, "bf16"), (34, 40, "bf16"), (40, 64, "bf16"),
+                                        (50, 100, "bf16"), (60, 600, "bf16"), (65, 600, "fp8"), (64, 70, "fp8")])
+def test_lists_with_room_for_every_row(ext, n, d, matmul):
+    """k + m ≥ n − 1: every other row is a candidate. Orthonormal rows have cosines of ~1e-8 with random
+    signs, so their exact order is far inside the coarse error: a row that a starting threshold left out
+    (the zero padding's score) shows."""
+    q = np.linalg.qr(np.random.default_rng(n).standard_normal((d, d)))[0]
+    x = np.ascontiguousarray(q[:n], dtype=np.float32)
+    for k in (1, n // 3, n // 2, n - 2):
+        want = ext._knn_bruteforce(x, k)
+        got, st = ext._knn_exact(x, k, matmul=matmul, margin=n)
+        assert st["coarse_kind"] != "fp32" and st["margin"] + k >= n - 1
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,d", [(17, 20), (34, 40), (40, 64)])
+def test_labels_of_lists_with_room_for_every_row(ext, n, d):
+    """The same in training: labels from lists of n − 1 candidates equal those from n − 2 (certified)."""
+    q = np.linalg.qr(np.random.default_rng(n).standard_normal((d, d)))[0]
+    x, k = np.ascontiguousarray(q[:n], dtype=np.float32), n // 2
+    trained = []
+    for margin in (n, n - 2 - k):
+        st = ext._mlp_train(x, k, sample=n, epochs=1, batch=32, margin=margin)
+        trained.append((st["loss"], st["mae"], st["coverage"]))
+    assert trained[0] == trained[1]
