@@ -219,6 +219,18 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 // 40,000 × 20 2.5 / 4.4, 80,000 × 32 6.5 / 12.6, 161,443 × 32 14.9 / 39.8).
 bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 16384; }
 
+// How many candidates a row the coarse passes keep at most: 128, and 64 for 40 < d ≤ 64 where k leaves
+// room. The tensor-core pass holds 64, so 64 keeps such a call there (160,000 × 64, k = 40: 9.3 ms with
+// 64 candidates, 118.6 with 80 on the FP32 pass); in the FP32 pass 128 rows' buffers of more than 64
+// candidates and a tile this deep leave one CTA to an SM (16,383 × 64, k = 60: 3.4 ms with 64, 4.9 with 120;
+// 60,000 × 64, k = 56: 20.6 and 25.1). With fewer than 4 candidates to spare the rows that the certificate
+// fails cost more than the buffers once lists cut the pass short (60,000 × 64 clustered, k = 63: 18.9 ms with
+// 64, 12.2 with 126; 16,383 × 64: 3.8 and 4.9).
+int coarse_most(int n, int d, int k, bool tensor_cores) {
+    if (d <= 40 || d > 64 || k >= 64) return 128;
+    return k <= 60 || tensor_cores || !fp32_lists_pay(n, d) ? 64 : 128;
+}
+
 // The tensor-core pass visits its tiles in row order below this many rows: the order stage costs more than
 // the lists and the earlier thresholds save (whole kNN on the device, row order / locality order:
 // 5,003 × 17 0.21 / 0.51 ms, 16,000 × 32 0.41 / 0.72, 24,000 × 15 0.80 / 0.96).
@@ -308,26 +320,18 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     int cap = (int)std::min<uint64_t>((uint64_t)k + margin, (uint64_t)n - 1);
     const int dp = coarse_dpad(d);
     const int np = round_up(n, 128);
-    // The coarse passes keep at most 128 candidates a row (fewer for 40 < d ≤ 64, where the query
-    // tile shares the shared memory). The over-selection m changes only how often the certificate
-    // holds, never the output (knn.rs:45-52), so a larger k + m runs with the largest candidate count
-    // the FP32 kernel holds that still exceeds k (rows the certificate then fails take the regather);
-    // when none does, every candidate is scanned exactly in f64 (knn.rs:884-924).
-    bool scan_all = false;
-    auto fits = [&](int c) { return coarse_fp32_holds(dp, c); };
-    if (!fits(cap)) {
-        int smaller = 0;
-        for (int c : {128, 64, 32})
-            if (c < cap && c > k && fits(c)) {
-                smaller = c;
-                break;
-            }
-        if (smaller) {
-            cap = smaller;
-            margin = (uint64_t)(cap - k);
-        } else {
-            scan_all = true;
-        }
+    // The over-selection m changes only how often the certificate holds, never the output (knn.rs:45-52),
+    // so a larger k + m runs with as many candidates as the passes hold (rows the certificate then fails
+    // take the regather); where k itself is beyond them, every candidate is scanned exactly in f64
+    // (knn.rs:884-924).
+    const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
+    const bool tc_backend = o.backend == COSTAL_BACKEND_BF16 || o.backend == COSTAL_BACKEND_BF16X3 ||
+                            o.backend == COSTAL_BACKEND_FP8;
+    const int most = coarse_most(n, d, k, tc_backend && !tanimoto);
+    const bool scan_all = cap > most && k >= most;
+    if (cap > most && !scan_all) {
+        cap = most;
+        margin = (uint64_t)(cap - k);
     }
     if (shard && o.select == COSTAL_SELECT_TANIMOTO)
         throw Fail{COSTAL_EUNSUPPORTED, "row shards support cosine selection only"};
@@ -352,9 +356,6 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     CK(ensure(c.fb_rows, (size_t)n * 4));
     CK(ensure(c.fb_minsim, (size_t)n * 8));
     CK(cudaEventRecord(c.ev[0], s));
-    const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
-    const bool tc_backend = o.backend == COSTAL_BACKEND_BF16 || o.backend == COSTAL_BACKEND_BF16X3 ||
-                            o.backend == COSTAL_BACKEND_FP8;
     // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
     const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
                             (tanimoto ? prune::supported(d) : !tc_backend && fp32_lists_pay(n, d));

@@ -68,3 +68,17 @@ def test_labels_of_lists_with_room_for_every_row(ext, n, d):
         st = ext._mlp_train(x, k, sample=n, epochs=1, batch=32, margin=margin)
         trained.append((st["loss"], st["mae"], st["coverage"]))
     assert trained[0] == trained[1]
+
+
+@pytest.mark.parametrize("matmul,d,k,margin,kept", [
+    ("bf16", 50, 40, None, 64), ("bf16", 64, 63, None, 64), ("bf16", 41, 33, 95, 64), ("fp8", 64, 50, 10, 64),
+    ("fp32", 64, 40, None, 64), ("fp32", 48, 60, 100, 64), ("fp32", 40, 40, None, 80), ("fp32", 65, 40, None, 80),
+    ("fp32", 64, 64, None, 128), ("fp32", 64, 30, None, 60)])
+def test_candidates_kept_where_the_passes_hold_64(ext, oracle, matmul, d, k, margin, kept):
+    """k + m above 64 at 40 < d ≤ 64: 64 candidates while k is below, which the tensor-core pass holds."""
+    x = clustered(700, d, d + k)
+    (idx, cos, norms), st = ext._knn_exact(x, k, margin=margin, matmul=matmul)
+    assert st["margin"] == kept - k
+    assert (st["coarse_kind"] == "fp32") == (matmul == "fp32")
+    for a, b in zip((idx.view(np.uint32), cos, norms), oracle.knn_bruteforce(x, k)):
+        np.testing.assert_array_equal(a, b)
