@@ -187,10 +187,15 @@ struct __align__(8) Barriers {
     float warp_floor[4];   // per epilogue warp: min over its rows of τ − E (never decreases)
 };
 
-// Entries of a query's buffer: 64 for cap ≤ 32, 128 for cap ≤ 64, and 80 for the split-FP8 kind (cap ≤ 64),
-// whose 48 KB stages then are three instead of two.
-__host__ __device__ constexpr int tc_bcap(int slots, bool fp8) { return fp8 && slots == 2 ? 80 : 64 * slots; }
-__host__ __device__ constexpr int tc_slots(int slots, bool fp8) { return (tc_bcap(slots, fp8) + 31) / 32; }
+// Entries of a query's buffer: 64 for cap ≤ 32, 128 for cap ≤ 64; narrow: 80 for cap ≤ 64 (fp8_narrow).
+__host__ __device__ constexpr int tc_bcap(int slots, bool narrow) { return narrow && slots == 2 ? 80 : 64 * slots; }
+__host__ __device__ constexpr int tc_slots(int slots, bool narrow) { return (tc_bcap(slots, narrow) + 31) / 32; }
+// The split-FP8 kind's 48 KB stages are three with 80-entry buffers, two with 128: the MMAs of n²·d products
+// then wait less for their operands, but a buffer is cut every 6 admissions instead of every 37, and a
+// query's admissions hardly grow with n. Coarse pass with 80 / 128 entries: 3,000 × 520 1.03 / 0.35 ms,
+// 20,000 × 520 3.50 / 1.60, 70,000 × 520 11.1 / 9.2, 40,000 × 1,000 7.6 / 7.3, 20,000 × 2,000 4.9 / 4.9,
+// 70,000 × 1,000 14.5 / 16.3, 40,000 × 2,000 12.4 / 14.2.
+static bool fp8_narrow(int n, int d) { return (long long)n * d >= 50'000'000; }
 
 // Per-query candidate buffer: BCAP entries in shared memory, [entry][query] with a row
 // stride of BLOCK_M + 1 words (appends of 32 lanes and the warp's reads of one query are both free
@@ -386,7 +391,7 @@ __device__ __forceinline__ void admit_slice(const uint32_t (&r)[64], int cb, int
     }
 }
 
-template <int SLOTS, bool KLOOP, bool FP8 = false, bool PAIR = false>
+template <int SLOTS, bool KLOOP, bool FP8 = false, bool PAIR = false, bool NARROW = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_coarse_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_bw, int n, int np,
@@ -398,13 +403,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 uint32_t* __restrict__ cand_idx, float* __restrict__ cand_score, float* __restrict__ tau_out,
                 unsigned long long* __restrict__ stopped_total, unsigned long long* __restrict__ timeout_flag,
                 int qb0) {
-    constexpr int SL = tc_slots(SLOTS, FP8);  // buffer slots per lane in a flush
+    constexpr int SL = tc_slots(SLOTS, NARROW);  // buffer slots per lane in a flush
     // The split-FP8 kind computes on the rows scaled by 2^8, so its accumulators hold 2^16 × the
     // coarse score: thresholds and admissions stay in those units, the lists and floors are scaled
     // back exactly.
     constexpr float OSCALE = FP8 ? 0x1p-16f : 1.0f;
     constexpr int KBE = FP8 ? 128 : KB;  // elements in one 128-byte K block (the TMA x coordinate step)
-    constexpr int BCAP = tc_bcap(SLOTS, FP8);
+    constexpr int BCAP = tc_bcap(SLOTS, NARROW);
     extern __shared__ unsigned char smem_raw[];
     // 1024-byte alignment for the swizzled tiles
     const uint32_t base_u32 = smem_u32(smem_raw);
@@ -1331,8 +1336,8 @@ static Shape shape_fp8(int d) {
     return s;
 }
 
-static size_t fixed_smem(const Shape& sh, int cap, bool fp8 = false) {
-    const int bcap = tc_bcap(cap <= 32 ? 1 : 2, fp8);
+static size_t fixed_smem(const Shape& sh, int cap, bool narrow = false) {
+    const int bcap = tc_bcap(cap <= 32 ? 1 : 2, narrow);
     return 1024 + (sh.resident ? (size_t)sh.nkb_a * A_KB_BYTES : 0) + (size_t)(BLOCK_M + 1) * bcap * 8 + sizeof(Barriers);
 }
 static size_t stage_smem(const Shape& sh) {
@@ -1348,7 +1353,7 @@ bool supported(int d, int cap) {
 bool supported_fp8(int d, int cap) {
     if (d < 1 || cap < 1 || cap > 64 || 3 * d <= 128) return false;
     const Shape sh = shape_fp8(d);
-    return fixed_smem(sh, cap, true) + stage_smem(sh) <= 227 * 1024;
+    return fixed_smem(sh, cap) + stage_smem(sh) <= 227 * 1024;
 }
 
 size_t workspace_bytes(int n, int d, bool fp8) {
@@ -1452,7 +1457,8 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
         !make_map(&mbw, plan.ops_b, plan.kpb, plan.np, BLOCK_N, plan.fp8))
         return cudaErrorInvalidValue;
     const Shape sh = plan.fp8 ? shape_fp8(plan.d) : shape_of(plan.d);
-    const size_t fixed = fixed_smem(sh, cap, plan.fp8), per = stage_smem(sh);
+    const bool narrow = plan.fp8 && fp8_narrow(plan.n, plan.d);
+    const size_t fixed = fixed_smem(sh, cap, narrow), per = stage_smem(sh);
     int stages = 4;
     while (stages > 1 && fixed + (size_t)stages * per > 227 * 1024) --stages;
     // (resident query tile) an even number of tiles in the ring, if two fit: one MMA warp per accumulator
@@ -1463,7 +1469,8 @@ cudaError_t launch_coarse(const Plan& plan, int cap, const uint32_t* lists, cons
     const int qblocks = (plan.n + BLOCK_M - 1) / BLOCK_M;
     if (qb1 < 0) qb1 = qblocks;
     if (qb0 < 0 || qb1 > qblocks || qb0 >= qb1) return cudaErrorInvalidValue;
-    auto kern = plan.fp8 ? (cap <= 32 ? k_coarse_tc<1, true, true> : k_coarse_tc<2, true, true>)
+    auto kern = plan.fp8 ? (cap <= 32 ? k_coarse_tc<1, true, true>
+                            : narrow ? k_coarse_tc<2, true, true, false, true> : k_coarse_tc<2, true, true>)
                 : !sh.resident ? (pair ? (cap <= 32 ? k_coarse_tc<1, true, false, true> : k_coarse_tc<2, true, false, true>)
                                        : (cap <= 32 ? k_coarse_tc<1, true> : k_coarse_tc<2, true>))
                                : (pair ? (cap <= 32 ? k_coarse_tc<1, false, false, true> : k_coarse_tc<2, false, false, true>)

@@ -82,3 +82,14 @@ def test_candidates_kept_where_the_passes_hold_64(ext, oracle, matmul, d, k, mar
     assert (st["coarse_kind"] == "fp32") == (matmul == "fp32")
     for a, b in zip((idx.view(np.uint32), cos, norms), oracle.knn_bruteforce(x, k)):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,d", [(24_400, 2048), (24_415, 2048), (97_657, 512)])
+def test_split_fp8_with_either_buffer(ext, n, d):
+    """Both sides of the size from which the split-FP8 kind takes three stages and 80-entry buffers
+    (n·d = 50,000,000): the answer equals the FP32 pass's."""
+    x = clustered(n, d, n + d, n_centers=40, noise=1.5)
+    got, st = ext._knn_exact(x, 10, matmul="bf16")
+    assert st["coarse_kind"] == "fp8" and st["max_err_ratio"] < 1.0
+    for a, b in zip(got, ext._knn_exact(x, 10)[0]):
+        np.testing.assert_array_equal(a, b)
