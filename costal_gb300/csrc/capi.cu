@@ -415,7 +415,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
         CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                           c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps_t, cap < n - 1, 1, nullptr,
                           nullptr, d_idx, d_cos, d_w, c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(),
-                          &dm->fb_count, dm->max_err_bits, s));
+                          &dm->fb_count, dm->max_err_bits, false, s));
         CK(cudaEventRecord(c.ev[3], s));
         if (cap < n - 1) {
             if (gather_smem(k, d, dp) > 227 * 1024)
@@ -496,7 +496,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                                   c.tau.as<float>(), d_norms, plan.row_eps, learned ? pp.row_ub : nullptr,
                                   &dm->prune_fail_count, 0.0, 1, 0, srows, scount, d_idx, d_cos, d_w,
                                   c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count,
-                                  dm->max_err_bits, s));
+                                  dm->max_err_bits, fp8, s));
             // How many rows failed decides the re-run's shape (few rows: the columns split across CTAs).
             CK(cudaMemcpyAsync(&c.h_misc->tc_fail_count, &dm->tc_fail_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
                                s));
@@ -510,7 +510,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                 CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                   c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps, cap < n - 1, 0,
                                   c.tc_rows.as<uint32_t>(), &dm->tc_fail_count, d_idx, d_cos, d_w,
-                                  c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, s));
+                                  c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, false, s));
             }
             CK(cudaEventRecord(c.ev[3], s));
         } else {
@@ -531,7 +531,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                 CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                   c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps, cap < n - 1, 0, srows,
                                   scount, d_idx, d_cos, d_w, c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(),
-                                  &dm->fb_count, dm->max_err_bits, s));
+                                  &dm->fb_count, dm->max_err_bits, false, s));
             CK(cudaEventRecord(c.ev[3], s));
         }
         if (cap < n - 1) {
@@ -1036,7 +1036,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
             CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                               c.tau.as<float>(), c.norms.as<double>(), plan.row_eps, nullptr, nullptr, 0.0, 1, 0, rows,
                               &dm->shard_rows, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
-                              c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count, nullptr, s));
+                              c.tc_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->tc_fail_count, nullptr, false, s));
             CK(cudaMemcpyAsync(&c.h_misc->tc_fail_count, &dm->tc_fail_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
                                s));
             CK(cudaStreamSynchronize(s));
@@ -1055,7 +1055,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
             CK(launch_rescore(c.x.as<float>(), N, D, K, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                               c.tau.as<float>(), c.norms.as<double>(), nullptr, nullptr, nullptr, eps, cap < N - 1, 0,
                               frows, fcount, c.out_idx.as<uint32_t>(), c.out_cos.as<double>(), nullptr,
-                              c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, s));
+                              c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, false, s));
         }
         if (cap < N - 1)
             CK(launch_gather(c.x.as<float>(), c.xsT.as<float>(), N, np, D, dp, K, c.norms.as<double>(),

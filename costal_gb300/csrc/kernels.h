@@ -58,12 +58,13 @@ cudaError_t launch_rerun_floor(const uint32_t* rows, const unsigned* count, int 
                                cudaStream_t st);
 // Self-check of the integer f32 → f64 conversion used by the f64 dot products (all 2³² patterns).
 cudaError_t launch_check_f64_of(unsigned long long* mismatches, int sm_count, cudaStream_t st);
+// wide_bound: the coarse scores' bound keeps most candidates (deep rows then drop some by f32 cosines).
 cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lstride, const uint32_t* cand_idx,
                            const float* cand_score, const float* tau, const double* norms, const double* row_eps,
                            const double* row_ub, unsigned* ub_fail, double eps, int certify, int select,
                            const uint32_t* rlist, const unsigned* rcount,
                            uint32_t* out_idx, double* out_cos, double* out_w, uint32_t* fb_rows, double* fb_minsim,
-                           unsigned* fb_count, unsigned long long* max_err_bits, cudaStream_t st);
+                           unsigned* fb_count, unsigned long long* max_err_bits, bool wide_bound, cudaStream_t st);
 int gather_capb(int k);
 size_t gather_smem(int k, int d, int dp);
 cudaError_t launch_gather(const float* x, const float* xsT, int n, int np, int d, int dp, int k, const double* norms,

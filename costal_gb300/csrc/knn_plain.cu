@@ -202,7 +202,7 @@ __device__ __forceinline__ uint32_t warp_kth_key(const uint32_t (&key)[SLOTS], i
 //     a candidate whose coarse score is below c_k − 2E scores below s_k exactly and can neither enter
 //     the top-k nor change s_k. Only the others are rescored (cosine selection; E the row's coarse
 //     error bound); they are packed into one list for the CTA.
-// (½) Deep rows: one warp per row takes each packed candidate's cosine in f32 over the normalised rows
+// (½) Deep rows of a coarse pass with a wide bound (the split-FP8 kind): one warp per row takes each packed candidate's cosine in f32 over the normalised rows
 //     (lanes over the dimensions, within δ = (d/32 + 22)·2⁻²³ of the exact one: a lane's chain of at most
 //     d/32 + 4 FMAs and five lane sums, 3 roundings for each normalised factor, Cauchy–Schwarz with unit
 //     rows, and a factor two) and drops by it what (0) could not by the coarse score: c'_k − 2δ in place
@@ -662,7 +662,7 @@ cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lst
                            const double* row_ub, unsigned* ub_fail, double eps, int certify, int select,
                            const uint32_t* rlist, const unsigned* rcount,
                            uint32_t* out_idx, double* out_cos, double* out_w, uint32_t* fb_rows, double* fb_minsim,
-                           unsigned* fb_count, unsigned long long* max_err_bits, cudaStream_t st) {
+                           unsigned* fb_count, unsigned long long* max_err_bits, bool wide_bound, cudaStream_t st) {
     const int slots = coarse_slots(cap);
     // deep rows: three CTAs per SM (their streamed rows fit L1); otherwise one CTA per group
     static int sms = 0;
@@ -674,8 +674,13 @@ cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lst
     }
     const int groups = (n + RS_ROWS - 1) / RS_ROWS;
     const int blocks = d >= 256 ? std::min(groups, 3 * sms) : groups;
-    auto kern = d >= 256 ? (slots == 1 ? k_rescore<1, true> : slots == 2 ? k_rescore<2, true> : k_rescore<4, true>)
-                         : (slots == 1 ? k_rescore<1, false> : slots == 2 ? k_rescore<2, false> : k_rescore<4, false>);
+    // Phase ½ where the coarse bound is wide (split FP8): 70,000 × 2,000, k = 10 345 ms of rescoring without
+    // it, 337 with, 100,000 × 2,000 of scRNA-like counts 33 and 19. Where the coarse scores are sharper it
+    // rules out too few: split BF16, 8,000 × 400, k = 15 0.41 without and 0.49 with, FP32, 8,000 × 1,000
+    // 0.40 and 0.50.
+    auto kern = wide_bound && d >= 256 && slots <= 2
+                    ? (slots == 1 ? k_rescore<1, true> : k_rescore<2, true>)
+                    : (slots == 1 ? k_rescore<1, false> : slots == 2 ? k_rescore<2, false> : k_rescore<4, false>);
     kern<<<blocks, 256, 0, st>>>(x, n, d, k, cap, lstride, cand_idx, cand_score, tau, norms, row_eps, row_ub, ub_fail, eps,
                                  certify, select, rlist, rcount, out_idx, out_cos, out_w, fb_rows, fb_minsim, fb_count,
                                  max_err_bits);
