@@ -213,17 +213,24 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
     return mlp::block_min(c.mlp_pred.as<float>(), pp.perm, n, pp.tq, s);
 }
 
-// Whether the FP32 pass visits its columns by lists, nearest blocks first with the exact early stop,
-// instead of all tiles in order: where the tiles and admissions it saves cost more than the order stage
-// (measured, whole kNN, lists / all tiles: 12,000 × 32 0.94 / 0.78 ms, 20,000 × 32 1.5 / 1.7,
-// 40,000 × 20 2.5 / 4.4, 80,000 × 32 6.5 / 12.6, 161,443 × 32 14.9 / 39.8).
-bool fp32_lists_pay(int n, int d) { return prune::supported(d) && n >= 16384; }
+// Whether the FP32 pass visits its columns by lists, nearest blocks first with the exact early stop, instead
+// of all tiles in order. With more query blocks than SMs the last wave of all tiles is nearly empty, and
+// clustered rows gain more with every row (whole kNN, lists / all tiles: 20,000 × 32 1.55 / 1.72 ms,
+// 40,000 × 20 2.5 / 4.4, 161,443 × 32 14.9 / 39.8; Gaussian rows lose the order stage, 22,000 × 32 2.12 / 1.85,
+// 160,000 × 64 64.6 / 63). With fewer, the order stage costs about what the lists save of clustered shallow
+// rows (16,384 × 8 0.92 / 0.97, 19,000 × 16 1.18 / 1.15), and deeper rows only lose by it (19,000 × 32 1.43 /
+// 1.34, Gaussian 1.77 / 1.34; 19,000 × 64 2.02 / 1.77, Gaussian 2.36 / 1.77).
+bool fp32_lists_pay(int n, int d) {
+    return prune::supported(d) && n >= (d <= 16 ? 16384 : 152 * 128 + 1);
+}
+// Tanimoto selection takes the norm order below this many rows.
+constexpr int TANI_LIST_ROWS = 16384;
 
 // How many candidates a row the coarse passes keep at most: 128, and 64 for 40 < d ≤ 64 where k leaves
 // room. The tensor-core pass holds 64, so 64 keeps such a call there (160,000 × 64, k = 40: 9.3 ms with
 // 64 candidates, 118.6 with 80 on the FP32 pass); in the FP32 pass 128 rows' buffers of more than 64
-// candidates and a tile this deep leave one CTA to an SM (16,383 × 64, k = 60: 3.4 ms with 64, 4.9 with 120;
-// 60,000 × 64, k = 56: 20.6 and 25.1). With fewer than 4 candidates to spare the rows that the certificate
+// candidates and a tile this deep leave one CTA to an SM (16,383 × 64, k = 60: 2.6 ms with 64, 4.9 with 120;
+// 60,000 × 64, k = 60: 18.1 and 26.3). With fewer than 4 candidates to spare the rows that the certificate
 // fails cost more than the buffers once lists cut the pass short (60,000 × 64 clustered, k = 63: 18.9 ms with
 // 64, 12.2 with 126; 16,383 × 64: 3.8 and 4.9).
 int coarse_most(int n, int d, int k, bool tensor_cores) {
@@ -249,7 +256,7 @@ void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani
     Misc* dm = c.misc.as<Misc>();
     prune::Plan pp{};
     CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
-    bool by_norm = tani_norms && !fp32_lists_pay(n, d);
+    bool by_norm = tani_norms && n < TANI_LIST_ROWS;
     if (tani_norms && !by_norm) {
         CK(prune::norm_window_share(tani_norms, n, dm->norm_share, s));
         CK(cudaMemcpyAsync(c.h_misc->norm_share, dm->norm_share, 8, cudaMemcpyDeviceToHost, s));

@@ -574,36 +574,41 @@ __global__ void k_merge_parts(const uint32_t* __restrict__ qlist, int count, int
 
 // The launch shape for a depth and a candidate count: the query operand resident or streamed, the
 // buffer's entries, the dimensions and number of the ring's stages, CTAs per SM. Two CTAs per SM with
-// buffers of cap + 32 entries if they fit, else down to cap + 16, else one CTA per SM.
+// buffers of cap + 32 entries if they fit, else down to cap + 16. Where a resident query operand leaves room
+// for one only (about 48 candidates and more at d = 64): with more query blocks than SMs (many) the query
+// operand is streamed so that two fit (60,000 × 64 Gaussian rows, k = 30 20.0 -> 16.8 ms, Tanimoto 29.6 ->
+// 22.6); with fewer, one wave of single CTAs starts cold once for a query block where two CTAs would be two
+// halves of one (8,000 × 48, k = 40 1.15 with one, 1.41 with two; 16,383 × 48 2.35 and 3.12).
 struct Shape {
     bool stream;
     int bcap, kc, stages, ctas;
     size_t smem;
 };
 
-static Shape shape_of(int dp, int cap) {
+static Shape shape_of(int dp, int cap, bool many) {
     for (int ctas = 2; ctas >= 1; --ctas)
-        for (int extra = 32; extra >= 16; extra -= 8) {
-            Shape s{};
-            s.ctas = ctas;
-            s.stream = dp > 64;
-            s.bcap = (cap + extra + 3) / 4 * 4;
-            const size_t lim = ctas == 2 ? SMEM_TWO : SMEM_ONE;
-            const size_t fixed = 128 + (size_t)BM * s.bcap * 8 + BM * 12 + sizeof(Bars) + (s.stream ? 0 : (size_t)dp * BM * 4);
-            if (fixed >= lim) continue;
-            // the deepest stage of which two fit (whole tiles), else three
-            const int most = s.stream ? 16 : dp;
-            for (int kc = most; kc >= 8; kc -= 8) {
-                if (!s.stream && dp % kc) continue;
-                const size_t per = (size_t)kc * BN * 4 * (s.stream ? 2 : 1);
-                const int stages = (int)std::min<size_t>(MAX_STAGES, (lim - fixed) / per);
-                if (stages < (kc == dp ? 2 : 3)) continue;
-                s.kc = kc;
-                s.stages = stages;
-                s.smem = fixed + stages * per;
-                return s;
+        for (int stream = dp > 64; stream < (dp > 64 || (ctas == 2 && many) ? 2 : 1); ++stream)
+            for (int extra = 32; extra >= 16; extra -= 8) {
+                Shape s{};
+                s.ctas = ctas;
+                s.stream = stream;
+                s.bcap = (cap + extra + 3) / 4 * 4;
+                const size_t lim = ctas == 2 ? SMEM_TWO : SMEM_ONE;
+                const size_t fixed = 128 + (size_t)BM * s.bcap * 8 + BM * 12 + sizeof(Bars) + (stream ? 0 : (size_t)dp * BM * 4);
+                if (fixed >= lim) continue;
+                // the deepest stage of which two fit (whole tiles), else three
+                const int most = stream ? 16 : dp;
+                for (int kc = most; kc >= 8; kc -= 8) {
+                    if (!stream && dp % kc) continue;
+                    const size_t per = (size_t)kc * BN * 4 * (stream ? 2 : 1);
+                    const int stages = (int)std::min<size_t>(MAX_STAGES, (lim - fixed) / per);
+                    if (stages < (kc == dp ? 2 : 3)) continue;
+                    s.kc = kc;
+                    s.stages = stages;
+                    s.smem = fixed + stages * per;
+                    return s;
+                }
             }
-        }
     return Shape{};
 }
 
@@ -622,10 +627,11 @@ static bool make_map(CUtensorMap* m, const void* base, size_t cols, int rows, in
 
 // Column segments for nq queries against `tiles` column tiles: the number whose last wave of CTAs
 // (`slots` at a time) ends first, a CTA costing its tiles plus `start` tiles' worth of time for loading
-// its queries, seeding and writing its lists (and the merge reading one more list).
-static int segments(int nq, int tiles, int dp, int slots) {
+// its queries, seeding, its first admissions (they grow with cap) and writing its lists (and the merge
+// reading one more list).
+static int segments(int nq, int tiles, int dp, int cap, int slots) {
     const int blocks = (nq + BM - 1) / BM;
-    const double start = 1.0 + 64.0 / dp;
+    const double start = 1.0 + 64.0 / dp + cap / 32.0;
     int best = 1;
     double best_t = 1e300;
     for (int s = 1; s <= std::min(256, tiles); ++s) {
@@ -639,6 +645,10 @@ static int segments(int nq, int tiles, int dp, int slots) {
         }
     }
     return best;
+}
+
+static Shape shape_of(const Fp32Job& J, int sm_count) {
+    return shape_of(J.dp, J.cap, (J.nq + BM - 1) / BM > sm_count);
 }
 
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -682,16 +692,17 @@ cudaError_t launch_work_cols(const float* xsR, const uint32_t* perm, int n, int 
 }
 
 // With lists the CTAs' lengths differ and fill each other's gaps: two waves of them are enough (every
-// segment starts cold: 100,003 × 15 Tanimoto 5.1 ms with 1 segment, 6.8 with 3), and a segment keeps at
-// least 24 entries (its stop comes a ring of stages after its thresholds have risen).
+// segment starts cold: 100,003 × 15 Tanimoto 5.1 ms with 1 segment, 6.8 with 3), and one wave of single CTAs,
+// whose start nothing hides (18,000 × 64 Tanimoto, k = 30 5.17 -> 4.34). A segment keeps at least 24 entries (its
+// stop comes a ring of stages after its thresholds have risen).
 static int segs_of(const Fp32Job& J, const fp32::Shape& sh, int sm_count) {
     const int blocks = (J.nq + fp32::BM - 1) / fp32::BM, slots = sm_count * sh.ctas;
-    if (!J.lists) return fp32::segments(J.nq, J.np / fp32::BN, J.dp, slots);
-    return std::max(1, std::min((2 * slots + blocks - 1) / blocks, J.ncb / 24));
+    if (!J.lists) return fp32::segments(J.nq, J.np / fp32::BN, J.dp, J.cap, slots);
+    return std::max(1, std::min(sh.ctas == 1 ? slots / blocks : (2 * slots + blocks - 1) / blocks, J.ncb / 24));
 }
 
 size_t coarse_fp32_ws_bytes(const Fp32Job& J, int sm_count) {
-    const fp32::Shape sh = fp32::shape_of(J.dp, J.cap);
+    const fp32::Shape sh = fp32::shape_of(J, sm_count);
     const int segs = segs_of(J, sh, sm_count);
     return fp32::carve(nullptr, J.dp, J.cap, J.rows != nullptr, J.nq, segs).bytes;
 }
@@ -730,7 +741,7 @@ cudaError_t launch_rerun_floor(const uint32_t* rows, const unsigned* count, int 
 cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStream_t st) {
     using namespace fp32;
     if (J.nq <= 0) return cudaSuccess;
-    const Shape sh = shape_of(J.dp, J.cap);
+    const Shape sh = shape_of(J, sm_count);
     if (sh.stages < 2) return cudaErrorInvalidValue;
     const int mp = (J.nq + BM - 1) / BM * BM, tiles = J.np / BN;
     const int segs = segs_of(J, sh, sm_count);
@@ -764,7 +775,7 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     P.counts = J.counts;
     // longest lists first (161,443 × 32 12.7 -> 11.5 ms); with segments the blocks' segments fill the last
     // wave already, and the order costs (30,000 × 15 1.2 -> 1.4 ms)
-    P.order = J.lists && segs == 1 && !sh.stream ? J.order : nullptr;
+    P.order = J.lists && segs == 1 ? J.order : nullptr;
     P.ncb = J.ncb;
     P.epc = J.list_cb / BN;
     P.eps = J.eps;
@@ -779,7 +790,7 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     P.timeout_flag = J.timeout_flag;
     const int slb = (sh.bcap + 31) / 32;
 #define COSTAL_T(S, ST, O) (J.norms ? k_fp32_tiles<S, ST, true, O> : k_fp32_tiles<S, ST, false, O>)
-#define COSTAL_K(S) (sh.stream ? COSTAL_T(S, true, false) : P.order ? COSTAL_T(S, false, true) : COSTAL_T(S, false, false))
+#define COSTAL_K(S) (sh.stream ? (P.order ? COSTAL_T(S, true, true) : COSTAL_T(S, true, false)) : P.order ? COSTAL_T(S, false, true) : COSTAL_T(S, false, false))
     auto kern = slb <= 2 ? COSTAL_K(2) : slb == 3 ? COSTAL_K(3) : COSTAL_K(5);
 #undef COSTAL_T
 #undef COSTAL_K
@@ -793,6 +804,6 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
 
 int coarse_dpad(int d) { return d <= 64 ? ((d < 1 ? 1 : d) + 7) / 8 * 8 : (d + 3) / 4 * 4; }
 
-bool coarse_fp32_holds(int dp, int cap) { return cap <= 128 && fp32::shape_of(dp, cap).stages >= 2; }
+bool coarse_fp32_holds(int dp, int cap) { return cap <= 128 && fp32::shape_of(dp, cap, false).stages >= 2; }
 
 }  // namespace costal

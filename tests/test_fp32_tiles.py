@@ -78,3 +78,22 @@ def test_tanimoto_by_lists(ext, oracle, n, d, k, spread, signed):
         for a, b in zip((got[0].view(np.uint32), got[1], got[2]), want):
             np.testing.assert_array_equal(a, b)
         assert prune or st["blocks_skipped"] == 0
+
+
+@pytest.mark.parametrize("n,d,k,margin", [(19_456, 30, 10, None), (19_457, 30, 10, None),  # all tiles | lists
+                                          (19_456, 64, 30, None), (19_457, 64, 30, None),  # one CTA an SM | two, streamed
+                                          (20_001, 41, 60, None), (21_000, 56, 63, None), (16_001, 48, 64, None)])
+@pytest.mark.parametrize("select", ["cosine", "tanimoto"])
+def test_fp32_pass_on_either_shape(ext, oracle, n, d, k, margin, select):
+    """Both sides of the size from which the lists are taken and a query operand that leaves room for one CTA
+    to an SM is streamed instead; the candidates kept (60, 64, 126, 128) decide the buffers."""
+    x = clustered(n, d, n + d)
+    if select == "tanimoto":
+        x = np.ascontiguousarray(x * np.random.default_rng(n).uniform(0.5, 2.0, size=(n, 1)).astype(np.float32))
+    want, _ = oracle.knn_exact(x, k, select=select)
+    got, st = ext._knn_exact(x, k, margin=margin, select=select)
+    for a, b in zip((got[0].view(np.uint32), got[1], got[2]), want):
+        np.testing.assert_array_equal(a, b)
+    assert st["max_err_ratio"] < 1.0
+    if select == "cosine":
+        assert (st["blocks_stopped"] > 0) == (n > 19_456)
