@@ -220,10 +220,12 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 // 160,000 × 64 64.6 / 63). With fewer, the order stage costs about what the lists save of clustered shallow
 // rows (16,384 × 8 0.92 / 0.97, 19,000 × 16 1.18 / 1.15), and deeper rows only lose by it (19,000 × 32 1.43 /
 // 1.34, Gaussian 1.77 / 1.34; 19,000 × 64 2.02 / 1.77, Gaussian 2.36 / 1.77).
+// And no further than the lists' sort: beyond, they would be in block order, without a stop, and cost 12 bytes
+// a block pair for nothing.
 bool fp32_lists_pay(int n, int d) {
-    return prune::supported(d) && n >= (d <= 16 ? 16384 : 152 * 128 + 1);
+    return prune::supported(d) && n >= (d <= 16 ? 16384 : 152 * 128 + 1) && prune::sortable(n);
 }
-// Tanimoto selection takes the norm order below this many rows.
+// Tanimoto selection takes the walk in the norm order below this many rows.
 constexpr int TANI_LIST_ROWS = 16384;
 
 // How many candidates a row the coarse passes keep at most: 128, and 64 for 40 < d ≤ 64 where k leaves
@@ -243,26 +245,68 @@ int coarse_most(int n, int d, int k, bool tensor_cores) {
 // 5,003 × 17 0.21 / 0.51 ms, 16,000 × 32 0.41 / 0.72, 24,000 × 15 0.80 / 0.96).
 constexpr int TC_ORDER_ROWS = 24576;
 
+// The buffers that the lists take beyond the plain pass (xsR, xsW and the order stage's in O(n); lists, bounds
+// and row maxima 12 bytes for every pair of query block and column block: 6.4 GB at 4,194,304 rows).
+struct ListBytes {
+    size_t xsR, xsW, prune_ws, tc_ws, rm_ws, rm_out;
+    size_t total() const { return xsR + xsW + prune_ws + tc_ws + rm_ws + rm_out; }
+};
+ListBytes list_bytes(int n, int d) {
+    const size_t nqb = ((size_t)n + 127) / 128, ncb = ((size_t)n + prune::col_block(n) - 1) / prune::col_block(n);
+    return {(size_t)n * d * 4, (size_t)coarse_dpad(d) * nqb * 128 * 4, prune::workspace_bytes(n, d),
+            tc::workspace_bytes(n, d, false), tc::rowmax_bytes((int)ncb, d), nqb * ncb * 4};
+}
+// Whether that much memory leaves a sixteenth of what is free, the buffers that it replaces included.
+bool lists_fit(size_t need, size_t held, size_t free_bytes) {
+    const size_t avail = free_bytes + held;
+    return need <= avail - avail / 16;
+}
+bool lists_fit_now(const Context& c, int n, int d) {
+    const ListBytes b = list_bytes(n, d);
+    size_t need = 0, held = 0;
+    auto grow = [&](const DevBuf& buf, size_t bytes) {
+        if (buf.bytes >= bytes) return;
+        need += bytes;
+        held += buf.bytes;
+    };
+    grow(c.xsR, b.xsR);
+    grow(c.xsW, b.xsW);
+    grow(c.prune_ws, b.prune_ws);
+    grow(c.tc_ws, b.tc_ws);
+    grow(c.rm_ws, b.rm_ws);
+    grow(c.rm_out, b.rm_out);
+    if (need < (256u << 20)) return true;  // (the query costs more than it could tell)
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return true;
+    return lists_fit(need, held, free_bytes);
+}
+
+// Tanimoto selection in the norm order, without lists: the rows sorted by norm, walked outward from each query
+// block's own tile until the norms alone bound every further score below its queries' thresholds
+// (knn.rs:595-644).
+void fp32_walk_job(Context& c, int n, int np, int d, int dp, const double* norms, double eps, Fp32Job& j, cudaStream_t s) {
+    prune::Walk w{};
+    CK(ensure(c.tani_ws, prune::norm_walk_bytes(n)));
+    CK(prune::norm_walk(c.tani_ws.p, norms, n, s, w));
+    CK(ensure(c.xsW, (size_t)dp * np * 4));
+    CK(launch_work_cols(c.xsR.as<float>(), w.perm, n, np, d, dp, c.xsW.as<float>(), s));
+    j.xsT = c.xsW.as<float>();
+    j.perm = w.perm;
+    j.walk = w.ranges;
+    j.walk_ends = w.ends;
+    j.eps = std::nextafterf((float)eps, INFINITY);
+    j.stopped_total = &c.misc.as<Misc>()->blocks_skipped;
+}
+
 // The FP32 pass by lists: the working order, the column lists and the rows' transposed copy in that order
-// (c.xsW) into the job. Cosine selection, and Tanimoto selection of enough rows, use the cells, bounds
-// and lists of the tensor-core path (the per-row bounds come from its split operands, with their
-// margin); Tanimoto selection bounds each block pair's score by its cosine bound and norm ranges, or
-// by the norm ranges alone in the norm order (knn.rs:595-644): with few rows, or where the norms are
-// spread so far that the window of a score of 0.9 leaves out more than half of all pairs (a block of
-// one cell spans its rows' whole norm range, so the cells' order cannot use the window: of 20,000 × 12
-// rows spread 8-fold in norm the norm order leaves out 60 % of the tiles, the cells' order 0.1 %;
-// of 100,003 × 15 cytometry-like rows the norm order 6 %, the cells' order 64 %).
-void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani_norms, double eps, Fp32Job& j, cudaStream_t s) {
+// (c.xsW) into the job. The cells, bounds and lists are those of the tensor-core path (the per-row bounds
+// come from its split operands, with their margin); Tanimoto selection bounds each block pair's score by its
+// cosine bound and norm ranges, or, in the norm order (by_norm), by the norm ranges alone.
+void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani_norms, bool by_norm, double eps, Fp32Job& j,
+                    cudaStream_t s) {
     Misc* dm = c.misc.as<Misc>();
     prune::Plan pp{};
     CK(ensure(c.prune_ws, prune::workspace_bytes(n, d)));
-    bool by_norm = tani_norms && n < TANI_LIST_ROWS;
-    if (tani_norms && !by_norm) {
-        CK(prune::norm_window_share(tani_norms, n, dm->norm_share, s));
-        CK(cudaMemcpyAsync(c.h_misc->norm_share, dm->norm_share, 8, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        by_norm = 2ull * c.h_misc->norm_share[1] < c.h_misc->norm_share[0];
-    }
     if (by_norm) {
         CK(ensure(c.tani_ws, prune::norm_order_bytes(n)));
         CK(prune::norm_plan(c.prune_ws.p, tani_norms, n, d, c.tani_ws.p, s, pp));
@@ -298,6 +342,26 @@ void fp32_lists_job(Context& c, int n, int np, int d, int dp, const double* tani
     j.eps = std::nextafterf((float)eps, INFINITY);
     // (Tanimoto selection's left-out blocks are reported as skipped, as its norm window's are)
     j.stopped_total = tani_norms ? &dm->blocks_skipped : &dm->blocks_stopped;
+}
+
+// Tanimoto selection by lists or by the walk: the walk with few rows (there it costs what norm lists cost, and
+// the cells' order stage more than it saves) and where lists would not be sorted or not fit. Lists in the norm
+// order where the norms are spread so far that the window of a score of 0.9 leaves out more than half of all
+// pairs (a block of one cell spans its rows' whole norm range, so the cells' order cannot use the window: of
+// 20,000 × 12 rows spread 8-fold in norm the norm order leaves out 60 % of the tiles, the cells' order 0.1 %;
+// of 100,003 × 15 cytometry-like rows the norm order 6 %, the cells' order 64 %); 400,000 × 15 rows spread
+// 7-fold take 134 ms by norm lists and 154 by the walk for the same tiles, 100,000 × 15 18.5 and 17.4.
+void tani_job(Context& c, int n, int np, int d, int dp, const double* norms, double eps, Fp32Job& j, cudaStream_t s) {
+    if (n < TANI_LIST_ROWS || !prune::sortable(n) || !lists_fit_now(c, n, d)) {
+        fp32_walk_job(c, n, np, d, dp, norms, eps, j, s);
+        return;
+    }
+    Misc* dm = c.misc.as<Misc>();
+    CK(prune::norm_window_share(norms, n, dm->norm_share, s));
+    CK(cudaMemcpyAsync(c.h_misc->norm_share, dm->norm_share, 8, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    const bool by_norm = 2ull * c.h_misc->norm_share[1] < c.h_misc->norm_share[0];
+    fp32_lists_job(c, n, np, d, dp, norms, by_norm, eps, j, s);
 }
 
 // One shard of the query rows (a multi-GPU run gives each rank one): the rows are cut into query
@@ -365,7 +429,8 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     CK(cudaEventRecord(c.ev[0], s));
     // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
     const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
-                            (tanimoto ? prune::supported(d) : !tc_backend && fp32_lists_pay(n, d));
+                            (tanimoto ? prune::supported(d)
+                                      : !tc_backend && fp32_lists_pay(n, d) && lists_fit_now(c, n, d));
     // the tensor-core pass in the locality order, with lists (a shard is a range of that order)
     const bool tc_ordered = tc_backend && !tanimoto && !scan_all && prune::supported(d) &&
                             (n >= TC_ORDER_ROWS || shard || (o.learned_prune && c.mlp.ready && c.mlp.d == d && c.mlp.k == k));
@@ -413,7 +478,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
         Fp32Job j = fp32_job(c, n, np, dp, cap);
         j.norms = d_norms;
         if (fp32_lists) {
-            fp32_lists_job(c, n, np, d, dp, d_norms, eps_t, j, s);
+            tani_job(c, n, np, d, dp, d_norms, eps_t, j, s);
             list_cb = j.list_cb;
             CK(cudaEventRecord(c.ev[5], s));
         }
@@ -524,7 +589,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             if (!shard) {
                 Fp32Job j = fp32_job(c, n, np, dp, cap);
                 if (fp32_lists) {
-                    fp32_lists_job(c, n, np, d, dp, nullptr, eps, j, s);
+                    fp32_lists_job(c, n, np, d, dp, nullptr, false, eps, j, s);
                     list_cb = j.list_cb;
                     CK(cudaEventRecord(c.ev[5], s));
                 }
@@ -659,6 +724,24 @@ int costal_check_f64_conversion(uint64_t* mismatches, char* err, size_t errlen) 
         CK(cudaStreamSynchronize(s));
         *mismatches = c.h_misc->conv_mismatches;
     });
+}
+
+int costal_fp32_list_bytes(uint64_t n, uint32_t d, const costal_knn_opts* opts, uint64_t free_bytes, uint64_t* bytes,
+                           char* err, size_t errlen) {
+    const costal_knn_opts o = opts ? *opts : defaults();
+    if (n == 0 || n > (uint64_t)INT32_MAX || d == 0 || !bytes) {
+        put_err(err, errlen, "n or d out of range");
+        return COSTAL_EINVAL;
+    }
+    *bytes = 0;
+    const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
+    if (!o.prune || !prune::supported((int)std::min<uint32_t>(d, 65))) return COSTAL_OK;
+    if (tanimoto ? (int64_t)n < TANI_LIST_ROWS || !prune::sortable((int)n)
+                 : o.backend != COSTAL_BACKEND_FP32 || !fp32_lists_pay((int)n, (int)d))
+        return COSTAL_OK;
+    const size_t need = list_bytes((int)n, (int)d).total();
+    if (lists_fit(need, 0, free_bytes)) *bytes = need;
+    return COSTAL_OK;
 }
 
 int costal_row_l2_norms(const float* x, uint64_t n, uint32_t d, float* out, char* err, size_t errlen) {

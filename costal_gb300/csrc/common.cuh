@@ -79,6 +79,19 @@ __device__ __forceinline__ float tani_coarse_f32(float c, float2 qn, float2 cn) 
     return (dn == 0.0f || den <= 0.0f) ? 0.0f : __fdiv_rn(dn, den);
 }
 
+// Tanimoto selection (knn.rs:239-283): with ρ the quotient of two rows' norms, T = c / (ρ + 1/ρ − c) grows
+// with their cosine c > 0, so over two blocks whose cosines are ≤ u and whose norms lie in [a.x, a.y] and
+// [b.x, b.y], T ≤ u / (m − u) with m = the smallest ρ + 1/ρ there (2 where the ranges meet), and T ≤ 0 for
+// u ≤ 0. Roundings go outward (the ranges arrive rounded outward to f32).
+__device__ __forceinline__ float tani_ub_f32(float u, float2 a, float2 b) {
+    if (u <= 0.0f) return 0.0f;
+    float r = 1.0f;
+    if (a.x > b.y) r = __fdiv_rd(a.x, b.y);
+    else if (b.x > a.y) r = __fdiv_rd(b.x, a.y);
+    const float m = r > 1.0f ? __fadd_rd(r, __fdiv_rd(1.0f, r)) : 2.0f;  // (r = +inf: no pair of live rows)
+    return fminf(1.0f, __fdiv_ru(u, __fsub_rd(fmaxf(m, 2.0f), u)));
+}
+
 // Rust's f64::total_cmp as a signed integer key (knn.rs:589-591 sorts with it).
 __device__ __forceinline__ long long total_key(double v) {
     long long b = __double_as_longlong(v);

@@ -28,6 +28,10 @@
 //             tiles, and the CTA stops at the first block whose bound is below every query's τ − ε (its
 //             columns' coarse scores are ≤ bound + ε, so none could be admitted; later bounds are no
 //             larger).
+//   walk      Tanimoto selection in the norm order (knn.rs:595-644): a CTA visits its own tile first and
+//             then outward on both sides, and leaves a side where the bound that the norms alone give is
+//             below every query's τ − ε. O(n) memory at any n, where lists take 12 bytes for every pair of
+//             blocks.
 //   segments  Few query blocks: the columns are split over gridDim.y CTAs per block and the segments'
 //             lists merged per row (k_merge_parts), so that no SM idles in a nearly empty last wave.
 //             The segments of a query share their thresholds whenever one of them cuts its buffer.
@@ -196,6 +200,8 @@ struct Args {
     const uint32_t* order; // the query block of each CTA (NULL: in order)
     int ncb, epc;          // list stride; 128-column tiles per list entry
     float eps;             // the coarse error bound, rounded up
+    const float2* walk;      // norm ranges of the tiles, and what lies after and before them (kernels.h)
+    const float2* walk_ends;
     unsigned long long* stopped_total;
     uint32_t* tau_shared;  // with segments: order key of each slot's largest threshold so far
     const float* tfloor;   // by row: no column at or below it can be among the best cap (NULL: none)
@@ -222,7 +228,13 @@ __device__ __forceinline__ float tani_cos_floor(float tau) {
                                  : 2.0f * __fdividef(tau, 1.0f + tau) * (1.0f - 0x1p-16f);
 }
 
-template <int SLB, bool STREAM, bool TANI, bool ORDER>
+enum Visit {
+    IN_ORDER,  // all tiles in order, or the lists of the query blocks in order
+    BY_ORDER,  // the lists, the query block of each CTA from P.order
+    WALK       // outward in the norm order
+};
+
+template <int SLB, bool STREAM, bool TANI, Visit VISIT>
 __global__ void __launch_bounds__(NT, 2)
     k_fp32_tiles(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Args P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -240,7 +252,7 @@ __global__ void __launch_bounds__(NT, 2)
     Bars* bars = reinterpret_cast<Bars*>(own_s + BM);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // (a template parameter: with the choice made at run time the whole kernel was 7 % slower)
-    const int qb = ORDER ? (int)P.order[blockIdx.x] : (int)blockIdx.x, q0 = qb * BM;
+    const int qb = VISIT == BY_ORDER ? (int)P.order[blockIdx.x] : (int)blockIdx.x, q0 = qb * BM;
     const int nch = (P.dp + kc - 1) / kc;
     if (tid == 0) {
         mbar_init(&bars->a_full, 1);
@@ -288,7 +300,35 @@ __global__ void __launch_bounds__(NT, 2)
             return true;
         };
         const int seg = (int)blockIdx.y, segs = (int)gridDim.y;
-        if (P.lists) {  // the segment's list entries: every segs-th one
+        if (VISIT == WALK) {  // the segment's steps of the walk: every segs-th one
+            // Steps alternate between the sides while both last, own tile first, so that a step's tile needs no
+            // other step's bound (chosen by bound, a segment had to follow all steps: 3 to 7 % slower). A side
+            // ends at its first tile whose bound is below the floors: later ones are no larger.
+            const float2 nq = P.walk[qb];
+            const int nl = qb + 1, nr = P.tiles - nl, both = 2 * min(nl, nr);
+            bool l_out = false, r_out = false;
+            unsigned out = 0;
+            for (int e = seg; e < P.tiles; e += segs) {
+                const bool left = e < both ? !(e & 1) : nl > nr;
+                const int i = e < both ? e >> 1 : e - both / 2, t = left ? qb - i : nl + i;
+                if (!(left ? l_out : r_out)) {
+                    const float2 ends = P.walk_ends[t];
+                    const float ub = tani_ub_f32(1.0f, nq, left ? make_float2(0.0f, ends.y) : make_float2(ends.x, CUDART_INF_F));
+                    volatile float* wf = bars->warp_floor;  // may be stale, i.e. lower: that only delays the stop
+                    if (!(ub < fminf(fminf(wf[0], wf[1]), fminf(wf[2], wf[3])))) {
+                        if (!send_tile(t * BN)) return;
+                        continue;
+                    }
+                    (left ? l_out : r_out) = true;
+                }
+                if ((l_out && r_out) || e >= both) {  // only tiles of a side that has ended are left
+                    out += (unsigned)((P.tiles - e + segs - 1) / segs);
+                    break;
+                }
+                ++out;
+            }
+            if (P.stopped_total && out) atomicAdd(P.stopped_total, (unsigned long long)out);
+        } else if (P.lists) {  // the segment's list entries: every segs-th one
             const uint32_t* list = P.lists + (size_t)qb * P.ncb;
             const float* ub = P.list_ub ? P.list_ub + (size_t)qb * P.ncb : nullptr;
             const int count = min((int)P.counts[qb], P.ncb);
@@ -460,7 +500,7 @@ __global__ void __launch_bounds__(NT, 2)
             }
         }
         __syncwarp();  // every lane sees the thresholds before the next tile's test
-        if (P.list_ub) {  // the warp's floor for the producer's stop test (signed-int order of the f32)
+        if (VISIT == WALK || P.list_ub) {  // the warp's floor for the producer's stop test (signed-int order of the f32)
             int key = __float_as_int(__fsub_rd(tau_s[qi_at(lane & 15, ty)], P.eps));
             key = __reduce_min_sync(COSTAL_FULL_MASK, key >= 0 ? key : key ^ 0x7fffffff);
             if (lane == 0)
@@ -691,14 +731,14 @@ cudaError_t launch_work_cols(const float* xsR, const uint32_t* perm, int n, int 
     return cudaGetLastError();
 }
 
-// With lists the CTAs' lengths differ and fill each other's gaps: two waves of them are enough (every
+// With lists (and in the walk) the CTAs' lengths differ and fill each other's gaps: two waves of them are enough (every
 // segment starts cold: 100,003 × 15 Tanimoto 5.1 ms with 1 segment, 6.8 with 3), and one wave of single CTAs,
 // whose start nothing hides (18,000 × 64 Tanimoto, k = 30 5.17 -> 4.34). A segment keeps at least 24 entries (its
 // stop comes a ring of stages after its thresholds have risen).
 static int segs_of(const Fp32Job& J, const fp32::Shape& sh, int sm_count) {
     const int blocks = (J.nq + fp32::BM - 1) / fp32::BM, slots = sm_count * sh.ctas;
-    if (!J.lists) return fp32::segments(J.nq, J.np / fp32::BN, J.dp, J.cap, slots);
-    return std::max(1, std::min(sh.ctas == 1 ? slots / blocks : (2 * slots + blocks - 1) / blocks, J.ncb / 24));
+    if (!J.lists && !J.walk) return fp32::segments(J.nq, J.np / fp32::BN, J.dp, J.cap, slots);
+    return std::max(1, std::min(sh.ctas == 1 ? slots / blocks : (2 * slots + blocks - 1) / blocks, (J.walk ? blocks : J.ncb) / 24));
 }
 
 size_t coarse_fp32_ws_bytes(const Fp32Job& J, int sm_count) {
@@ -742,7 +782,7 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     using namespace fp32;
     if (J.nq <= 0) return cudaSuccess;
     const Shape sh = shape_of(J, sm_count);
-    if (sh.stages < 2) return cudaErrorInvalidValue;
+    if (sh.stages < 2 || (J.walk && !J.norms)) return cudaErrorInvalidValue;
     const int mp = (J.nq + BM - 1) / BM * BM, tiles = J.np / BN;
     const int segs = segs_of(J, sh, sm_count);
     const Ws w = carve(ws, J.dp, J.cap, J.rows != nullptr, J.nq, segs);
@@ -779,6 +819,8 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     P.ncb = J.ncb;
     P.epc = J.list_cb / BN;
     P.eps = J.eps;
+    P.walk = J.walk;
+    P.walk_ends = J.walk_ends;
     P.stopped_total = J.stopped_total;
     P.part_stride = segs > 1 ? J.nq : 0;
     P.tau_shared = segs > 1 ? w.tau_shared : nullptr;
@@ -789,10 +831,13 @@ cudaError_t launch_coarse_fp32(const Fp32Job& J, void* ws, int sm_count, cudaStr
     P.tau_out = segs > 1 ? w.part_tau : J.tau;
     P.timeout_flag = J.timeout_flag;
     const int slb = (sh.bcap + 31) / 32;
-#define COSTAL_T(S, ST, O) (J.norms ? k_fp32_tiles<S, ST, true, O> : k_fp32_tiles<S, ST, false, O>)
-#define COSTAL_K(S) (sh.stream ? (P.order ? COSTAL_T(S, true, true) : COSTAL_T(S, true, false)) : P.order ? COSTAL_T(S, false, true) : COSTAL_T(S, false, false))
+#define COSTAL_T(S, ST, V) (J.norms ? k_fp32_tiles<S, ST, true, V> : k_fp32_tiles<S, ST, false, V>)
+#define COSTAL_V(S, ST) \
+    (J.walk ? k_fp32_tiles<S, ST, true, WALK> : P.order ? COSTAL_T(S, ST, BY_ORDER) : COSTAL_T(S, ST, IN_ORDER))
+#define COSTAL_K(S) (sh.stream ? COSTAL_V(S, true) : COSTAL_V(S, false))
     auto kern = slb <= 2 ? COSTAL_K(2) : slb == 3 ? COSTAL_K(3) : COSTAL_K(5);
 #undef COSTAL_T
+#undef COSTAL_V
 #undef COSTAL_K
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem)) != cudaSuccess) return e;
     kern<<<dim3(mp / BM, segs), NT, sh.smem, st>>>(ma, mb, P); note_launch();

@@ -37,6 +37,11 @@ struct Fp32Job {
     const uint32_t* order;  // the query blocks, longest lists first
     int ncb, list_cb;
     float eps;
+    // Tanimoto selection without lists, xsT in the norm order perm (prune::norm_walk): the norm ranges of the
+    // tiles' 128 rows, and for each tile (the smallest norm of it and the tiles after it, the largest of it
+    // and the tiles before it). The tiles are visited outward from the query block's own.
+    const float2* walk;
+    const float2* walk_ends;
     unsigned long long* stopped_total;
     uint32_t* cand_idx;    // [n][cap], by original row, original column ids
     float* cand_score;

@@ -487,19 +487,6 @@ __device__ __forceinline__ float row_ub_f32(float m, float delta, float rb) {
     return fminf(1.0f, __fadd_ru(cosf(th), 1e-6f));
 }
 
-// Tanimoto selection (knn.rs:239-283): with ρ the quotient of two rows' norms, T = c / (ρ + 1/ρ − c) grows
-// with their cosine c > 0, so over two blocks whose cosines are ≤ u and whose norms lie in [a.x, a.y] and
-// [b.x, b.y], T ≤ u / (m − u) with m = the smallest ρ + 1/ρ there (2 where the ranges meet), and T ≤ 0 for
-// u ≤ 0. Roundings go outward (the ranges arrive rounded outward to f32).
-__device__ __forceinline__ float tani_ub_f32(float u, float2 a, float2 b) {
-    if (u <= 0.0f) return 0.0f;
-    float r = 1.0f;
-    if (a.x > b.y) r = __fdiv_rd(a.x, b.y);
-    else if (b.x > a.y) r = __fdiv_rd(b.x, a.y);
-    const float m = r > 1.0f ? __fadd_rd(r, __fdiv_rd(1.0f, r)) : 2.0f;  // (r = +inf: no pair of live rows)
-    return fminf(1.0f, __fdiv_ru(u, __fsub_rd(fmaxf(m, 2.0f), u)));
-}
-
 // Compare-exchange of list keys (descending) at a register distance S within a thread's run.
 template <int S, int KPT>
 __device__ __forceinline__ void cx_regs(uint32_t (&v)[KPT], int base, int size) {
@@ -950,19 +937,12 @@ cudaError_t norm_window_share(const double* norms, int n, unsigned* share, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& P) {
-    Scratch S{};
-    carve(ws, n, d, P, S);
-    P.norm_only = true;
-    return norm_order(norms, n, norm_ws, P.perm, st);
-}
-
 size_t norm_order_bytes(int n) {
     const size_t nch = (size_t)(n + CHUNK - 1) / CHUNK;
     return a256((size_t)n * 4) + a256(nch * NORM_BUCKETS * 4) + a256((NORM_BUCKETS + 1) * 4) + 256;
 }
 
-cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cudaStream_t st) {
+static cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cudaStream_t st) {
     char* p = static_cast<char*>(ws);
     const int nch = (n + CHUNK - 1) / CHUNK;
     uint32_t* cell = reinterpret_cast<uint32_t*>(p);
@@ -980,6 +960,59 @@ cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cud
     return sort_by_cell(cell, n, NORM_BUCKETS, hist, start, perm, st);
 }
 
+cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& P) {
+    Scratch S{};
+    carve(ws, n, d, P, S);
+    P.norm_only = true;
+    return norm_order(norms, n, norm_ws, P.perm, st);
+}
+
+// ends[t] = (the smallest lower end of ranges[t …], the largest upper end of ranges[… t]). One CTA.
+__global__ void __launch_bounds__(1024) k_walk_ends(const float2* __restrict__ ranges, int tiles, float2* __restrict__ ends) {
+    __shared__ float lo_s[1024], hi_s[1024];
+    const int tid = threadIdx.x, per = (tiles + 1023) / 1024;
+    const long long a = min((long long)tid * per, (long long)tiles), b = min(a + per, (long long)tiles);
+    float lo = CUDART_INF_F, hi = 0.0f;
+    for (long long t = a; t < b; ++t) {
+        lo = fminf(lo, ranges[t].x);
+        hi = fmaxf(hi, ranges[t].y);
+    }
+    lo_s[tid] = lo;
+    hi_s[tid] = hi;
+    __syncthreads();
+    lo = CUDART_INF_F;
+    hi = 0.0f;
+    for (int t = 0; t < tid; ++t) hi = fmaxf(hi, hi_s[t]);
+    for (int t = 1023; t > tid; --t) lo = fminf(lo, lo_s[t]);
+    for (long long t = a; t < b; ++t) ends[t].y = hi = fmaxf(hi, ranges[t].y);
+    for (long long t = b - 1; t >= a; --t) ends[t].x = lo = fminf(lo, ranges[t].x);
+}
+
+size_t norm_walk_bytes(int n) {
+    const size_t tiles = ((size_t)n + QB - 1) / QB;
+    return a256((size_t)n * 4) + 2 * a256(tiles * 8) + norm_order_bytes(n);
+}
+
+cudaError_t norm_walk(void* ws, const double* norms, int n, cudaStream_t st, Walk& W) {
+    const int tiles = (n + QB - 1) / QB;
+    char* p = static_cast<char*>(ws);
+    uint32_t* perm = reinterpret_cast<uint32_t*>(p);
+    p += a256((size_t)n * 4);
+    float2* ranges = reinterpret_cast<float2*>(p);
+    p += a256((size_t)tiles * 8);
+    float2* ends = reinterpret_cast<float2*>(p);
+    p += a256((size_t)tiles * 8);
+    cudaError_t e = norm_order(norms, n, p, perm, st);
+    if (e != cudaSuccess) return e;
+    k_block_norms<<<(tiles + 7) / 8, 256, 0, st>>>(norms, perm, n, QB, tiles, ranges); note_launch();
+    k_walk_ends<<<1, 1024, 0, st>>>(ranges, tiles, ends); note_launch();
+    W.perm = perm;
+    W.ranges = ranges;
+    W.ends = ends;
+    return cudaGetLastError();
+}
+
+static_assert(ListShape<16>::N == LIST_FAST && ListShape<32>::N == LIST_MAX, "the lists' limits are their sorts'");
 cudaError_t build_lists(Plan& P, unsigned long long* skipped_total, cudaStream_t st) {
     // up to 8,192 column blocks: 16 keys a thread, two CTAs per SM; up to 16,384: 32 keys a thread;
     // beyond that (n > 4,194,304 with blocks of 256) the lists stay in block order (no early stop)

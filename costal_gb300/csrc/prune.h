@@ -19,7 +19,9 @@ constexpr int QB = 128;           // query block (rows of one tensor-core CTA)
 // 2,000,000 (+5.5 %), where the lists need the 32-keys-a-thread sort.
 constexpr int CB_FINE = 128, CB_WIDE = 256;
 constexpr int LIST_FAST = 8192;  // the widest list of the 16-keys-a-thread sort
-inline int col_block(int n) { return (n + CB_FINE - 1) / CB_FINE <= LIST_FAST ? CB_FINE : CB_WIDE; }
+constexpr int LIST_MAX = 16384;  // the widest list that is sorted at all (n ≤ 4,194,304): longer ones stay in block order
+inline int col_block(int n) { return (n - 1) / CB_FINE < LIST_FAST ? CB_FINE : CB_WIDE; }
+inline bool sortable(int n) { return (n - 1) / col_block(n) + 1 <= LIST_MAX; }
 constexpr int SAMPLE = 65536;     // rows of the k-means sample
 constexpr int LLOYD_STEPS = 8;
 
@@ -58,18 +60,27 @@ cudaError_t build_order(void* ws, const float* xsT, const float* xsR, int n, int
 // Per-query-block column lists with the thresholds in plan.tq (NULL: keep all, nearest first).
 cudaError_t build_lists(Plan& plan, unsigned long long* skipped_total, cudaStream_t st);
 
-// Rows grouped by norm for Tanimoto selection's norm window (knn.rs:413-418 sorts by norm): a stable
+// Rows grouped by norm for Tanimoto selection's norm window (knn.rs:413-418 sorts by norm): perm, a stable
 // counting sort into NORM_BUCKETS buckets spaced evenly in log(norm) between the smallest and the
-// largest positive norm (zero rows first). Within a bucket rows keep their input order; the bounds
-// only need each block's exact norm range, so the order inside a bucket does not matter.
+// largest positive norm (zero rows first; within a bucket rows keep their input order). ranges: the norm
+// range of every 128 rows of that order, rounded outward; ends: for every such block the smallest norm of it
+// and all after it, and the largest of it and all before it, so that a walk outward has bounds that do not
+// increase although neighbouring blocks of one bucket overlap.
 constexpr int NORM_BUCKETS = 1024;
 size_t norm_order_bytes(int n);
-cudaError_t norm_order(const double* norms, int n, void* ws, uint32_t* perm, cudaStream_t st);
+struct Walk {
+    const uint32_t* perm;   // working -> original [n]
+    const float2* ranges;   // [⌈n/128⌉]
+    const float2* ends;     // [⌈n/128⌉]
+};
+size_t norm_walk_bytes(int n);
+cudaError_t norm_walk(void* ws, const double* norms, int n, cudaStream_t st, Walk& walk);
+// A plan whose working order is that order (no cells, no geometry; norm_ws holds norm_order_bytes(n)), for
+// lists by norm ranges alone.
+cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& plan);
 // How much of the data a norm window leaves: of the pairs of a row sample (share[0], zeroed by the
 // caller), those inside the window of a Tanimoto score of 0.9 (share[1]).
 cudaError_t norm_window_share(const double* norms, int n, unsigned* share, cudaStream_t st);
-// A plan whose working order is that norm order (no cells, no geometry), for lists by norm ranges alone.
-cudaError_t norm_plan(void* ws, const double* norms, int n, int d, void* norm_ws, cudaStream_t st, Plan& plan);
 // The blocks' norm ranges into ranges[ncb + nqb], and into the plan: build_lists then bounds the
 // Tanimoto score instead of the cosine.
 cudaError_t block_norms(const double* norms, Plan& plan, float2* ranges, cudaStream_t st);
