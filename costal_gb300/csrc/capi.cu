@@ -11,6 +11,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "costal_gb300.h"
@@ -71,6 +72,7 @@ struct Context {
     DevBuf mlp_params, mlp_params_bf, mlp_m1, mlp_m2, mlp_feat, mlp_y, mlp_pred, mlp_partial, mlp_grad, mlp_rows, mlp_perm;
     DevBuf fp32_ws, tfloor, xsW, xsR;
     DevBuf csr_ws, csr_indptr, csr_src, csr_nbr, csr_w, tnorm, shard_rows, tani_ws, tani_ranges, rm_ws, rm_out;
+    DevBuf mlp_next, mlp_next_bf;  // a model being trained or loaded (install_model)
     MlpState mlp;
 };
 
@@ -190,6 +192,21 @@ void coarse_fp32_rows(Context& c, int n, int np, int dp, int cap, const uint32_t
     j.nq = nq;
     j.tfloor = tfloor;
     coarse_fp32(c, j, s);
+}
+
+// The parameters in mlp_next and mlp_next_bf become the loaded model. Until then the one loaded before stays as
+// it is, whatever fails on the way.
+void install_model(Context& c, int d, int k, float quantile) {
+    std::swap(c.mlp_params, c.mlp_next);
+    std::swap(c.mlp_params_bf, c.mlp_next_bf);
+    c.mlp.ready = true;
+    c.mlp.d = d;
+    c.mlp.k = k;
+    c.mlp.F = d + MLP_TOPC;
+    c.mlp.quantile = quantile;
+    c.mlp.params = c.mlp_params.as<float>();
+    c.mlp.params_bf = c.mlp_params_bf.as<float>();
+    c.mlp.nparams = mlp_param_count(c.mlp.F);
 }
 
 // Learned thresholds: the model's prediction for every row, then t_Q = min over each query block.
@@ -1085,8 +1102,8 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(ensure(c.mlp_y, (size_t)m * 4));
         CK(ensure(c.mlp_feat, (size_t)std::max(m, std::min(N, MLP_CHUNK)) * F * 4));
         CK(ensure(c.mlp_pred, std::max<size_t>(n, m) * 4));
-        CK(ensure(c.mlp_params, P * 4));
-        CK(ensure(c.mlp_params_bf, P * 4));
+        CK(ensure(c.mlp_next, P * 4));
+        CK(ensure(c.mlp_next_bf, P * 4));
         CK(ensure(c.mlp_m1, P * 4));
         CK(ensure(c.mlp_m2, P * 4));
         CK(ensure(c.mlp_partial, (size_t)((std::max<uint32_t>(32, o.batch) + 31) / 32) * P * 4));
@@ -1155,7 +1172,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         CK(mlp::features(c.xsT.as<float>(), np, D, pp.centroids, pp.K, rows, m, c.mlp_feat.as<float>(), s));
         CK(cudaEventRecord(c.ev[1], s));
         // Adam on the pinball loss, minibatches in sample order
-        CK(launch_init_params(c.mlp_params.as<float>(), F, (unsigned long long)o.seed, s));
+        CK(launch_init_params(c.mlp_next.as<float>(), F, (unsigned long long)o.seed, s));
         CK(cudaMemsetAsync(c.mlp_m1.p, 0, P * 4, s));
         CK(cudaMemsetAsync(c.mlp_m2.p, 0, P * 4, s));
         int t = 0;
@@ -1163,13 +1180,13 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
         for (uint32_t ep = 0; ep < o.epochs; ++ep) {
             for (int b0 = 0; b0 < m; b0 += B) {
                 const int mb = std::min(B, m - b0);
-                CK(mlp::train_step(c.mlp_params.as<float>(), F, c.mlp_feat.as<float>() + (size_t)b0 * F,
+                CK(mlp::train_step(c.mlp_next.as<float>(), F, c.mlp_feat.as<float>() + (size_t)b0 * F,
                                    c.mlp_y.as<float>() + b0, mb, o.quantile, c.mlp_partial.as<float>(),
                                    c.mlp_m1.as<float>(), c.mlp_m2.as<float>(), o.lr, ++t, s));
             }
         }
-        CK(mlp::round_bf16(c.mlp_params.as<float>(), c.mlp_params_bf.as<float>(), P, s));
-        CK(mlp::forward(c.mlp_params_bf.as<float>(), F, c.mlp_feat.as<float>(), m, c.mlp_pred.as<float>(), s));
+        CK(mlp::round_bf16(c.mlp_next.as<float>(), c.mlp_next_bf.as<float>(), P, s));
+        CK(mlp::forward(c.mlp_next_bf.as<float>(), F, c.mlp_feat.as<float>(), m, c.mlp_pred.as<float>(), s));
         CK(cudaEventRecord(c.ev[2], s));
         std::vector<float> pred(m), y(m);
         CK(cudaMemcpyAsync(pred.data(), c.mlp_pred.p, (size_t)m * 4, cudaMemcpyDeviceToHost, s));
@@ -1187,14 +1204,7 @@ int costal_mlp_train(const float* x, uint64_t n, uint32_t d, uint32_t k, const c
             mae += std::fabs(r);
             below += pred[i] <= y[i];
         }
-        c.mlp.ready = true;
-        c.mlp.d = D;
-        c.mlp.k = K;
-        c.mlp.F = F;
-        c.mlp.quantile = o.quantile;
-        c.mlp.params = c.mlp_params.as<float>();
-        c.mlp.params_bf = c.mlp_params_bf.as<float>();
-        c.mlp.nparams = P;
+        install_model(c, D, K, o.quantile);
         if (stats) {
             stats->samples = (uint64_t)m;
             stats->steps = (uint64_t)t;
@@ -1229,19 +1239,12 @@ int costal_mlp_set(const float* params, uint64_t count, uint32_t d, uint32_t k, 
         const size_t P = mlp_param_count(F);
         if (!prune::supported((int)d) || count != P)
             throw Fail{COSTAL_EINVAL, "parameter block does not match d (expected " + std::to_string(P) + " values)"};
-        CK(ensure(c.mlp_params, P * 4));
-        CK(ensure(c.mlp_params_bf, P * 4));
-        CK(cudaMemcpy(c.mlp_params.p, params, P * 4, cudaMemcpyHostToDevice));
-        CK(mlp::round_bf16(c.mlp_params.as<float>(), c.mlp_params_bf.as<float>(), P, c.stream));
+        CK(ensure(c.mlp_next, P * 4));
+        CK(ensure(c.mlp_next_bf, P * 4));
+        CK(cudaMemcpy(c.mlp_next.p, params, P * 4, cudaMemcpyHostToDevice));
+        CK(mlp::round_bf16(c.mlp_next.as<float>(), c.mlp_next_bf.as<float>(), P, c.stream));
         CK(cudaStreamSynchronize(c.stream));
-        c.mlp.ready = true;
-        c.mlp.d = (int)d;
-        c.mlp.k = (int)k;
-        c.mlp.F = F;
-        c.mlp.quantile = quantile;
-        c.mlp.params = c.mlp_params.as<float>();
-        c.mlp.params_bf = c.mlp_params_bf.as<float>();
-        c.mlp.nparams = P;
+        install_model(c, (int)d, (int)k, quantile);
     });
 }
 

@@ -172,3 +172,31 @@ def test_model_trained_on_one_draw_prunes_another(ext, zipf_case):
     assert st["pruned_fallback_rows"] < 0.01 * len(x2), st
     print("other draw: learned skips", st["blocks_skipped"], "of", st["blocks_total"], "rescanned rows",
           st["pruned_fallback_rows"])
+
+
+@pytest.mark.gpu
+def test_a_failed_training_leaves_the_loaded_model(ext):
+    """Training that ends in an error, on deeper rows than the loaded model's (whose buffers would have to
+    grow), keeps that model: its parameters and what a learned call does with it. So does a refused load."""
+    from conftest import clustered
+
+    x = clustered(40_000, 8, 3)
+    ext._mlp_train(x, 5, sample=4000, epochs=3)
+    before = ext._mlp_get()
+    got, st = ext._knn_exact(x, 5, matmul="bf16", learned_prune=True)
+    bad = clustered(3_000, 64, 4)
+    bad[2_999, 63] = np.inf
+    for rows, d in ((bad, 64), (bad[:, :8], 8)):
+        rows = np.ascontiguousarray(rows)
+        rows[-1, -1] = np.nan
+        with pytest.raises(ValueError, match="row 2999 contains NaN or inf"):
+            ext._mlp_train(rows, 5, sample=500, epochs=2)
+        with pytest.raises(ValueError, match="does not match d"):
+            ext._mlp_set(np.zeros(7, np.float32), d, 5)
+        after = ext._mlp_get()
+        np.testing.assert_array_equal(after[0], before[0])
+        assert after[1:] == before[1:]
+        again, st2 = ext._knn_exact(x, 5, matmul="bf16", learned_prune=True)
+        for a, b in zip(again, got):
+            np.testing.assert_array_equal(a, b)
+        assert st2["blocks_skipped"] == st["blocks_skipped"]
