@@ -675,7 +675,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // The descriptors of the first K step; a step is 32 bytes further (2 in their 16-byte units).
             const uint64_t a_desc = sw128_desc(smem_u32(a_tile)), b_desc = sw128_desc(smem_u32(b_tiles));
             volatile int* stop = &bars->stop_tile;
-            long long budget = 0;
             int s = 0;
             uint32_t ph = 0;
             auto advance = [&](int k) {
@@ -695,10 +694,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 // those steps also cover). 16 bf16 = 32 bytes inside a swizzle row.
                 for (int kb = 0; kb < nkb_b; ++kb) {
                     // (a stop at an earlier visit, the other warp's, leaves this one's tile unloaded)
+                    long long polls = 0;  // of this wait alone
                     while (ok && !mbar_try_wait(&bars->b_full[s], ph)) {
                         if (kb == 0 && *stop < v) ok = false;
                         else if (kb == 0 && *stop == v) break;
-                        else if (!wait_budget(timeout_flag, budget)) ok = false;
+                        else if (!wait_budget(timeout_flag, polls)) ok = false;
                     }
                     if (!ok) break;
                     // (the accumulator last: it is what the visit waits for, and its MMAs start at once)
