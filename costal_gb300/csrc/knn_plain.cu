@@ -216,6 +216,12 @@ __device__ __forceinline__ uint32_t warp_kth_key(const uint32_t (&key)[SLOTS], i
 constexpr int RS_ROWS = 8;
 constexpr int RS_MAXCAP = 128;
 
+// An f32 at or below a non-negative f64 given by its bits (truncated; integer operations only).
+__device__ __forceinline__ float f32_below(unsigned long long bits) {
+    const uint32_t hi = (uint32_t)(bits >> 32);
+    return hi < 0x38100000u ? 0.0f : __uint_as_float(((hi - 0x38000000u) << 3) | ((uint32_t)bits >> 29));
+}
+
 template <int SLOTS, bool DEEP>
 __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x, int n, int d, int k, int cap, int lstride,
               const uint32_t* __restrict__ cand_idx, const float* __restrict__ cand_score,
@@ -398,7 +404,9 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
     }
     // phase 1: the f64 rescoring of the packed entries
     unsigned long long err = 0;  // (non-negative doubles order like their bits)
-    float ratio = 0.0f;          // rounded up
+    // The ratio's f64 division only where its f32 upper bound could still beat the largest of the call so far.
+    unsigned long long ratio = 0;
+    float known = max_err_bits ? f32_below(*reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) : CUDART_INF_F;
     for (int w = tid; w < total; w += blockDim.x) {
         const int code = work_s[w], r = code / RS_MAXCAP, p = code - r * RS_MAXCAP, e = r * cap + p;
         const int i = row_s[r];
@@ -424,8 +432,12 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
         const double diff = fabs((double)cand_score[(size_t)i * lstride + p] - score);
         const unsigned long long db = (unsigned long long)__double_as_longlong(diff);
         err = db > err ? db : err;
-        // against the bound the certificate used
-        ratio = fmaxf(ratio, __fdiv_ru(__double2float_ru(diff), __double2float_rd(row_eps ? row_eps[i] : eps)));
+        const double bound = row_eps ? row_eps[i] : eps;  // the one the certificate uses
+        if (__fdiv_ru(__double2float_ru(diff), __double2float_rd(bound)) > known) {
+            const unsigned long long q = (unsigned long long)__double_as_longlong(__ddiv_rn(diff, bound));
+            ratio = q > ratio ? q : ratio;
+            known = fmaxf(known, f32_below(q));
+        }
         sc_s[e] = score;
         cs_s[e] = c;
         id_s[e] = j;
@@ -434,15 +446,15 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long oe = __shfl_xor_sync(COSTAL_FULL_MASK, err, o);
         err = oe > err ? oe : err;
-        ratio = fmaxf(ratio, __shfl_xor_sync(COSTAL_FULL_MASK, ratio, o));
+        const unsigned long long oq = __shfl_xor_sync(COSTAL_FULL_MASK, ratio, o);
+        ratio = oq > ratio ? oq : ratio;
     }
     // max_err_bits[0]: the largest |coarse − rescored|, [1]: the largest ratio of it to the row's bound
     // (non-negative doubles order like their bits). One address for the whole grid: read it first,
     // so that only a new maximum pays for the atomic.
     if (lane == 0 && max_err_bits && err > 0) {
         if (err > *reinterpret_cast<volatile unsigned long long*>(max_err_bits)) atomicMax(max_err_bits, err);
-        const unsigned long long rb = (unsigned long long)__double_as_longlong((double)ratio);
-        if (rb > *reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) atomicMax(max_err_bits + 1, rb);
+        if (ratio > *reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) atomicMax(max_err_bits + 1, ratio);
     }
     __syncthreads();
     if (warp < nr) {

@@ -93,3 +93,16 @@ def test_split_fp8_with_either_buffer(ext, n, d):
     assert st["coarse_kind"] == "fp8" and st["max_err_ratio"] < 1.0
     for a, b in zip(got, ext._knn_exact(x, 10)[0]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("matmul,n,d", [("fp32", 1500, 24), ("bf16", 1500, 24), ("fp8", 900, 600)])
+def test_error_ratio_is_the_f64_quotient(ext, matmul, n, d):
+    """max_err_ratio is the largest f64 quotient itself, not an f32 above it: 29 and more of its low bits are
+    zero only by a chance of 2⁻²⁹. (FP32: the bound is one number, so the quotient of the maxima.)"""
+    x = clustered(n, d, n + d)
+    for seed in range(3):
+        _, st = ext._knn_exact(x + np.float32(0.01 * seed), 10, matmul=matmul)
+        r = st["max_err_ratio"]
+        assert 0.0 < r < 1.0 and float(np.float32(r)) != r
+        if matmul == "fp32":
+            assert r == st["max_coarse_err"] / ((d + 4.0) * 2.0**-23)
