@@ -36,7 +36,8 @@
 //             lists merged per row (k_merge_parts), so that no SM idles in a nearly empty last wave.
 //             The segments of a query share their thresholds whenever one of them cuts its buffer.
 //
-// Every mbarrier wait is bounded (ptx.cuh); a wait that gives up raises timeout_flag.
+// Every mbarrier wait is bounded (ptx.cuh); a wait that gives up raises timeout_flag, and the producer, the last
+// to leave, waits for the loads in flight.
 
 #include <cuda_runtime.h>
 
@@ -287,9 +288,15 @@ __global__ void __launch_bounds__(NT, 2)
                 ph ^= 1u;
             }
         };
+        auto wait_empty = [&]() -> bool {
+            if (mbar_wait(&bars->empty[s], ph, P.timeout_flag, true)) return true;
+            drain_ring(bars->full, P.stages, s, ph);
+            if (!STREAM) mbar_drain(&bars->a_full, 0);
+            return false;
+        };
         auto send_tile = [&](int c0) -> bool {
             for (int ch = 0; ch < nch; ++ch) {
-                if (!mbar_wait(&bars->empty[s], ph, P.timeout_flag, true)) return false;
+                if (!wait_empty()) return false;
                 unsigned char* dst = ring + (size_t)s * stage_bytes;
                 bars->c0[s] = c0;
                 mbar_expect_tx(&bars->full[s], stage_bytes);
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(NT, 2)
             for (int t = seg * tps; t < min(P.tiles, (seg + 1) * tps); ++t)
                 if (!send_tile(t * BN)) return;
         }
-        if (!mbar_wait(&bars->empty[s], ph, P.timeout_flag, true)) return;
+        if (!wait_empty()) return;
         bars->c0[s] = -1;
         mbar_arrive(&bars->full[s]);  // completes the phase without data (release)
         return;

@@ -185,6 +185,7 @@ struct __align__(8) Barriers {
     uint32_t tmem_base;
     int stop_tile;         // the list position at which the CTA stops (set by the TMA warp)
     float warp_floor[4];   // per epilogue warp: min over its rows of τ − E (never decreases)
+    uint64_t drain[2];     // per MMA warp that has given up: its issued MMAs are done
 };
 
 // Entries of a query's buffer: 64 for cap ≤ 32, 128 for cap ≤ 64; narrow: 80 for cap ≤ 64 (fp8_narrow).
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(&bars->t_full[b], 1);
             mbar_init(&bars->t_empty[b], EPI_WARPS);
         }
+        for (int w = 0; w < 2; ++w) mbar_init(&bars->drain[w], 1);
         bars->stop_tile = nvisits;
         for (int w = 0; w < EPI_WARPS; ++w) bars->warp_floor[w] = -CUDART_INF_F;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -515,6 +517,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (ok) tile_cols(t, en, c0, c1);
                 for (int kb = 0; kb < nkb; ++kb) {
                     if (!mbar_wait(&bars->b_empty[s], ph, timeout_flag, false)) {
+                        drain_ring(bars->b_full, stages, s, ph);
+                        if (!KLOOP) mbar_drain(&bars->a_full, 0);
                         go = false;
                         break;
                     }
@@ -573,6 +577,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 int c0 = 0, c1 = 0;
                 for (int kb = 0; kb < nkb_b; ++kb) {
                     if (!mbar_wait(&bars->b_empty[s], ph, timeout_flag, false)) {
+                        drain_ring(bars->b_full, stages, s, ph);
+                        if (!KLOOP) mbar_drain(&bars->a_full, 0);
                         go = false;
                         break;
                     }
@@ -623,17 +629,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     } else if (KLOOP && warp == EPI_WARPS + 1) {
         // ------------------------------------------------------------------ MMA issuer, K loop
         if (lane == 0) {
-            bool go = true;
+            bool go = true, lost = false;  // lost: a wait gave up
             const uint64_t st_desc = sw128_desc(smem_u32(b_tiles));
             int s = 0;
             uint32_t ph = 0;
             for (int t = 0; go && t < ntiles; ++t) {
                 const int buf = t & 1;
                 const uint32_t bph = (uint32_t)(t >> 1) & 1u;
-                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, false)) break;
+                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, false)) {
+                    lost = true;
+                    break;
+                }
                 const uint32_t d = tmem + (uint32_t)(buf * BLOCK_N);
                 for (int kb = 0; kb < nkb; ++kb) {
                     if (!mbar_wait(&bars->b_full[s], ph, timeout_flag, false)) {
+                        lost = true;
                         go = false;
                         break;
                     }
@@ -658,6 +668,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (!go) break;
                 mma_commit(&bars->t_full[buf]);
             }
+            if (lost) {
+                mma_commit(&bars->drain[0]);
+                mbar_drain(&bars->drain[0], 0);
+            }
         }
     }
     if (!KLOOP && warp > EPI_WARPS) {
@@ -670,7 +684,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // two warps need a ring of an even number of tiles, else warp 5 issues every visit.
         const int mw = warp - (EPI_WARPS + 1);
         if (lane == 0 && mw < mma_warps) {
-            bool ok = mbar_wait(&bars->a_full, 0, timeout_flag, true);
+            bool ok = mbar_wait(&bars->a_full, 0, timeout_flag, true), lost = !ok;  // lost: a wait gave up
             tc_fence_after();
             // The descriptors of the first K step; a step is 32 bytes further (2 in their 16-byte units).
             const uint64_t a_desc = sw128_desc(smem_u32(a_tile)), b_desc = sw128_desc(smem_u32(b_tiles));
@@ -698,11 +712,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     while (ok && !mbar_try_wait(&bars->b_full[s], ph)) {
                         if (kb == 0 && *stop < v) ok = false;
                         else if (kb == 0 && *stop == v) break;
-                        else if (!wait_budget(timeout_flag, polls)) ok = false;
+                        else if (!wait_budget(timeout_flag, polls)) lost = true, ok = false;
                     }
                     if (!ok) break;
                     // (the accumulator last: it is what the visit waits for, and its MMAs start at once)
                     if (kb == 0 && !mbar_wait(&bars->t_empty[buf], ((uint32_t)(v >> 1) & 1u) ^ 1u, timeout_flag, false)) {
+                        lost = true;
                         ok = false;
                         break;
                     }
@@ -725,6 +740,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (!ok) break;
                 mma_commit(&bars->t_full[buf]);
                 if (mma_warps == 2) advance(nkb_b);  // the other warp's visit
+            }
+            if (lost) {
+                mma_commit(&bars->drain[mw]);
+                mbar_drain(&bars->drain[mw], 0);
             }
         }
     }
@@ -922,6 +941,7 @@ struct __align__(8) RmBars {
     uint64_t c_empty[4];
     uint64_t t_full[2];
     uint64_t t_empty[2];
+    uint64_t drain;        // as in Barriers
     uint32_t tmem_base;
 };
 
@@ -950,6 +970,7 @@ __global__ void __launch_bounds__(RM_THREADS, 1)
 
     if (threadIdx.x == 0) {
         mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->drain, 1);
         for (int s = 0; s < stages; ++s) {
             mbar_init(&bars->c_full[s], 1);
             mbar_init(&bars->c_empty[s], 1);
@@ -979,7 +1000,11 @@ __global__ void __launch_bounds__(RM_THREADS, 1)
             for (int t = 0; t < ntiles; ++t) {
                 const int s = t % stages;
                 const uint32_t ph = (uint32_t)(t / stages) & 1u;
-                if (!mbar_wait(&bars->c_empty[s], ph ^ 1u, timeout_flag, true)) break;
+                if (!mbar_wait(&bars->c_empty[s], ph ^ 1u, timeout_flag, true)) {
+                    drain_ring(bars->c_full, stages, s, ph ^ 1u);
+                    mbar_drain(&bars->q_full, 0);
+                    break;
+                }
                 mbar_expect_tx(&bars->c_full[s], c_bytes);
                 unsigned char* dst = c_tiles + (size_t)s * c_bytes;
                 for (int kb = 0; kb < nkb_c; ++kb)
@@ -988,14 +1013,17 @@ __global__ void __launch_bounds__(RM_THREADS, 1)
         }
     } else if (warp == EPI_WARPS + 1) {
         if (lane == 0) {
-            const bool ok = mbar_wait(&bars->q_full, 0, timeout_flag, true);
+            bool lost = !mbar_wait(&bars->q_full, 0, timeout_flag, true);
             tc_fence_after();
             const uint32_t q_base = smem_u32(q_tile);
-            for (int t = 0; ok && t < ntiles; ++t) {
+            for (int t = 0; !lost && t < ntiles; ++t) {
                 const int s = t % stages, buf = t & 1;
                 const uint32_t ph = (uint32_t)(t / stages) & 1u, bph = (uint32_t)(t >> 1) & 1u;
-                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, true)) break;
-                if (!mbar_wait(&bars->c_full[s], ph, timeout_flag, true)) break;
+                if (!mbar_wait(&bars->t_empty[buf], bph ^ 1u, timeout_flag, true) ||
+                    !mbar_wait(&bars->c_full[s], ph, timeout_flag, true)) {
+                    lost = true;
+                    break;
+                }
                 tc_fence_after();
                 const uint32_t c_base = smem_u32(c_tiles + (size_t)s * c_bytes);
                 const uint32_t dt = tmem + (uint32_t)(buf * RM_N);
@@ -1009,6 +1037,10 @@ __global__ void __launch_bounds__(RM_THREADS, 1)
                 }
                 mma_commit(&bars->c_empty[s]);
                 mma_commit(&bars->t_full[buf]);
+            }
+            if (lost) {
+                mma_commit(&bars->drain);
+                mbar_drain(&bars->drain, 0);
             }
         }
     } else {

@@ -60,6 +60,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     return mbar_try_wait(bar, parity) || mbar_wait_long(bar, parity, timeout_flag, sleep);
 }
 
+// The wait of a role that has given up for copies or MMAs of its own that are still in flight, which must not
+// outlive the CTA's shared memory: bounded too (65,536 polls of 64 ns and more, where they take microseconds).
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    for (int polls = 0; polls < 65536 && !mbar_try_wait(bar, parity); ++polls) __nanosleep(64);
+}
+// The loads of a ring whose next stage is s with producer parity ph (full[q] of an unused stage passes at once).
+__device__ __forceinline__ void drain_ring(uint64_t* full, int stages, int s, uint32_t ph) {
+    for (int q = 0; q < stages; ++q) mbar_drain(&full[q], q < s ? ph ^ 1u : ph);
+}
+
 // ---- TMA ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile(

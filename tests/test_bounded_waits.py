@@ -24,3 +24,17 @@ def test_every_wait_counts_its_own_polls():
             calls += 1
     assert calls >= 2
 
+
+def test_a_role_that_gives_up_waits_for_its_own_work():
+    """Every kernel that starts bulk copies or MMAs waits for those in flight before a role that has given up
+    lets the CTA end: they read and write its shared memory."""
+    kernels = 0
+    for name, text in _sources().items():
+        for body in text.split("__global__")[1:]:
+            body = body[:body.find("\n}\n")]
+            if "tma_load_2d(" in body:
+                kernels += 1
+                assert "drain_ring(" in body, name
+            if "mma_commit(" in body:
+                assert "mbar_drain(&bars->drain" in body, name
+    assert kernels == 3
