@@ -110,3 +110,72 @@ def test_above_the_longest_sorted_lists(ext, select):
     env = dict(os.environ, PYTHONPATH=str(ROOT))
     r = subprocess.run([sys.executable, "-c", _ABOVE, select], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("matmul,select,n,d", [
+    ("fp32", "cosine", 20_001, 12), ("fp32", "cosine", 20_001, 40), ("fp32", "cosine", 9_000, 70),  # lists, all tiles
+    ("fp32", "tanimoto", 300, 5), ("fp32", "tanimoto", 20_001, 12),                                 # walk, lists
+    ("bf16", "cosine", 5_000, 12), ("bf16", "cosine", 25_000, 40), ("bf16", "cosine", 3_000, 520)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_rows_on_every_route(ext, matmul, select, n, d, bad):
+    """The error names the first bad row wherever the rows have been by then, and the next call is right."""
+    x = clustered(n, d, n + d)
+    want, _ = ext._knn_exact(x, 5, matmul=matmul, select=select)
+    y = x.copy()
+    y[n - 7, d - 1] = bad
+    y[n - 3] = np.nan
+    with pytest.raises(ValueError, match=f"row {n - 7} contains NaN or inf"):
+        ext._knn_exact(y, 5, matmul=matmul, select=select)
+    got, _ = ext._knn_exact(x, 5, matmul=matmul, select=select)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.gpu
+def test_non_finite_rows_in_training(ext):
+    x = clustered(20_001, 12, 9)
+    ext._mlp_train(x, 5, sample=2000, epochs=1)
+    before = ext._mlp_get()
+    x[17_000, 3] = np.inf
+    with pytest.raises(ValueError, match="row 17000 contains NaN or inf"):
+        ext._mlp_train(x, 5, sample=2000, epochs=1)
+    np.testing.assert_array_equal(ext._mlp_get()[0], before[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("select,spread", [("cosine", 1.0), ("tanimoto", 1.2), ("tanimoto", 400.0)])
+def test_lists_of_256_row_blocks(ext, select, spread):
+    """Above 1,048,576 rows a list entry is two column tiles (their own geometry and norm ranges beside the
+    query blocks'), with a last entry of one: the answer equals the pass over all tiles, in the cells' order and (norms
+    spread 400-fold) in the norm order."""
+    n, d, k = 1_048_577 + 128 * 3 + 40, 8, 3
+    rng = np.random.default_rng(3)
+    centres = rng.standard_normal((60, d))
+    x = centres[rng.integers(0, 60, n)] + 0.15 * rng.standard_normal((n, d), dtype=np.float32)
+    x = np.ascontiguousarray(x * np.exp(rng.uniform(0, np.log(spread), (n, 1))), dtype=np.float32)
+    got, st = ext._knn_exact(x, k, select=select)
+    want, st0 = ext._knn_exact(x, k, select=select, prune=False)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    left_out = "blocks_stopped" if select == "cosine" else "blocks_skipped"
+    assert st["col_block"] == 256 and st[left_out] > st["blocks_total"] // 4
+    assert st0["col_block"] == 128 and st0[left_out] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", ["cells", "norms"])
+def test_the_two_orders_of_tanimoto_selection(ext, order):
+    """Enough rows for lists. Forty tight clusters with norms within 5 %: only the cells' order leaves blocks out.
+    One cluster with norms spread 55-fold: only the norm order does."""
+    n, d, k = 30_000, 12, 10
+    rng = np.random.default_rng(8)
+    x = clustered(n, d, 8, n_centers=40 if order == "cells" else 1, noise=0.1 if order == "cells" else 0.5).astype(np.float64)
+    x *= (rng.uniform(1.0, 1.05, n) if order == "cells" else np.exp(rng.uniform(0.0, 4.0, n)))[:, None] / np.linalg.norm(
+        x, axis=1, keepdims=True)
+    x = np.ascontiguousarray(x, dtype=np.float32)
+    got, st = ext._knn_exact(x, k, select="tanimoto")
+    want, _ = ext._knn_exact(x, k, select="tanimoto", prune=False)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    assert st["blocks_skipped"] > 0.3 * st["blocks_total"]
