@@ -258,8 +258,11 @@ int coarse_most(int n, int d, int k, bool tensor_cores) {
 }
 
 // The tensor-core pass visits its tiles in row order below this many rows: the order stage costs more than
-// the lists and the earlier thresholds save (whole kNN on the device, row order / locality order:
-// 5,003 × 17 0.21 / 0.51 ms, 16,000 × 32 0.41 / 0.72, 24,000 × 15 0.80 / 0.96).
+// the lists and the earlier thresholds save (whole kNN on clustered rows, row order / locality order:
+// 5,003 × 17 0.21 / 0.51 ms, 16,000 × 32 0.40 / 0.75, 24,000 × 32 0.82 / 1.01). Shallow clustered rows are even
+// from 20,000 (× 10 0.70 / 0.69); deeper ones cross where the row order starts its third wave of CTAs (32,000 × 32
+// 0.97 / 1.16, 40,000 × 32 1.53 / 1.40, k = 30 × 40 2.73 / 2.18, 60,000 × 32 2.52 / 1.88), Gaussian rows later
+// (60,000 × 40 2.67 / 2.95).
 constexpr int TC_ORDER_ROWS = 24576;
 
 // The buffers that the lists take beyond the plain pass (xsR, xsW and the order stage's in O(n); lists, bounds

@@ -754,7 +754,8 @@ size_t coarse_fp32_ws_bytes(const Fp32Job& J, int sm_count) {
     return fp32::carve(nullptr, J.dp, J.cap, J.rows != nullptr, J.nq, segs).bytes;
 }
 
-cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
+// The lists of `segs` column segments (segs × count × cap entries, τ: segs × count) merged per row.
+static cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
                                const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
                                float* tau, cudaStream_t st) {
     fp32::k_merge_parts<<<(count + 7) / 8, 256, 0, st>>>(rows, count, segs, cap, part_idx, part_score, tfloor, cap,

@@ -12,7 +12,6 @@ namespace costal {
 cudaError_t launch_prep(const float* x, int n, int d, int np, int dp, double* norms, float* xsT, float* xsR,
                         unsigned long long* bad_row, cudaStream_t st);
 cudaError_t launch_row_l2_norms_f32(const float* x, int n, int d, float* out, cudaStream_t st);
-int coarse_slots(int cap);
 // d_pad of the working copy: a multiple of 8 up to 64 (compile-time tile depths), else of 4.
 int coarse_dpad(int d);
 // Whether the FP32 pass holds cap candidates a row at this depth (up to 128 at any).
@@ -53,10 +52,6 @@ cudaError_t launch_coarse_fp32(const Fp32Job& job, void* ws, int sm_count, cudaS
 // The transposed copy in working order: xsW [dp][np] from the row-major rows xsR [n][d].
 cudaError_t launch_work_cols(const float* xsR, const uint32_t* perm, int n, int np, int d, int dp, float* xsW,
                              cudaStream_t st);
-// The lists of `segs` column segments (segs × count × cap entries, τ: segs × count) merged per row.
-cudaError_t launch_merge_parts(const uint32_t* rows, int count, int segs, int cap, const uint32_t* part_idx,
-                               const float* part_score, const float* tfloor, uint32_t* cand_idx, float* cand_score,
-                               float* tau, cudaStream_t st);
 // The floor of rows re-run after the tensor-core pass (rows[0..*count), cand_* and tau of that pass).
 cudaError_t launch_rerun_floor(const uint32_t* rows, const unsigned* count, int nmax, int cap, const float* tau,
                                const float* cand_score, const double* row_eps, double eps, float* tfloor,

@@ -100,15 +100,6 @@ __global__ void __launch_bounds__(PREP_ROWS) k_prep(const float* __restrict__ x,
     }
 }
 
-// Rows of the padded range [n, np) in a block that has no real row still need zero columns.
-__global__ void k_zero_pad_cols(float* __restrict__ xsT, int n, int np, int dp) {
-    const int pad = np - n;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < pad * dp; e += gridDim.x * blockDim.x) {
-        const int t = e / pad, c = n + e % pad;
-        xsT[(size_t)t * np + c] = 0.0f;
-    }
-}
-
 // lib.rs:94-102 / crates/costal-core/src/lib.rs:34-47: f32 row norms, sequential f32 sum.
 __global__ void k_row_l2_norms_f32(const float* __restrict__ x, int n, int d, float* __restrict__ out) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -667,7 +658,7 @@ cudaError_t launch_check_f64_of(unsigned long long* mismatches, int sm_count, cu
     return cudaGetLastError();
 }
 
-int coarse_slots(int cap) { return cap <= 32 ? 1 : (cap <= 64 ? 2 : (cap <= 128 ? 4 : 0)); }
+static int coarse_slots(int cap) { return cap <= 32 ? 1 : (cap <= 64 ? 2 : (cap <= 128 ? 4 : 0)); }
 
 cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lstride, const uint32_t* cand_idx,
                            const float* cand_score, const float* tau, const double* norms, const double* row_eps,
@@ -717,12 +708,6 @@ cudaError_t launch_gather(const float* x, const float* xsT, int n, int np, int d
     if (e != cudaSuccess) return e;
     k_gather<<<grid, GT, smem, st>>>(x, xsT, n, np, d, dp, k, norms, rows, minsim, count, all_rows, select, capb,
                                      out_idx, out_cos, out_w); note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_zero_pad(float* xsT, int n, int np, int dp, cudaStream_t st) {
-    if (np == n) return cudaSuccess;
-    k_zero_pad_cols<<<64, 256, 0, st>>>(xsT, n, np, dp); note_launch();
     return cudaGetLastError();
 }
 

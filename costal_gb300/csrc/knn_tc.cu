@@ -46,7 +46,6 @@
 #include "kernels.h"
 #include "knn_tc.h"
 #include "ptx.cuh"
-#include "topk.cuh"
 
 namespace costal {
 namespace tc {

@@ -17,7 +17,6 @@
 
 #include "common.cuh"
 #include "mlp.h"
-#include "topk.cuh"
 
 namespace costal {
 namespace mlp {

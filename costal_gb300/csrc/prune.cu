@@ -1,4 +1,5 @@
-// Locality order and block pruning for the tensor-core coarse pass.
+// Locality order and block pruning: the column lists of the tensor-core and FP32 coarse passes, and the norm
+// order of Tanimoto selection.
 //
 // The reference visits column blocks in index order and prunes only for Tanimoto selection, by norm
 // windows (crates/costal-core/src/knn.rs:603-644, :272-283). This file gives the cosine path the same
@@ -7,7 +8,7 @@
 //   cells     spherical k-means (K = 256 centroids, a seeded sample of rows, a few Lloyd steps with
 //             deterministic centroid sums) and the cell of every row;
 //   order     a working order: rows stably sorted by cell (ties by original index). The tensor
-//             operands are laid out in this order; candidates are mapped back to original indices.
+//             operands (or the FP32 pass's rows) are laid out in this order; candidates are mapped back to original indices.
 //   geometry  for every 128-row query block Q and every column block B (128 working rows, or 256 for
 //             lists longer than the sort takes; prune.h col_block) a
 //             unit centre c and an angular radius r = max angle(row, c), in f64;

@@ -1,4 +1,4 @@
-// Locality order and block pruning for the tensor-core coarse pass (prune.cu).
+// Locality order and block pruning for the coarse passes (prune.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,9 +14,10 @@ constexpr int QB = 128;           // query block (rows of one tensor-core CTA)
 // list entries) while a query block's list fits the 16-keys-a-thread sort (≤ 8,192 blocks, n ≤
 // 1,048,576), else 256 (one tile per entry). Blocks of 128 straddle fewer k-means cells, so their
 // bounds skip more columns (visited pairs 25 % instead of 36 % at 200,000 rows of the Zipf mixture, 14.1
-// instead of 15.1 % at 2,000,000), but twice as many list entries cost more to bound and sort: measured
-// per step they win up to 1,000,000 rows (−6.6 % at 200,000, −1.9 % at 1,000,000) and lose at
-// 2,000,000 (+5.5 %), where the lists need the 32-keys-a-thread sort.
+// instead of 15.1 % at 2,000,000), but twice as many list entries cost more to bound and sort. Whole tensor-core
+// kNN with 128 / 256: 100,000 × 40 3.06 / 3.48 ms, 600,000 × 40 24.1 / 25.0, 1,000,000 × 40 52.2 / 53.0; above,
+// where the lists of 128 need the 32-keys-a-thread sort, 1,500,000 × 40 109 / 103, 2,000,000 × 40 176 / 164. (The
+// FP32 pass, which pays more for a pair, would keep 128: 1,500,000 × 32 427 / 444.)
 constexpr int CB_FINE = 128, CB_WIDE = 256;
 constexpr int LIST_FAST = 8192;  // the widest list of the 16-keys-a-thread sort
 constexpr int LIST_MAX = 16384;  // the widest list that is sorted at all (n ≤ 4,194,304): longer ones stay in block order
