@@ -227,6 +227,7 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
     __shared__ uint16_t work_s[RS_ROWS * RS_MAXCAP];  // packed (row, slot) entries to rescore
     __shared__ float r_s[DEEP ? RS_ROWS * RS_MAXCAP : 1];
     __shared__ int row_s[RS_ROWS], cnt_s[RS_ROWS], ok_s[RS_ROWS];
+    __shared__ float top_s[RS_ROWS];  // (a warp a row)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nrows = rlist ? (int)*rcount : n;
     const int w0 = g * RS_ROWS;
@@ -395,9 +396,11 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
     }
     // phase 1: the f64 rescoring of the packed entries
     unsigned long long err = 0;  // (non-negative doubles order like their bits)
-    // The ratio's f64 division only where its f32 upper bound could still beat the largest of the call so far.
-    unsigned long long ratio = 0;
-    float known = max_err_bits ? f32_below(*reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) : CUDART_INF_F;
+    // The thread's largest ratio of such an error to its row's bound, as the pair and the quotient's f32 upper bound:
+    // the f64 division runs for the CTA's largest alone (in every warp it cost a small call 5 us of 373).
+    double top_diff = 0.0, top_bound = 1.0;
+    float top = 0.0f;
+    constexpr float NEAR = 1.0f - 0x1p-20f;  // upper bounds further apart than this tell the quotients' order
     for (int w = tid; w < total; w += blockDim.x) {
         const int code = work_s[w], r = code / RS_MAXCAP, p = code - r * RS_MAXCAP, e = r * cap + p;
         const int i = row_s[r];
@@ -424,30 +427,38 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
         const unsigned long long db = (unsigned long long)__double_as_longlong(diff);
         err = db > err ? db : err;
         const double bound = row_eps ? row_eps[i] : eps;  // the one the certificate uses
-        if (__fdiv_ru(__double2float_ru(diff), __double2float_rd(bound)) > known) {
-            const unsigned long long q = (unsigned long long)__double_as_longlong(__ddiv_rn(diff, bound));
-            ratio = q > ratio ? q : ratio;
-            known = fmaxf(known, f32_below(q));
+        const float up = __fdiv_ru(__double2float_ru(diff), __double2float_rd(bound));
+        if (up > top * NEAR && (up * NEAR >= top || __ddiv_rn(diff, bound) > __ddiv_rn(top_diff, top_bound))) {
+            top = fmaxf(top, up);
+            top_diff = diff;
+            top_bound = bound;
         }
         sc_s[e] = score;
         cs_s[e] = c;
         id_s[e] = j;
     }
+    float warp_top = top;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long oe = __shfl_xor_sync(COSTAL_FULL_MASK, err, o);
         err = oe > err ? oe : err;
-        const unsigned long long oq = __shfl_xor_sync(COSTAL_FULL_MASK, ratio, o);
-        ratio = oq > ratio ? oq : ratio;
+        warp_top = fmaxf(warp_top, __shfl_xor_sync(COSTAL_FULL_MASK, warp_top, o));
     }
     // max_err_bits[0]: the largest |coarse − rescored|, [1]: the largest ratio of it to the row's bound
     // (non-negative doubles order like their bits). One address for the whole grid: read it first,
     // so that only a new maximum pays for the atomic.
-    if (lane == 0 && max_err_bits && err > 0) {
-        if (err > *reinterpret_cast<volatile unsigned long long*>(max_err_bits)) atomicMax(max_err_bits, err);
-        if (ratio > *reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)) atomicMax(max_err_bits + 1, ratio);
+    if (lane == 0) {
+        top_s[warp] = warp_top;
+        if (max_err_bits && err > *reinterpret_cast<volatile unsigned long long*>(max_err_bits)) atomicMax(max_err_bits, err);
     }
     __syncthreads();
+    if (max_err_bits && top > 0.0f) {
+        float cta_top = 0.0f;
+#pragma unroll
+        for (int w = 0; w < RS_ROWS; ++w) cta_top = fmaxf(cta_top, top_s[w]);
+        if (top >= cta_top * NEAR && top > f32_below(*reinterpret_cast<volatile unsigned long long*>(max_err_bits + 1)))
+            atomicMax(max_err_bits + 1, (unsigned long long)__double_as_longlong(__ddiv_rn(top_diff, top_bound)));
+    }
     if (warp < nr) {
         const int i = row_s[warp];
         double sc[SLOTS], cs[SLOTS];
@@ -502,7 +513,7 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
 // Row groups of RS_ROWS, grid-stride: one group per CTA, or (deep rows) a few CTAs per SM walking
 // many groups, so that the rows each thread streams through stay in L1.
 template <int SLOTS, bool DEEP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, DEEP ? 4 : 5)
     k_rescore(const float* __restrict__ x, int n, int d, int k, int cap, int lstride,
               const uint32_t* __restrict__ cand_idx, const float* __restrict__ cand_score,
               const float* __restrict__ tau, const double* __restrict__ norms, const double* __restrict__ row_eps,
@@ -677,10 +688,10 @@ cudaError_t launch_rescore(const float* x, int n, int d, int k, int cap, int lst
     }
     const int groups = (n + RS_ROWS - 1) / RS_ROWS;
     const int blocks = d >= 256 ? std::min(groups, 3 * sms) : groups;
-    // Phase ½ where the coarse bound is wide (split FP8): 70,000 × 2,000, k = 10 345 ms of rescoring without
-    // it, 337 with, 100,000 × 2,000 of scRNA-like counts 33 and 19. Where the coarse scores are sharper it
-    // rules out too few: split BF16, 8,000 × 400, k = 15 0.41 without and 0.49 with, FP32, 8,000 × 1,000
-    // 0.40 and 0.50.
+    // Phase ½ where the coarse bound is wide (split FP8, and the FP32 re-run of its failing rows with the same 64
+    // candidates): 70,000 × 2,000, k = 10 345 ms of rescoring without it, 337 with, 100,000 × 2,000 of scRNA-like
+    // counts 33 and 19. Where the coarse scores are sharper it rules out too few: split BF16, 8,000 × 400, k = 15
+    // 0.41 without and 0.49 with, FP32, 8,000 × 1,000 0.40 and 0.50.
     auto kern = wide_bound && d >= 256 && slots <= 2
                     ? (slots == 1 ? k_rescore<1, true> : k_rescore<2, true>)
                     : (slots == 1 ? k_rescore<1, false> : slots == 2 ? k_rescore<2, false> : k_rescore<4, false>);
