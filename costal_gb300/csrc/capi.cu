@@ -602,7 +602,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
                 CK(launch_rescore(d_x, n, d, k, cap, cap, c.cand_idx.as<uint32_t>(), c.cand_score.as<float>(),
                                   c.tau.as<float>(), d_norms, nullptr, nullptr, nullptr, eps, cap < n - 1, 0,
                                   c.tc_rows.as<uint32_t>(), &dm->tc_fail_count, d_idx, d_cos, d_w,
-                                  c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, false, s));
+                                  c.fb_rows.as<uint32_t>(), c.fb_minsim.as<double>(), &dm->fb_count, nullptr, fp8, s));
             }
             CK(cudaEventRecord(c.ev[3], s));
         } else {

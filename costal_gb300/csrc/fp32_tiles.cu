@@ -674,11 +674,11 @@ static bool make_map(CUtensorMap* m, const void* base, size_t cols, int rows, in
 
 // Column segments for nq queries against `tiles` column tiles: the number whose last wave of CTAs
 // (`slots` at a time) ends first, a CTA costing its tiles plus `start` tiles' worth of time for loading
-// its queries, seeding, its first admissions (they grow with cap) and writing its lists (and the merge
-// reading one more list).
+// its queries, seeding, its first admissions (they grow with cap; next to a deep tile they are little) and
+// writing its lists (and the merge reading one more list).
 static int segments(int nq, int tiles, int dp, int cap, int slots) {
     const int blocks = (nq + BM - 1) / BM;
-    const double start = 1.0 + 64.0 / dp + cap / 32.0;
+    const double start = 1.0 + 64.0 / dp + cap / 32.0 * std::min(1.0, 64.0 / dp);
     int best = 1;
     double best_t = 1e300;
     for (int s = 1; s <= std::min(256, tiles); ++s) {
