@@ -447,23 +447,6 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     CK(ensure(c.fb_rows, (size_t)n * 4));
     CK(ensure(c.fb_minsim, (size_t)n * 8));
     CK(cudaEventRecord(c.ev[0], s));
-    // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
-    const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
-                            (tanimoto ? prune::supported(d)
-                                      : !tc_backend && fp32_lists_pay(n, d) && lists_fit_now(c, n, d));
-    // the tensor-core pass in the locality order, with lists (a shard is a range of that order)
-    const bool tc_ordered = tc_backend && !tanimoto && !scan_all && prune::supported(d) &&
-                            (n >= TC_ORDER_ROWS || shard || (o.learned_prune && c.mlp.ready && c.mlp.d == d && c.mlp.k == k));
-    float* xsR = nullptr;
-    if (fp32_lists || tc_ordered) {
-        CK(ensure(c.xsR, (size_t)n * d * 4));
-        xsR = c.xsR.as<float>();
-    }
-    CK(launch_prep(d_x, n, d, np, dp, d_norms, c.xsT.as<float>(), xsR, &dm->bad_row, s));
-    CK(cudaEventRecord(c.ev[1], s));
-    CK(cudaEventRecord(c.ev[5], s));
-    bool used_tc = false;
-    int list_cb = 0;  // rows of a column block of the tensor-core path's lists (0: no lists)
     // The split-FP8 kind: its coarse scores are ~2⁻⁸ coarser than split BF16's, so it keeps 64
     // candidates a row whatever the margin (the output does not depend on it) to let the certificate
     // hold for nearly every row.
@@ -477,6 +460,24 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
             fp8 = false;
         }
     }
+    // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
+    const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
+                            (tanimoto ? prune::supported(d)
+                                      : !tc_backend && fp32_lists_pay(n, d) && lists_fit_now(c, n, d));
+    // the tensor-core pass in the locality order, with lists (a shard is a range of that order; the split-FP8 kind,
+    // forced at 43 ≤ d ≤ 64, has no lists)
+    const bool tc_ordered = tc_backend && !tanimoto && !scan_all && !fp8 && prune::supported(d) &&
+                            (n >= TC_ORDER_ROWS || shard || (o.learned_prune && c.mlp.ready && c.mlp.d == d && c.mlp.k == k));
+    float* xsR = nullptr;
+    if (fp32_lists || tc_ordered) {
+        CK(ensure(c.xsR, (size_t)n * d * 4));
+        xsR = c.xsR.as<float>();
+    }
+    CK(launch_prep(d_x, n, d, np, dp, d_norms, c.xsT.as<float>(), xsR, &dm->bad_row, s));
+    CK(cudaEventRecord(c.ev[1], s));
+    CK(cudaEventRecord(c.ev[5], s));
+    bool used_tc = false;
+    int list_cb = 0;  // rows of a column block of the tensor-core path's lists (0: no lists)
     if (scan_all) {
         if (shard) throw Fail{COSTAL_EUNSUPPORTED, "row shards need k + margin within the coarse pass's 128 candidates"};
         if (gather_smem(k, d, dp) > 227 * 1024) throw Fail{COSTAL_EUNSUPPORTED, "k too large for the GPU scan kernel"};

@@ -106,3 +106,13 @@ def test_error_ratio_is_the_f64_quotient(ext, matmul, n, d):
         assert 0.0 < r < 1.0 and float(np.float32(r)) != r
         if matmul == "fp32":
             assert r == st["max_coarse_err"] / ((d + 4.0) * 2.0**-23)
+
+
+@pytest.mark.parametrize("n,d", [(25_000, 43), (25_000, 64), (40_001, 50)])
+def test_split_fp8_forced_where_bf16_has_lists(ext, n, d):
+    """The split-FP8 kind has no lists: forced at 43 ≤ d ≤ 64 it runs its tiles in row order at any size."""
+    x = clustered(n, d, n + d)
+    got, st = ext._knn_exact(x, 10, matmul="fp8")
+    assert st["coarse_kind"] == "fp8" and st["blocks_stopped"] == 0
+    for a, b in zip(got, ext._knn_exact(x, 10)[0]):
+        np.testing.assert_array_equal(a, b)
