@@ -305,9 +305,7 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
             const float inv_i = __fdiv_rn(1.0f, nf);
             const bool row_ok = nf > 1e-15f && nf < 1e15f;
             const float* xi = x + (size_t)i * d;
-            // (few more than k left by the coarse score: the f64 dots are cheaper than the pass)
-            const bool worth = hi - lo > k + k / 4;
-            for (int w = lo; worth && w < hi; ++w) {
+            for (int w = lo; w < hi; ++w) {
                 const int p = work_s[w] & (RS_MAXCAP - 1);
                 const uint32_t j = cand_idx[(size_t)i * lstride + p];
                 const float mf = (float)norms[j];
@@ -342,7 +340,7 @@ __device__ __forceinline__ void rescore_group(int g, const float* __restrict__ x
             for (int s = 0; s < SLOTS; ++s) {
                 const int p = s * 32 + lane;
                 key[s] = 0;  // no estimate, or not packed
-                if (worth && (keep[s] >> lane & 1u)) {
+                if (keep[s] >> lane & 1u) {
                     const uint32_t u = __float_as_uint(r_s[warp * RS_MAXCAP + p]);
                     if ((u & 0x7fffffffu) < 0x7f800000u) key[s] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
                 }
