@@ -104,7 +104,7 @@ SIGNATURES = {
     "costal_device_ok": [STR, SZ],
     "costal_check_f64_conversion": [P, STR, SZ],
     "costal_row_l2_norms": [P, U64, U32, P, STR, SZ],
-    "costal_fp32_list_bytes": [U64, U32, P, U64, P, STR, SZ],
+    "costal_fp32_list_bytes": [U64, U32, U32, P, U64, P, STR, SZ],
     "costal_knn_exact": [P, U64, U32, U32, P, P, P, P, P, STR, SZ],
     "costal_knn_exact_device": [P, U64, U32, U32, P, P, P, P, P, P, STR, SZ],
     "costal_knn_bruteforce": [P, U64, U32, U32, U32, P, P, P, STR, SZ],

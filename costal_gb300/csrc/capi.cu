@@ -235,12 +235,14 @@ cudaError_t mlp_predict_thresholds(Context& c, prune::Plan& pp, cudaStream_t s) 
 // clustered rows gain more with every row (whole kNN, lists / all tiles: 20,000 × 32 1.55 / 1.72 ms,
 // 40,000 × 20 2.5 / 4.4, 161,443 × 32 14.9 / 39.8; Gaussian rows lose the order stage, 22,000 × 32 2.12 / 1.85,
 // 160,000 × 64 64.6 / 63). With fewer, the order stage costs about what the lists save of clustered shallow
-// rows (16,384 × 8 0.92 / 0.97, 19,000 × 16 1.18 / 1.15), and deeper rows only lose by it (19,000 × 32 1.43 /
-// 1.34, Gaussian 1.77 / 1.34; 19,000 × 64 2.02 / 1.77, Gaussian 2.36 / 1.77).
+// rows (16,384 × 8 0.92 / 0.97, 19,000 × 16 1.18 / 1.15) or of the admissions of more than 20 candidates
+// (clustered 17,443 × 35, k = 12 1.79 / 1.86, 16,384 × 32, k = 30 2.07 / 2.22, Gaussian 2.70 / 2.25); else rows only lose
+// by it (19,000 × 32, k = 10 1.43 / 1.34, Gaussian 1.77 / 1.34; 19,000 × 64 2.02 / 1.77, Gaussian 2.36 / 1.77).
 // And no further than the lists' sort: beyond, they would be in block order, without a stop, and cost 12 bytes
 // a block pair for nothing.
-bool fp32_lists_pay(int n, int d) {
-    return prune::supported(d) && n >= (d <= 16 ? 16384 : 152 * 128 + 1) && prune::sortable(n);
+bool fp32_lists_pay(int n, int d, int cap) {
+    const bool few = d <= 16 || (d <= 40 && cap > 20);
+    return prune::supported(d) && n >= (few ? 16384 : 152 * 128 + 1) && prune::sortable(n);
 }
 // Tanimoto selection takes the walk in the norm order below this many rows.
 constexpr int TANI_LIST_ROWS = 16384;
@@ -254,7 +256,7 @@ constexpr int TANI_LIST_ROWS = 16384;
 // 64, 12.2 with 126; 16,383 × 64: 3.8 and 4.9).
 int coarse_most(int n, int d, int k, bool tensor_cores) {
     if (d <= 40 || d > 64 || k >= 64) return 128;
-    return k <= 60 || tensor_cores || !fp32_lists_pay(n, d) ? 64 : 128;
+    return k <= 60 || tensor_cores || !fp32_lists_pay(n, d, 128) ? 64 : 128;
 }
 
 // The tensor-core pass visits its tiles in row order below this many rows: the order stage costs more than
@@ -463,7 +465,7 @@ void run_knn(Context& c, const float* d_x, int n, int d, int k, const costal_knn
     // the FP32 pass by lists; the order stage (also the tensor-core path's) gathers row-major rows
     const bool fp32_lists = !scan_all && !shard && o.prune && cap < n - 1 &&
                             (tanimoto ? prune::supported(d)
-                                      : !tc_backend && fp32_lists_pay(n, d) && lists_fit_now(c, n, d));
+                                      : !tc_backend && fp32_lists_pay(n, d, cap) && lists_fit_now(c, n, d));
     // the tensor-core pass in the locality order, with lists (a shard is a range of that order; the split-FP8 kind,
     // forced at 43 ≤ d ≤ 64, has no lists)
     const bool tc_ordered = tc_backend && !tanimoto && !scan_all && !fp8 && prune::supported(d) &&
@@ -747,18 +749,19 @@ int costal_check_f64_conversion(uint64_t* mismatches, char* err, size_t errlen) 
     });
 }
 
-int costal_fp32_list_bytes(uint64_t n, uint32_t d, const costal_knn_opts* opts, uint64_t free_bytes, uint64_t* bytes,
-                           char* err, size_t errlen) {
+int costal_fp32_list_bytes(uint64_t n, uint32_t d, uint32_t k, const costal_knn_opts* opts, uint64_t free_bytes,
+                           uint64_t* bytes, char* err, size_t errlen) {
     const costal_knn_opts o = opts ? *opts : defaults();
-    if (n == 0 || n > (uint64_t)INT32_MAX || d == 0 || !bytes) {
-        put_err(err, errlen, "n or d out of range");
+    if (n > (uint64_t)INT32_MAX || d == 0 || k == 0 || k >= n || !bytes) {
+        put_err(err, errlen, "n, d or k out of range");
         return COSTAL_EINVAL;
     }
     *bytes = 0;
     const bool tanimoto = o.select == COSTAL_SELECT_TANIMOTO;
     if (!o.prune || !prune::supported((int)std::min<uint32_t>(d, 65))) return COSTAL_OK;
     if (tanimoto ? (int64_t)n < TANI_LIST_ROWS || !prune::sortable((int)n)
-                 : o.backend != COSTAL_BACKEND_FP32 || !fp32_lists_pay((int)n, (int)d))
+                 : o.backend != COSTAL_BACKEND_FP32 ||
+                       !fp32_lists_pay((int)n, (int)d, (int)std::min<uint64_t>(k + (o.margin == UINT32_MAX ? (uint64_t)k : o.margin), n - 1)))
         return COSTAL_OK;
     const size_t need = list_bytes((int)n, (int)d).total();
     if (lists_fit(need, 0, free_bytes)) *bytes = need;

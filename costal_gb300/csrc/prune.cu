@@ -978,13 +978,19 @@ __global__ void __launch_bounds__(1024) k_walk_ends(const float2* __restrict__ r
         lo = fminf(lo, ranges[t].x);
         hi = fmaxf(hi, ranges[t].y);
     }
+    for (int o = 1; o < 1024; o <<= 1) {  // the threads' shares, scanned from both ends
+        lo_s[tid] = lo;
+        hi_s[tid] = hi;
+        __syncthreads();
+        if (tid + o < 1024) lo = fminf(lo, lo_s[tid + o]);
+        if (tid >= o) hi = fmaxf(hi, hi_s[tid - o]);
+        __syncthreads();
+    }
     lo_s[tid] = lo;
     hi_s[tid] = hi;
     __syncthreads();
-    lo = CUDART_INF_F;
-    hi = 0.0f;
-    for (int t = 0; t < tid; ++t) hi = fmaxf(hi, hi_s[t]);
-    for (int t = 1023; t > tid; --t) lo = fminf(lo, lo_s[t]);
+    lo = tid < 1023 ? lo_s[tid + 1] : CUDART_INF_F;
+    hi = tid > 0 ? hi_s[tid - 1] : 0.0f;
     for (long long t = a; t < b; ++t) ends[t].y = hi = fmaxf(hi, ranges[t].y);
     for (long long t = b - 1; t >= a; --t) ends[t].x = lo = fminf(lo, ranges[t].x);
 }

@@ -55,7 +55,8 @@ typedef struct costal_knn_opts {
     uint32_t col_block;    /* idem */
     int32_t sort_by_norm;  /* idem (knn.rs:41): output-independent */
     int32_t prune;         /* idem (knn.rs:44): output-independent; it enables the exact early stop of each
-                              query block's column list (bf16 backend; FP32 above 19,456 rows, from 16,384 at d <= 16; d <= 64) */
+                              query block's column list (bf16 backend; FP32 above 19,456 rows, from 16,384 at d <= 16
+                              or d <= 40 with more than 20 candidates; d <= 64) */
     int32_t learned_prune; /* 1 = use the trained block-pruning model if one is loaded (bf16 backend) */
 } costal_knn_opts;
 
@@ -102,8 +103,8 @@ int costal_row_l2_norms(const float* x, uint64_t n, uint32_t d, float* out, char
  * norm order, in O(n) memory - as it does with prune = 0, d > 64, few rows, more than 4,194,304 rows (the
  * longest lists that are sorted), or where the lists would not leave a sixteenth of the free memory. No
  * reference counterpart. */
-int costal_fp32_list_bytes(uint64_t n, uint32_t d, const costal_knn_opts* opts, uint64_t free_bytes, uint64_t* bytes,
-                           char* err, size_t errlen);
+int costal_fp32_list_bytes(uint64_t n, uint32_t d, uint32_t k, const costal_knn_opts* opts, uint64_t free_bytes,
+                           uint64_t* bytes, char* err, size_t errlen);
 /* lib.rs:114-167 `_knn_exact` -> knn.rs:365 knn_exact_with_stats. Host buffers: x n*d f32;
  * idx n*k, cos n*k, norms n. */
 int costal_knn_exact(const float* x, uint64_t n, uint32_t d, uint32_t k, const costal_knn_opts* opts,

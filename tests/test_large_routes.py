@@ -12,12 +12,12 @@ import pytest
 from conftest import ROOT, clustered
 
 
-def _list_bytes(n, d, select="cosine", free=1 << 40, prune=1, backend=0):
+def _list_bytes(n, d, select="cosine", free=1 << 40, prune=1, backend=0, k=10):
     from costal_gb300 import _lib as L
 
     o = L.KnnOpts(margin=0xFFFFFFFF, select=L.SELECT[select], backend=backend, sort_by_norm=1, prune=prune, learned_prune=0)
     out, (err, size) = C.c_uint64(1), L.errbuf()
-    L.check(L.lib().costal_fp32_list_bytes(n, d, C.byref(o), free, C.byref(out), err, size), err)
+    L.check(L.lib().costal_fp32_list_bytes(n, d, k, C.byref(o), free, C.byref(out), err, size), err)
     return out.value
 
 
@@ -37,6 +37,9 @@ def test_lists_are_bounded(ext):
             assert _list_bytes(n, 10, select) == 0
         assert _list_bytes(161_443, 65, select) == 0
     assert _list_bytes(161_443, 32, backend=1) == 0
+    # few query blocks: shallow rows, or more than 20 candidates at d ≤ 40
+    assert [_list_bytes(16_384, d, k=k) > 0 for d, k in ((16, 5), (17, 10), (40, 11), (41, 30))] == [True, False, True, False]
+    assert _list_bytes(16_383, 10, k=30) == 0
     with pytest.raises(ValueError):
         _list_bytes(0, 5)
 
